@@ -21,6 +21,7 @@
 // fixed sequence of launches on one stream (capturable in a CUDA graph).
 #include <string.h>
 
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include "accx_internal.h"
@@ -36,7 +37,9 @@
 #define C_OWNER 9  // + kind: owner-side elements
 #define C_MATCH 12 // + kind: common ids found (oriented counts)
 #define C_PROBED 15 // ids probed by the oriented bitmap kernel
-#define C_NUM 16
+#define C_HEAVY 16  // work items of the oriented bitmap kernel
+#define C_LIGHT 17  // owners of the warp-per-owner kernel
+#define C_NUM 18
 
 #define MERGE_WARPS 8        // warps per merge/gallop CTA
 #define ITEM_TARGET_DEFAULT (1u << 20)  // probe elements per bitmap work item
@@ -362,23 +365,27 @@ __device__ __forceinline__ void accx_item_shape(uint32_t du, uint32_t nsp, unsig
 __global__ void k_item_counts(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst, uint32_t n,
                               const unsigned long long *__restrict__ work_u, uint32_t W, uint32_t chs,
                               uint32_t target, unsigned long long *__restrict__ icnt,
-                              unsigned long long *__restrict__ ctr, const uint32_t *__restrict__ pre) {
+                              unsigned long long *__restrict__ ctr) {
+  unsigned long long staged = 0;
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u <= n; u += gridDim.x * blockDim.x) {
     unsigned long long c = 0;
     if (u < n) {
       unsigned long long w = work_u[u];
       if (w) {
         uint32_t ub = off[u], ue = off[u + 1];
-        // oriented owners stage only their prefix, all of it in the dense window
-        uint32_t us = pre ? ue : accx_lower_bound(dst, ub, ue, (int32_t)min(W, 0x7fffffffu));
+        uint32_t us = accx_lower_bound(dst, ub, ue, (int32_t)min(W, 0x7fffffffu));
         uint32_t nc, ns;
         accx_item_shape(ue - ub, ue - us, w, chs, target, &nc, &ns);
         c = (unsigned long long)nc * ns;
-        atomicAdd(&ctr[C_OWNER + ACCX_KIND_BITMAP], (unsigned long long)(pre ? pre[u] : ue - ub) * ns);
+        staged += (unsigned long long)(ue - ub) * ns;
       }
     }
     icnt[u] = c;
   }
+  __syncwarp();
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) staged += __shfl_xor_sync(ACCX_FULL_MASK, staged, d);
+  if ((threadIdx.x & 31) == 0 && staged) atomicAdd(&ctr[C_OWNER + ACCX_KIND_BITMAP], staged);
 }
 
 __device__ __forceinline__ uint32_t accx_slot_hash(uint32_t word, uint32_t S) {
@@ -880,17 +887,6 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     k_classify<true><<<classify_grid(sms, m), 256, 0, s>>>(off, tilerow, dst, n, m, policy, g->d_table, g->d_edge_list,
                                                           list_cap, work_u, ctr, g->d_pre, W, pcap, g->d_or_sl, g->d_rev,
                                                           cnt, bias, g->d_vinfo);  // classify also fills cnt with the bias
-    k_item_counts<<<sms * 4, 256, 0, s>>>(off, dst, n, work_u, W, 1, target, g->d_icnt, ctr, g->d_pre);
-    ACCX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(g->d_scan_tmp, g->scan_tmp_bytes, g->d_icnt, g->d_prefix,
-                                                (int64_t)n + 1, s));
-    k_item_fill<<<sms * 4, 256, 0, s>>>(g->d_icnt, g->d_prefix, n, items_cap, g->d_or_items);
-    ACCX_MARK(1);
-    k_merge_or<<<sms * 8, MERGE_WARPS * 32, 0, s>>>(off, dst, g->d_pre, g->d_rev, g->d_edge_list, list_cap, ctr,
-                                                    cnt);
-    ACCX_MARK(2);
-    k_gallop_or<GALLOP_OR_GROUP><<<sms * 8, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list, list_cap, ctr,
-                                                     cnt);
-    ACCX_MARK(3);
     // the instance whose per-round arrays fit the block: 256 threads (four CTAs per
     // SM with the default 24 KiB window), 512 (two per SM with windows up to ~60
     // KiB) or 1024
@@ -899,8 +895,22 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     int per_sm = 0;
     ACCX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kb, warps * 32, smem));
     if (per_sm < 1) return ACCX_ERR_INVALID_ARG;
-    kb<<<sms * per_sm, warps * 32, smem, s>>>(off, dst, g->d_pre, n, g->d_or_items, items_cap, work_u, g->d_prefix,
-                                              g->d_or_sl, W, pcap, target, cnt, ctr);
+    const uint32_t ctas = (uint32_t)(sms * per_sm);
+    k_owner_items<<<OI_CTAS, OI_THREADS, 0, s>>>(off, g->d_pre, n < W ? n : W, work_u, target, ctas, items_cap, g->d_prefix, g->d_or_items,
+                                          ctr);
+    ACCX_MARK(1);
+    k_merge_or<<<sms * 8, MERGE_WARPS * 32, 0, s>>>(off, dst, g->d_pre, g->d_rev, g->d_edge_list, list_cap, ctr,
+                                                    cnt);
+    ACCX_MARK(2);
+    k_gallop_or<GALLOP_OR_GROUP><<<sms * 8, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list, list_cap, ctr,
+                                                     cnt);
+    ACCX_MARK(3);
+    const size_t ow_smem = sizeof(ow_warp) * OW_WARPS;
+    ACCX_CUDA_TRY(cudaFuncSetAttribute(k_owner_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ow_smem));
+    kb<<<ctas, warps * 32, smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, work_u, g->d_prefix, g->d_or_sl, W,
+                                      pcap, target, cnt, ctr);
+    k_owner_warp<<<sms * 4, OW_WARPS * 32, ow_smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, g->d_or_sl, cnt,
+                                                         ctr);
     ACCX_MARK(4);
     // suffix entries take their prefix entry's count.  One thread per entry in
     // entry order, so the reads of the prefix entries sweep the array upwards;
@@ -916,7 +926,7 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     const uint32_t S = (uint32_t)skb * 1024u / 8u;   // sparse 8-byte slots
     const size_t smem = (size_t)W / 8u + (size_t)S * 8u;
     const uint32_t target = ITEM_TARGET_DEFAULT;
-    k_item_counts<<<sms * 4, 256, 0, s>>>(off, dst, n, work_u, W, S / 2, target, g->d_icnt, ctr, nullptr);
+    k_item_counts<<<sms * 4, 256, 0, s>>>(off, dst, n, work_u, W, S / 2, target, g->d_icnt, ctr);
     ACCX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(g->d_scan_tmp, g->scan_tmp_bytes, g->d_icnt, g->d_prefix,
                                                 (int64_t)n + 1, s));
     ACCX_MARK(1);

@@ -161,12 +161,267 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
   if (gl == 0 && found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_GALLOP], found);
 }
 
-// items[i] = the owner of bitmap work item i (items of one owner are contiguous).
-__global__ void k_item_fill(const unsigned long long *__restrict__ icnt, const unsigned long long *__restrict__ prefix,
-                            uint32_t n, uint32_t cap, uint32_t *__restrict__ items) {
-  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-    const unsigned long long c = icnt[u], p0 = prefix[u];
-    for (unsigned long long j = 0; j < c && p0 + j < cap; j++) items[p0 + j] = u;
+// Work items of the bitmap owners.  An owner with little probe work is one entry of
+// the light list (a warp each, k_owner_warp); the others become items of the CTA
+// kernel, cut into slices of about `target` probes.  items[] holds the CTA items from
+// the front and the light owners from the back, slot[u] the first item of owner u.
+// Together they never exceed n + m/32, as an owner has at most max(1, degree/32)
+// slices.
+//
+// Light: at most OW_CAP prefix ids (the warp's table and counters), OW_WORK probes
+// and OW_DEG entries.  A CTA spends ~4 us of barriers on an item however small it
+// is, a warp well under 1 us; with many probes one warp becomes the tail of a small
+// graph.  Counts (us) by OW_WORK 0 (no light owners) / 512 / 1024 / 2048 / 4096:
+// R-MAT 15 187 / 187 / 183 / 183 / 218, Chung-Lu 3M 5825 / 5144 / 5004 / 4978 / 5058,
+// a batch of 48 small graphs 1929 / 994 / 999 / 998 / 1024.
+//
+// n here is the number of vertices that can own (ids below the dense window).  One
+// cluster of eight CTAs counts and then fills in id order: the heavy owners come
+// first, and neighbours in time share partner lists in L2 (slots handed out by
+// atomics in a grid of 64 CTAs, about 16K ids out of order, cost the CTA kernel 1.3 %
+// at R-MAT 24).  A count, device scan and fill over all n vertices were four launches,
+// and one 64-bit atomic per owner for the owner-work statistic took 139 us of a
+// 3M-vertex power-law count.
+#define OW_CAP 256u
+#define OW_WORK 2048u
+#define OW_DEG 4096u
+// CTA items aim at a 16th of a CTA's share of all probes, within these bounds (a
+// smaller item costs its staging more often, a larger one ends later than the rest)
+#define ITEM_TARGET_MIN 16384u
+__device__ __forceinline__ uint32_t accx_item_target(const unsigned long long *__restrict__ ctr, uint32_t target_max,
+                                                     uint32_t ctas) {
+  const unsigned long long t = ctr[C_WORK + ACCX_KIND_BITMAP] / (16ull * ctas);
+  return (uint32_t)(t < ITEM_TARGET_MIN ? ITEM_TARGET_MIN : t > target_max ? target_max : t);
+}
+
+__device__ __forceinline__ uint32_t accx_warp_incl_sum(uint32_t v, int lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t a = __shfl_up_sync(ACCX_FULL_MASK, v, d);
+    if (lane >= d) v += a;
+  }
+  return v;
+}
+
+// an owner's CTA slices (0: none or light)
+__device__ __forceinline__ uint32_t ow_shape(const uint32_t *__restrict__ off, const uint32_t *__restrict__ pre,
+                                             const unsigned long long *__restrict__ work_u, uint32_t u, uint32_t n,
+                                             uint32_t target, bool *light, uint32_t *px) {
+  const unsigned long long w = u < n ? work_u[u] : 0ull;
+  uint32_t ns = 0;
+  *light = false;
+  *px = 0;
+  if (w) {
+    const uint32_t du = off[u + 1] - off[u];
+    *px = pre[u];
+    *light = *px <= OW_CAP && w <= OW_WORK && du <= OW_DEG;
+    uint32_t nc;
+    if (!*light) accx_item_shape(du, 0, w, 1, target, &nc, &ns);
+  }
+  return ns;
+}
+
+#define OI_CTAS 8
+#define OI_THREADS 1024
+__global__ void __cluster_dims__(OI_CTAS, 1, 1) __launch_bounds__(OI_THREADS)
+    k_owner_items(const uint32_t *__restrict__ off, const uint32_t *__restrict__ pre, uint32_t n,
+                  const unsigned long long *__restrict__ work_u, uint32_t target_max, uint32_t ctas, uint32_t cap,
+                  unsigned long long *__restrict__ slot, uint32_t *__restrict__ items,
+                  unsigned long long *__restrict__ ctr) {
+  __shared__ uint32_t s_h[32], s_l[32], s_tot[2];
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t target = accx_item_target(ctr, target_max, ctas);
+  // a run of `span` vertices (a multiple of 32) per warp of the cluster
+  const uint32_t nw = OI_CTAS * OI_THREADS / 32, span = ((n + nw - 1) / nw + 31u) & ~31u;
+  const uint32_t b = min(n, (cl.block_rank() * (OI_THREADS / 32) + warp) * span), e = min(n, b + span);
+  unsigned long long staged = 0;
+  uint32_t h = 0, l = 0;
+  for (uint32_t u0 = b; u0 < e; u0 += 32) {
+    bool light;
+    uint32_t px;
+    const uint32_t ns = ow_shape(off, pre, work_u, u0 + lane, e, target, &light, &px);
+    h += ns;
+    l += light;
+    staged += (unsigned long long)px * (light ? 1u : ns);
+  }
+  h = __reduce_add_sync(ACCX_FULL_MASK, h);
+  l = __reduce_add_sync(ACCX_FULL_MASK, l);
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) staged += __shfl_xor_sync(ACCX_FULL_MASK, staged, d);
+  if (lane == 0) {
+    if (staged) atomicAdd(&ctr[C_OWNER + ACCX_KIND_BITMAP], staged);
+    s_h[warp] = h;
+    s_l[warp] = l;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t vh = s_h[lane], vl = s_l[lane];
+    const uint32_t ih = accx_warp_incl_sum(vh, lane), il = accx_warp_incl_sum(vl, lane);
+    s_h[lane] = ih - vh;
+    s_l[lane] = il - vl;
+    if (lane == 31) {
+      s_tot[0] = ih;
+      s_tot[1] = il;
+    }
+  }
+  cl.sync();
+  uint32_t h0 = s_h[warp], l0 = s_l[warp];
+  for (unsigned r = 0; r < cl.block_rank(); r++) {
+    const uint32_t *t = cl.map_shared_rank(s_tot, r);
+    h0 += t[0];
+    l0 += t[1];
+  }
+  if (cl.block_rank() == OI_CTAS - 1 && threadIdx.x == 0) {
+    ctr[C_HEAVY] = h0 + s_tot[0];  // warp 0: the CTA's first slots
+    ctr[C_LIGHT] = l0 + s_tot[1];
+  }
+  cl.sync();  // the totals are not read after this
+  for (uint32_t u0 = b; u0 < e; u0 += 32) {
+    const uint32_t u = u0 + lane;
+    bool light;
+    uint32_t px;
+    const uint32_t ns = ow_shape(off, pre, work_u, u, e, target, &light, &px);
+    const unsigned lm = __ballot_sync(ACCX_FULL_MASK, light);
+    const uint32_t incl = accx_warp_incl_sum(ns, lane), p = h0 + incl - ns;
+    const uint32_t q = l0 + __popc(lm & ((1u << lane) - 1u));
+    if (light && q < cap) items[cap - 1 - q] = u;
+    if (ns) {
+      slot[u] = p;
+      for (uint32_t j = 0; j < ns && p + j < cap; j++) items[p + j] = u;
+    }
+    h0 += __shfl_sync(ACCX_FULL_MASK, incl, 31);
+    l0 += __popc(lm);
+  }
+}
+
+// Light bitmap owners: a warp per owner, no barriers.  The owner's prefix goes into
+// a hash table of packed (id << 8 | position) words in the warp's shared memory (at
+// least four slots an id, so most look-ups read one word), with one counter per
+// position; ids are below 2^24 as bitmap owners lie inside the dense window.  The
+// row is walked 32 entries at a time: their partner ranges are concatenated (warp
+// scan) and streamed 32 ids a step, four steps' loads in flight, as the CTA kernel
+// streams its short lists.  Credits are the CTA kernel's.  Bound by latency and
+// instruction issue.
+#define OW_WARPS 8
+struct ow_warp {
+  uint32_t tab[4 * OW_CAP];
+  uint32_t oc[OW_CAP];
+  uint32_t pre[33], beg[32], hit[32];
+};
+
+__device__ __forceinline__ uint32_t ow_hash(uint32_t id, int sh) { return (id * 0x9E3779B1u) >> sh; }
+
+__global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__restrict__ off,
+                                                              const int32_t *__restrict__ dst,
+                                                              const uint32_t *__restrict__ pre,
+                                                              const uint32_t *__restrict__ items, uint32_t cap,
+                                                              const uint2 *__restrict__ sl, int32_t *__restrict__ cnt,
+                                                              unsigned long long *__restrict__ ctr) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  const int lane = threadIdx.x & 31;
+  ow_warp &S = reinterpret_cast<ow_warp *>(smem)[threadIdx.x >> 5];
+  unsigned long long total = ctr[C_LIGHT];
+  if (total > cap) total = cap;
+  unsigned long long found = 0, probed = 0;
+  const unsigned long long nw = (unsigned long long)gridDim.x * OW_WARPS;
+  for (unsigned long long it = (unsigned long long)blockIdx.x * OW_WARPS + (threadIdx.x >> 5); it < total; it += nw) {
+    const uint32_t x = items[cap - 1 - it];
+    const uint32_t ub = off[x], ue = off[x + 1], px = min(pre[x], OW_CAP);
+    // the table: 64 to 1024 slots
+    int lg = 6;
+    while (lg < 10 && (1u << lg) < 4u * px) lg++;
+    const uint32_t mask = (1u << lg) - 1u;
+    const int sh = 32 - lg;
+    for (uint32_t i = lane; i <= mask; i += 32) S.tab[i] = 0xffffffffu;
+    for (uint32_t i = lane; i < px; i += 32) S.oc[i] = 0;
+    __syncwarp();
+    for (uint32_t i = lane; i < px; i += 32) {
+      const uint32_t id = (uint32_t)__ldg(dst + ub + i);
+      uint32_t h = ow_hash(id, sh);
+      while (atomicCAS(&S.tab[h], 0xffffffffu, (id << 8) | i) != 0xffffffffu) h = (h + 1) & mask;
+    }
+    __syncwarp();
+    for (uint32_t r0 = ub; r0 < ue; r0 += 32) {
+      const uint32_t k = r0 + lane;
+      uint32_t sst = 0, len = 0;
+      if (k < ue) {
+        const uint2 e = sl[k];
+        sst = e.x;
+        len = (e.y & OR_SL_GALLOP) ? 0u : e.y;
+      }
+      const unsigned act = __ballot_sync(ACCX_FULL_MASK, len > 0);
+      if (!act) continue;
+      probed += len;
+      const uint32_t incl = accx_warp_incl_sum(len, lane);
+      const uint32_t tot = __shfl_sync(ACCX_FULL_MASK, incl, 31), nseg = __popc(act);
+      const uint32_t me = __popc(act & ((1u << lane) - 1u));
+      if (len) {
+        S.pre[me] = incl - len;
+        S.beg[me] = sst;
+        S.hit[me] = 0;
+      }
+      if (lane == 0) S.pre[nseg] = tot;
+      __syncwarp();
+      uint32_t segb = 0;
+      for (uint32_t c0 = 0; c0 < tot; c0 += 32u * PROBE_UNROLL) {
+        int32_t xs[PROBE_UNROLL];
+        uint32_t sg[PROBE_UNROLL], gi[PROBE_UNROLL];
+#pragma unroll
+        for (int r = 0; r < PROBE_UNROLL; r++) {
+          // 32 ids meet at most 31 segment starts after segb: each lane loads one
+          // start, and a lane's segment is segb + the starts at or before its id
+          const uint32_t i0 = c0 + 32u * r, i = i0 + lane;
+          const uint32_t kb = segb + 1u + lane;
+          const uint32_t o = (kb <= nseg ? S.pre[kb] : 0xffffffffu) - i0;
+          const unsigned M = __reduce_or_sync(ACCX_FULL_MASK, o < 32u ? (1u << o) : 0u);
+          const uint32_t sj = min(segb + __popc(M & (0xffffffffu >> (31 - lane))), 31u);
+          sg[r] = sj;
+          gi[r] = (i < tot) ? S.beg[sj] + (i - S.pre[sj]) : 0u;
+          xs[r] = (i < tot) ? __ldg(dst + gi[r]) : -1;
+          segb += __popc(M) + (__ballot_sync(ACCX_FULL_MASK, o == 32u) ? 1u : 0u);
+        }
+#pragma unroll
+        for (int r = 0; r < PROBE_UNROLL; r++) {
+          if (xs[r] < 0) continue;
+          const uint32_t id = (uint32_t)xs[r];
+          uint32_t h = ow_hash(id, sh), t = S.tab[h];
+          while ((t >> 8) != id && t != 0xffffffffu) {
+            h = (h + 1) & mask;
+            t = S.tab[h];
+          }
+          if (t != 0xffffffffu) {
+            atomicAdd(cnt + gi[r], 1);
+            atomicAdd(&S.oc[t & 255u], 1u);
+            atomicAdd(&S.hit[sg[r]], 1u);
+          }
+        }
+      }
+      __syncwarp();
+      if (len) {  // the edge's credit, to its prefix entry
+        const uint32_t h = S.hit[me];
+        found += h;
+        if (h) {
+          if (k - ub < px) atomicAdd(&S.oc[k - ub], h);
+          else atomicAdd(cnt + sst + len, (int32_t)h);
+        }
+      }
+      __syncwarp();
+    }
+    for (uint32_t i = lane; i < px; i += 32) {
+      const uint32_t h = S.oc[i];
+      if (h) atomicAdd(cnt + ub + i, (int32_t)h);
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) {
+    found += __shfl_xor_sync(ACCX_FULL_MASK, found, d);
+    probed += __shfl_xor_sync(ACCX_FULL_MASK, probed, d);
+  }
+  if (lane == 0) {
+    if (found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_BITMAP], found);
+    if (probed) atomicAdd(&ctr[C_PROBED], probed);
   }
 }
 
@@ -232,12 +487,12 @@ __device__ __forceinline__ uint32_t or_piece(const int32_t *__restrict__ dst, ui
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__restrict__ off,
                                                        const int32_t *__restrict__ dst,
-                                                       const uint32_t *__restrict__ pre, uint32_t n,
+                                                       const uint32_t *__restrict__ pre,
                                                        const uint32_t *__restrict__ items, uint32_t items_cap,
                                                        const unsigned long long *__restrict__ work_u,
-                                                       const unsigned long long *__restrict__ prefix,
+                                                       const unsigned long long *__restrict__ slot,
                                                        const uint2 *__restrict__ sl, uint32_t W, uint32_t pcap,
-                                                       uint32_t target, int32_t *__restrict__ cnt,
+                                                       uint32_t target_max, int32_t *__restrict__ cnt,
                                                        unsigned long long *__restrict__ ctr) {
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t nwords = W / 32;
@@ -247,17 +502,20 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
   uint32_t *ocnt = smem + nwords + 4;
   uint16_t *wbase = reinterpret_cast<uint16_t *>(ocnt + pcap + 32);  // nwords first-id positions
   __shared__ unsigned long long s_it;
-  __shared__ uint32_t s_tot, s_nseg, s_nlong, s_next;
+  __shared__ uint32_t s_tot, s_nseg, s_nlong, s_next, s_target;
   __shared__ uint32_t s_wsum[32], s_wcnt[32], s_wlong[32];
   __shared__ uint32_t s_pre[NT + 1], s_beg[NT], s_ent[NT], s_hit[NT];
   __shared__ uint32_t s_lbeg[NT], s_llen[NT], s_lent[NT], s_lhit[NT];
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
   for (uint32_t i = tid; i <= nwords; i += nt) words[i] = 0;
-  unsigned long long total = prefix[n];
+  unsigned long long total = ctr[C_HEAVY];
   if (total > items_cap) total = items_cap;
   unsigned long long found = 0, probed = 0;  // this thread's share, summed per warp at the end
-  if (tid == 0) s_it = atomicAdd(&ctr[C_ITEMS], 1ull);
+  if (tid == 0) {
+    s_it = atomicAdd(&ctr[C_ITEMS], 1ull);
+    s_target = accx_item_target(ctr, target_max, gridDim.x);
+  }
   __syncthreads();
   for (;;) {
     const unsigned long long it = s_it;
@@ -265,8 +523,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
     const uint32_t x = items[it];
     const uint32_t ub = off[x], ue = off[x + 1], du = ue - ub, px = pre[x];
     uint32_t nchunks, nsplit;
-    accx_item_shape(du, 0, work_u[x], 1, target, &nchunks, &nsplit);
-    const uint32_t sp = (uint32_t)(it - prefix[x]);
+    accx_item_shape(du, 0, work_u[x], 1, s_target, &nchunks, &nsplit);
+    const uint32_t sp = (uint32_t)(it - slot[x]);
     const uint32_t pa = ub + (uint32_t)((unsigned long long)du * sp / nsplit);
     const uint32_t pb = ub + (uint32_t)((unsigned long long)du * (sp + 1) / nsplit);
     const uint32_t pxs = px <= pcap ? px : 0;  // the classifier guarantees px <= pcap for bitmap owners

@@ -1,0 +1,92 @@
+"""GPU parity of the oriented bitmap kind's tiers at their edges: owners walked by a
+warp or by a CTA (prefix lengths around the warp's table, probe work and degree
+around its limits), against the oracle's counts.  Counts are whole numbers: equal
+or wrong."""
+import numpy as np
+import pytest
+
+from conftest import has_gpu
+
+pytestmark = pytest.mark.gpu
+
+if has_gpu():
+    from acctricnt_gb300 import accx
+    from oracle import oracle
+
+
+def _csr(n, u, v):
+    keep = u != v
+    u, v = u[keep].astype(np.int64), v[keep].astype(np.int64)
+    k = np.unique(np.concatenate([u * n + v, v * n + u]))
+    off = np.searchsorted(k, np.arange(n + 1) * n).astype(np.uint32)
+    return off, (k % n).astype(np.int32)
+
+
+def _hubs_and_leaves(hubs, leaf_prefixes, density, seed, satellites=0):
+    """`hubs` vertices joined pairwise with probability `density` (each with enough
+    satellites to stay ahead of the leaves in degree order), and per entry p of
+    leaf_prefixes one vertex joined to p random hubs."""
+    rng = np.random.default_rng(seed)
+    a, b = np.triu_indices(hubs, 1)
+    m = rng.random(len(a)) < density
+    us, vs = [a[m]], [b[m]]
+    n = hubs
+    for p in leaf_prefixes:
+        us.append(np.full(p, n))
+        vs.append(rng.permutation(hubs)[:p])
+        n += 1
+    for h in range(hubs):
+        us.append(np.full(satellites, h))
+        vs.append(np.arange(n, n + satellites))
+        n += satellites
+    u, v = np.concatenate(us), np.concatenate(vs)
+    p = rng.permutation(n)  # the relabel has to find the order
+    return _csr(n, p[u], p[v])
+
+
+def _check(off, dst, **kw):
+    ref = oracle.cn_count(off, dst, nthreads=8)
+    G = accx.Graph.from_csr(off, dst)
+    G.relabel()
+    assert np.array_equal(G.count(policy="bitmap", bias=2, orient=True, **kw), ref)
+    st = G.last_stats()
+    matches, _ = G.last_matches()
+    assert sum(matches.values()) == (int(ref.sum()) - 2 * len(ref)) // 6  # every triangle once
+    assert sum(s["edges"] for s in st.values()) <= len(dst) // 2
+
+
+# the warp's table takes 256 prefix ids and 64 to 1024 slots (four an id)
+@pytest.mark.parametrize("p", [1, 2, 15, 16, 17, 31, 32, 33, 64, 65, 127, 128, 129, 255, 256, 257, 300])
+def test_prefix_length_edges(p):
+    _check(*_hubs_and_leaves(320, [p] * 5 + [p - 1 or 1] * 3, 0.1, seed=p, satellites=60))
+
+
+# probe work around the light limit (2048 probes): a leaf of p hubs probes about
+# p * density * hubs / 2 ids
+@pytest.mark.parametrize("density", [0.02, 0.05, 0.1, 0.2, 0.5, 1.0])
+def test_probe_work_edges(density):
+    _check(*_hubs_and_leaves(256, list(range(1, 257, 5)) * 2, density, seed=11, satellites=40))
+
+
+# rows around the light owners' 4096 entries: few prefix ids, long suffixes
+@pytest.mark.parametrize("sats", [4000, 4090, 4096, 4100])
+def test_row_length_edges(sats):
+    rng = np.random.default_rng(sats)
+    hubs, n = 6, 6
+    us, vs = [], []
+    for h in range(hubs):
+        us.append(np.full(sats, h))
+        vs.append(rng.permutation(sats + 200)[:sats] + hubs)
+    a, b = np.triu_indices(hubs, 1)
+    us.append(a)
+    vs.append(b)
+    n = hubs + sats + 200
+    _check(*_csr(n, np.concatenate(us), np.concatenate(vs)))
+
+
+@pytest.mark.parametrize("kw", [{"window_kb": 1, "sparse_kb": 1, "block_warps": 4}, {"window_kb": 8, "block_warps": 16},
+                                {"window_kb": 64, "sparse_kb": 16, "block_warps": 32}])
+def test_shapes(kw):
+    G = accx.Graph.generate(accx.chung_lu_params(60000, 20, 2.1, 6000, seed=5))
+    off, dst = G.download()
+    _check(off, dst, **kw)

@@ -79,6 +79,12 @@ struct accx_graph {
   uint32_t *d_or_items = nullptr;          // n + m/32 + 1 oriented bitmap work items: owner of each
   uint32_t *d_rev = nullptr;               // m reverse entry of every entry of the counting CSR (oriented counts)
   uint32_t *d_rev_orig = nullptr;          // m reverse entries of the handle's own CSR, recorded by full validation
+  // dense rows of the relabeled CSR (planned by the relabel; 0 rows: none worth it)
+  uint32_t dense_k = 0, dense_m = 0;       // hub ids (bits a row) and rows
+  uint32_t dense_maxpre = 0;               // the longest prefix of those rows
+  uint32_t *d_dense_t = nullptr;           // dense_m x dense_k bits
+  uint32_t *d_dense_low = nullptr;         // dense_m: set bits of each row
+  uint4 *d_dense_items = nullptr;          // (row, first entry, entries) pieces of the rows
   bool symmetric = false;                  // known symmetric: validated, generated or built from an edge list
   const uint32_t *rev_csr = nullptr;       // the offsets array d_rev was built for
   void *d_scan_tmp = nullptr;

@@ -36,10 +36,11 @@
 #define C_WORK 6   // + kind
 #define C_OWNER 9  // + kind: owner-side elements
 #define C_MATCH 12 // + kind: common ids found (oriented counts)
-#define C_PROBED 15 // ids probed by the oriented bitmap kernel
+#define C_PROBED 15 // partner ids of the oriented bitmap kind's edges (probed, or covered by dense rows)
 #define C_HEAVY 16  // work items of the oriented bitmap kernel
 #define C_LIGHT 17  // owners of the warp-per-owner kernel
-#define C_NUM 18
+#define C_DENSE 18  // work items of the dense rows
+#define C_NUM 19
 
 #define MERGE_WARPS 8        // warps per merge/gallop CTA
 #define ITEM_TARGET_DEFAULT (1u << 20)  // probe elements per bitmap work item
@@ -56,6 +57,16 @@ __device__ __forceinline__ int accx_edge_kind(int policy, const uint8_t *table, 
     case ACCX_POLICY_BITMAP: return ACCX_KIND_BITMAP;
     default: return table[accx_bucket(du) * ACCX_NB + accx_bucket(dv)];
   }
+}
+
+// Whether the edge between rows x and y (prefix lengths px, py), both below the dense
+// rows' M, is counted with the dense rows: its kind is bitmap, by the rules of classify
+// (M is at most the bitmap window, so the owner's id is inside it).
+__device__ __forceinline__ bool accx_dense_edge(int policy, const uint8_t *table, uint32_t x, uint32_t px, uint32_t y,
+                                                uint32_t py, uint32_t pcap) {
+  const bool own = accx_owns(x, px, y, py);
+  const uint32_t po = own ? px : py, pp = own ? py : px;
+  return pp > 0 && po <= pcap && accx_edge_kind(policy, table, po, pp) == ACCX_KIND_BITMAP;
 }
 
 // ---------------------------------------------------------------------------
@@ -99,7 +110,8 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
                                                   unsigned long long *__restrict__ ctr, const uint32_t *__restrict__ pre,
                                                   uint32_t bm_idlim, uint32_t bm_pcap, uint2 *__restrict__ or_sl,
                                                   const uint32_t *__restrict__ rev, int32_t *__restrict__ fill,
-                                                  int32_t bias, const uint2 *__restrict__ vinfo) {
+                                                  int32_t bias, const uint2 *__restrict__ vinfo, uint32_t dense_m,
+                                                  const uint32_t *__restrict__ dense_low) {
   static_assert(256 % CL_EPT == 0, "chunks inside tile-row tiles");
   __shared__ uint8_t s_table[ACCX_NB * ACCX_NB];
   __shared__ uint32_t s_wc[2][8];              // per-warp merge / gallop entries of the block
@@ -110,7 +122,10 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
   if (policy == ACCX_POLICY_TABLE || policy == ACCX_POLICY_MODEL)
     for (int i = tid; i < ACCX_NB * ACCX_NB; i += 256) s_table[i] = table[i];
   __syncthreads();
+  // direct: an owner with empty lists still has an item; oriented: nothing to do
+  constexpr unsigned long long extra = ORIENT ? 0 : 1;
   cl_stats st;
+  unsigned long long probed = 0;
   const uint32_t span = 256u * CL_EPT;
   const uint32_t nblk = (uint32_t)(((unsigned long long)m + span - 1) / span);
   for (uint32_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
@@ -187,11 +202,16 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
           // walks (zero for the other kinds), and every galloping entry
           uint2 sl = make_uint2(0u, 0u);
           if (kind == ACCX_KIND_BITMAP || kind == ACCX_KIND_GALLOP) {
-            const uint32_t sst = ss[j];
+            uint32_t sst = ss[j];
             uint32_t tt = sst + dv;
             if (v > u) {  // cut P(v) at u: u's position in N(v) is the reverse entry
               const uint32_t r = __ldg(rev + e);
               tt = (r >= sst && r < tt) ? r : sst;
+            }
+            if (kind == ACCX_KIND_BITMAP) {
+              probed += tt - sst;
+              // between dense rows the hub ids are counted there: the list starts behind them
+              if (u < dense_m && v < dense_m) sst = min(sst + __ldg(dense_low + v), tt);
             }
             sl = make_uint2(sst, (tt - sst) | (kind == ACCX_KIND_GALLOP ? OR_SL_GALLOP : 0u));
             bwork = tt - sst;
@@ -203,7 +223,7 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
         cg += kind == ACCX_KIND_GALLOP;
         if (kind == ACCX_KIND_BITMAP) {
           if (u != run_u) {
-            if (run_u != 0xffffffffu) atomicAdd(&work_u[run_u], run_w + 1ull);
+            if (run_u != 0xffffffffu && run_w + extra) atomicAdd(&work_u[run_u], run_w + extra);
             run_u = u;
             run_w = 0;
           }
@@ -218,7 +238,8 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
       const unsigned peers = __match_any_sync(ACCX_FULL_MASK, run_u);
       const unsigned long long hi = __reduce_add_sync(peers, (unsigned)(run_w >> 32));
       const unsigned long long lo = __reduce_add_sync(peers, (unsigned)(run_w & 0xffffffffu));
-      if (run_u != 0xffffffffu && lane == __ffs(peers) - 1) atomicAdd(&work_u[run_u], (hi << 32) + lo + 1ull);
+      if (run_u != 0xffffffffu && lane == __ffs(peers) - 1 && (hi | lo | extra))
+        atomicAdd(&work_u[run_u], (hi << 32) + lo + extra);
     }
     // list slots: exclusive scan of the threads' counts over the block
     uint32_t im = cm, ig = cg;
@@ -275,6 +296,11 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
       for (int d = 16; d >= 1; d >>= 1) x += __shfl_xor_sync(ACCX_FULL_MASK, x, d);
       if (lane == 0 && x) atomicAdd(&s_st[q * ACCX_NUM_KINDS + k], x);
     }
+  }
+  if (ORIENT) {
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) probed += __shfl_xor_sync(ACCX_FULL_MASK, probed, d);
+    if (lane == 0 && probed) atomicAdd(&ctr[C_PROBED], probed);
   }
   __syncthreads();
   if (tid < 3 * ACCX_NUM_KINDS && s_st[tid]) atomicAdd(&ctr[C_EDGES + tid], s_st[tid]);
@@ -768,6 +794,25 @@ static int g_or_counter_kb = 8;
 static int g_or_block_warps = 8;
 
 
+// Dense rows' scratch: item size, item capacity and the arrays (all or none).
+static uint32_t dense_chunk(const accx_graph *g) { return g->m < (1ull << 25) ? 256u : 512u; }
+static uint32_t dense_cap(const accx_graph *g) { return g->dense_m + (uint32_t)(g->m / dense_chunk(g)) + 1u; }
+static bool alloc_dense(accx_graph *g) {
+  const size_t tb = (size_t)g->dense_m * (g->dense_k / 8u);
+  bool ok = accx_dev_alloc((void **)&g->d_dense_t, tb, g->home) == cudaSuccess &&
+            accx_dev_alloc((void **)&g->d_dense_low, sizeof(uint32_t) * (size_t)g->dense_m, g->home) == cudaSuccess &&
+            accx_dev_alloc((void **)&g->d_dense_items, sizeof(uint4) * (size_t)dense_cap(g), g->home) == cudaSuccess;
+  if (ok && g->home) ok = cudaStreamSynchronize(g->home) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    for (void **p : {(void **)&g->d_dense_t, (void **)&g->d_dense_low, (void **)&g->d_dense_items}) {
+      accx_dev_free(*p, g->home);
+      *p = nullptr;
+    }
+  }
+  return ok;
+}
+
 // Persistent classify CTAs: four per SM (64 registers a thread), at most one per
 // block of entries.
 static unsigned classify_grid(int sms, uint32_t m) {
@@ -884,9 +929,21 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
       }
       g->rev_csr = off;
     }
+    // dense rows, where the relabel planned some and bitmap-kind edges can occur
+    const uint32_t wpl = g->dense_k / 1024u;
+    uint32_t dm = rel && policy != ACCX_POLICY_HEURISTIC && policy != ACCX_POLICY_MERGE && policy != ACCX_POLICY_GALLOP
+                      ? (g->dense_m < W ? g->dense_m : W) : 0u;
+    const uint32_t dchunk = dense_chunk(g), dcap = dense_cap(g);
+    if (dm && !g->d_dense_t && !alloc_dense(g)) dm = 0;  // no room: every id is probed
+    if (dm) {
+      auto kr = wpl == 4 ? k_dense_rows<4> : wpl == 2 ? k_dense_rows<2> : k_dense_rows<1>;
+      kr<<<sms * 8, 256, 0, s>>>(off, dst, g->d_pre, dm, dchunk, g->d_dense_t, g->d_dense_low, g->d_dense_items, dcap,
+                                 ctr);
+    }
     k_classify<true><<<classify_grid(sms, m), 256, 0, s>>>(off, tilerow, dst, n, m, policy, g->d_table, g->d_edge_list,
                                                           list_cap, work_u, ctr, g->d_pre, W, pcap, g->d_or_sl, g->d_rev,
-                                                          cnt, bias, g->d_vinfo);  // classify also fills cnt with the bias
+                                                          cnt, bias, g->d_vinfo, dm,
+                                                          g->d_dense_low);  // classify also fills cnt with the bias
     // the instance whose per-round arrays fit the block: 256 threads (four CTAs per
     // SM with the default 24 KiB window), 512 (two per SM with windows up to ~60
     // KiB) or 1024
@@ -905,6 +962,14 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     k_gallop_or<GALLOP_OR_GROUP><<<sms * 8, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list, list_cap, ctr,
                                                      cnt);
     ACCX_MARK(3);
+    if (dm) {
+      const bool all = policy == ACCX_POLICY_BITMAP && g->dense_maxpre <= pcap;
+      auto kd = wpl == 4 ? (all ? k_dense_pairs<4, true> : k_dense_pairs<4, false>)
+              : wpl == 2 ? (all ? k_dense_pairs<2, true> : k_dense_pairs<2, false>)
+                         : (all ? k_dense_pairs<1, true> : k_dense_pairs<1, false>);
+      kd<<<sms * 2, DENSE_WARPS * 32, 0, s>>>(off, dst, g->d_pre, g->d_dense_low, g->d_dense_t, g->d_dense_items, dcap,
+                                              policy, g->d_table, pcap, cnt, ctr);
+    }
     const size_t ow_smem = sizeof(ow_warp) * OW_WARPS;
     ACCX_CUDA_TRY(cudaFuncSetAttribute(k_owner_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ow_smem));
     kb<<<ctas, warps * 32, smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, work_u, g->d_prefix, g->d_or_sl, W,
@@ -921,7 +986,7 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   } else {
     k_classify<false><<<classify_grid(sms, m), 256, 0, s>>>(off, tilerow, dst, n, m, policy, g->d_table, g->d_edge_list,
                                                            list_cap, work_u, ctr, nullptr, 0u, 0u, nullptr, nullptr,
-                                                           nullptr, 0, nullptr);
+                                                           nullptr, 0, nullptr, 0u, nullptr);
     const uint32_t W = (uint32_t)dkb * 8192u;        // dense ids (bits)
     const uint32_t S = (uint32_t)skb * 1024u / 8u;   // sparse 8-byte slots
     const size_t smem = (size_t)W / 8u + (size_t)S * 8u;

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
   ow_warp &S = reinterpret_cast<ow_warp *>(smem)[threadIdx.x >> 5];
   unsigned long long total = ctr[C_LIGHT];
   if (total > cap) total = cap;
-  unsigned long long found = 0, probed = 0;
+  unsigned long long found = 0;
   const unsigned long long nw = (unsigned long long)gridDim.x * OW_WARPS;
   for (unsigned long long it = (unsigned long long)blockIdx.x * OW_WARPS + (threadIdx.x >> 5); it < total; it += nw) {
     const uint32_t x = items[cap - 1 - it];
@@ -352,7 +352,6 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
       }
       const unsigned act = __ballot_sync(ACCX_FULL_MASK, len > 0);
       if (!act) continue;
-      probed += len;
       const uint32_t incl = accx_warp_incl_sum(len, lane);
       const uint32_t tot = __shfl_sync(ACCX_FULL_MASK, incl, 31), nseg = __popc(act);
       const uint32_t me = __popc(act & ((1u << lane) - 1u));
@@ -415,14 +414,221 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
     __syncwarp();
   }
 #pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    found += __shfl_xor_sync(ACCX_FULL_MASK, found, d);
-    probed += __shfl_xor_sync(ACCX_FULL_MASK, probed, d);
+  for (int d = 16; d >= 1; d >>= 1) found += __shfl_xor_sync(ACCX_FULL_MASK, found, d);
+  if (lane == 0 && found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_BITMAP], found);
+}
+
+// Dense rows: the triangles a < b < c of bitmap-kind edges with a among the first K
+// ids (the hubs after the degree relabel) and c among the first M, counted a word at
+// a time.  T[x] is a K-bit mask of P(x) ∩ [0, K) for every row x < M.  The row x of a
+// triangle's b or c meets the other one, y, as a neighbour, so over all neighbours
+// y < M of x
+//   * sum over y of T[y], taken at the bits of T[x], is the number of these triangles
+//     on the edge (x, a), for every hub a at once;
+//   * popc(T[x] & T[y]), for y < x, is their number on the edge (x, y).
+// The sums are kept as vertical (bit-sliced) counters: a lane holds K/1024 words of
+// each of ten bit planes and adds a neighbour's word to 32 counters with about 2.3
+// three-input logic operations (carry-save adders, 32 neighbours a round), so no
+// common id is ever enumerated and nothing is credited by atomics until the row's
+// end, where each of its entries below K takes its counter's value.  The list-probing
+// kernels then start a partner's list behind its ids below K for these edges.
+//
+// Probing spent ~54 thread instructions an id (a hit costs a rank, a RED and a shared
+// atomic); at R-MAT 24 the 61 % of all probes that lie on edges with c < 65536 have
+// 65-98 % of their ids below 4096.  K and M come from k_dense_plan.  Measured at
+// R-MAT 24 (K 4096, M 131072): list probing 71.2 -> 39.6 ms for 9.8 ms here, bound by
+// L2 (512 bytes an entry, 8.2 TB/s); Chung-Lu 3M: 4.2 -> 2.4 ms for both.
+#define DENSE_PLANES 10   // a counter holds at most DENSE_CHUNK neighbours: < 2^10
+#define DENSE_CHUNK_MAX 960u
+#define DENSE_WARPS 8
+
+// T, low[x] = |T[x]| and the work items of the rows below M: a warp per row.
+// item = (row, first entry, entries), at most `chunk` entries below M of the row.
+template <int WPL>
+__global__ void __launch_bounds__(256) k_dense_rows(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst,
+                                                    const uint32_t *__restrict__ pre, uint32_t M, uint32_t chunk,
+                                                    uint32_t *__restrict__ T, uint32_t *__restrict__ low,
+                                                    uint4 *__restrict__ items, uint32_t cap,
+                                                    unsigned long long *__restrict__ ctr) {
+  constexpr uint32_t K = WPL * 1024u;
+  __shared__ uint32_t s_t[8][WPL * 32];
+  const int lane = threadIdx.x & 31;
+  uint32_t *t = s_t[threadIdx.x >> 5];
+  const uint32_t nw = gridDim.x * 8u;
+  for (uint32_t x = blockIdx.x * 8u + (threadIdx.x >> 5); x < M; x += nw) {
+    const uint32_t b = off[x], px = pre[x];
+#pragma unroll
+    for (int k = 0; k < WPL; k++) t[k * 32 + lane] = 0;
+    __syncwarp();
+    uint32_t lw = 0;
+    for (uint32_t i0 = 0; i0 < px; i0 += 32) {
+      const uint32_t id = i0 + lane < px ? (uint32_t)__ldg(dst + b + i0 + lane) : 0xffffffffu;
+      if (id < K) atomicOr(&t[id >> 5], 1u << (id & 31u));
+      const unsigned in = __ballot_sync(ACCX_FULL_MASK, id < K);
+      lw += __popc(in);
+      if (in != ACCX_FULL_MASK) break;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < WPL; k++) T[(size_t)x * (WPL * 32) + k * 32 + lane] = t[k * 32 + lane];
+    if (lane == 0) {
+      low[x] = lw;
+      if (lw) {
+        const uint32_t e = off[x + 1], c = accx_lower_bound(dst, b, e, (int32_t)M) - b;
+        const uint32_t nch = (c + chunk - 1) / chunk;
+        const unsigned long long p = atomicAdd(&ctr[C_DENSE], (unsigned long long)nch);
+        for (uint32_t j = 0; j < nch && p + j < cap; j++)
+          items[p + j] = make_uint4(x, b + j * chunk, min(chunk, c - j * chunk), 0u);
+      }
+    }
+    __syncwarp();
   }
-  if (lane == 0) {
-    if (found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_BITMAP], found);
-    if (probed) atomicAdd(&ctr[C_PROBED], probed);
+}
+
+// full adder on 32 counters' bits: l += a + b, the carries to h
+__device__ __forceinline__ void accx_csa(uint32_t &h, uint32_t &l, uint32_t a, uint32_t b) {
+  h = (l & a) | (l & b) | (a & b);
+  l = l ^ a ^ b;
+}
+
+template <int WPL>
+__device__ __forceinline__ void dense_load(uint32_t (&w)[WPL], const uint32_t *__restrict__ T, uint32_t y, int lane) {
+  const uint32_t *p = T + (size_t)y * (WPL * 32) + lane * WPL;
+  if (WPL == 4) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+    w[0] = q.x; w[1 % WPL] = q.y; w[2 % WPL] = q.z; w[3 % WPL] = q.w;
+  } else if (WPL == 2) {
+    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+    w[0] = q.x; w[1 % WPL] = q.y;
+  } else {
+    w[0] = __ldg(p);
   }
+}
+
+// Eight neighbours (lanes g0..g0+7 of y, the set ones of act) into the low planes;
+// the carries of weight eight to e8.  POP: also popc(T[x] & T[y]), kept by the lane
+// of y in `pc`, for y below x.
+template <int WPL, bool POP>
+__device__ __forceinline__ void dense_eight(const uint32_t *__restrict__ T, uint32_t y, unsigned act, int g0, int lane,
+                                            const uint32_t (&tx)[WPL], uint32_t (&pl)[DENSE_PLANES][WPL],
+                                            uint32_t (&e8)[WPL], uint32_t x, uint32_t &pc) {
+  uint32_t w[8][WPL];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const uint32_t yi = __shfl_sync(ACCX_FULL_MASK, y, g0 + i);
+    if ((act >> (g0 + i)) & 1u) {
+      dense_load<WPL>(w[i], T, yi, lane);
+    } else {
+#pragma unroll
+      for (int k = 0; k < WPL; k++) w[i][k] = 0;
+    }
+  }
+  if (POP) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      uint32_t c = 0;
+#pragma unroll
+      for (int k = 0; k < WPL; k++) c += __popc(w[i][k] & tx[k]);
+      c = __reduce_add_sync(ACCX_FULL_MASK, c);
+      if (lane == g0 + i) pc = c;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < WPL; k++) {
+    uint32_t ta, tb, fa, fb;
+    accx_csa(ta, pl[0][k], w[0][k], w[1][k]);
+    accx_csa(tb, pl[0][k], w[2][k], w[3][k]);
+    accx_csa(fa, pl[1][k], ta, tb);
+    accx_csa(ta, pl[0][k], w[4][k], w[5][k]);
+    accx_csa(tb, pl[0][k], w[6][k], w[7][k]);
+    accx_csa(fb, pl[1][k], ta, tb);
+    accx_csa(e8[k], pl[2][k], fa, fb);
+  }
+}
+
+// A warp per item.  ALL: every edge between rows below M is of the bitmap kind;
+// otherwise each neighbour's kind is looked up as classify does.
+template <int WPL, bool ALL>
+__global__ void __launch_bounds__(DENSE_WARPS * 32, 2) k_dense_pairs(
+    const uint32_t *__restrict__ off, const int32_t *__restrict__ dst, const uint32_t *__restrict__ pre,
+    const uint32_t *__restrict__ low, const uint32_t *__restrict__ T, const uint4 *__restrict__ items, uint32_t cap,
+    int policy, const uint8_t *__restrict__ table, uint32_t pcap, int32_t *__restrict__ cnt,
+    unsigned long long *__restrict__ ctr) {
+  __shared__ uint32_t s_pl[DENSE_WARPS][DENSE_PLANES][WPL * 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long total = ctr[C_DENSE];
+  if (total > cap) total = cap;
+  unsigned long long found = 0;
+  const unsigned long long nw = (unsigned long long)gridDim.x * DENSE_WARPS;
+  for (unsigned long long it = (unsigned long long)blockIdx.x * DENSE_WARPS + warp; it < total; it += nw) {
+    const uint4 item = __ldg(items + it);
+    const uint32_t x = item.x, eb = item.y, ec = item.z;
+    const uint32_t px = ALL ? 0u : __ldg(pre + x);
+    uint32_t tx[WPL], pl[DENSE_PLANES][WPL];
+    dense_load<WPL>(tx, T, x, lane);
+#pragma unroll
+    for (int p = 0; p < DENSE_PLANES; p++)
+#pragma unroll
+      for (int k = 0; k < WPL; k++) pl[p][k] = 0;
+    uint32_t yn = (uint32_t)lane < ec ? (uint32_t)__ldg(dst + eb + lane) : 0xffffffffu;
+    for (uint32_t j = 0; j < ec; j += 32) {
+      const uint32_t y = yn;
+      yn = j + 32 + lane < ec ? (uint32_t)__ldg(dst + eb + j + 32 + lane) : 0xffffffffu;
+      bool on = y != 0xffffffffu;
+      if (!ALL && on) on = accx_dense_edge(policy, table, x, px, y, __ldg(pre + y), pcap);
+      const unsigned act = __ballot_sync(ACCX_FULL_MASK, on);
+      if (!act) continue;
+      const unsigned below = __ballot_sync(ACCX_FULL_MASK, on && y < x);
+      uint32_t pc = 0;
+      uint32_t e8[4][WPL], c16[2][WPL];
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        if ((below >> (8 * g)) & 0xffu) {
+          dense_eight<WPL, true>(T, y, act, 8 * g, lane, tx, pl, e8[g], x, pc);
+        } else if ((act >> (8 * g)) & 0xffu) {
+          dense_eight<WPL, false>(T, y, act, 8 * g, lane, tx, pl, e8[g], x, pc);
+        } else {
+#pragma unroll
+          for (int k = 0; k < WPL; k++) e8[g][k] = 0;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < WPL; k++) {
+        uint32_t c;
+        accx_csa(c16[0][k], pl[3][k], e8[0][k], e8[1][k]);
+        accx_csa(c16[1][k], pl[3][k], e8[2][k], e8[3][k]);
+        accx_csa(c, pl[4][k], c16[0][k], c16[1][k]);
+#pragma unroll
+        for (int p = 5; p < DENSE_PLANES; p++) {
+          const uint32_t o = pl[p][k];
+          pl[p][k] = o ^ c;
+          c &= o;
+        }
+      }
+      if (((below >> lane) & 1u) && pc) {
+        found += pc;
+        atomicAdd(cnt + eb + j + lane, (int32_t)pc);
+      }
+    }
+    // the counters of the row's hub entries, through shared memory
+#pragma unroll
+    for (int p = 0; p < DENSE_PLANES; p++)
+#pragma unroll
+      for (int k = 0; k < WPL; k++) s_pl[warp][p][lane * WPL + k] = pl[p][k];
+    __syncwarp();
+    const uint32_t ub = __ldg(off + x), lw = __ldg(low + x);
+    for (uint32_t i = lane; i < lw; i += 32) {
+      const uint32_t a = (uint32_t)__ldg(dst + ub + i), wd = (a >> 5) & (WPL * 32 - 1), bit = a & 31u;
+      uint32_t v = 0;
+#pragma unroll
+      for (int p = 0; p < DENSE_PLANES; p++) v |= ((s_pl[warp][p][wd] >> bit) & 1u) << p;
+      if (v) atomicAdd(cnt + ub + i, (int32_t)v);
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) found += __shfl_xor_sync(ACCX_FULL_MASK, found, d);
+  if (lane == 0 && found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_BITMAP], found);
 }
 
 // One piece of a long list for one warp: G pair groups (64 G ids) from the
@@ -511,7 +717,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
   for (uint32_t i = tid; i <= nwords; i += nt) words[i] = 0;
   unsigned long long total = ctr[C_HEAVY];
   if (total > items_cap) total = items_cap;
-  unsigned long long found = 0, probed = 0;  // this thread's share, summed per warp at the end
+  unsigned long long found = 0;  // this thread's share, summed per warp at the end
   if (tid == 0) {
     s_it = atomicAdd(&ctr[C_ITEMS], 1ull);
     s_target = accx_item_target(ctr, target_max, gridDim.x);
@@ -546,7 +752,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
         sst = e.x;
         len = (e.y & OR_SL_GALLOP) ? 0u : e.y;  // galloping entries are not this kernel's
       }
-      probed += len;
       const bool is_short = len > 0 && len < LONG_SEG, is_long = len >= LONG_SEG;
       const unsigned bs = __ballot_sync(ACCX_FULL_MASK, is_short), bl = __ballot_sync(ACCX_FULL_MASK, is_long);
       uint32_t incl = is_short ? len : 0u;
@@ -700,14 +905,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
     __syncthreads();
   }
 #pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    found += __shfl_xor_sync(ACCX_FULL_MASK, found, d);
-    probed += __shfl_xor_sync(ACCX_FULL_MASK, probed, d);
-  }
-  if (lane == 0) {
-    if (found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_BITMAP], found);
-    if (probed) atomicAdd(&ctr[C_PROBED], probed);
-  }
+  for (int d = 16; d >= 1; d >>= 1) found += __shfl_xor_sync(ACCX_FULL_MASK, found, d);
+  if (lane == 0 && found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_BITMAP], found);
 }
 
 // Every credit lands on an edge's prefix entry (the entry in the larger id's

@@ -90,3 +90,32 @@ def test_shapes(kw):
     G = accx.Graph.generate(accx.chung_lu_params(60000, 20, 2.1, 6000, seed=5))
     off, dst = G.download()
     _check(off, dst, **kw)
+
+
+# dense rows (hub ids as bit masks): 1024, 2048 and 4096 bits a row by the graph's
+# size, every edge of the bitmap kind or only some (tables, few owner counters), rows
+# cut by the window, and graphs too small or flat for any
+@pytest.mark.parametrize("scale,ef", [(11, 40), (13, 24), (15, 16), (16, 32), (18, 16), (20, 8)])
+def test_dense_rows_rmat(scale, ef):
+    G = accx.Graph.generate(accx.rmat_params(scale, ef, seed=scale))
+    off, dst = G.download()
+    ref = oracle.cn_count(off, dst, nthreads=16)
+    G.relabel()
+    rng = np.random.default_rng(scale)
+    for kw in ({"policy": "bitmap"}, {"policy": "bitmap", "sparse_kb": 1}, {"policy": "bitmap", "window_kb": 1},
+               {"policy": "table", "table": rng.integers(0, 3, size=(24, 24)).astype(np.uint8)}):
+        assert np.array_equal(G.count(bias=2, orient=True, **kw), ref), kw
+        matches, _ = G.last_matches()
+        assert sum(matches.values()) == (int(ref.sum()) - 2 * len(ref)) // 6, kw
+
+
+@pytest.mark.parametrize("n,hubs", [(1500, 1023), (1500, 1024), (1500, 1025), (2600, 2049), (5200, 4097)])
+def test_dense_rows_around_k(n, hubs):
+    """Cliques of hubs around the mask's 1024, 2048 and 4096 ids, with leaves on them:
+    counters near their ten bits, rows of every word."""
+    rng = np.random.default_rng(hubs)
+    a, b = np.triu_indices(hubs, 1)
+    m = rng.random(len(a)) < (1.0 if hubs < 1100 else 0.3)
+    k = (n - hubs) * 200
+    off, dst = _csr(n, np.concatenate([a[m], rng.integers(hubs, n, k)]), np.concatenate([b[m], rng.integers(0, hubs, k)]))
+    _check(off, dst)

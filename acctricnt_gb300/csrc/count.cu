@@ -967,7 +967,9 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
       auto kd = wpl == 4 ? (all ? k_dense_pairs<4, true> : k_dense_pairs<4, false>)
               : wpl == 2 ? (all ? k_dense_pairs<2, true> : k_dense_pairs<2, false>)
                          : (all ? k_dense_pairs<1, true> : k_dense_pairs<1, false>);
-      kd<<<sms * 2, DENSE_WARPS * 32, 0, s>>>(off, dst, g->d_pre, g->d_dense_low, g->d_dense_t, g->d_dense_items, dcap,
+      const size_t dsmem = (size_t)DENSE_WARPS * 2u * 8u * 32u * wpl * 4u;
+      ACCX_CUDA_TRY(cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
+      kd<<<sms * 2, DENSE_WARPS * 32, dsmem, s>>>(off, dst, g->d_pre, g->d_dense_low, g->d_dense_t, g->d_dense_items, dcap,
                                               policy, g->d_table, pcap, cnt, ctr);
     }
     const size_t ow_smem = sizeof(ow_warp) * OW_WARPS;

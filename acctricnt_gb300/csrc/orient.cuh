@@ -436,8 +436,8 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
 // Probing spent ~54 thread instructions an id (a hit costs a rank, a RED and a shared
 // atomic); at R-MAT 24 the 61 % of all probes that lie on edges with c < 65536 have
 // 65-98 % of their ids below 4096.  K and M come from k_dense_plan.  Measured at
-// R-MAT 24 (K 4096, M 131072): list probing 71.2 -> 39.6 ms for 9.8 ms here, bound by
-// L2 (512 bytes an entry, 8.2 TB/s); Chung-Lu 3M: 4.2 -> 2.4 ms for both.
+// R-MAT 24 (K 4096, M 131072): list probing 71.2 -> 39.6 ms for 8.6 ms here; Chung-Lu 3M:
+// 4.2 -> 2.4 ms for both.
 #define DENSE_PLANES 10   // a counter holds at most DENSE_CHUNK neighbours: < 2^10
 #define DENSE_CHUNK_MAX 960u
 #define DENSE_WARPS 8
@@ -491,46 +491,64 @@ __device__ __forceinline__ void accx_csa(uint32_t &h, uint32_t &l, uint32_t a, u
   l = l ^ a ^ b;
 }
 
+// The masks of eight neighbours (lanes g0..g0+7 of y, the set ones of act) on their
+// way into shared memory, one asynchronous copy of 4 WPL bytes a lane and row; rows that
+// are not active, and words past the smaller of x and y (no triangle there), arrive as
+// zeros without a read.
 template <int WPL>
-__device__ __forceinline__ void dense_load(uint32_t (&w)[WPL], const uint32_t *__restrict__ T, uint32_t y, int lane) {
-  const uint32_t *p = T + (size_t)y * (WPL * 32) + lane * WPL;
-  if (WPL == 4) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
-    w[0] = q.x; w[1 % WPL] = q.y; w[2 % WPL] = q.z; w[3 % WPL] = q.w;
-  } else if (WPL == 2) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
-    w[0] = q.x; w[1 % WPL] = q.y;
-  } else {
-    w[0] = __ldg(p);
-  }
-}
-
-// Eight neighbours (lanes g0..g0+7 of y, the set ones of act) into the low planes;
-// the carries of weight eight to e8.  POP: also popc(T[x] & T[y]), kept by the lane
-// of y in `pc`, for y below x.
-template <int WPL, bool POP>
-__device__ __forceinline__ void dense_eight(const uint32_t *__restrict__ T, uint32_t y, unsigned act, int g0, int lane,
-                                            const uint32_t (&tx)[WPL], uint32_t (&pl)[DENSE_PLANES][WPL],
-                                            uint32_t (&e8)[WPL], uint32_t x, uint32_t &pc) {
-  uint32_t w[8][WPL];
+__device__ __forceinline__ void dense_issue(uint32_t sbuf, const uint32_t *__restrict__ T, uint32_t x, uint32_t y,
+                                            unsigned act, int g0, int lane) {
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const uint32_t yi = __shfl_sync(ACCX_FULL_MASK, y, g0 + i);
-    if ((act >> (g0 + i)) & 1u) {
-      dense_load<WPL>(w[i], T, yi, lane);
-    } else {
-#pragma unroll
-      for (int k = 0; k < WPL; k++) w[i][k] = 0;
-    }
+    const bool in = ((act >> (g0 + i)) & 1u) && (uint32_t)lane * (WPL * 32) < min(x, yi);
+    const uint32_t *src = T + (in ? (size_t)yi * (WPL * 32) + lane * WPL : 0);
+    const int bytes = in ? WPL * 4 : 0;
+    const uint32_t to = sbuf + (uint32_t)(i * 32 + lane) * (WPL * 4);
+    if (WPL == 4)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(bytes) : "memory");
+    else if (WPL == 2)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(to), "l"(src), "r"(bytes) : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src), "r"(bytes) : "memory");
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int WPL>
+__device__ __forceinline__ void dense_read(uint32_t (&w)[WPL], const uint32_t *p) {
+  if (WPL == 4) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(p);
+    w[0] = q.x; w[1 % WPL] = q.y; w[2 % WPL] = q.z; w[3 % WPL] = q.w;
+  } else if (WPL == 2) {
+    const uint2 q = *reinterpret_cast<const uint2 *>(p);
+    w[0] = q.x; w[1 % WPL] = q.y;
+  } else {
+    w[0] = *p;
+  }
+}
+
+// Eight neighbours' masks into the low planes; the carries of weight eight to e8.  POP:
+// also popc(T[x] & T[y]), kept by the lane of y in `pc` (two sums to a warp reduction:
+// each is at most 4096).
+template <int WPL, bool POP>
+__device__ __forceinline__ void dense_eight(const uint32_t *buf, int g0, int lane, const uint32_t (&tx)[WPL],
+                                            uint32_t (&pl)[DENSE_PLANES][WPL], uint32_t (&e8)[WPL], uint32_t &pc) {
+  uint32_t w[8][WPL];
+#pragma unroll
+  for (int i = 0; i < 8; i++) dense_read<WPL>(w[i], buf + (i * 32 + lane) * WPL);
   if (POP) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      uint32_t c = 0;
+    for (int i = 0; i < 8; i += 2) {
+      uint32_t c = 0, d = 0;
 #pragma unroll
-      for (int k = 0; k < WPL; k++) c += __popc(w[i][k] & tx[k]);
-      c = __reduce_add_sync(ACCX_FULL_MASK, c);
-      if (lane == g0 + i) pc = c;
+      for (int k = 0; k < WPL; k++) {
+        c += __popc(w[i][k] & tx[k]);
+        d += __popc(w[i + 1][k] & tx[k]);
+      }
+      c = __reduce_add_sync(ACCX_FULL_MASK, c + (d << 16));
+      if (lane == g0 + i) pc = c & 0xffffu;
+      if (lane == g0 + i + 1) pc = c >> 16;
     }
   }
 #pragma unroll
@@ -546,16 +564,29 @@ __device__ __forceinline__ void dense_eight(const uint32_t *__restrict__ T, uint
   }
 }
 
-// A warp per item.  ALL: every edge between rows below M is of the bitmap kind;
-// otherwise each neighbour's kind is looked up as classify does.
+// A warp per item.  The neighbours' masks come through a ring of two groups of eight in
+// the warp's shared memory: the next group is copied while this one is added, so the
+// loads in flight do not cost registers (R-MAT 24 count 70.7 -> 69.2 ms against loads
+// into registers; three CTAs an SM instead of two spill at K 4096: 70.0).  The ALU pipe
+// is the busiest (60 %), L2 at a third of its peak.  ALL: every edge between rows below
+// M is of the bitmap kind; otherwise each neighbour's kind is looked up as classify
+// does.
+template <int WPL>
+struct dense_ring {
+  uint32_t w[2][8 * 32 * WPL];  // also takes the planes at the item's end: DENSE_PLANES x 32 WPL words
+};
 template <int WPL, bool ALL>
 __global__ void __launch_bounds__(DENSE_WARPS * 32, 2) k_dense_pairs(
     const uint32_t *__restrict__ off, const int32_t *__restrict__ dst, const uint32_t *__restrict__ pre,
     const uint32_t *__restrict__ low, const uint32_t *__restrict__ T, const uint4 *__restrict__ items, uint32_t cap,
     int policy, const uint8_t *__restrict__ table, uint32_t pcap, int32_t *__restrict__ cnt,
     unsigned long long *__restrict__ ctr) {
-  __shared__ uint32_t s_pl[DENSE_WARPS][DENSE_PLANES][WPL * 32];
+  static_assert(DENSE_PLANES <= 16, "planes fit the ring");
+  extern __shared__ __align__(16) uint32_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t *ring = reinterpret_cast<dense_ring<WPL> *>(smem)[warp].w[0];
+  const uint32_t sring = (uint32_t)__cvta_generic_to_shared(ring);
+  constexpr uint32_t GROUP = 8 * 32 * WPL;  // words of a group
   unsigned long long total = ctr[C_DENSE];
   if (total > cap) total = cap;
   unsigned long long found = 0;
@@ -565,39 +596,49 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, 2) k_dense_pairs(
     const uint32_t x = item.x, eb = item.y, ec = item.z;
     const uint32_t px = ALL ? 0u : __ldg(pre + x);
     uint32_t tx[WPL], pl[DENSE_PLANES][WPL];
-    dense_load<WPL>(tx, T, x, lane);
+    dense_read<WPL>(tx, T + (size_t)x * (WPL * 32) + lane * WPL);
 #pragma unroll
     for (int p = 0; p < DENSE_PLANES; p++)
 #pragma unroll
       for (int k = 0; k < WPL; k++) pl[p][k] = 0;
-    uint32_t yn = (uint32_t)lane < ec ? (uint32_t)__ldg(dst + eb + lane) : 0xffffffffu;
-    for (uint32_t j = 0; j < ec; j += 32) {
-      const uint32_t y = yn;
-      yn = j + 32 + lane < ec ? (uint32_t)__ldg(dst + eb + j + 32 + lane) : 0xffffffffu;
+    auto active = [&](uint32_t y) {
       bool on = y != 0xffffffffu;
       if (!ALL && on) on = accx_dense_edge(policy, table, x, px, y, __ldg(pre + y), pcap);
-      const unsigned act = __ballot_sync(ACCX_FULL_MASK, on);
-      if (!act) continue;
-      const unsigned below = __ballot_sync(ACCX_FULL_MASK, on && y < x);
+      return __ballot_sync(ACCX_FULL_MASK, on);
+    };
+    uint32_t y = (uint32_t)lane < ec ? (uint32_t)__ldg(dst + eb + lane) : 0xffffffffu;
+    uint32_t yn = 32u + lane < ec ? (uint32_t)__ldg(dst + eb + 32 + lane) : 0xffffffffu;
+    unsigned act = active(y);
+    dense_issue<WPL>(sring, T, x, y, act, 0, lane);
+    for (uint32_t j = 0; j < ec; j += 32) {
+      const unsigned actn = active(yn);
+      const unsigned below = __ballot_sync(ACCX_FULL_MASK, y < x) & act;
       uint32_t pc = 0;
-      uint32_t e8[4][WPL], c16[2][WPL];
+      uint32_t e8[4][WPL];
 #pragma unroll
       for (int g = 0; g < 4; g++) {
+        // the next group on its way (at the end of the row: an empty one), then this one
+        if (g < 3) dense_issue<WPL>(sring + ((g + 1) & 1) * GROUP * 4, T, x, y, act, 8 * (g + 1), lane);
+        else dense_issue<WPL>(sring, T, x, yn, actn, 0, lane);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const uint32_t *buf = ring + (g & 1) * GROUP;
         if ((below >> (8 * g)) & 0xffu) {
-          dense_eight<WPL, true>(T, y, act, 8 * g, lane, tx, pl, e8[g], x, pc);
+          dense_eight<WPL, true>(buf, 8 * g, lane, tx, pl, e8[g], pc);
         } else if ((act >> (8 * g)) & 0xffu) {
-          dense_eight<WPL, false>(T, y, act, 8 * g, lane, tx, pl, e8[g], x, pc);
+          dense_eight<WPL, false>(buf, 8 * g, lane, tx, pl, e8[g], pc);
         } else {
 #pragma unroll
           for (int k = 0; k < WPL; k++) e8[g][k] = 0;
         }
+        __syncwarp();
       }
 #pragma unroll
       for (int k = 0; k < WPL; k++) {
-        uint32_t c;
-        accx_csa(c16[0][k], pl[3][k], e8[0][k], e8[1][k]);
-        accx_csa(c16[1][k], pl[3][k], e8[2][k], e8[3][k]);
-        accx_csa(c, pl[4][k], c16[0][k], c16[1][k]);
+        uint32_t a, b, c;
+        accx_csa(a, pl[3][k], e8[0][k], e8[1][k]);
+        accx_csa(b, pl[3][k], e8[2][k], e8[3][k]);
+        accx_csa(c, pl[4][k], a, b);
 #pragma unroll
         for (int p = 5; p < DENSE_PLANES; p++) {
           const uint32_t o = pl[p][k];
@@ -609,19 +650,24 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, 2) k_dense_pairs(
         found += pc;
         atomicAdd(cnt + eb + j + lane, (int32_t)pc);
       }
+      y = yn;
+      act = actn;
+      yn = j + 64 + lane < ec ? (uint32_t)__ldg(dst + eb + j + 64 + lane) : 0xffffffffu;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
     // the counters of the row's hub entries, through shared memory
 #pragma unroll
     for (int p = 0; p < DENSE_PLANES; p++)
 #pragma unroll
-      for (int k = 0; k < WPL; k++) s_pl[warp][p][lane * WPL + k] = pl[p][k];
+      for (int k = 0; k < WPL; k++) ring[p * (WPL * 32) + lane * WPL + k] = pl[p][k];
     __syncwarp();
     const uint32_t ub = __ldg(off + x), lw = __ldg(low + x);
     for (uint32_t i = lane; i < lw; i += 32) {
       const uint32_t a = (uint32_t)__ldg(dst + ub + i), wd = (a >> 5) & (WPL * 32 - 1), bit = a & 31u;
       uint32_t v = 0;
 #pragma unroll
-      for (int p = 0; p < DENSE_PLANES; p++) v |= ((s_pl[warp][p][wd] >> bit) & 1u) << p;
+      for (int p = 0; p < DENSE_PLANES; p++) v |= ((ring[p * (WPL * 32) + wd] >> bit) & 1u) << p;
       if (v) atomicAdd(cnt + ub + i, (int32_t)v);
     }
     __syncwarp();

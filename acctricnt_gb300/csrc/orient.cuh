@@ -715,27 +715,29 @@ __device__ __forceinline__ uint32_t or_piece(const int32_t *__restrict__ dst, ui
   return h;
 }
 
-#define SHORT_PIECE (32u * PROBE_UNROLL)  // ids per short piece (concatenated short lists)
 #define LONG_PIECE (32u * LONG_UNROLL)    // ids per piece of a long list
 
-// Bitmap kind.  CTAs take work items (an owner x, or a slice of its list when
-// the owner's probe work is large) from a device counter.  The owner's prefix
-// -- ids below x, which the classifier keeps below W -- is staged as a dense
-// bitmap over [0, W) plus, per non-empty 32-bit word, the prefix position of
-// the word's first id (rank of an id = that base + popcount of the lower bits).
-// The slice is walked in rounds of blockDim entries; the classifier stored, per
-// bitmap entry (x,y), where P(y) starts and its length cut at min(x,y) (0 for
-// other entries), so a round starts with one coalesced load per entry.  Short
-// probe lists are concatenated (CTA prefix sum) and cut into chunks; warps take
-// whole long lists (at most the owner counters' size, walked in pieces of
-// LONG_PIECE ids) and then the short chunks from one shared queue, so the
-// small grains even out the round's end.  A hit at partner entry j
-// credits cnt[j] (RED), the owner's shared counter of the id's rank, and the
-// edge (shared per-entry counters, credited after the round).
-// NT = the block size the per-round arrays are sized for (blockDim.x <= NT); a
-// 512-thread instance needs half the static shared memory, so two CTAs fit an
-// SM when the window is small enough, and a 256-thread one with a small window
-// runs four per SM.
+// Bitmap kind.  CTAs take work items (an owner x, or a slice of its list when the
+// owner's probe work is large) from a device counter.  The owner's prefix -- ids below
+// x, which the classifier keeps below W -- is staged as a dense bitmap over [0, W)
+// plus, per non-empty 32-bit word, the prefix position of the word's first id (rank of
+// an id = that base + popcount of the lower bits).  The warps then take the slice's
+// entries 32 at a time from a shared queue and need no barrier until its end: the
+// classifier stored, per bitmap entry (x,y), where P(y) starts and its length cut at
+// min(x,y) (0 for other entries), one coalesced load.  A long probe list is walked by
+// the whole warp in pieces of LONG_PIECE ids, its bounds and hits staying in registers;
+// short ones are concatenated (warp scan) and streamed 32 ids a step.  A hit at partner
+// entry j credits cnt[j] (RED), the owner's shared counter of the id's rank, and the
+// edge (after the 32 entries).
+// NT = the largest block size (blockDim.x <= NT); four 256-thread CTAs an SM with the
+// default window, two of 512 threads with windows up to ~60 KiB.
+// Bound by instruction issue and latency.  The earlier form took rounds of blockDim
+// entries with CTA scans and four barriers each, and one queue entry per long list:
+// ~0.15 ns a list and 0.84 ps an id at R-MAT 22 and 24 (R-MAT 24 count 69.2 -> 64.0 ms,
+// Chung-Lu 3M 4.12 -> 3.90).
+struct or_seg {
+  uint32_t pre[33], beg[32], hit[32];
+};
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__restrict__ off,
                                                        const int32_t *__restrict__ dst,
@@ -753,32 +755,38 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
   // base (< pxs) + 31, so the counter add needs no bounds test even on unsorted input
   uint32_t *ocnt = smem + nwords + 4;
   uint16_t *wbase = reinterpret_cast<uint16_t *>(ocnt + pcap + 32);  // nwords first-id positions
-  __shared__ unsigned long long s_it;
-  __shared__ uint32_t s_tot, s_nseg, s_nlong, s_next, s_target;
-  __shared__ uint32_t s_wsum[32], s_wcnt[32], s_wlong[32];
-  __shared__ uint32_t s_pre[NT + 1], s_beg[NT], s_ent[NT], s_hit[NT];
-  __shared__ uint32_t s_lbeg[NT], s_llen[NT], s_lent[NT], s_lhit[NT];
+  __shared__ or_seg s_seg[NT / 32];
+  // the next item, fetched while the current one is walked: x, its first and last entry
+  // to walk, row start and prefix length (x = 0xffffffff: none)
+  __shared__ uint32_t s_item[5], s_next;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
+  const int lane = tid & 31;
+  or_seg &S = s_seg[tid >> 5];
+  auto fetch = [&]() {
+    unsigned long long total = ctr[C_HEAVY];
+    if (total > items_cap) total = items_cap;
+    const unsigned long long it = atomicAdd(&ctr[C_ITEMS], 1ull);
+    uint32_t x = 0xffffffffu;
+    if (it < total) {
+      x = items[it];
+      const uint32_t ub = off[x], du = off[x + 1] - ub;
+      uint32_t nchunks, nsplit;
+      accx_item_shape(du, 0, work_u[x], 1, accx_item_target(ctr, target_max, gridDim.x), &nchunks, &nsplit);
+      const uint32_t sp = (uint32_t)(it - slot[x]);
+      s_item[1] = ub + (uint32_t)((unsigned long long)du * sp / nsplit);
+      s_item[2] = ub + (uint32_t)((unsigned long long)du * (sp + 1) / nsplit);
+      s_item[3] = ub;
+      s_item[4] = pre[x];
+    }
+    s_item[0] = x;
+  };
   for (uint32_t i = tid; i <= nwords; i += nt) words[i] = 0;
-  unsigned long long total = ctr[C_HEAVY];
-  if (total > items_cap) total = items_cap;
   unsigned long long found = 0;  // this thread's share, summed per warp at the end
-  if (tid == 0) {
-    s_it = atomicAdd(&ctr[C_ITEMS], 1ull);
-    s_target = accx_item_target(ctr, target_max, gridDim.x);
-  }
+  if (tid == 0) fetch();
   __syncthreads();
   for (;;) {
-    const unsigned long long it = s_it;
-    if (it >= total) break;
-    const uint32_t x = items[it];
-    const uint32_t ub = off[x], ue = off[x + 1], du = ue - ub, px = pre[x];
-    uint32_t nchunks, nsplit;
-    accx_item_shape(du, 0, work_u[x], 1, s_target, &nchunks, &nsplit);
-    const uint32_t sp = (uint32_t)(it - slot[x]);
-    const uint32_t pa = ub + (uint32_t)((unsigned long long)du * sp / nsplit);
-    const uint32_t pb = ub + (uint32_t)((unsigned long long)du * (sp + 1) / nsplit);
+    const uint32_t x = s_item[0], pa = s_item[1], pb = s_item[2], ub = s_item[3], px = s_item[4];
+    if (x == 0xffffffffu) break;
     const uint32_t pxs = px <= pcap ? px : 0;  // the classifier guarantees px <= pcap for bitmap owners
     for (uint32_t i = tid; i < pxs; i += nt) {
       const uint32_t id = (uint32_t)__ldg(dst + ub + i);
@@ -788,98 +796,70 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
       }
       ocnt[i] = 0;
     }
+    if (tid == 0) s_next = 0;
     __syncthreads();
-    if (tid == 0) s_it = atomicAdd(&ctr[C_ITEMS], 1ull);  // the next item, read after this one
-    for (uint32_t r0 = pa; r0 < pb; r0 += (uint32_t)nt) {
-      const uint32_t k = r0 + (uint32_t)tid;
+    if (tid == 0) fetch();  // read by all after this item's last barrier
+    __syncwarp();
+    for (;;) {
+      uint32_t r0 = 0;
+      if (lane == 0) r0 = atomicAdd(&s_next, 32u);
+      r0 = pa + __shfl_sync(ACCX_FULL_MASK, r0, 0);
+      if (r0 >= pb) break;
+      const uint32_t k = r0 + (uint32_t)lane;
       uint32_t sst = 0, len = 0;
       if (k < pb) {
         const uint2 e = sl[k];
         sst = e.x;
         len = (e.y & OR_SL_GALLOP) ? 0u : e.y;  // galloping entries are not this kernel's
       }
-      const bool is_short = len > 0 && len < LONG_SEG, is_long = len >= LONG_SEG;
-      const unsigned bs = __ballot_sync(ACCX_FULL_MASK, is_short), bl = __ballot_sync(ACCX_FULL_MASK, is_long);
-      uint32_t incl = is_short ? len : 0u;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t a = __shfl_up_sync(ACCX_FULL_MASK, incl, d);
-        if (lane >= d) incl += a;
-      }
-      if (lane == 31) {
-        s_wsum[warp] = incl;
-        s_wcnt[warp] = __popc(bs);
-        s_wlong[warp] = __popc(bl);
-      }
-      __syncthreads();
-      if (warp == 0) {
-        const uint32_t ws = lane < nwarps ? s_wsum[lane] : 0u, wc = lane < nwarps ? s_wcnt[lane] : 0u;
-        const uint32_t wl = lane < nwarps ? s_wlong[lane] : 0u;
-        uint32_t is = ws, ic = wc, il = wl;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const uint32_t a = __shfl_up_sync(ACCX_FULL_MASK, is, d), b = __shfl_up_sync(ACCX_FULL_MASK, ic, d);
-          const uint32_t c = __shfl_up_sync(ACCX_FULL_MASK, il, d);
-          if (lane >= d) { is += a; ic += b; il += c; }
+      uint32_t hits = 0;
+      for (unsigned lm = __ballot_sync(ACCX_FULL_MASK, len >= LONG_SEG); lm; lm &= lm - 1) {
+        // a long list, walked in pieces of LONG_PIECE ids from the even entry at or
+        // before its start
+        const int src = __ffs(lm) - 1;
+        const uint32_t a0 = __shfl_sync(ACCX_FULL_MASK, sst, src);
+        const uint32_t a1 = a0 + __shfl_sync(ACCX_FULL_MASK, len, src);
+        uint32_t h = 0;
+        for (uint32_t j0 = a0 & ~1u; j0 < a1; j0 += LONG_PIECE) {
+          // the last piece loads only the pair groups it needs (the size class is
+          // warp-uniform, and each class issues all its loads at once)
+          const uint32_t rem = a1 - j0;
+          if (rem > 256u) h += or_piece<LONG_UNROLL / 2>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
+          else if (rem > 128u) h += or_piece<4>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
+          else if (rem > 64u) h += or_piece<2>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
+          else h += or_piece<1>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
         }
-        if (lane < nwarps) {
-          s_wsum[lane] = is - ws;
-          s_wcnt[lane] = ic - wc;
-          s_wlong[lane] = il - wl;
+        h = __reduce_add_sync(ACCX_FULL_MASK, h);
+        if (lane == src) hits = h;
+      }
+      const bool is_short = len > 0 && len < LONG_SEG;
+      const unsigned bs = __ballot_sync(ACCX_FULL_MASK, is_short);
+      if (bs) {
+        const uint32_t incl = accx_warp_incl_sum(is_short ? len : 0u, lane);
+        const uint32_t tot = __shfl_sync(ACCX_FULL_MASK, incl, 31), nseg = __popc(bs);
+        const uint32_t me = __popc(bs & ((1u << lane) - 1u));
+        if (is_short) {
+          S.pre[me] = incl - len;
+          S.beg[me] = sst;
+          S.hit[me] = 0;
         }
-        if (lane == 31) { s_tot = is; s_nseg = ic; s_nlong = il; s_next = 0; }
-      }
-      __syncthreads();
-      if (is_short) {
-        const uint32_t idx = s_wcnt[warp] + __popc(bs & ((1u << lane) - 1u));
-        s_pre[idx] = s_wsum[warp] + incl - len;
-        s_beg[idx] = sst;
-        s_ent[idx] = k;
-        s_hit[idx] = 0;
-      }
-      if (is_long) {
-        const uint32_t idx = s_wlong[warp] + __popc(bl & ((1u << lane) - 1u));
-        s_lbeg[idx] = sst;
-        s_llen[idx] = len;
-        s_lent[idx] = k;
-        s_lhit[idx] = 0;
-      }
-      if (tid == 0) s_pre[s_nseg] = s_tot;
-      __syncthreads();
-      const uint32_t tot = s_tot, nseg = s_nseg, nlong = s_nlong;
-      // the queue: whole long lists first (the larger grains), then short chunks
-      const uint32_t nsp = (tot + SHORT_PIECE - 1) / SHORT_PIECE, npieces = nlong + nsp;
-      for (;;) {
-        uint32_t p = 0;
-        if (lane == 0) p = atomicAdd(&s_next, 1u);
-        p = __shfl_sync(ACCX_FULL_MASK, p, 0);
-        if (p >= npieces) break;
-        if (p >= nlong) {
-          // short chunk: SHORT_PIECE consecutive ids of the concatenation
-          const uint32_t c0 = (p - nlong) * SHORT_PIECE;
-          uint32_t lo = 0, hi = nseg;
-          while (hi - lo > 1) {
-            const uint32_t step = (hi - lo + 31) / 32;
-            const uint32_t q = lo + (uint32_t)lane * step;
-            const unsigned b = __ballot_sync(ACCX_FULL_MASK, q < hi && s_pre[q] <= c0);
-            lo += (31 - __clz(b)) * step;
-            const uint32_t nh = lo + step;
-            hi = nh < hi ? nh : hi;
-          }
-          uint32_t segb = lo;
+        if (lane == 0) S.pre[nseg] = tot;
+        __syncwarp();
+        uint32_t segb = 0;
+        for (uint32_t c0 = 0; c0 < tot; c0 += 32u * PROBE_UNROLL) {
           int32_t xs[PROBE_UNROLL];
           uint32_t sg[PROBE_UNROLL], gi[PROBE_UNROLL];
 #pragma unroll
           for (int r = 0; r < PROBE_UNROLL; r++) {
-            const uint32_t i0 = c0 + 32u * r;
-            const uint32_t i = i0 + (uint32_t)lane;
+            // 32 ids meet at most 31 segment starts after segb: each lane loads one
+            // start, and a lane's segment is segb + the starts at or before its id
+            const uint32_t i0 = c0 + 32u * r, i = i0 + (uint32_t)lane;
             const uint32_t kb = segb + 1u + (uint32_t)lane;
-            const uint32_t bnd = kb <= nseg ? s_pre[kb] : 0xffffffffu;
-            const uint32_t o = bnd - i0;
+            const uint32_t o = (kb <= nseg ? S.pre[kb] : 0xffffffffu) - i0;
             const unsigned M = __reduce_or_sync(ACCX_FULL_MASK, o < 32u ? (1u << o) : 0u);
-            const uint32_t sj = segb + __popc(M & (lane == 31 ? 0xffffffffu : ((2u << lane) - 1u)));
+            const uint32_t sj = min(segb + __popc(M & (0xffffffffu >> (31 - lane))), 31u);
             sg[r] = sj;
-            gi[r] = (i < tot) ? s_beg[sj] + (i - s_pre[sj]) : 0u;
+            gi[r] = (i < tot) ? S.beg[sj] + (i - S.pre[sj]) : 0u;
             xs[r] = (i < tot) ? __ldg(dst + gi[r]) : -1;
             segb += __popc(M) + (__ballot_sync(ACCX_FULL_MASK, o == 32u) ? 1u : 0u);
           }
@@ -892,48 +872,24 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
               const uint32_t rk = wbase[id >> 5] + __popc(wd << (~id & 31u)) - 1u;
               atomicAdd(cnt + gi[r], 1);
               atomicAdd(&ocnt[rk], 1u);  // rk < pxs on a sorted CSR, < pxs + 31 always (spare counters)
-              atomicAdd(&s_hit[sg[r]], 1u);
+              atomicAdd(&S.hit[sg[r]], 1u);
             }
           }
-        } else {
-          // a long list, walked in pieces of LONG_PIECE ids from the even entry at
-          // or before its start
-          const uint32_t q = p;
-          const uint32_t a0 = s_lbeg[q], a1 = a0 + s_llen[q];
-          uint32_t h = 0;
-          for (uint32_t j0 = a0 & ~1u; j0 < a1; j0 += LONG_PIECE) {
-            // the last piece loads only the pair groups it needs (the size
-            // class is warp-uniform, and each class issues all its loads at once)
-            const uint32_t rem = a1 - j0;
-            if (rem > 256u) h += or_piece<LONG_UNROLL / 2>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
-            else if (rem > 128u) h += or_piece<4>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
-            else if (rem > 64u) h += or_piece<2>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
-            else h += or_piece<1>(dst, j0, a0, a1, lane, W, words, wbase, ocnt, pxs, cnt);
-          }
-          h = __reduce_add_sync(ACCX_FULL_MASK, h);
-          if (lane == 0 && h) atomicAdd(&s_lhit[q], h);
         }
+        __syncwarp();
+        if (is_short) hits = S.hit[me];
+        __syncwarp();
       }
-      __syncthreads();
       // edge credits go to the edge's prefix entry: the entry itself when y < x
-      // (through the owner's counters), else x's position in N(y), which is where
-      // the partner range was cut
-      for (uint32_t q = tid; q < nseg + nlong; q += nt) {
-        const bool sh = q < nseg;
-        const uint32_t h = sh ? s_hit[q] : s_lhit[q - nseg], kk = sh ? s_ent[q] : s_lent[q - nseg];
-        found += h;
-        if (h) {
-          if (kk - ub < px) {
-            if (kk - ub < pxs) atomicAdd(&ocnt[kk - ub], h);
-            else atomicAdd(cnt + kk, (int32_t)h);
-          } else {
-            const uint32_t cut = sh ? s_beg[q] + (s_pre[q + 1] - s_pre[q]) : s_lbeg[q - nseg] + s_llen[q - nseg];
-            atomicAdd(cnt + cut, (int32_t)h);
-          }
-        }
+      // (through the owner's counters), else x's position in N(y), which is where the
+      // partner range was cut
+      found += hits;
+      if (hits) {
+        if (k - ub < pxs) atomicAdd(&ocnt[k - ub], hits);
+        else atomicAdd(cnt + (k - ub < px ? k : sst + len), (int32_t)hits);
       }
-      __syncthreads();
     }
+    __syncthreads();
     // owner-side credits to HBM, then clear what was staged
     for (uint32_t i = tid; i < pxs; i += nt) {
       const uint32_t h = ocnt[i];

@@ -79,6 +79,7 @@ struct accx_graph {
   uint32_t *d_or_items = nullptr;          // n + m/32 + 1 oriented bitmap work items: owner of each
   uint32_t *d_rev = nullptr;               // m reverse entry of every entry of the counting CSR (oriented counts)
   uint32_t *d_rev_orig = nullptr;          // m reverse entries of the handle's own CSR, recorded by full validation
+  uint32_t *d_dg = nullptr;                // the default policy's degree-ordered count
   // dense rows of the relabeled CSR (planned by the relabel; 0 rows: none worth it)
   uint32_t dense_k = 0, dense_m = 0;       // hub ids (bits a row) and rows
   uint32_t dense_maxpre = 0;               // the longest prefix of those rows

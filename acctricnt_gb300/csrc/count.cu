@@ -40,7 +40,8 @@
 #define C_HEAVY 16  // work items of the oriented bitmap kernel
 #define C_LIGHT 17  // owners of the warp-per-owner kernel
 #define C_DENSE 18  // work items of the dense rows
-#define C_NUM 19
+#define C_DGBIG 19  // long rows of the default policy's degree-ordered count
+#define C_NUM 20
 
 #define MERGE_WARPS 8        // warps per merge/gallop CTA
 #define ITEM_TARGET_DEFAULT (1u << 20)  // probe elements per bitmap work item
@@ -715,6 +716,7 @@ __global__ void __launch_bounds__(1024, 1) k_bitmap(const uint32_t *__restrict__
 }
 
 #include "orient.cuh"
+#include "degree.cuh"
 
 // ---------------------------------------------------------------------------
 // Mirror: each owned entry e=(u,v) adds the bias and copies its count to the
@@ -813,6 +815,17 @@ static bool alloc_dense(accx_graph *g) {
   return ok;
 }
 
+// Scratch of the degree-ordered count: entries and counters of the F lists (m each), two
+// lists of rows (n each), and the CTAs' items: at most a slice for each row of more than
+// DG_ROW_SMALL entries and one more per DG_SLICE entries.
+static bool alloc_degree(accx_graph *g) {
+  const size_t words = 2 * (size_t)g->m + 2 * (size_t)g->n + 2 + 2 * ((size_t)g->m / DG_ROW_SMALL + (size_t)g->m / DG_SLICE + 2);
+  bool ok = accx_dev_alloc((void **)&g->d_dg, sizeof(uint32_t) * words, g->home) == cudaSuccess;
+  if (ok && g->home) ok = cudaStreamSynchronize(g->home) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
 // Persistent classify CTAs: four per SM (64 registers a thread), at most one per
 // block of entries.
 static unsigned classify_grid(int sms, uint32_t m) {
@@ -865,8 +878,13 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   const uint32_t *tilerow = rel ? g->d_rtilerow : g->d_tilerow;
   unsigned long long *ctr = g->d_counters;
   unsigned long long *work_u = g->d_counters + C_NUM;
-  ACCX_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * (C_NUM + (size_t)n + 1), s));
-  if (!orient) ACCX_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(m ? m : 1), s));
+  // the default policy on a CSR known to be symmetric (degree.cuh): ids in the warps'
+  // tables have 24 bits; without that, or without room, an intersection per edge
+  bool degree = !orient && policy == ACCX_POLICY_HEURISTIC && g->symmetric && n <= OW_MAX_N && m;
+  const bool small = degree && m <= DG_SMALL_M;
+  if (degree && !small && !g->d_dg && !alloc_degree(g)) degree = false;
+  ACCX_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * (C_NUM + (degree ? 0 : (size_t)n + 1)), s));
+  if (!orient && !degree) ACCX_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(m ? m : 1), s));
   if (m == 0) {
     g->cnt_bias = bias;
     g->cnt_valid = true;
@@ -883,7 +901,33 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   ACCX_MARK(0);
   int sms = accx_sm_count(g->device);
   if (o && o->sm_limit > 0 && o->sm_limit < sms) sms = o->sm_limit;
-  if (orient) {
+  if (small) {
+    ACCX_MARK(1);
+    k_count_small<<<(m + DS_TILE - 1) / DS_TILE, 256, 0, s>>>(off, tilerow, dst, n, m, bias, cnt, ctr);
+    ACCX_MARK(2);
+    ACCX_MARK(3);
+    ACCX_MARK(4);
+  } else if (degree) {
+    // F lists in the owned-edge list's place; entries, counters and row lists in d_dg
+    int32_t *f = reinterpret_cast<int32_t *>(g->d_edge_list), *fc = reinterpret_cast<int32_t *>(g->d_dg) + m;
+    const uint32_t row = m < DG_ROW_M ? DG_ROW_SMALL : DG_ROW;
+    uint32_t *ent = g->d_dg, *mid = ent + 2 * (size_t)m, *big = mid + n;
+    uint2 *heavy = reinterpret_cast<uint2 *>(g->d_dg + ((2 * (size_t)m + 2 * (size_t)n + 1) & ~(size_t)1));
+    k_dg_rows<<<sms * 8, DG_THREADS, 0, s>>>(off, dst, n, f, ent, fc, g->d_pre, big, mid, row, ctr);
+    k_dg_big<<<sms * 4, DG_THREADS, 0, s>>>(off, dst, f, ent, fc, g->d_pre, big, heavy, ctr);
+    ACCX_MARK(1);
+    const size_t smem = DG_SLOTS * 6u + DG_CAP * 4u;
+    const size_t smid = sizeof(dg_warp<DG_WARP>) * DG_WARPS, slight = sizeof(dg_warp<DG_LIGHT>) * DG_WARPS;
+    ACCX_CUDA_TRY(cudaFuncSetAttribute(k_dg_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ACCX_CUDA_TRY(cudaFuncSetAttribute(k_dg_warp<DG_WARP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smid));
+    k_dg_cta<<<sms * 6, DG_THREADS, smem, s>>>(off, dst, f, g->d_pre, heavy, fc, ctr);
+    k_dg_warp<DG_WARP><<<sms * 4, DG_THREADS, smid, s>>>(off, dst, f, g->d_pre, n, mid, fc, row, ctr);
+    k_dg_warp<DG_LIGHT><<<sms * 8, DG_THREADS, slight, s>>>(off, dst, f, g->d_pre, n, nullptr, fc, row, ctr);
+    ACCX_MARK(2);
+    ACCX_MARK(3);
+    ACCX_MARK(4);
+    k_dg_out<256><<<tiles, 256, 0, s>>>(off, tilerow, dst, n, m, bias, f, ent, fc, g->d_pre, cnt);
+  } else if (orient) {
     const uint32_t W = (uint32_t)dkb * 8192u;       // dense ids (bits); bitmap owners have ids below W
     const uint32_t pcap = (uint32_t)skb * 256u;     // owner-prefix counters
     // words + the zero word (padded), owner counters + 32 spares, word ranks

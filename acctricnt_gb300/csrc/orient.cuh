@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
 #define OW_CAP 256u
 #define OW_WORK 2048u
 #define OW_DEG 4096u
+#define OW_MAX_N (1u << 24)  // ids must fit 24 bits of a table word
 // CTA items aim at a 16th of a CTA's share of all probes, within these bounds (a
 // smaller item costs its staging more often, a larger one ends later than the rest)
 #define ITEM_TARGET_MIN 16384u

@@ -188,7 +188,11 @@ typedef struct {
   int sparse_table_kb;    /* hashed bitmap-word table for the other ids, KiB (0 = tuned default) */
   int sm_limit;           /* run the persistent counting kernels on at most this many SMs (0 = all);
                              leaves SMs free for latency-critical work on other streams */
-  int orient;             /* 0: direct -- every owned edge intersects the two full lists.
+  int orient;             /* 0: direct -- every owned edge intersects the two full lists.  (The default
+                             policy, ACCX_POLICY_HEURISTIC, on a graph known to be symmetric --
+                             validated, generated or built from edges -- gets the same counts and the
+                             rule's statistics from triangles on degree-ordered prefixes, or from one
+                             kernel when the graph is small; its time is ACCX_PHASE_MERGE's.)
                              1: oriented -- |N(u) ∩ N(v)| is the number of triangles on (u,v); each
                              triangle a<b<c is found once, from the edge (c,b), by intersecting the
                              prefix lists N(c) ∩ [0,b) and N(b) ∩ [0,b), and credited to its three

@@ -19,7 +19,8 @@
 // resident graph at once (each on its own stream).
 struct accx_query_ctx {
   uint32_t *d_simbits = nullptr;  // ceil(m/32) words
-  int32_t *d_core_count = nullptr;
+  uint32_t *d_corelist = nullptr;             // n: cores with short rows
+  uint2 *d_push = nullptr;                    // slices of the longer core rows
   int32_t *d_label = nullptr;
   int32_t *d_parent = nullptr;
   int32_t *d_hubmin = nullptr;

@@ -33,7 +33,9 @@
 #define Q_PAIRS 5
 #define Q_DIGEST 6
 #define Q_BIG 7
-#define Q_NUM 8
+#define Q_CORELIST 8   // cores with short rows, in the core list
+#define Q_PUSH 9       // slices of the other cores' rows
+#define Q_NUM 10
 
 __device__ __forceinline__ unsigned long long accx_mix64_dev(unsigned long long x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -42,133 +44,242 @@ __device__ __forceinline__ unsigned long long accx_mix64_dev(unsigned long long 
   return x ^ (x >> 31);
 }
 
+// The float nearest to c^2 / (du dv) but for rare last-bit ties (error below 2^-24
+// (1 + 2^-20) relative): the quotient of the products' leading floats, corrected once by
+// the exact remainder of their float pairs.  FP64 and conversions of 64-bit integers run
+// at a small fraction of the FP32 rate here: the keys of 128M entries took 3.27 ms with
+// FP64 division and 1.32 ms through 64-bit integers; now 0.90.  Operands of 2^24 and more
+// (no float holds them exactly) take the 64-bit way.
+__device__ __noinline__ float accx_ratio_wide(uint32_t c, uint32_t du, uint32_t dv) {
+  const unsigned long long a = (unsigned long long)c * c, d = (unsigned long long)du * dv;
+  const float ah = __ull2float_rn(a), dh = __ull2float_rn(d);
+  // |a - ah| < 2^40, exact as a signed difference (mod 2^64: ah may round up to 2^64)
+  const float al = __ll2float_rn((long long)(a - (ah >= 18446744073709551616.0f ? 0ull : (unsigned long long)ah)));
+  const float dl = __ll2float_rn((long long)(d - (dh >= 18446744073709551616.0f ? 0ull : (unsigned long long)dh)));
+  const float q = __fdiv_rn(ah, dh);
+  const float r = __fmaf_rn(-q, dl, __fmaf_rn(-q, dh, ah) + al);
+  return __fadd_rn(q, __fdividef(r, dh));
+}
+__device__ __forceinline__ float accx_ratio(uint32_t c, uint32_t du, uint32_t dv) {
+  if ((c | du | dv) >> 24) return accx_ratio_wide(c, du, dv);
+  const float cf = __uint2float_rn(c), uf = __uint2float_rn(du), vf = __uint2float_rn(dv);
+  const float ah = __fmul_rn(cf, cf), al = __fmaf_rn(cf, cf, -ah), dh = __fmul_rn(uf, vf), dl = __fmaf_rn(uf, vf, -dh);
+  const float i = __fdividef(1.f, dh), q = __fmul_rn(ah, i);
+  const float r = __fmaf_rn(-q, dl, __fmaf_rn(-q, dh, ah) + al);
+  return __fmaf_rn(r, i, q);
+}
+
 // Per-entry similarity key, built once after each count: the float nearest to
 // x^2 = cnn^2 / (du * dv).  A query compares it with the squared threshold M^2
 // of its eps; only keys within 2^-21 (relative) of M^2 -- where float rounding
 // could matter -- take the exact-integer test (simpred.h) with cnn, du, dv read
 // back from the graph.
-template <int TILE>
-__global__ void __launch_bounds__(TILE) k_simkey(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
-                                                 const int32_t *__restrict__ dst, const int32_t *__restrict__ cnt,
-                                                 uint32_t n, uint32_t m, int32_t bias, float *__restrict__ key,
-                                                 uint32_t *__restrict__ src) {
-  __shared__ accx_tile_rows<TILE> sh;
-  uint32_t base = blockIdx.x * (uint32_t)TILE;
-  uint32_t e = base + threadIdx.x;
-  uint32_t u = accx_tile_row<TILE>(off, tilerow, n, m, base, e, &sh);
-  if (e >= m) return;
-  const uint32_t v = (uint32_t)dst[e];
-  const double c = (double)(uint32_t)(cnt[e] - bias + 2);
-  const double du = (double)(off[u + 1] - off[u] + 1), dv = (double)(off[v + 1] - off[v] + 1);
-  key[e] = (float)(c * c / (du * dv));
-  src[e] = u;
+// A thread takes eight consecutive entries: one row search inside their 256-entry tile
+// (tilerow), the neighbours' offsets gathered together.
+__global__ void __launch_bounds__(256) k_simkey(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
+                                                const int32_t *__restrict__ dst, const int32_t *__restrict__ cnt,
+                                                uint32_t m, int32_t bias, float *__restrict__ key,
+                                                uint32_t *__restrict__ src) {
+  const uint32_t nb = m / 8 + (m % 8 ? 1 : 0);
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nb; c += gridDim.x * blockDim.x) {
+    const uint32_t e0 = c * 8, k = min(m - e0, 8u), t = e0 / 256u;
+    uint32_t v[8], n[8], dv[8];
+    if (k == 8) {
+      const int4 a = __ldg(reinterpret_cast<const int4 *>(dst + e0)), b = __ldg(reinterpret_cast<const int4 *>(dst + e0) + 1);
+      const int4 p = __ldg(reinterpret_cast<const int4 *>(cnt + e0)), q = __ldg(reinterpret_cast<const int4 *>(cnt + e0) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      n[0] = p.x; n[1] = p.y; n[2] = p.z; n[3] = p.w; n[4] = q.x; n[5] = q.y; n[6] = q.z; n[7] = q.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        v[i] = (uint32_t)i < k ? (uint32_t)__ldg(dst + e0 + i) : 0u;
+        n[i] = (uint32_t)i < k ? (uint32_t)__ldg(cnt + e0 + i) : 0u;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) dv[i] = __ldg(off + v[i] + 1) - __ldg(off + v[i]) + 1;
+    uint32_t u = accx_row_of(off, __ldg(tilerow + t), __ldg(tilerow + t + 1) + 1, e0);
+    uint32_t re = __ldg(off + u + 1), du = re - __ldg(off + u) + 1;
+    float x[8];
+    uint32_t r[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      while ((uint32_t)i < k && re <= e0 + i) {  // the next non-empty row
+        const uint32_t rb = re;
+        u++;
+        re = __ldg(off + u + 1);
+        du = re - rb + 1;
+      }
+      x[i] = accx_ratio((uint32_t)((int32_t)n[i] - bias + 2), du, dv[i]);
+      r[i] = u;
+    }
+    if (k == 8) {
+      reinterpret_cast<float4 *>(key + e0)[0] = make_float4(x[0], x[1], x[2], x[3]);
+      reinterpret_cast<float4 *>(key + e0)[1] = make_float4(x[4], x[5], x[6], x[7]);
+      reinterpret_cast<uint4 *>(src + e0)[0] = make_uint4(r[0], r[1], r[2], r[3]);
+      reinterpret_cast<uint4 *>(src + e0)[1] = make_uint4(r[4], r[5], r[6], r[7]);
+    } else {
+      for (uint32_t i = 0; i < k; i++) {
+        key[e0 + i] = x[i];
+        src[e0 + i] = r[i];
+      }
+    }
+  }
 }
 
-// Similarity bits from the keys: a streaming pass, one 32-bit word per warp.
-__global__ void k_sim_keys(const float *__restrict__ key, const uint32_t *__restrict__ off,
-                           const uint32_t *__restrict__ src, const int32_t *__restrict__ dst,
-                           const int32_t *__restrict__ cnt, uint32_t n, uint32_t m, int32_t bias, accx_simq q,
-                           float lo, float hi, uint32_t *__restrict__ simbits, unsigned long long *__restrict__ qc) {
-  const uint32_t stride = gridDim.x * blockDim.x;  // a multiple of 32
-  unsigned long long similar = 0;
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < ((m + 31) & ~31u); e += stride) {
-    bool sim = false;
-    if (e < m) {
+// Similarity bits from the keys: a streaming pass, eight entries a thread (two 16-byte
+// loads, one byte of the bit array), and in the same pass the caller's 0/1 bytes when
+// wanted (out, 8-byte aligned).  Bound by HBM: 4 bytes read an entry.  128M entries: 452
+// us with one entry a thread and a ballot, plus 189 for the bytes in a pass of their own; now
+// 125 for both (5.1 TB/s).
+__global__ void __launch_bounds__(256) k_sim_keys(const float *__restrict__ key, const uint32_t *__restrict__ off,
+                                                  const uint32_t *__restrict__ src, const int32_t *__restrict__ dst,
+                                                  const int32_t *__restrict__ cnt, uint32_t m, int32_t bias,
+                                                  accx_simq q, float lo, float hi, uint8_t *__restrict__ simbits,
+                                                  uint8_t *__restrict__ out, unsigned long long *__restrict__ qc) {
+  const uint32_t stride = gridDim.x * blockDim.x;
+  const uint32_t nb = ((m + 31) / 32) * 4;  // bytes of whole words: bits past m are zero
+  uint32_t similar = 0;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nb; c += stride) {
+    const uint32_t e0 = c * 8;
+    uint32_t bits = 0;
+    if (e0 < m) {
+      const uint32_t valid = m - e0 >= 8 ? 0xffu : (1u << (m - e0)) - 1u;
       if (q.mode != 0) {
-        sim = q.mode == 1;
+        bits = q.mode == 1 ? 0xffu : 0u;
       } else {
-        const float k = __ldg(key + e);
-        if (k > hi) sim = true;
-        else if (k >= lo) {
-          // ambiguous band (exact ties x == eps land here): exact test with the
-          // entry's own numbers
-          const uint32_t u = __ldg(src + e);
-          const uint32_t v = (uint32_t)dst[e];
-          sim = accx_similar(q, (uint32_t)(cnt[e] - bias + 2), off[u + 1] - off[u] + 1, off[v + 1] - off[v] + 1);
+        float k[8];
+        if (valid == 0xffu) {
+          const float4 a = __ldg(reinterpret_cast<const float4 *>(key + e0));
+          const float4 b = __ldg(reinterpret_cast<const float4 *>(key + e0) + 1);
+          k[0] = a.x; k[1] = a.y; k[2] = a.z; k[3] = a.w;
+          k[4] = b.x; k[5] = b.y; k[6] = b.z; k[7] = b.w;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++) k[i] = (valid >> i) & 1u ? __ldg(key + e0 + i) : -1.f;
+        }
+        uint32_t band = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          bits |= (k[i] > hi ? 1u : 0u) << i;
+          band |= (k[i] >= lo && k[i] <= hi ? 1u : 0u) << i;
+        }
+        for (band &= valid; band; band &= band - 1) {
+          // ambiguous band (exact ties x == eps land here): exact test with the entry's
+          // own numbers
+          const uint32_t i = __ffs(band) - 1, e = e0 + i, u = __ldg(src + e), v = (uint32_t)dst[e];
+          if (accx_similar(q, (uint32_t)(cnt[e] - bias + 2), off[u + 1] - off[u] + 1, off[v + 1] - off[v] + 1))
+            bits |= 1u << i;
+        }
+      }
+      bits &= valid;
+      if (out) {
+        // four bits to four 0/1 bytes: copies shifted by 7, 14 and 21 put bit i at byte i
+        const uint2 y = make_uint2(((bits & 15u) * 0x00204081u) & 0x01010101u, ((bits >> 4) * 0x00204081u) & 0x01010101u);
+        if (valid == 0xffu) {
+          *reinterpret_cast<uint2 *>(out + e0) = y;
+        } else {
+          for (uint32_t i = 0; e0 + i < m; i++) out[e0 + i] = (uint8_t)((bits >> i) & 1u);
         }
       }
     }
-    const unsigned w = __ballot_sync(ACCX_FULL_MASK, sim);
-    if ((threadIdx.x & 31) == 0) {
-      simbits[e >> 5] = w;
-      similar += __popc(w);
-    }
+    simbits[c] = (uint8_t)bits;
+    similar += __popc(bits);
   }
-  if ((threadIdx.x & 31) == 0 && similar) atomicAdd(&qc[Q_SIMILAR], similar);
+  similar = __reduce_add_sync(ACCX_FULL_MASK, similar);
+  if ((threadIdx.x & 31) == 0 && similar) atomicAdd(&qc[Q_SIMILAR], (unsigned long long)similar);
 }
 
 // Cores from the similarity bits: core_count[u] = popcount of row u's bits.
-// One thread per vertex; rows longer than BIG_ROW are left to k_cores_big (one
-// CTA each).  Also resets labels, union-find roots, hub ranges and writes the
-// core bitmap (n/8 bytes, kept in L2 for the random lookups that follow).
+// One thread per vertex, four words' loads in flight (a warp for each row above 256
+// entries measured slower: hubs' ids lie together); rows above BIG_ROW by a CTA
+// (k_cores_big).  Also resets labels, union-find roots
+// and hub ranges, writes the core bitmap (n/8 bytes, kept in L2 for the random lookups
+// that follow), and lists the cores for k_hub_push: short rows as vertices, longer ones
+// as slices.
 #define BIG_ROW 4096
-__device__ __forceinline__ uint32_t accx_row_popc(const uint32_t *__restrict__ bits, uint32_t b, uint32_t e) {
-  uint32_t c = 0;
-  if (b >= e) return 0;
-  const uint32_t w0 = b >> 5, w1 = (e - 1) >> 5;
-  for (uint32_t w = w0; w <= w1; w++) {
-    uint32_t x = __ldg(bits + w);
-    if (w == w0) x &= 0xffffffffu << (b & 31);
-    if (w == w1 && (e & 31)) x &= 0xffffffffu >> (32 - (e & 31));
-    c += __popc(x);
-  }
-  return c;
+#define PUSH_ROW 256u     // cores with rows up to this are one warp's work
+#define PUSH_SLICE 512u   // entries of a longer core row a warp pushes
+__device__ __forceinline__ uint32_t accx_row_word(const uint32_t *__restrict__ bits, uint32_t w, uint32_t b,
+                                                  uint32_t e) {
+  uint32_t x = __ldg(bits + w);
+  if (w == b >> 5) x &= 0xffffffffu << (b & 31);
+  if (w == (e - 1) >> 5 && (e & 31)) x &= 0xffffffffu >> (32 - (e & 31));
+  return __popc(x);
 }
 
-__global__ void k_cores(const uint32_t *__restrict__ off, uint32_t n, int mu, const uint32_t *__restrict__ simbits,
-                        int32_t *__restrict__ core_count, int32_t *__restrict__ label, int32_t *__restrict__ parent,
-                        int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax, uint32_t *__restrict__ corebits,
-                        uint32_t *__restrict__ big, unsigned long long *__restrict__ qc) {
+__device__ __forceinline__ void accx_push_slices(uint32_t u, uint32_t deg, uint2 *__restrict__ push,
+                                                 unsigned long long *__restrict__ qc) {
+  const uint32_t ns = (deg + PUSH_SLICE - 1) / PUSH_SLICE;
+  const unsigned long long p = atomicAdd(&qc[Q_PUSH], (unsigned long long)ns);
+  for (uint32_t j = 0; j < ns; j++) push[p + j] = make_uint2(u, j);
+}
+
+__global__ void __launch_bounds__(256) k_cores(const uint32_t *__restrict__ off, uint32_t n, int mu,
+                                               const uint32_t *__restrict__ simbits, int32_t *__restrict__ label,
+                                               int32_t *__restrict__ parent, int32_t *__restrict__ hubmin,
+                                               int32_t *__restrict__ hubmax, uint32_t *__restrict__ corebits,
+                                               uint32_t *__restrict__ big, uint32_t *__restrict__ corelist,
+                                               uint2 *__restrict__ push, unsigned long long *__restrict__ qc) {
   const uint32_t stride = gridDim.x * blockDim.x;  // a multiple of 32
+  const int lane = threadIdx.x & 31;
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < ((n + 31) & ~31u); u += stride) {
-    bool core = false;
+    uint32_t b = 0, e = 0, c = 0;
     if (u < n) {
-      const uint32_t b = off[u], e = off[u + 1];
-      if (e - b > BIG_ROW) {
-        const unsigned long long p = atomicAdd(&qc[Q_BIG], 1ull);
-        big[p] = u;  // counted by k_cores_big
-      } else {
-        const uint32_t c = accx_row_popc(simbits, b, e);
-        core_count[u] = (int32_t)c;
-        core = (int)c >= mu;
-        label[u] = core ? ACCX_CORE : ACCX_UNCLASSIFIED;
-      }
+      b = __ldg(off + u);
+      e = __ldg(off + u + 1);
       parent[u] = (int32_t)u;
       hubmin[u] = 0x7fffffff;
       hubmax[u] = -1;
     }
+    const uint32_t deg = e - b;
+    const bool is_big = deg > BIG_ROW;
+    if (deg && !is_big)
+      for (uint32_t w = b >> 5, w1 = (e - 1) >> 5; w <= w1; w += 4) {
+        uint32_t t[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) t[i] = w + i <= w1 ? accx_row_word(simbits, w + i, b, e) : 0u;
+        c += t[0] + t[1] + t[2] + t[3];
+      }
+    const bool core = u < n && !is_big && (int)c >= mu;
+    if (is_big) big[atomicAdd(&qc[Q_BIG], 1ull)] = u;  // decided by k_cores_big
+    else if (u < n) label[u] = core ? ACCX_CORE : ACCX_UNCLASSIFIED;
     const unsigned w = __ballot_sync(ACCX_FULL_MASK, core);
-    if ((threadIdx.x & 31) == 0 && u < n) corebits[u >> 5] = w;
+    if (lane == 0 && u < n) corebits[u >> 5] = w;
+    const bool brief = core && deg <= PUSH_ROW;
+    const unsigned bw = __ballot_sync(ACCX_FULL_MASK, brief);
+    if (bw) {
+      unsigned long long p = 0;
+      if (lane == 0) p = atomicAdd(&qc[Q_CORELIST], (unsigned long long)__popc(bw));
+      p = __shfl_sync(ACCX_FULL_MASK, p, 0);
+      if (brief) corelist[p + __popc(bw & ((1u << lane) - 1u))] = u;
+    }
+    if (core && !brief) accx_push_slices(u, deg, push, qc);
   }
 }
 
 __global__ void __launch_bounds__(256) k_cores_big(const uint32_t *__restrict__ off, int mu,
                                                    const uint32_t *__restrict__ simbits, const uint32_t *__restrict__ big,
-                                                   const unsigned long long *__restrict__ qc,
-                                                   int32_t *__restrict__ core_count, int32_t *__restrict__ label,
-                                                   uint32_t *__restrict__ corebits) {
+                                                   int32_t *__restrict__ label, uint32_t *__restrict__ corebits,
+                                                   uint2 *__restrict__ push, unsigned long long *__restrict__ qc) {
   __shared__ uint32_t part[8];
   const unsigned long long nb = qc[Q_BIG];
   for (unsigned long long i = blockIdx.x; i < nb; i += gridDim.x) {
     const uint32_t u = big[i], b = off[u], e = off[u + 1];
     uint32_t c = 0;
-    const uint32_t w0 = b >> 5, w1 = (e - 1) >> 5;
-    for (uint32_t w = w0 + threadIdx.x; w <= w1; w += blockDim.x) {
-      uint32_t x = __ldg(simbits + w);
-      if (w == w0) x &= 0xffffffffu << (b & 31);
-      if (w == w1 && (e & 31)) x &= 0xffffffffu >> (32 - (e & 31));
-      c += __popc(x);
-    }
+    for (uint32_t w = (b >> 5) + threadIdx.x; w <= (e - 1) >> 5; w += blockDim.x) c += accx_row_word(simbits, w, b, e);
     c = __reduce_add_sync(ACCX_FULL_MASK, c);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
       uint32_t t = 0;
       for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += part[k];
-      core_count[u] = (int32_t)t;
       const bool core = (int)t >= mu;
       label[u] = core ? ACCX_CORE : ACCX_UNCLASSIFIED;
-      if (core) atomicOr(&corebits[u >> 5], 1u << (u & 31));
+      if (core) {
+        atomicOr(&corebits[u >> 5], 1u << (u & 31));
+        accx_push_slices(u, e - b, push, qc);
+      }
     }
     __syncthreads();
   }
@@ -192,30 +303,53 @@ __device__ __forceinline__ int32_t uf_find(volatile int32_t *parent, int32_t x) 
   return cur;
 }
 
-// Union over similar core-core entries: one thread per similarity word, only
-// set bits do work.  UnionThreadSafe (union_find.h:22-35): hook the larger root
-// under the smaller.
-__global__ void k_hook_words(const uint32_t *__restrict__ src, const int32_t *__restrict__ dst, uint32_t m,
-                             const uint32_t *__restrict__ simbits,
-                             const uint32_t *__restrict__ corebits, int32_t *parent) {
+// Union over similar core-core entries.  A warp takes 32 similarity words, gathers the
+// entries of their set bits in shared memory and then gives every lane one entry: an
+// entry is a chain of dependent random reads, so a thread working off a word's bits alone
+// left most of the machine waiting (R-MAT 22: 96 us; R-MAT 16: 61).  UnionThreadSafe
+// (union_find.h:22-35): hook the larger root under the smaller.
+// FIRST: a first pass that only lowers each core's parent to its smallest similar core
+// neighbour (one atomic minimum an entry, nothing to wait for or to retry).  It loses
+// links, but the second pass unites over every entry again and finds nearly all of them
+// done, where without it the cores of one big cluster fight over the same roots (both
+// passes: R-MAT 22 55 us, R-MAT 16 27; the second alone 112 and 73).
+#define HOOK_WARPS 4
+template <bool FIRST>
+__global__ void __launch_bounds__(HOOK_WARPS * 32) k_hook_words(const uint32_t *__restrict__ src,
+                                                                const int32_t *__restrict__ dst, uint32_t m,
+                                                                const uint32_t *__restrict__ simbits,
+                                                                const uint32_t *__restrict__ corebits,
+                                                                int32_t *parent) {
+  __shared__ uint32_t s_q[HOOK_WARPS][1024];
   volatile int32_t *vp = parent;
-  const uint32_t words = (m + 31) / 32;
-  for (uint32_t wi = blockIdx.x * blockDim.x + threadIdx.x; wi < words; wi += gridDim.x * blockDim.x) {
-    uint32_t w = __ldg(simbits + wi);
-    while (w) {
-      const uint32_t e = wi * 32u + (uint32_t)(__ffs(w) - 1);
-      w &= w - 1;
-      const uint32_t v = (uint32_t)dst[e];
-      if (!accx_is_core(corebits, v)) continue;
-      const uint32_t u = __ldg(src + e);
-      if (u >= v || !accx_is_core(corebits, u)) continue;
-      for (;;) {
+  const int lane = threadIdx.x & 31;
+  uint32_t *q = s_q[threadIdx.x >> 5];
+  const uint32_t words = (m + 31) / 32, nw = gridDim.x * HOOK_WARPS;
+  for (unsigned long long w0 = 32ull * (blockIdx.x * HOOK_WARPS + (threadIdx.x >> 5)); w0 < words; w0 += 32ull * nw) {
+    const uint32_t wi = (uint32_t)w0 + lane;
+    uint32_t w = wi < words ? __ldg(simbits + wi) : 0u;
+    uint32_t at = __popc(w);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t a = __shfl_up_sync(ACCX_FULL_MASK, at, d);
+      if (lane >= d) at += a;
+    }
+    const uint32_t total = __shfl_sync(ACCX_FULL_MASK, at, 31);
+    at -= __popc(w);
+    for (; w; w &= w - 1) q[at++] = wi * 32u + (uint32_t)(__ffs(w) - 1);
+    __syncwarp();
+    for (uint32_t i = lane; i < total; i += 32) {
+      const uint32_t e = q[i], u = __ldg(src + e), v = (uint32_t)__ldg(dst + e);
+      if (u >= v || !accx_is_core(corebits, v) || !accx_is_core(corebits, u)) continue;
+      if (FIRST) atomicMin(&parent[v], (int32_t)u);
+      while (!FIRST) {
         int32_t ru = uf_find(vp, (int32_t)u), rv = uf_find(vp, (int32_t)v);
         if (ru == rv) break;
         int32_t lo = ru < rv ? ru : rv, hi = ru < rv ? rv : ru;
         if (atomicCAS(&parent[hi], hi, lo) == hi) break;
       }
     }
+    __syncwarp();
   }
 }
 
@@ -227,57 +361,50 @@ __global__ void k_compress(uint32_t n, const uint32_t *__restrict__ corebits, in
   }
 }
 
-// Hubs, pushed from the core side: a warp per core vertex v streams N(v) and
-// folds v's cluster root into the [min, max] range of every non-core neighbour
-// (CheckHub ignores similarity: any core neighbour counts).
-__global__ void k_hub_push(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst, uint32_t n,
-                           const uint32_t *__restrict__ corebits, const int32_t *__restrict__ parent,
-                           int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t words = (n + 31) / 32;
-  for (uint32_t wi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; wi < words; wi += nw) {
-    uint32_t cw = __ldg(corebits + wi);
-    while (cw) {
-      const uint32_t v = wi * 32u + (uint32_t)(__ffs(cw) - 1);
-      cw &= cw - 1;
-      const uint32_t b = off[v], e = off[v + 1];
-      if (e - b > BIG_ROW) continue;  // k_hub_push_big spreads long rows over many CTAs
-      const int32_t r = parent[v];
-      for (uint32_t j = b + lane; j < e; j += 32) {
-        const uint32_t u = (uint32_t)dst[j];
-        if (accx_is_core(corebits, u)) continue;
-        atomicMin(&hubmin[u], r);
-        atomicMax(&hubmax[u], r);
-      }
+// Hubs, pushed from the core side: core vertex v streams N(v) and folds its cluster root
+// into the [min, max] range of every non-core neighbour (CheckHub ignores similarity: any
+// core neighbour counts).  A warp per listed core with a short row, or per slice of a
+// longer row: walking the core bitmap instead, one warp had all the cores of a word,
+// whose rows can be hubs' (R-MAT 13: 86 us, now 8; R-MAT 22, with a grid of CTAs for the
+// longest rows: 97, now 70).
+__device__ __forceinline__ void accx_hub_range(const int32_t *__restrict__ dst, uint32_t b, uint32_t e, int32_t r,
+                                               int lane, const uint32_t *__restrict__ corebits,
+                                               int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax) {
+  for (uint32_t j0 = b; j0 < e; j0 += 128) {
+    uint32_t u[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) u[k] = j0 + 32 * k + lane < e ? (uint32_t)__ldg(dst + j0 + 32 * k + lane) : 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (u[k] == 0xffffffffu || accx_is_core(corebits, u[k])) continue;
+      atomicMin(&hubmin[u[k]], r);
+      atomicMax(&hubmax[u[k]], r);
     }
   }
 }
-
-// The long core rows (the big list of k_cores): blockIdx.y walks the list,
-// blockIdx.x and the threads split each row.
-__global__ void k_hub_push_big(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst,
-                               const uint32_t *__restrict__ big, const unsigned long long *__restrict__ qc,
-                               const uint32_t *__restrict__ corebits, const int32_t *__restrict__ parent,
-                               int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax) {
-  const unsigned long long nb = qc[Q_BIG];
-  for (unsigned long long i = blockIdx.y; i < nb; i += gridDim.y) {
-    const uint32_t v = big[i];
-    if (!accx_is_core(corebits, v)) continue;
-    const int32_t r = parent[v];
-    const uint32_t b = off[v], e = off[v + 1];
-    for (uint32_t j = b + blockIdx.x * blockDim.x + threadIdx.x; j < e; j += gridDim.x * blockDim.x) {
-      const uint32_t u = (uint32_t)dst[j];
-      if (accx_is_core(corebits, u)) continue;
-      atomicMin(&hubmin[u], r);
-      atomicMax(&hubmax[u], r);
-    }
+__global__ void __launch_bounds__(256) k_hub_push(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst,
+                                                  const uint32_t *__restrict__ corelist, const uint2 *__restrict__ push,
+                                                  const unsigned long long *__restrict__ qc,
+                                                  const uint32_t *__restrict__ corebits,
+                                                  const int32_t *__restrict__ parent, int32_t *__restrict__ hubmin,
+                                                  int32_t *__restrict__ hubmax) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long nw = (gridDim.x * blockDim.x) >> 5, w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long np = qc[Q_PUSH], nc = qc[Q_CORELIST];
+  for (unsigned long long i = w0; i < np; i += nw) {
+    const uint2 it = __ldg(push + i);
+    const uint32_t b = __ldg(off + it.x) + it.y * PUSH_SLICE, e = min(b + PUSH_SLICE, __ldg(off + it.x + 1));
+    accx_hub_range(dst, b, e, parent[it.x], lane, corebits, hubmin, hubmax);
+  }
+  for (unsigned long long i = w0; i < nc; i += nw) {
+    const uint32_t v = __ldg(corelist + i);
+    accx_hub_range(dst, __ldg(off + v), __ldg(off + v + 1), parent[v], lane, corebits, hubmin, hubmax);
   }
 }
 
 __global__ void k_finish(uint32_t n, int32_t *__restrict__ label, const int32_t *__restrict__ parent,
-                         const int32_t *__restrict__ hubmin, const int32_t *__restrict__ hubmax,
-                         int32_t *__restrict__ cluster_out, unsigned long long *__restrict__ qc) {
+                         const int32_t *hubmin, const int32_t *__restrict__ hubmax,
+                         int32_t *cluster_out, unsigned long long *__restrict__ qc) {  // cluster_out may be hubmin
   unsigned long long cores = 0, clusters = 0, hubs = 0, outl = 0, dig = 0;
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
     int32_t l = label[u];
@@ -347,8 +474,8 @@ __global__ void __launch_bounds__(TILE) k_pairs(const uint32_t *__restrict__ off
 }
 
 void accx_query_ctx_release(accx_query_ctx *q) {
-  void *ptrs[] = {q->d_simbits, q->d_core_count, q->d_label,     q->d_parent, q->d_hubmin,
-                  q->d_hubmax,  q->d_qcounters,  q->d_pairs,     q->d_pairs_tmp, q->d_corebits, q->d_big};
+  void *ptrs[] = {q->d_simbits, q->d_corelist,  q->d_label, q->d_parent,    q->d_hubmin,   q->d_hubmax,
+                  q->d_push,    q->d_qcounters, q->d_pairs, q->d_pairs_tmp, q->d_corebits, q->d_big};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   *q = accx_query_ctx();
@@ -360,7 +487,9 @@ static int ensure_query_arrays(const accx_graph *g, accx_query_ctx *q) {
   q->m = g->m;
   const size_t n = g->n ? g->n : 1, words = (g->m + 31) / 32 + 1;
   if (!q->d_simbits) ACCX_CUDA_TRY(cudaMalloc(&q->d_simbits, sizeof(uint32_t) * words));
-  if (!q->d_core_count) ACCX_CUDA_TRY(cudaMalloc(&q->d_core_count, sizeof(int32_t) * n));
+  if (!q->d_corelist) ACCX_CUDA_TRY(cudaMalloc(&q->d_corelist, sizeof(uint32_t) * n));
+  // rows above PUSH_ROW have at most 1 + degree/PUSH_SLICE slices
+  if (!q->d_push) ACCX_CUDA_TRY(cudaMalloc(&q->d_push, sizeof(uint2) * (g->m / PUSH_ROW + g->m / PUSH_SLICE + 2)));
   if (!q->d_label) ACCX_CUDA_TRY(cudaMalloc(&q->d_label, sizeof(int32_t) * n));
   if (!q->d_parent) ACCX_CUDA_TRY(cudaMalloc(&q->d_parent, sizeof(int32_t) * n));
   if (!q->d_hubmin) ACCX_CUDA_TRY(cudaMalloc(&q->d_hubmin, sizeof(int32_t) * n));
@@ -383,7 +512,6 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
   const accx_simq sq = accx_simq_make(eps);
   const int sms = accx_sm_count(g->device);
   ACCX_CUDA_TRY(cudaMemsetAsync(q->d_qcounters, 0, sizeof(unsigned long long) * Q_NUM, s));
-  const uint32_t tiles = (m + 255) / 256;
   if (m && !g->key_valid.load(std::memory_order_acquire)) {
     // once per count; several threads may query one const handle, so the key
     // array is built under a lock
@@ -396,8 +524,8 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
         ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_src, sizeof(uint32_t) * (size_t)m, g->home));
         if (g->home) ACCX_CUDA_TRY(cudaStreamSynchronize(g->home));
       }
-      k_simkey<256><<<tiles, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->d_cnt, n, m, g->cnt_bias, gm->d_simkey,
-                                          gm->d_src);
+      k_simkey<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->d_cnt, m, g->cnt_bias, gm->d_simkey,
+                                       gm->d_src);
       ACCX_CUDA_TRY(cudaStreamSynchronize(s));
       gm->key_valid.store(true, std::memory_order_release);
     }
@@ -405,53 +533,58 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
   // threshold band on the keys: exact outside, simpred.h inside
   const float klo = sq.mode == 0 ? (float)sq.m2_lo * (1.0f - 4e-7f) : 0.f;
   const float khi = sq.mode == 0 ? (float)sq.m2_hi * (1.0f + 4e-7f) : 0.f;
-  if (m) k_sim_keys<<<sms * 8, 256, 0, s>>>(g->d_simkey, g->d_off, g->d_src, g->d_dst, g->d_cnt, n, m, g->cnt_bias,
-                                            sq, klo, khi, q->d_simbits, q->d_qcounters);
-  if (n) {
-    k_cores<<<sms * 8, 256, 0, s>>>(g->d_off, n, mu, q->d_simbits, q->d_core_count, q->d_label, q->d_parent,
-                                    q->d_hubmin, q->d_hubmax, q->d_corebits, q->d_big, q->d_qcounters);
-    k_cores_big<<<sms * 2, 256, 0, s>>>(g->d_off, mu, q->d_simbits, q->d_big, q->d_qcounters, q->d_core_count,
-                                        q->d_label, q->d_corebits);
+  // the caller's similarity bytes come from the same pass: into device memory that allows
+  // 8-byte stores, or into a buffer that is then copied to the host
+  const bool sim_dev = sim && m && accx_is_device_ptr(sim);
+  uint8_t *sim_tmp = nullptr, *sim_out = sim_dev && !((uintptr_t)sim & 7) ? sim : nullptr;
+  if (sim && m && !sim_dev) {
+    ACCX_CUDA_TRY(accx_dev_alloc((void **)&sim_tmp, m, s));
+    sim_out = sim_tmp;
   }
-  if (m) k_hook_words<<<sms * 8, 256, 0, s>>>(g->d_src, g->d_dst, m, q->d_simbits, q->d_corebits, q->d_parent);
+  if (m) k_sim_keys<<<sms * 8, 256, 0, s>>>(g->d_simkey, g->d_off, g->d_src, g->d_dst, g->d_cnt, m, g->cnt_bias, sq, klo,
+                                            khi, reinterpret_cast<uint8_t *>(q->d_simbits), sim_out, q->d_qcounters);
+  if (n) {
+    k_cores<<<sms * 8, 256, 0, s>>>(g->d_off, n, mu, q->d_simbits, q->d_label, q->d_parent, q->d_hubmin, q->d_hubmax,
+                                    q->d_corebits, q->d_big, q->d_corelist, q->d_push, q->d_qcounters);
+    if (m > BIG_ROW)
+      k_cores_big<<<sms * 2, 256, 0, s>>>(g->d_off, mu, q->d_simbits, q->d_big, q->d_label, q->d_corebits, q->d_push,
+                                          q->d_qcounters);
+  }
+  if (m) {
+    k_hook_words<true><<<sms * 12, HOOK_WARPS * 32, 0, s>>>(g->d_src, g->d_dst, m, q->d_simbits, q->d_corebits,
+                                                           q->d_parent);
+    k_hook_words<false><<<sms * 12, HOOK_WARPS * 32, 0, s>>>(g->d_src, g->d_dst, m, q->d_simbits, q->d_corebits,
+                                                            q->d_parent);
+  }
   if (n) k_compress<<<sms * 4, 256, 0, s>>>(n, q->d_corebits, q->d_parent);
-  if (n) {
-    k_hub_push<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_dst, n, q->d_corebits, q->d_parent, q->d_hubmin, q->d_hubmax);
-    k_hub_push_big<<<dim3(16, 64), 256, 0, s>>>(g->d_off, g->d_dst, q->d_big, q->d_qcounters, q->d_corebits,
-                                                 q->d_parent, q->d_hubmin, q->d_hubmax);
-  }
+  if (n) k_hub_push<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_dst, q->d_corelist, q->d_push, q->d_qcounters, q->d_corebits,
+                                            q->d_parent, q->d_hubmin, q->d_hubmax);
   bool cl_dev = cluster && accx_is_device_ptr(cluster);
-  int32_t *cl_target = cl_dev ? cluster : nullptr;
+  // host clusters: through the hub minima's array, which nothing reads after this
+  int32_t *cl_target = cl_dev ? cluster : cluster ? q->d_hubmin : nullptr;
   if (n) k_finish<<<sms * 4, 256, 0, s>>>(n, q->d_label, q->d_parent, q->d_hubmin, q->d_hubmax, cl_target, q->d_qcounters);
   ACCX_CUDA_TRY(cudaGetLastError());
   q->query_valid = true;
   q->pairs_valid = false;
   q->last_eps = eps;
   q->last_mu = mu;
-  if (sim && m) {
-    if (accx_is_device_ptr(sim)) {
-      k_bits_to_bytes<<<sms * 8, 256, 0, s>>>(q->d_simbits, m, sim);
-      ACCX_CUDA_TRY(cudaGetLastError());
-    } else {
-      uint8_t *tmp = nullptr;
-      ACCX_CUDA_TRY(cudaMalloc(&tmp, m));
-      k_bits_to_bytes<<<sms * 8, 256, 0, s>>>(q->d_simbits, m, tmp);
-      cudaError_t e1 = cudaMemcpyAsync(sim, tmp, m, cudaMemcpyDeviceToHost, s);
-      cudaError_t e2 = cudaStreamSynchronize(s);
-      cudaFree(tmp);
-      if (e1 != cudaSuccess || e2 != cudaSuccess) return ACCX_ERR_CUDA;
-    }
+  if (sim_dev && !sim_out) {
+    k_bits_to_bytes<<<sms * 8, 256, 0, s>>>(q->d_simbits, m, sim);
+    ACCX_CUDA_TRY(cudaGetLastError());
+  }
+  if (sim_tmp) {
+    cudaError_t e1 = cudaMemcpyAsync(sim, sim_tmp, m, cudaMemcpyDeviceToHost, s);
+    cudaError_t e2 = cudaStreamSynchronize(s);
+    accx_dev_free(sim_tmp, s);
+    if (e1 != cudaSuccess || e2 != cudaSuccess) return ACCX_ERR_CUDA;
   }
   if (label) {
     rc = accx_copy_out(label, q->d_label, sizeof(int32_t) * n, s);
     if (rc) return rc;
   }
   if (cluster && !cl_dev && n) {
-    std::vector<int32_t> lab(n), par(n);
-    rc = accx_copy_out(lab.data(), q->d_label, sizeof(int32_t) * n, s);
-    if (!rc) rc = accx_copy_out(par.data(), q->d_parent, sizeof(int32_t) * n, s);
+    rc = accx_copy_out(cluster, q->d_hubmin, sizeof(int32_t) * n, s);
     if (rc) return rc;
-    for (uint32_t u = 0; u < n; u++) cluster[u] = lab[u] == ACCX_CORE ? par[u] : -1;
   }
   unsigned long long h[Q_NUM];
   ACCX_CUDA_TRY(cudaMemcpyAsync(h, q->d_qcounters, sizeof(h), cudaMemcpyDeviceToHost, s));

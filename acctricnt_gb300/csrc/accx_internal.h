@@ -83,12 +83,14 @@ struct accx_graph {
   uint32_t *d_dg = nullptr;                // the default policy's degree-ordered count
   // dense rows of the relabeled CSR (planned by the relabel; 0 rows: none worth it)
   uint32_t dense_k = 0, dense_m = 0;       // hub ids (bits a row) and rows
-  uint32_t dense_maxpre = 0;               // the longest prefix of those rows
+  uint32_t plan_rows = 0, plan_maxpre = 0; // rows the relabel's plan looked at, and their longest prefix
+  uint32_t dense_built = 0;                // rows the arrays below were built for
   uint32_t *d_dense_t = nullptr;           // dense_m x dense_k bits
   uint32_t *d_dense_low = nullptr;         // dense_m: set bits of each row
   uint4 *d_dense_items = nullptr;          // (row, first entry, entries) pieces of the rows
   bool symmetric = false;                  // known symmetric: validated, generated or built from an edge list
   const uint32_t *rev_csr = nullptr;       // the offsets array d_rev was built for
+  const uint32_t *pre_csr = nullptr;       // ... and d_pre with d_vinfo
   void *d_scan_tmp = nullptr;
   size_t scan_tmp_bytes = 0;
   unsigned long long *d_counters = nullptr;  // [0] merge, [1] gallop, [2] bitmap items, [3..5] work per kind
@@ -158,9 +160,10 @@ int accx_rev_by_sort(accx_graph *g, const uint32_t *off, const uint32_t *tilerow
                      cudaStream_t s, uint32_t **rev_out);
 
 // Relabeled counts -> the handle's entry order (relabel.cu).
-int accx_relabel_gather(accx_graph *g, int32_t *host, cudaStream_t s);
-// The device address of pinned (mapped) host memory, or nullptr (graph.cu).
-void *accx_mapped_host(const void *p);
+int accx_relabel_gather(accx_graph *g, int32_t *out, cudaStream_t s);
+// The address at which kernels on `device` can write p: mapped host memory or memory of
+// that device (*on_device), else nullptr (graph.cu).
+void *accx_writable(const void *p, int device, bool *on_device);
 
 int accx_build_csr_from_keys(accx_graph *g, unsigned long long *d_keys, uint64_t nkeys, uint32_t n,
                              cudaStream_t s);

@@ -39,7 +39,7 @@
 #define C_PROBED 15 // partner ids of the oriented bitmap kind's edges (probed, or covered by dense rows)
 #define C_HEAVY 16  // work items of the oriented bitmap kernel
 #define C_LIGHT 17  // owners of the warp-per-owner kernel
-#define C_DENSE 18  // work items of the dense rows
+#define C_TICKET 18 // rows taken from the degree-ordered count's list
 #define C_DGBIG 19  // long rows of the default policy's degree-ordered count
 #define C_NUM 20
 
@@ -799,10 +799,14 @@ static int g_or_block_warps = 8;
 // Dense rows' scratch: item size, item capacity and the arrays (all or none).
 static uint32_t dense_chunk(const accx_graph *g) { return g->m < (1ull << 25) ? 256u : 512u; }
 static uint32_t dense_cap(const accx_graph *g) { return g->dense_m + (uint32_t)(g->m / dense_chunk(g)) + 1u; }
+// the item counter lies behind the rows' lengths, 8-byte aligned
+static unsigned long long *dense_ctr(const accx_graph *g) {
+  return reinterpret_cast<unsigned long long *>(g->d_dense_low + ((g->dense_m + 1u) & ~1u));
+}
 static bool alloc_dense(accx_graph *g) {
   const size_t tb = (size_t)g->dense_m * (g->dense_k / 8u);
   bool ok = accx_dev_alloc((void **)&g->d_dense_t, tb, g->home) == cudaSuccess &&
-            accx_dev_alloc((void **)&g->d_dense_low, sizeof(uint32_t) * (size_t)g->dense_m, g->home) == cudaSuccess &&
+            accx_dev_alloc((void **)&g->d_dense_low, sizeof(uint32_t) * ((size_t)g->dense_m + 4), g->home) == cudaSuccess &&
             accx_dev_alloc((void **)&g->d_dense_items, sizeof(uint4) * (size_t)dense_cap(g), g->home) == cudaSuccess;
   if (ok && g->home) ok = cudaStreamSynchronize(g->home) == cudaSuccess;
   if (!ok) {
@@ -815,11 +819,11 @@ static bool alloc_dense(accx_graph *g) {
   return ok;
 }
 
-// Scratch of the degree-ordered count: entries and counters of the F lists (m each), two
-// lists of rows (n each), and the CTAs' items: at most a slice for each row of more than
+// Scratch of the degree-ordered count: entries and counters of the F lists (m each), the
+// F lengths and two lists of rows (n each), and the CTAs' items: at most a slice for each row of more than
 // DG_ROW_SMALL entries and one more per DG_SLICE entries.
 static bool alloc_degree(accx_graph *g) {
-  const size_t words = 2 * (size_t)g->m + 2 * (size_t)g->n + 2 + 2 * ((size_t)g->m / DG_ROW_SMALL + (size_t)g->m / DG_SLICE + 2);
+  const size_t words = 2 * (size_t)g->m + 3 * (size_t)g->n + 2 + 2 * ((size_t)g->m / DG_ROW_SMALL + (size_t)g->m / DG_SLICE + 2);
   bool ok = accx_dev_alloc((void **)&g->d_dg, sizeof(uint32_t) * words, g->home) == cudaSuccess;
   if (ok && g->home) ok = cudaStreamSynchronize(g->home) == cudaSuccess;
   if (!ok) cudaGetLastError();
@@ -834,10 +838,11 @@ static unsigned classify_grid(int sms, uint32_t m) {
   return (unsigned)(blocks < g ? (blocks ? blocks : 1) : g);
 }
 
-// host_out (optional): the caller's output as a device-mapped pointer; a count
-// on the relabeled CSR then writes it in its final gather (*host_done = true).
-static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s, int32_t *host_out = nullptr,
-                        bool *host_done = nullptr) {
+// copy (optional): the caller's output as a pointer this device can write: its own
+// memory (on_device) or mapped host memory.  Counts on the relabeled CSR write it in their
+// final gather, small ones with the counts if it is device memory (*copied = true).
+static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s, int32_t *copy = nullptr,
+                        bool on_device = false, bool *copied = nullptr) {
   const uint32_t n = g->n, m = (uint32_t)g->m;
   int policy = o ? o->policy : ACCX_POLICY_HEURISTIC;
   int32_t bias = o ? o->bias : 0;
@@ -849,6 +854,16 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   if (o && (o->orient < 0 || o->orient > 1)) return ACCX_ERR_INVALID_ARG;
   if (warps < 1 || warps > 32 || dkb < 1 || skb < 1) return ACCX_ERR_INVALID_ARG;
   if (orient ? (dkb + dkb / 2 + skb > 196 || skb > 200) : (dkb + skb > 200)) return ACCX_ERR_INVALID_ARG;
+  // shapes past a block's 227 KB are refused for every policy, whether or not this count
+  // launches a bitmap kernel: windows and tables plus the per-round arrays (direct 29664
+  // bytes; oriented 32 a thread of the instance and 416)
+  const uint32_t inst = warps <= 8 ? 256u : warps <= 16 ? 512u : 1024u;
+  const size_t need = orient ? (size_t)dkb * 1536u + (size_t)skb * 1024u + 144u + 32u * inst + 416u
+                             : ((size_t)dkb + skb) * 1024u + 29664u;
+  if (n && g->m && need > 227u * 1024u) {
+    accx_set_cuda_error(cudaErrorInvalidValue, "shared memory of the bitmap kernel", __FILE__, __LINE__);
+    return ACCX_ERR_CUDA;
+  }
   if (n == 0) {
     g->cnt_bias = bias;
     g->cnt_valid = true;
@@ -883,7 +898,14 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   bool degree = !orient && policy == ACCX_POLICY_HEURISTIC && g->symmetric && n <= OW_MAX_N && m;
   const bool small = degree && m <= DG_SMALL_M;
   if (degree && !small && !g->d_dg && !alloc_degree(g)) degree = false;
-  ACCX_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * (C_NUM + (degree ? 0 : (size_t)n + 1)), s));
+  // which kinds can occur; oriented bitmap owners lie below the dense window, so only
+  // their part of work_u is used
+  const bool any = policy == ACCX_POLICY_TABLE || policy == ACCX_POLICY_MODEL;
+  const bool can_merge = any || policy == ACCX_POLICY_HEURISTIC || policy == ACCX_POLICY_MERGE;
+  const bool can_bitmap = any || policy == ACCX_POLICY_BITMAP;
+  const uint32_t window = (uint32_t)dkb * 8192u;
+  const size_t works = degree ? 0 : !orient ? (size_t)n + 1 : !can_bitmap ? 0 : n < window ? n : window;
+  ACCX_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * (C_NUM + works), s));
   if (!orient && !degree) ACCX_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(m ? m : 1), s));
   if (m == 0) {
     g->cnt_bias = bias;
@@ -902,8 +924,11 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   int sms = accx_sm_count(g->device);
   if (o && o->sm_limit > 0 && o->sm_limit < sms) sms = o->sm_limit;
   if (small) {
+    int32_t *direct = !rel && on_device ? copy : nullptr;
     ACCX_MARK(1);
-    k_count_small<<<(m + DS_TILE - 1) / DS_TILE, 256, 0, s>>>(off, tilerow, dst, n, m, bias, cnt, ctr);
+    k_count_small<<<(m + DS_TILE - 1) / DS_TILE, 256, 0, s>>>(off, tilerow, dst, n, m, bias, cnt,
+                                                                direct, ctr);
+    if (direct) *copied = true;
     ACCX_MARK(2);
     ACCX_MARK(3);
     ACCX_MARK(4);
@@ -911,24 +936,24 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     // F lists in the owned-edge list's place; entries, counters and row lists in d_dg
     int32_t *f = reinterpret_cast<int32_t *>(g->d_edge_list), *fc = reinterpret_cast<int32_t *>(g->d_dg) + m;
     const uint32_t row = m < DG_ROW_M ? DG_ROW_SMALL : DG_ROW;
-    uint32_t *ent = g->d_dg, *mid = ent + 2 * (size_t)m, *big = mid + n;
-    uint2 *heavy = reinterpret_cast<uint2 *>(g->d_dg + ((2 * (size_t)m + 2 * (size_t)n + 1) & ~(size_t)1));
-    k_dg_rows<<<sms * 8, DG_THREADS, 0, s>>>(off, dst, n, f, ent, fc, g->d_pre, big, mid, row, ctr);
-    k_dg_big<<<sms * 4, DG_THREADS, 0, s>>>(off, dst, f, ent, fc, g->d_pre, big, heavy, ctr);
+    uint32_t *ent = g->d_dg, *mid = ent + 2 * (size_t)m, *big = mid + n, *flen = big + n;
+    uint2 *heavy = reinterpret_cast<uint2 *>(g->d_dg + ((2 * (size_t)m + 3 * (size_t)n + 1) & ~(size_t)1));
+    k_dg_rows<<<sms * 8, DG_THREADS, 0, s>>>(off, dst, n, f, ent, fc, flen, big, mid, row, ctr);
+    k_dg_big<<<sms * 4, DG_THREADS, 0, s>>>(off, dst, f, ent, fc, flen, big, heavy, ctr);
     ACCX_MARK(1);
     const size_t smem = DG_SLOTS * 6u + DG_CAP * 4u;
     const size_t smid = sizeof(dg_warp<DG_WARP>) * DG_WARPS, slight = sizeof(dg_warp<DG_LIGHT>) * DG_WARPS;
     ACCX_CUDA_TRY(cudaFuncSetAttribute(k_dg_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ACCX_CUDA_TRY(cudaFuncSetAttribute(k_dg_warp<DG_WARP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smid));
-    k_dg_cta<<<sms * 6, DG_THREADS, smem, s>>>(off, dst, f, g->d_pre, heavy, fc, ctr);
-    k_dg_warp<DG_WARP><<<sms * 4, DG_THREADS, smid, s>>>(off, dst, f, g->d_pre, n, mid, fc, row, ctr);
-    k_dg_warp<DG_LIGHT><<<sms * 8, DG_THREADS, slight, s>>>(off, dst, f, g->d_pre, n, nullptr, fc, row, ctr);
+    k_dg_cta<<<sms * 6, DG_THREADS, smem, s>>>(off, dst, f, flen, heavy, fc, ctr);
+    k_dg_warp<DG_WARP><<<sms * 4, DG_THREADS, smid, s>>>(off, dst, f, flen, n, mid, fc, row, ctr);
+    k_dg_warp<DG_LIGHT><<<sms * 8, DG_THREADS, slight, s>>>(off, dst, f, flen, n, nullptr, fc, row, ctr);
     ACCX_MARK(2);
     ACCX_MARK(3);
     ACCX_MARK(4);
-    k_dg_out<256><<<tiles, 256, 0, s>>>(off, tilerow, dst, n, m, bias, f, ent, fc, g->d_pre, cnt);
+    k_dg_out<256><<<tiles, 256, 0, s>>>(off, tilerow, dst, n, m, bias, f, ent, fc, flen, cnt);
   } else if (orient) {
-    const uint32_t W = (uint32_t)dkb * 8192u;       // dense ids (bits); bitmap owners have ids below W
+    const uint32_t W = can_bitmap ? window : 0u;    // dense ids (bits); bitmap owners have ids below W
     const uint32_t pcap = (uint32_t)skb * 256u;     // owner-prefix counters
     // words + the zero word (padded), owner counters + 32 spares, word ranks
     const size_t smem = (size_t)W / 8u + 16u + ((size_t)pcap + 32u) * 4u + (size_t)W / 16u;
@@ -943,7 +968,11 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
         ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_or_items, sizeof(uint32_t) * (size_t)items_cap, g->home));
       if (g->home) ACCX_CUDA_TRY(cudaStreamSynchronize(g->home));
     }
-    k_pre<<<sms * 8, 256, 0, s>>>(off, dst, n, g->d_pre, g->d_vinfo);
+    // prefix lengths: an index of the counting CSR, built on its first oriented count
+    if (g->pre_csr != off) {
+      k_pre<<<sms * 8, 256, 0, s>>>(off, dst, n, g->d_pre, g->d_vinfo);
+      g->pre_csr = off;
+    }
     // reverse entries: built on the first oriented count of this CSR and kept
     // (an index of the graph, like the tile rows).  The original CSR's comes
     // from validation; a known-symmetric CSR's from the sort (accx_rev_by_sort);
@@ -975,53 +1004,60 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     }
     // dense rows, where the relabel planned some and bitmap-kind edges can occur
     const uint32_t wpl = g->dense_k / 1024u;
-    uint32_t dm = rel && policy != ACCX_POLICY_HEURISTIC && policy != ACCX_POLICY_MERGE && policy != ACCX_POLICY_GALLOP
-                      ? (g->dense_m < W ? g->dense_m : W) : 0u;
+    uint32_t dm = rel && can_bitmap ? (g->dense_m < W ? g->dense_m : W) : 0u;
     const uint32_t dchunk = dense_chunk(g), dcap = dense_cap(g);
     if (dm && !g->d_dense_t && !alloc_dense(g)) dm = 0;  // no room: every id is probed
-    if (dm) {
+    if (dm && g->dense_built != dm) {  // an index of the relabeled CSR, for this many rows
       auto kr = wpl == 4 ? k_dense_rows<4> : wpl == 2 ? k_dense_rows<2> : k_dense_rows<1>;
+      ACCX_CUDA_TRY(cudaMemsetAsync(dense_ctr(g), 0, sizeof(unsigned long long), s));
       kr<<<sms * 8, 256, 0, s>>>(off, dst, g->d_pre, dm, dchunk, g->d_dense_t, g->d_dense_low, g->d_dense_items, dcap,
-                                 ctr);
+                                 dense_ctr(g));
+      g->dense_built = dm;
     }
     k_classify<true><<<classify_grid(sms, m), 256, 0, s>>>(off, tilerow, dst, n, m, policy, g->d_table, g->d_edge_list,
                                                           list_cap, work_u, ctr, g->d_pre, W, pcap, g->d_or_sl, g->d_rev,
                                                           cnt, bias, g->d_vinfo, dm,
                                                           g->d_dense_low);  // classify also fills cnt with the bias
-    // the instance whose per-round arrays fit the block: 256 threads (four CTAs per
-    // SM with the default 24 KiB window), 512 (two per SM with windows up to ~60
-    // KiB) or 1024
+    // the instance for the block: 256 threads (four CTAs per SM with the default 24 KiB
+    // window), 512 (two per SM with windows up to ~60 KiB) or 1024
     auto kb = warps <= 8 ? k_bitmap_or<256> : warps <= 16 ? k_bitmap_or<512> : k_bitmap_or<1024>;
     ACCX_CUDA_TRY(cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     ACCX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kb, warps * 32, smem));
     if (per_sm < 1) return ACCX_ERR_INVALID_ARG;
     const uint32_t ctas = (uint32_t)(sms * per_sm);
-    k_owner_items<<<OI_CTAS, OI_THREADS, 0, s>>>(off, g->d_pre, n < W ? n : W, work_u, target, ctas, items_cap, g->d_prefix, g->d_or_items,
-                                          ctr);
+    if (can_bitmap)
+      k_owner_items<<<OI_CTAS, OI_THREADS, 0, s>>>(off, g->d_pre, n < W ? n : W, work_u, target, ctas, items_cap,
+                                                   g->d_prefix, g->d_or_items, ctr);
     ACCX_MARK(1);
-    k_merge_or<<<sms * 8, MERGE_WARPS * 32, 0, s>>>(off, dst, g->d_pre, g->d_rev, g->d_edge_list, list_cap, ctr,
-                                                    cnt);
+    if (can_merge)
+      k_merge_or<<<sms * 8, MERGE_WARPS * 32, 0, s>>>(off, dst, g->d_pre, g->d_rev, g->d_edge_list, list_cap, ctr, cnt);
     ACCX_MARK(2);
-    k_gallop_or<GALLOP_OR_GROUP><<<sms * 8, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list, list_cap, ctr,
-                                                     cnt);
+    // an all-bitmap count gallops only where an owner is outside the window or the counters
+    const bool can_gallop = policy != ACCX_POLICY_MERGE &&
+                            !(policy == ACCX_POLICY_BITMAP && rel && n <= W && n <= g->plan_rows && g->plan_maxpre <= pcap);
+    if (can_gallop)
+      k_gallop_or<GALLOP_OR_GROUP><<<sms * 8, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list,
+                                                                        list_cap, ctr, cnt);
     ACCX_MARK(3);
     if (dm) {
-      const bool all = policy == ACCX_POLICY_BITMAP && g->dense_maxpre <= pcap;
+      const bool all = policy == ACCX_POLICY_BITMAP && g->plan_maxpre <= pcap;
       auto kd = wpl == 4 ? (all ? k_dense_pairs<4, true> : k_dense_pairs<4, false>)
               : wpl == 2 ? (all ? k_dense_pairs<2, true> : k_dense_pairs<2, false>)
                          : (all ? k_dense_pairs<1, true> : k_dense_pairs<1, false>);
       const size_t dsmem = (size_t)DENSE_WARPS * 2u * 8u * 32u * wpl * 4u;
       ACCX_CUDA_TRY(cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
       kd<<<sms * 2, DENSE_WARPS * 32, dsmem, s>>>(off, dst, g->d_pre, g->d_dense_low, g->d_dense_t, g->d_dense_items, dcap,
-                                              policy, g->d_table, pcap, cnt, ctr);
+                                                  dense_ctr(g), policy, g->d_table, pcap, cnt, ctr);
     }
-    const size_t ow_smem = sizeof(ow_warp) * OW_WARPS;
-    ACCX_CUDA_TRY(cudaFuncSetAttribute(k_owner_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ow_smem));
-    kb<<<ctas, warps * 32, smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, work_u, g->d_prefix, g->d_or_sl, W,
-                                      pcap, target, cnt, ctr);
-    k_owner_warp<<<sms * 4, OW_WARPS * 32, ow_smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, g->d_or_sl, cnt,
-                                                         ctr);
+    if (can_bitmap) {
+      const size_t ow_smem = sizeof(ow_warp) * OW_WARPS;
+      ACCX_CUDA_TRY(cudaFuncSetAttribute(k_owner_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ow_smem));
+      kb<<<ctas, warps * 32, smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, work_u, g->d_prefix, g->d_or_sl, W,
+                                        pcap, target, cnt, ctr);
+      k_owner_warp<<<sms * 4, OW_WARPS * 32, ow_smem, s>>>(off, dst, g->d_pre, g->d_or_items, items_cap, g->d_or_sl, cnt,
+                                                           ctr);
+    }
     ACCX_MARK(4);
     // suffix entries take their prefix entry's count.  One thread per entry in
     // entry order, so the reads of the prefix entries sweep the array upwards;
@@ -1055,9 +1091,9 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     k_mirror<256><<<tiles, 256, 0, s>>>(off, tilerow, dst, n, m, bias, cnt);
   }
   if (rel) {
-    rc = accx_relabel_gather(g, host_out, s);
+    rc = accx_relabel_gather(g, copy, s);
     if (rc) return rc;
-    if (host_out && host_done) *host_done = true;
+    if (copy && copied) *copied = true;
   }
   ACCX_MARK(5);
 #undef ACCX_MARK
@@ -1074,17 +1110,19 @@ extern "C" int accx_cn_count(accx_graph *g, const accx_count_opts *opts, int32_t
   if (!g) return ACCX_ERR_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   ACCX_CUDA_TRY(cudaSetDevice(g->device));
-  // pinned host output, 16-byte aligned: written by the count's last pass itself
-  int32_t *mapped = out ? static_cast<int32_t *>(accx_mapped_host(out)) : nullptr;
-  if (mapped && ((uintptr_t)mapped & 15)) mapped = nullptr;
+  // pinned host output (16-byte aligned) and output in this device's memory: written by
+  // the count's last pass itself where it can
+  bool on_device = false;
+  int32_t *target = out ? static_cast<int32_t *>(accx_writable(out, g->device, &on_device)) : nullptr;
+  if (target && ((uintptr_t)target & (on_device ? 3 : 15))) target = nullptr;
   bool done = false;
-  int rc = launch_count(g, opts, s, mapped, &done);
+  int rc = launch_count(g, opts, s, target, on_device, &done);
   if (rc) {
     g->cnt_valid = false;
     return rc;
   }
   if (out && done) {
-    ACCX_CUDA_TRY(cudaStreamSynchronize(s));
+    if (!on_device) ACCX_CUDA_TRY(cudaStreamSynchronize(s));
   } else if (out) {
     rc = accx_copy_out(out, g->d_cnt, sizeof(int32_t) * (size_t)g->m, s);
     if (rc) return rc;

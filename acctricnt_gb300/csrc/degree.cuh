@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_warp(const uint32_t *__restri
     const uint32_t total = (uint32_t)ctr[C_LIGHT];
     for (;;) {
       uint32_t it = 0;
-      if (lane == 0) it = (uint32_t)atomicAdd(&ctr[C_DENSE], 1ull);
+      if (lane == 0) it = (uint32_t)atomicAdd(&ctr[C_TICKET], 1ull);
       it = __shfl_sync(ACCX_FULL_MASK, it, 0);
       if (it >= total) break;
       const uint32_t x = __ldg(mid + it);
@@ -438,8 +438,7 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_cta(const uint32_t *__restric
   }
 }
 
-// Every edge's count, from its place in F to both of its entries (and to the caller's
-// device array when there is one).
+// Every edge's count, from its place in F to both of its entries.
 template <int TILE>
 __global__ void __launch_bounds__(TILE) k_dg_out(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
                                                  const int32_t *__restrict__ dst, uint32_t n, uint32_t m, int32_t bias,
@@ -467,7 +466,7 @@ __global__ void __launch_bounds__(TILE) k_dg_out(const uint32_t *__restrict__ of
 __global__ void __launch_bounds__(256) k_count_small(const uint32_t *__restrict__ off,
                                                      const uint32_t *__restrict__ tilerow,
                                                      const int32_t *__restrict__ dst, uint32_t n, uint32_t m,
-                                                     int32_t bias, int32_t *__restrict__ cnt,
+                                                     int32_t bias, int32_t *cnt, int32_t *copy,
                                                      unsigned long long *__restrict__ ctr) {
   __shared__ unsigned long long s_st[9];
   __shared__ uint4 s_own[DS_TILE];
@@ -506,8 +505,12 @@ __global__ void __launch_bounds__(256) k_count_small(const uint32_t *__restrict_
       lo = __shfl_sync(ACCX_FULL_MASK, p, (int)min(o.w - j0 - 1u, 31u));
     }
     c = __reduce_add_sync(ACCX_FULL_MASK, c);
-    if (lane == 0) cnt[s_list[i].y] = (int32_t)c + bias;
-    if (lane == 31 && r < o.w && __ldg(dst + r) == (int32_t)s_list[i].x) cnt[r] = (int32_t)c + bias;
+    // lane 0: the entry, lane 31: its reverse
+    if (lane == 0) r = s_list[i].y;
+    if (lane == 0 || (lane == 31 && r < o.w && __ldg(dst + r) == (int32_t)s_list[i].x)) {
+      cnt[r] = (int32_t)c + bias;
+      if (copy) copy[r] = (int32_t)c + bias;
+    }
   }
   dg_stat_flush(st, s_st, ctr);
 }

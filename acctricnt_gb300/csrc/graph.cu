@@ -131,7 +131,16 @@ static void *mapped_host(const void *p) {
   return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-void *accx_mapped_host(const void *p) { return mapped_host(p); }
+void *accx_writable(const void *p, int device, bool *on_device) {
+  cudaPointerAttributes a;
+  *on_device = false;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  *on_device = a.type == cudaMemoryTypeDevice && a.device == device;
+  return a.type == cudaMemoryTypeHost || *on_device ? a.devicePointer : nullptr;
+}
 
 static cudaError_t copy_via_kernel(void *d, const void *sp, size_t bytes, cudaStream_t s) {
   const size_t n16 = bytes / 16, head = n16 * 16;

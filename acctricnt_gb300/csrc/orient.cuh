@@ -168,8 +168,9 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
 // Together they never exceed n + m/32, as an owner has at most max(1, degree/32)
 // slices.
 //
-// Light: at most OW_CAP prefix ids (the warp's table and counters), OW_WORK probes
-// and OW_DEG entries.  A CTA spends ~4 us of barriers on an item however small it
+// Light: at most OW_CAP prefix ids (the warp's table and counters), OW_DEG entries and
+// OW_WORK probes, but no more than an OW_SHARE'th of all (a small graph's owners are fewer
+// than the machine's warps).  A CTA spends ~4 us of barriers on an item however small it
 // is, a warp well under 1 us; with many probes one warp becomes the tail of a small
 // graph.  Counts (us) by OW_WORK 0 (no light owners) / 512 / 1024 / 2048 / 4096:
 // R-MAT 15 187 / 187 / 183 / 183 / 218, Chung-Lu 3M 5825 / 5144 / 5004 / 4978 / 5058,
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
 // 3M-vertex power-law count.
 #define OW_CAP 256u
 #define OW_WORK 2048u
+#define OW_SHARE 4096u
 #define OW_DEG 4096u
 #define OW_MAX_N (1u << 24)  // ids must fit 24 bits of a table word
 // CTA items aim at a 16th of a CTA's share of all probes, within these bounds (a
@@ -204,26 +206,32 @@ __device__ __forceinline__ uint32_t accx_warp_incl_sum(uint32_t v, int lane) {
   return v;
 }
 
-// an owner's CTA slices (0: none or light)
-__device__ __forceinline__ uint32_t ow_shape(const uint32_t *__restrict__ off, const uint32_t *__restrict__ pre,
-                                             const unsigned long long *__restrict__ work_u, uint32_t u, uint32_t n,
-                                             uint32_t target, bool *light, uint32_t *px) {
-  const unsigned long long w = u < n ? work_u[u] : 0ull;
-  uint32_t ns = 0;
-  *light = false;
-  *px = 0;
-  if (w) {
-    const uint32_t du = off[u + 1] - off[u];
-    *px = pre[u];
-    *light = *px <= OW_CAP && w <= OW_WORK && du <= OW_DEG;
-    uint32_t nc;
-    if (!*light) accx_item_shape(du, 0, w, 1, target, &nc, &ns);
-  }
-  return ns;
-}
-
 #define OI_CTAS 8
 #define OI_THREADS 1024
+#define OI_STEP 4  // vertices a lane takes at once: their loads are in flight together
+// The CTA slices (0: none or light) of the vertices u0 + 32 r, r < OI_STEP, of this lane.
+__device__ __forceinline__ void ow_shape(const uint32_t *__restrict__ off, const uint32_t *__restrict__ pre,
+                                         const unsigned long long *__restrict__ work_u, uint32_t u0, uint32_t e,
+                                         uint32_t target, uint32_t light_max, uint32_t (&ns)[OI_STEP],
+                                         bool (&light)[OI_STEP], uint32_t (&px)[OI_STEP]) {
+  unsigned long long w[OI_STEP];
+  uint32_t du[OI_STEP];
+#pragma unroll
+  for (int r = 0; r < OI_STEP; r++) {
+    const uint32_t u = u0 + 32u * r;
+    w[r] = u < e ? work_u[u] : 0ull;
+    du[r] = u < e ? __ldg(off + u + 1) - __ldg(off + u) : 0u;
+    px[r] = u < e ? __ldg(pre + u) : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < OI_STEP; r++) {
+    light[r] = w[r] && px[r] <= OW_CAP && w[r] <= light_max && du[r] <= OW_DEG;
+    uint32_t nc;
+    ns[r] = 0;
+    if (w[r] && !light[r]) accx_item_shape(du[r], 0, w[r], 1, target, &nc, &ns[r]);
+  }
+}
+
 __global__ void __cluster_dims__(OI_CTAS, 1, 1) __launch_bounds__(OI_THREADS)
     k_owner_items(const uint32_t *__restrict__ off, const uint32_t *__restrict__ pre, uint32_t n,
                   const unsigned long long *__restrict__ work_u, uint32_t target_max, uint32_t ctas, uint32_t cap,
@@ -233,18 +241,23 @@ __global__ void __cluster_dims__(OI_CTAS, 1, 1) __launch_bounds__(OI_THREADS)
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t target = accx_item_target(ctr, target_max, ctas);
+  const unsigned long long share = ctr[C_WORK + ACCX_KIND_BITMAP] / OW_SHARE;
+  const uint32_t light_max = share < OW_WORK ? (uint32_t)share : OW_WORK;
   // a run of `span` vertices (a multiple of 32) per warp of the cluster
   const uint32_t nw = OI_CTAS * OI_THREADS / 32, span = ((n + nw - 1) / nw + 31u) & ~31u;
   const uint32_t b = min(n, (cl.block_rank() * (OI_THREADS / 32) + warp) * span), e = min(n, b + span);
   unsigned long long staged = 0;
   uint32_t h = 0, l = 0;
-  for (uint32_t u0 = b; u0 < e; u0 += 32) {
-    bool light;
-    uint32_t px;
-    const uint32_t ns = ow_shape(off, pre, work_u, u0 + lane, e, target, &light, &px);
-    h += ns;
-    l += light;
-    staged += (unsigned long long)px * (light ? 1u : ns);
+  for (uint32_t u0 = b; u0 < e; u0 += 32 * OI_STEP) {
+    bool light[OI_STEP];
+    uint32_t ns[OI_STEP], px[OI_STEP];
+    ow_shape(off, pre, work_u, u0 + lane, e, target, light_max, ns, light, px);
+#pragma unroll
+    for (int r = 0; r < OI_STEP; r++) {
+      h += ns[r];
+      l += light[r];
+      staged += (unsigned long long)px[r] * (light[r] ? 1u : ns[r]);
+    }
   }
   h = __reduce_add_sync(ACCX_FULL_MASK, h);
   l = __reduce_add_sync(ACCX_FULL_MASK, l);
@@ -278,21 +291,24 @@ __global__ void __cluster_dims__(OI_CTAS, 1, 1) __launch_bounds__(OI_THREADS)
     ctr[C_LIGHT] = l0 + s_tot[1];
   }
   cl.sync();  // the totals are not read after this
-  for (uint32_t u0 = b; u0 < e; u0 += 32) {
-    const uint32_t u = u0 + lane;
-    bool light;
-    uint32_t px;
-    const uint32_t ns = ow_shape(off, pre, work_u, u, e, target, &light, &px);
-    const unsigned lm = __ballot_sync(ACCX_FULL_MASK, light);
-    const uint32_t incl = accx_warp_incl_sum(ns, lane), p = h0 + incl - ns;
-    const uint32_t q = l0 + __popc(lm & ((1u << lane) - 1u));
-    if (light && q < cap) items[cap - 1 - q] = u;
-    if (ns) {
-      slot[u] = p;
-      for (uint32_t j = 0; j < ns && p + j < cap; j++) items[p + j] = u;
+  for (uint32_t u0 = b; u0 < e; u0 += 32 * OI_STEP) {
+    bool light[OI_STEP];
+    uint32_t ns[OI_STEP], px[OI_STEP];
+    ow_shape(off, pre, work_u, u0 + lane, e, target, light_max, ns, light, px);
+#pragma unroll
+    for (int r = 0; r < OI_STEP; r++) {
+      const uint32_t u = u0 + 32u * r + lane;
+      const unsigned lm = __ballot_sync(ACCX_FULL_MASK, light[r]);
+      const uint32_t incl = accx_warp_incl_sum(ns[r], lane), p = h0 + incl - ns[r];
+      const uint32_t q = l0 + __popc(lm & ((1u << lane) - 1u));
+      if (light[r] && q < cap) items[cap - 1 - q] = u;
+      if (ns[r]) {
+        slot[u] = p;
+        for (uint32_t j = 0; j < ns[r] && p + j < cap; j++) items[p + j] = u;
+      }
+      h0 += __shfl_sync(ACCX_FULL_MASK, incl, 31);
+      l0 += __popc(lm);
     }
-    h0 += __shfl_sync(ACCX_FULL_MASK, incl, 31);
-    l0 += __popc(lm);
   }
 }
 
@@ -326,9 +342,18 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
   if (total > cap) total = cap;
   unsigned long long found = 0;
   const unsigned long long nw = (unsigned long long)gridDim.x * OW_WARPS;
-  for (unsigned long long it = (unsigned long long)blockIdx.x * OW_WARPS + (threadIdx.x >> 5); it < total; it += nw) {
-    const uint32_t x = items[cap - 1 - it];
-    const uint32_t ub = off[x], ue = off[x + 1], px = min(pre[x], OW_CAP);
+  unsigned long long it = (unsigned long long)blockIdx.x * OW_WARPS + (threadIdx.x >> 5);
+  // a row is a chain of dependent loads: the next row's bounds, and this row's first ids
+  // and ranges, are loaded ahead of where they are used
+  uint32_t x = it < total ? items[cap - 1 - it] : 0u;
+  uint32_t nb = it < total ? __ldg(off + x) : 0u, ne = it < total ? __ldg(off + x + 1) : 0u;
+  uint32_t np = it < total ? __ldg(pre + x) : 0u;
+  for (; it < total; it += nw) {
+    const uint32_t ub = nb, ue = ne, px = min(np, OW_CAP);
+    const uint32_t id0 = (uint32_t)lane < px ? (uint32_t)__ldg(dst + ub + lane) : 0u;
+    uint2 sn = ub + lane < ue ? __ldg(sl + ub + lane) : make_uint2(0u, 0u);
+    const bool more = it + nw < total;
+    x = more ? items[cap - 1 - (it + nw)] : 0u;
     // the table: 64 to 1024 slots
     int lg = 6;
     while (lg < 10 && (1u << lg) < 4u * px) lg++;
@@ -338,19 +363,18 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
     for (uint32_t i = lane; i < px; i += 32) S.oc[i] = 0;
     __syncwarp();
     for (uint32_t i = lane; i < px; i += 32) {
-      const uint32_t id = (uint32_t)__ldg(dst + ub + i);
+      const uint32_t id = i < 32 ? id0 : (uint32_t)__ldg(dst + ub + i);
       uint32_t h = ow_hash(id, sh);
       while (atomicCAS(&S.tab[h], 0xffffffffu, (id << 8) | i) != 0xffffffffu) h = (h + 1) & mask;
     }
     __syncwarp();
+    nb = more ? __ldg(off + x) : 0u;
+    ne = more ? __ldg(off + x + 1) : 0u;
+    np = more ? __ldg(pre + x) : 0u;
     for (uint32_t r0 = ub; r0 < ue; r0 += 32) {
       const uint32_t k = r0 + lane;
-      uint32_t sst = 0, len = 0;
-      if (k < ue) {
-        const uint2 e = sl[k];
-        sst = e.x;
-        len = (e.y & OR_SL_GALLOP) ? 0u : e.y;
-      }
+      const uint32_t sst = sn.x, len = (sn.y & OR_SL_GALLOP) ? 0u : sn.y;
+      sn = k + 32 < ue ? __ldg(sl + k + 32) : make_uint2(0u, 0u);
       const unsigned act = __ballot_sync(ACCX_FULL_MASK, len > 0);
       if (!act) continue;
       const uint32_t incl = accx_warp_incl_sum(len, lane);
@@ -450,7 +474,7 @@ __global__ void __launch_bounds__(256) k_dense_rows(const uint32_t *__restrict__
                                                     const uint32_t *__restrict__ pre, uint32_t M, uint32_t chunk,
                                                     uint32_t *__restrict__ T, uint32_t *__restrict__ low,
                                                     uint4 *__restrict__ items, uint32_t cap,
-                                                    unsigned long long *__restrict__ ctr) {
+                                                    unsigned long long *__restrict__ nitems) {
   constexpr uint32_t K = WPL * 1024u;
   __shared__ uint32_t s_t[8][WPL * 32];
   const int lane = threadIdx.x & 31;
@@ -477,7 +501,7 @@ __global__ void __launch_bounds__(256) k_dense_rows(const uint32_t *__restrict__
       if (lw) {
         const uint32_t e = off[x + 1], c = accx_lower_bound(dst, b, e, (int32_t)M) - b;
         const uint32_t nch = (c + chunk - 1) / chunk;
-        const unsigned long long p = atomicAdd(&ctr[C_DENSE], (unsigned long long)nch);
+        const unsigned long long p = atomicAdd(nitems, (unsigned long long)nch);
         for (uint32_t j = 0; j < nch && p + j < cap; j++)
           items[p + j] = make_uint4(x, b + j * chunk, min(chunk, c - j * chunk), 0u);
       }
@@ -580,7 +604,7 @@ template <int WPL, bool ALL>
 __global__ void __launch_bounds__(DENSE_WARPS * 32, 2) k_dense_pairs(
     const uint32_t *__restrict__ off, const int32_t *__restrict__ dst, const uint32_t *__restrict__ pre,
     const uint32_t *__restrict__ low, const uint32_t *__restrict__ T, const uint4 *__restrict__ items, uint32_t cap,
-    int policy, const uint8_t *__restrict__ table, uint32_t pcap, int32_t *__restrict__ cnt,
+    const unsigned long long *__restrict__ nitems, int policy, const uint8_t *__restrict__ table, uint32_t pcap, int32_t *__restrict__ cnt,
     unsigned long long *__restrict__ ctr) {
   static_assert(DENSE_PLANES <= 16, "planes fit the ring");
   extern __shared__ __align__(16) uint32_t smem[];
@@ -588,7 +612,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32, 2) k_dense_pairs(
   uint32_t *ring = reinterpret_cast<dense_ring<WPL> *>(smem)[warp].w[0];
   const uint32_t sring = (uint32_t)__cvta_generic_to_shared(ring);
   constexpr uint32_t GROUP = 8 * 32 * WPL;  // words of a group
-  unsigned long long total = ctr[C_DENSE];
+  unsigned long long total = *nitems;
   if (total > cap) total = cap;
   unsigned long long found = 0;
   const unsigned long long nw = (unsigned long long)gridDim.x * DENSE_WARPS;

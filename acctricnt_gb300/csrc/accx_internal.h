@@ -165,5 +165,20 @@ int accx_relabel_gather(accx_graph *g, int32_t *out, cudaStream_t s);
 // that device (*on_device), else nullptr (graph.cu).
 void *accx_writable(const void *p, int device, bool *on_device);
 
-int accx_build_csr_from_keys(accx_graph *g, unsigned long long *d_keys, uint64_t nkeys, uint32_t n,
+// Entry keys (gen.cu): (source << b) | neighbour, b = the bits of an id below n; 4 bytes
+// when both fit, else 8.
+static inline int accx_key_bits(uint32_t n) {
+  int b = 1;
+  while (b < 32 && (1ull << b) < n) b++;
+  return b;
+}
+static inline size_t accx_key_size(uint32_t n) { return accx_key_bits(n) <= 16 ? 4 : 8; }
+#ifdef __CUDACC__
+template <typename K>
+__host__ __device__ inline K accx_key_none(int b) {  // the key of a dropped entry: sorts last
+  return (K)(~0ull >> (64 - 2 * b));
+}
+#endif
+// Sorted, deduplicated CSR of nkeys entry keys into g; *d_bad (optional) set: ACCX_ERR_RANGE.
+int accx_build_csr_from_keys(accx_graph *g, void *d_keys, uint64_t nkeys, uint32_t n, const int *d_bad,
                              cudaStream_t s);

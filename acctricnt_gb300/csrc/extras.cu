@@ -9,19 +9,16 @@
 #include "accx_internal.h"
 #include "devutil.cuh"
 
+template <typename K>
 __global__ void k_edge_keys(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint64_t k, uint32_t n,
-                            unsigned long long *__restrict__ keys, int *__restrict__ bad) {
+                            int b, K *__restrict__ keys, int *__restrict__ bad) {
+  const K none = accx_key_none<K>(b);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t u = src[i], v = dst[i];
-    unsigned long long a = ~0ull, b = ~0ull;  // self loops sort last and are dropped
-    if (u >= n || v >= n) {
-      atomicOr(bad, 1);
-    } else if (u != v) {
-      a = ((unsigned long long)u << 32) | v;
-      b = ((unsigned long long)v << 32) | u;
-    }
-    keys[2 * i] = a;
-    keys[2 * i + 1] = b;
+    const bool ok = u < n && v < n, keep = ok && u != v;  // self loops are dropped
+    if (!ok) atomicOr(bad, 1);
+    keys[2 * i] = keep ? ((K)u << b) | v : none;
+    keys[2 * i + 1] = keep ? ((K)v << b) | u : none;
   }
 }
 
@@ -40,31 +37,33 @@ extern "C" int accx_graph_from_edges(const uint32_t *src, const uint32_t *dst, u
   if (!g) return ACCX_ERR_OOM;
   cudaGetDevice(&g->device);
   g->symmetric = true;  // both directions of every edge are kept
-  unsigned long long *keys = nullptr;
-  uint32_t *ds = nullptr, *dd = nullptr;
-  int *bad = nullptr, hbad = 0;
+  // one block of the pool: keys, the host lists staged, the defect flag
+  char *block = nullptr;
+  const size_t key_bytes = (accx_key_size(n) * (2 * k + 1) + 255) & ~(size_t)255;
+  const size_t list = (sizeof(uint32_t) * k + 255) & ~(size_t)255;
+  const bool host = k && !accx_is_device_ptr(src);
   int rc = ACCX_OK;
   do {
-    if (cudaMalloc(&keys, sizeof(unsigned long long) * (2 * k + 1)) != cudaSuccess ||
-        cudaMalloc(&bad, sizeof(int)) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+    if (accx_dev_alloc((void **)&block, key_bytes + (host ? 2 * list : 0) + 256, s) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
     const uint32_t *s_src = src, *s_dst = dst;
-    if (k && !accx_is_device_ptr(src)) {  // stage host lists
-      if (cudaMalloc(&ds, sizeof(uint32_t) * k) != cudaSuccess || cudaMalloc(&dd, sizeof(uint32_t) * k) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+    if (host) {
+      uint32_t *ds = reinterpret_cast<uint32_t *>(block + key_bytes), *dd = reinterpret_cast<uint32_t *>(block + key_bytes + list);
       if (cudaMemcpyAsync(ds, src, sizeof(uint32_t) * k, cudaMemcpyHostToDevice, s) != cudaSuccess ||
           cudaMemcpyAsync(dd, dst, sizeof(uint32_t) * k, cudaMemcpyHostToDevice, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
       s_src = ds;
       s_dst = dd;
     }
+    int *bad = reinterpret_cast<int *>(block + key_bytes + (host ? 2 * list : 0));
     if (cudaMemsetAsync(bad, 0, sizeof(int), s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-    if (k) k_edge_keys<<<accx_sm_count(g->device) * 8, 256, 0, s>>>(s_src, s_dst, k, n, keys, bad);
-    if (cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-    if (hbad) { rc = ACCX_ERR_RANGE; break; }
-    rc = accx_build_csr_from_keys(g, keys, 2 * k, n, s);
+    const int grid = accx_sm_count(g->device) * 8, b = accx_key_bits(n);
+    if (k && accx_key_size(n) == 4)
+      k_edge_keys<<<grid, 256, 0, s>>>(s_src, s_dst, k, n, b, reinterpret_cast<uint32_t *>(block), bad);
+    else if (k)
+      k_edge_keys<<<grid, 256, 0, s>>>(s_src, s_dst, k, n, b, reinterpret_cast<unsigned long long *>(block), bad);
+    rc = accx_build_csr_from_keys(g, block, 2 * k, n, bad, s);
   } while (0);
   if (rc == ACCX_ERR_CUDA || rc == ACCX_ERR_OOM) cudaGetLastError();
-  for (void *p : {(void *)keys, (void *)ds, (void *)dd, (void *)bad})
-    if (p) cudaFree(p);
+  accx_dev_free(block, s);
   if (rc) {
     accx_graph_free(g);
     return rc;

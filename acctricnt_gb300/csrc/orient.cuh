@@ -169,12 +169,14 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
 // slices.
 //
 // Light: at most OW_CAP prefix ids (the warp's table and counters), OW_DEG entries and
-// OW_WORK probes, but no more than an OW_SHARE'th of all (a small graph's owners are fewer
-// than the machine's warps).  A CTA spends ~4 us of barriers on an item however small it
-// is, a warp well under 1 us; with many probes one warp becomes the tail of a small
-// graph.  Counts (us) by OW_WORK 0 (no light owners) / 512 / 1024 / 2048 / 4096:
-// R-MAT 15 187 / 187 / 183 / 183 / 218, Chung-Lu 3M 5825 / 5144 / 5004 / 4978 / 5058,
-// a batch of 48 small graphs 1929 / 994 / 999 / 998 / 1024.
+// OW_WORK probes -- up to OW_WORK_MAX on graphs whose owners average that much, so that
+// many warps have several (all probes / OW_SPREAD), but no more than an OW_SHARE'th of all
+// (a small graph's owners are fewer than the machine's warps).  A CTA spends ~4 us of
+// staging and barriers on an item however small it is, a warp well under 1 us; with many
+// probes one warp becomes the tail.  Counts (us) with 2048 / 4096 / 8192 / 16384: R-MAT 21
+// 5949 / 5706 / 5362 / 5499, Chung-Lu 3M 3704 / 3523 / 3579 / 3914, R-MAT 18 602 / 590 / 627 /
+// 628; without light owners a batch of 48 small graphs took 1929, with them 998.  Owners
+// from a counter instead of a fixed stride: Chung-Lu 3M 3744.
 //
 // n here is the number of vertices that can own (ids below the dense window).  One
 // cluster of eight CTAs counts and then fills in id order: the heavy owners come
@@ -183,9 +185,13 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
 // at R-MAT 24).  A count, device scan and fill over all n vertices were four launches,
 // and one 64-bit atomic per owner for the owner-work statistic took 139 us of a
 // 3M-vertex power-law count.
-#define OW_CAP 256u
-#define OW_WORK 2048u
+#define OW_CAP 512u
+#define OW_SLOTS 1024u
+#define OW_POS 11  // bits of a position in a table word; the ids, below the window, take the others
+#define OW_WORK 4096u
+#define OW_WORK_MAX 8192u
 #define OW_SHARE 4096u
+#define OW_SPREAD 400000u
 #define OW_DEG 4096u
 #define OW_MAX_N (1u << 24)  // ids must fit 24 bits of a table word
 // CTA items aim at a 16th of a CTA's share of all probes, within these bounds (a
@@ -242,7 +248,9 @@ __global__ void __cluster_dims__(OI_CTAS, 1, 1) __launch_bounds__(OI_THREADS)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t target = accx_item_target(ctr, target_max, ctas);
   const unsigned long long share = ctr[C_WORK + ACCX_KIND_BITMAP] / OW_SHARE;
-  const uint32_t light_max = share < OW_WORK ? (uint32_t)share : OW_WORK;
+  const unsigned long long mean = ctr[C_WORK + ACCX_KIND_BITMAP] / OW_SPREAD;
+  uint32_t light_max = mean < OW_WORK ? OW_WORK : mean > OW_WORK_MAX ? OW_WORK_MAX : (uint32_t)mean;
+  if (share < light_max) light_max = (uint32_t)share;
   // a run of `span` vertices (a multiple of 32) per warp of the cluster
   const uint32_t nw = OI_CTAS * OI_THREADS / 32, span = ((n + nw - 1) / nw + 31u) & ~31u;
   const uint32_t b = min(n, (cl.block_rank() * (OI_THREADS / 32) + warp) * span), e = min(n, b + span);
@@ -313,16 +321,16 @@ __global__ void __cluster_dims__(OI_CTAS, 1, 1) __launch_bounds__(OI_THREADS)
 }
 
 // Light bitmap owners: a warp per owner, no barriers.  The owner's prefix goes into
-// a hash table of packed (id << 8 | position) words in the warp's shared memory (at
-// least four slots an id, so most look-ups read one word), with one counter per
-// position; ids are below 2^24 as bitmap owners lie inside the dense window.  The
+// a hash table of packed (id << OW_POS | position) words in the warp's shared memory
+// (four slots an id up to 256 ids, so most look-ups read one word; at least two), with
+// one counter per position; ids are below 2^21 as bitmap owners lie inside the window.  The
 // row is walked 32 entries at a time: their partner ranges are concatenated (warp
 // scan) and streamed 32 ids a step, four steps' loads in flight, as the CTA kernel
 // streams its short lists.  Credits are the CTA kernel's.  Bound by latency and
 // instruction issue.
 #define OW_WARPS 8
 struct ow_warp {
-  uint32_t tab[4 * OW_CAP];
+  uint32_t tab[OW_SLOTS];
   uint32_t oc[OW_CAP];
   uint32_t pre[33], beg[32], hit[32];
 };
@@ -338,22 +346,22 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
   extern __shared__ __align__(16) uint32_t smem[];
   const int lane = threadIdx.x & 31;
   ow_warp &S = reinterpret_cast<ow_warp *>(smem)[threadIdx.x >> 5];
-  unsigned long long total = ctr[C_LIGHT];
-  if (total > cap) total = cap;
+  const uint32_t total = (uint32_t)(ctr[C_LIGHT] < cap ? ctr[C_LIGHT] : cap);
   unsigned long long found = 0;
-  const unsigned long long nw = (unsigned long long)gridDim.x * OW_WARPS;
-  unsigned long long it = (unsigned long long)blockIdx.x * OW_WARPS + (threadIdx.x >> 5);
+  const uint32_t nw = gridDim.x * OW_WARPS;
+  uint32_t it = blockIdx.x * OW_WARPS + (threadIdx.x >> 5);
   // a row is a chain of dependent loads: the next row's bounds, and this row's first ids
   // and ranges, are loaded ahead of where they are used
   uint32_t x = it < total ? items[cap - 1 - it] : 0u;
   uint32_t nb = it < total ? __ldg(off + x) : 0u, ne = it < total ? __ldg(off + x + 1) : 0u;
   uint32_t np = it < total ? __ldg(pre + x) : 0u;
-  for (; it < total; it += nw) {
+  while (it < total) {
     const uint32_t ub = nb, ue = ne, px = min(np, OW_CAP);
     const uint32_t id0 = (uint32_t)lane < px ? (uint32_t)__ldg(dst + ub + lane) : 0u;
     uint2 sn = ub + lane < ue ? __ldg(sl + ub + lane) : make_uint2(0u, 0u);
-    const bool more = it + nw < total;
-    x = more ? items[cap - 1 - (it + nw)] : 0u;
+    it += nw;
+    const bool more = it < total;
+    x = more ? items[cap - 1 - it] : 0u;
     // the table: 64 to 1024 slots
     int lg = 6;
     while (lg < 10 && (1u << lg) < 4u * px) lg++;
@@ -365,7 +373,7 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
     for (uint32_t i = lane; i < px; i += 32) {
       const uint32_t id = i < 32 ? id0 : (uint32_t)__ldg(dst + ub + i);
       uint32_t h = ow_hash(id, sh);
-      while (atomicCAS(&S.tab[h], 0xffffffffu, (id << 8) | i) != 0xffffffffu) h = (h + 1) & mask;
+      while (atomicCAS(&S.tab[h], 0xffffffffu, (id << OW_POS) | i) != 0xffffffffu) h = (h + 1) & mask;
     }
     __syncwarp();
     nb = more ? __ldg(off + x) : 0u;
@@ -410,13 +418,13 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
           if (xs[r] < 0) continue;
           const uint32_t id = (uint32_t)xs[r];
           uint32_t h = ow_hash(id, sh), t = S.tab[h];
-          while ((t >> 8) != id && t != 0xffffffffu) {
+          while ((t >> OW_POS) != id && t != 0xffffffffu) {
             h = (h + 1) & mask;
             t = S.tab[h];
           }
           if (t != 0xffffffffu) {
             atomicAdd(cnt + gi[r], 1);
-            atomicAdd(&S.oc[t & 255u], 1u);
+            atomicAdd(&S.oc[t & ((1u << OW_POS) - 1u)], 1u);
             atomicAdd(&S.hit[sg[r]], 1u);
           }
         }

@@ -55,13 +55,13 @@ def _check(off, dst, **kw):
     assert sum(s["edges"] for s in st.values()) <= len(dst) // 2
 
 
-# the warp's table takes 256 prefix ids and 64 to 1024 slots (four an id)
-@pytest.mark.parametrize("p", [1, 2, 15, 16, 17, 31, 32, 33, 64, 65, 127, 128, 129, 255, 256, 257, 300])
+# the warp's table takes 512 prefix ids and 64 to 1024 slots
+@pytest.mark.parametrize("p", [1, 2, 15, 16, 17, 31, 32, 33, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513])
 def test_prefix_length_edges(p):
-    _check(*_hubs_and_leaves(320, [p] * 5 + [p - 1 or 1] * 3, 0.1, seed=p, satellites=60))
+    _check(*_hubs_and_leaves(540, [p] * 5 + [p - 1 or 1] * 3, 0.1, seed=p, satellites=60))
 
 
-# probe work around the light limit (2048 probes): a leaf of p hubs probes about
+# probe work around the light limits (a share of all probes, 4096, 8192): a leaf of p hubs probes about
 # p * density * hubs / 2 ids
 @pytest.mark.parametrize("density", [0.02, 0.05, 0.1, 0.2, 0.5, 1.0])
 def test_probe_work_edges(density):

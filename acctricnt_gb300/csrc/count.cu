@@ -1036,9 +1036,12 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     // an all-bitmap count gallops only where an owner is outside the window or the counters
     const bool can_gallop = policy != ACCX_POLICY_MERGE &&
                             !(policy == ACCX_POLICY_BITMAP && rel && n <= W && n <= g->plan_rows && g->plan_maxpre <= pcap);
-    if (can_gallop)
+    if (can_gallop) {
       k_gallop_or<GALLOP_OR_GROUP><<<sms * 8, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list,
                                                                         list_cap, ctr, cnt);
+      k_gallop_lane<<<sms * GALLOP_CTAS, MERGE_WARPS * 32, 0, s>>>(g->d_vinfo, dst, g->d_or_sl, g->d_edge_list, list_cap,
+                                                                   ctr, cnt);
+    }
     ACCX_MARK(3);
     if (dm) {
       const bool all = policy == ACCX_POLICY_BITMAP && g->plan_maxpre <= pcap;

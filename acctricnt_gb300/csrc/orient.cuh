@@ -106,23 +106,62 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_merge_or(const uint32_t *_
   if (lane == 0 && found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_MERGE], found);
 }
 
-// Groups of G lanes take one edge each: the lanes take the partner's prefix ids
-// in order and binary-search each in the owner's prefix; every round starts at
-// the position the group's last lane reached.  Galloping edges mostly have
-// short partner lists (the low-degree owners outside the bitmap window), so a
-// warp works on 32/G edges at once.  The partner range comes from classify
-// (sl[e], already cut at min(x, y)), so an edge needs its list record, that
-// range and the owner's offset and prefix length (vinfo): y < x exactly when e lies in
-// x's prefix, and then the owner's range is cut at e and the edge's credit goes
-// to e; otherwise to the end of the partner range (x's position in N(y)).
+// One galloping edge by G lanes: the lanes take the partner's ids in order and
+// binary-search each in the owner's prefix; every round starts at the position the
+// group's last lane reached.  Credits both entries of a match; returns the matches.
 template <int G>
-__global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__restrict__ vinfo,
-                                                                 const int32_t *__restrict__ dst,
-                                                                 const uint2 *__restrict__ sl,
-                                                                 const uint2 *__restrict__ list, uint32_t list_cap,
-                                                                 unsigned long long *__restrict__ ctr,
-                                                                 int32_t *__restrict__ cnt) {
+__device__ __forceinline__ uint32_t or_gallop_group(const int32_t *__restrict__ dst, uint32_t xb, uint32_t xe,
+                                                    uint32_t yb, uint32_t ye, int gl, unsigned gmask,
+                                                    int32_t *__restrict__ cnt) {
+  uint32_t c = 0, lo = xb;
+  for (uint32_t j0 = yb; j0 < ye && lo < xe; j0 += G) {
+    const uint32_t j = j0 + (uint32_t)gl;
+    uint32_t pos = xe;
+    if (j < ye) {
+      const int32_t id = __ldg(dst + j);
+      pos = accx_lower_bound(dst, lo, xe, id);
+      if (pos < xe && __ldg(dst + pos) == id) {
+        c++;
+        atomicAdd(cnt + pos, 1);
+        atomicAdd(cnt + j, 1);
+      }
+    }
+    const uint32_t last = (ye - j0 >= (uint32_t)G) ? (uint32_t)G - 1u : (ye - j0 - 1);
+    lo = __shfl_sync(gmask, pos, (int)last, G);
+  }
+#pragma unroll
+  for (int d = G / 2; d >= 1; d >>= 1) c += __shfl_xor_sync(gmask, c, d, G);
+  return c;
+}
+
+// Galloping edges.  An edge's records are its list entry, the partner range that classify
+// wrote (sl[e], already cut at min(x, y)) and the owner's offset and prefix length
+// (vinfo): y < x exactly when e lies in x's prefix, and then the owner's range is cut at e
+// and the edge's credit goes to e; otherwise to the end of the partner range (x's
+// position in N(y)).  Two kernels, each of which returns at once when the edges are the
+// other's: where the partner lists average more than GALLOP_MEAN ids, groups of G lanes
+// take one edge each (k_gallop_or), else a lane does (k_gallop_lane).
+#define GALLOP_MEAN 24ull
+__device__ __forceinline__ bool or_gallop_long(const unsigned long long *__restrict__ ctr) {
+  return ctr[C_WORK + ACCX_KIND_GALLOP] > GALLOP_MEAN * ctr[C_EDGES + ACCX_KIND_GALLOP];
+}
+struct or_gallop_edge {
+  uint32_t xb, xe, yb, ye, at;  // owner range, partner range, the edge's prefix entry
+};
+__device__ __forceinline__ or_gallop_edge or_gallop_get(uint2 p, uint2 r, uint2 xi) {
+  const uint32_t xp = xi.x + xi.y, ye = r.x + (r.y & ~OR_SL_GALLOP);
+  return or_gallop_edge{xi.x, min(xp, p.y), r.x, ye, p.y < xp ? p.y : ye};
+}
+
+template <int G>
+__global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_gallop_or(const uint2 *__restrict__ vinfo,
+                                                                    const int32_t *__restrict__ dst,
+                                                                    const uint2 *__restrict__ sl,
+                                                                    const uint2 *__restrict__ list, uint32_t list_cap,
+                                                                    unsigned long long *__restrict__ ctr,
+                                                                    int32_t *__restrict__ cnt) {
   static_assert(G == 8 || G == 16 || G == 32, "group size");
+  if (!or_gallop_long(ctr)) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int sub = lane / G, gl = lane % G;
   const unsigned gmask = G == 32 ? ACCX_FULL_MASK : (((1u << G) - 1u) << (sub * G));
@@ -133,32 +172,116 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) k_gallop_or(const uint2 *__r
   for (unsigned long long it = ((unsigned long long)blockIdx.x * MERGE_WARPS + w) * (32 / G) + sub; it < total;
        it += ng) {
     const uint2 p = list[list_cap - 1 - it];
-    const uint32_t x = p.x, e = p.y;
-    const uint2 r = __ldg(sl + e), xi = __ldg(vinfo + x);
-    const uint32_t xb = xi.x, xp = xi.x + xi.y;
-    const uint32_t xe = min(xp, e), yb = r.x, ye = r.x + (r.y & ~OR_SL_GALLOP);
-    uint32_t c = 0, lo = xb;
-    for (uint32_t j0 = yb; j0 < ye && lo < xe; j0 += G) {
-      const uint32_t j = j0 + (uint32_t)gl;
-      uint32_t pos = xe;
-      if (j < ye) {
-        const int32_t id = __ldg(dst + j);
-        pos = accx_lower_bound(dst, lo, xe, id);
-        if (pos < xe && __ldg(dst + pos) == id) {
-          c++;
-          atomicAdd(cnt + pos, 1);
-          atomicAdd(cnt + j, 1);
-        }
-      }
-      const uint32_t last = (ye - j0 >= (uint32_t)G) ? (uint32_t)G - 1u : (ye - j0 - 1);
-      lo = __shfl_sync(gmask, pos, (int)last, G);
-    }
-#pragma unroll
-    for (int d = G / 2; d >= 1; d >>= 1) c += __shfl_xor_sync(gmask, c, d, G);
-    if (gl == 0 && c) atomicAdd(cnt + (e < xp ? e : ye), (int32_t)c);  // the edge's prefix entry
+    const or_gallop_edge d = or_gallop_get(p, __ldg(sl + p.y), __ldg(vinfo + p.x));
+    const uint32_t c = or_gallop_group<G>(dst, d.xb, d.xe, d.yb, d.ye, gl, gmask, cnt);
+    if (gl == 0 && c) atomicAdd(cnt + d.at, (int32_t)c);
     if (gl == 0) found += c;
   }
   if (gl == 0 && found) atomicAdd(&ctr[C_MATCH + ACCX_KIND_GALLOP], found);
+}
+
+// A warp takes 32 edges, a lane loading each one's records (the next 32 edges' while these
+// are walked).  Partner lists of up to GALLOP_LANE ids are the lane's own: both lists
+// walked together, or the partner's ids searched where the owner's list is much longer;
+// eight-lane groups take the longer ones.  A group for every edge spent ~25 warp
+// instructions on two lists of ten ids; walking with a branch per advance, 34.  Erdos-
+// Renyi with 16M entries 569 -> 330 us, with 120M, whose lists come from HBM,
+// 3.60 -> 2.23 ms; R-MAT 24, with 58 ids a list, would take 12.7 ms instead of 10.1.
+#define GALLOP_LANE 32u   // partner ids up to which a lane takes the edge alone
+#define GALLOP_MERGE 8u   // owner ids per partner id up to which it walks both lists
+// per SM: with more the partner lists push each other out of L1 (Erdos-Renyi with 120M
+// entries: 4 CTAs 2.55 ms, 5 2.23, 6 2.46, 8 3.1; a prefetch of the next lists into L2 cost
+// 0.6 ms)
+#define GALLOP_CTAS 5
+__global__ void __launch_bounds__(MERGE_WARPS * 32, GALLOP_CTAS) k_gallop_lane(const uint2 *__restrict__ vinfo,
+                                                                                const int32_t *__restrict__ dst,
+                                                                                const uint2 *__restrict__ sl,
+                                                                                const uint2 *__restrict__ list,
+                                                                                uint32_t list_cap,
+                                                                                unsigned long long *__restrict__ ctr,
+                                                                                int32_t *__restrict__ cnt) {
+  if (or_gallop_long(ctr)) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane / 8, gl = lane % 8;
+  const unsigned gmask = 0xffu << (sub * 8);
+  uint32_t found = 0;
+  const uint32_t total = (uint32_t)(ctr[C_GALLOP] < list_cap ? ctr[C_GALLOP] : list_cap);
+  const uint32_t step = gridDim.x * MERGE_WARPS * 32;
+  auto load = [&](uint32_t it, uint2 *p) {
+    *p = make_uint2(0u, 0u);
+    if (it >= total) return false;
+    *p = __ldg(list + (list_cap - 1 - it));
+    return true;
+  };
+  uint32_t it = (blockIdx.x * MERGE_WARPS + w) * 32 + lane;
+  uint2 p, r = make_uint2(0u, 0u), xi = make_uint2(0u, 0u);
+  if (load(it, &p)) {
+    r = __ldg(sl + p.y);
+    xi = __ldg(vinfo + p.x);
+  }
+  for (uint32_t it0 = it - lane; it0 < total; it0 += step) {
+    const or_gallop_edge d = or_gallop_get(p, r, xi);
+    it = it0 + lane < 0xffffffffu - step ? it0 + lane + step : 0xffffffffu;
+    if (load(it, &p)) {
+      r = __ldg(sl + p.y);
+      xi = __ldg(vinfo + p.x);
+    } else {
+      r = xi = make_uint2(0u, 0u);
+    }
+    const bool any = d.yb < d.ye && d.xb < d.xe, own = any && d.ye - d.yb <= GALLOP_LANE;
+    if (own) {
+      uint32_t c = 0;
+      if (d.xe - d.xb <= GALLOP_MERGE * (d.ye - d.yb)) {
+        // both ids loaded anew each step (mostly L1 hits; the array is padded past its
+        // end): the only branches are the loop's and the rare match's
+        uint32_t i = d.xb, j = d.yb;
+        do {
+          const int32_t a = __ldg(dst + i), b = __ldg(dst + j);
+          if (a == b) {
+            c++;
+            atomicAdd(cnt + i, 1);
+            atomicAdd(cnt + j, 1);
+          }
+          i += a <= b;
+          j += b <= a;
+        } while (i < d.xe && j < d.ye);
+      } else {
+        uint32_t lo = d.xb;
+        for (uint32_t j = d.yb; j < d.ye && lo < d.xe; j++) {
+          const int32_t id = __ldg(dst + j);
+          lo = accx_lower_bound(dst, lo, d.xe, id);
+          if (lo < d.xe && __ldg(dst + lo) == id) {
+            c++;
+            atomicAdd(cnt + lo, 1);
+            atomicAdd(cnt + j, 1);
+          }
+        }
+      }
+      if (c) atomicAdd(cnt + d.at, (int32_t)c);
+      found += c;
+    }
+    __syncwarp();
+    for (unsigned big = __ballot_sync(ACCX_FULL_MASK, any && !own); big;) {
+      // the group's edge: the sub-th of the next four
+      unsigned m = big;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (q < sub) m &= m - 1;
+        big &= big - 1;
+      }
+      const int src = m ? __ffs(m) - 1 : 0;
+      const uint32_t gxb = __shfl_sync(ACCX_FULL_MASK, d.xb, src), exe = __shfl_sync(ACCX_FULL_MASK, d.xe, src);
+      const uint32_t gyb = __shfl_sync(ACCX_FULL_MASK, d.yb, src), gye = __shfl_sync(ACCX_FULL_MASK, d.ye, src);
+      const uint32_t gat = __shfl_sync(ACCX_FULL_MASK, d.at, src);
+      const uint32_t c = or_gallop_group<8>(dst, gxb, m ? exe : gxb, gyb, gye, gl, gmask, cnt);
+      if (gl == 0 && c) atomicAdd(cnt + gat, (int32_t)c);
+      if (gl == 0) found += c;
+      __syncwarp();
+    }
+  }
+  unsigned long long f = found;
+#pragma unroll
+  for (int q = 16; q >= 1; q >>= 1) f += __shfl_xor_sync(ACCX_FULL_MASK, f, q);
+  if (lane == 0 && f) atomicAdd(&ctr[C_MATCH + ACCX_KIND_GALLOP], f);
 }
 
 // Work items of the bitmap owners.  An owner with little probe work is one entry of

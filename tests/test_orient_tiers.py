@@ -119,3 +119,30 @@ def test_dense_rows_around_k(n, hubs):
     k = (n - hubs) * 200
     off, dst = _csr(n, np.concatenate([a[m], rng.integers(hubs, n, k)]), np.concatenate([b[m], rng.integers(0, hubs, k)]))
     _check(off, dst)
+
+
+# galloping edges by lane (partner lists that average up to 24 ids) and by group: sparse
+# and dense graphs, partner lists around the lane's 32 ids, owners much longer
+@pytest.mark.parametrize("n,mean", [(40, 3), (3000, 6), (3000, 45), (2000, 62), (2000, 66), (1500, 140), (400, 300)])
+def test_gallop_random(n, mean):
+    rng = np.random.default_rng(n + mean)
+    k = n * mean // 2
+    off, dst = _csr(n, rng.integers(0, n, k), rng.integers(0, n, k))
+    ref = oracle.cn_count(off, dst, nthreads=8)
+    for relabel in (False, True):
+        G = accx.Graph.from_csr(off, dst)
+        if relabel:
+            G.relabel()
+        assert np.array_equal(G.count(policy="gallop", bias=2, orient=True), ref)
+        matches, _ = G.last_matches()
+        assert matches["gallop"] == (int(ref.sum()) - 2 * len(ref)) // 6
+
+
+@pytest.mark.parametrize("p", [1, 3, 8, 31, 32, 33, 40])
+def test_gallop_skewed(p):
+    """Leaves of p hubs on hubs with long prefixes: the searching side of both kernels."""
+    off, dst = _hubs_and_leaves(600, [p] * 900, 0.5, seed=p, satellites=45)
+    ref = oracle.cn_count(off, dst, nthreads=8)
+    G = accx.Graph.from_csr(off, dst)
+    G.relabel()
+    assert np.array_equal(G.count(policy="gallop", bias=2, orient=True), ref)

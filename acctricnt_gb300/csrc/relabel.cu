@@ -13,49 +13,38 @@
 #include "accx_internal.h"
 #include "devutil.cuh"
 
-__global__ void k_vertex_keys(const uint32_t *__restrict__ off, uint32_t n, unsigned long long *__restrict__ keys) {
+// Sort keys of the vertex order: the top of the key range less the degree, so that an
+// ascending stable sort of the ids by key gives degree descending, then id.  The keys have
+// the bits of the entry count: fewer radix passes than a 64-bit (degree, id) key.
+__global__ void k_vertex_keys(const uint32_t *__restrict__ off, uint32_t n, uint32_t top, uint32_t *__restrict__ keys,
+                              uint32_t *__restrict__ ids) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    uint32_t d = off[v + 1] - off[v];
-    keys[v] = ((unsigned long long)(0xffffffffu - d) << 32) | v;  // degree descending, then id
+    keys[v] = top - (off[v + 1] - off[v]);
+    ids[v] = v;
   }
 }
 
-__global__ void k_perm(const unsigned long long *__restrict__ sorted, uint32_t n, const uint32_t *__restrict__ off,
+__global__ void k_perm(const uint32_t *__restrict__ sorted, uint32_t n, const uint32_t *__restrict__ off,
                        uint32_t *__restrict__ oldid, uint32_t *__restrict__ newid, uint32_t *__restrict__ rdeg) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    uint32_t v = (uint32_t)(sorted[i] & 0xffffffffull);
+    const uint32_t v = sorted[i];
     oldid[i] = v;
     newid[v] = i;
     rdeg[i] = off[v + 1] - off[v];
   }
 }
 
-// Rows move whole: the row of old vertex u becomes row newid[u], so an entry's
-// new place is that row's start plus its old position in the row; it carries the
-// new id of its neighbour (the sort key) and its own old index.  Rows are sorted
-// by key afterwards.
-template <int TILE>
-__global__ void __launch_bounds__(TILE) k_row_scatter(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
-                                                      const int32_t *__restrict__ dst, uint32_t n, uint32_t m,
-                                                      const uint32_t *__restrict__ newid, const uint32_t *__restrict__ roff,
-                                                      uint32_t *__restrict__ key, uint32_t *__restrict__ val) {
-  __shared__ accx_tile_rows<TILE> sh;
-  uint32_t base = blockIdx.x * (uint32_t)TILE;
-  uint32_t e = base + threadIdx.x;
-  uint32_t u = accx_tile_row<TILE>(off, tilerow, n, m, base, e, &sh);
-  if (e >= m) return;
-  const uint32_t p = roff[newid[u]] + (e - off[u]);
-  const uint32_t v = (uint32_t)dst[e];
-  key[p] = v < n ? newid[v] : 0xffffffffu;
-  val[p] = e;
-}
+// Rows move whole: the row of old vertex u becomes row newid[u], sorted by its
+// neighbours' new ids.  Relabeled rows are in non-increasing degree order, so each degree
+// class is a range of rows, sorted by a kernel of its size straight from the original
+// entries: it reads the row, looks up the new ids and writes the sorted row and the map.
+// bounds[i] = the first row of degree <= RELABEL_CLASS[i], bounds[RELABEL_NCLASS + i] its
+// first entry.
+#define RELABEL_NCLASS 8
+__constant__ uint32_t RELABEL_CLASS[RELABEL_NCLASS] = {4096u, 1024u, 512u, 256u, 128u, 64u, 32u, 1u};
 
-// Relabeled rows are in non-increasing degree order, so each degree class is a
-// range of rows: bounds[i] = the first row of degree <= RELABEL_CLASS[i].
-#define RELABEL_NCLASS 5
-__constant__ uint32_t RELABEL_CLASS[RELABEL_NCLASS] = {4096u, 1024u, 256u, 32u, 1u};
-
-__global__ void k_class_bounds(const uint32_t *__restrict__ rdeg, uint32_t n, uint32_t *__restrict__ bounds) {
+__global__ void k_class_bounds(const uint32_t *__restrict__ rdeg, uint32_t n, const uint32_t *__restrict__ roff,
+                               uint32_t *__restrict__ bounds) {
   const int i = threadIdx.x;
   if (i >= RELABEL_NCLASS) return;
   uint32_t lo = 0, hi = n;
@@ -65,78 +54,152 @@ __global__ void k_class_bounds(const uint32_t *__restrict__ rdeg, uint32_t n, ui
     else lo = mid + 1;
   }
   bounds[i] = lo;
+  bounds[RELABEL_NCLASS + i] = roff[lo];
 }
 
-// Writes sorted row entries: the relabeled neighbour id and, for the entry's old
-// index, its new position.
-__device__ __forceinline__ void relabel_put(uint32_t p, uint32_t k, uint32_t v, int32_t *__restrict__ rdst,
-                                            uint32_t *__restrict__ map) {
-  rdst[p] = (int32_t)k;
-  map[v] = p;
+// The original and the relabeled graph, as the row kernels take them.
+struct relabel_view {
+  const uint32_t *off;    // original offsets
+  const int32_t *dst;     // original neighbours
+  const uint32_t *oldid, *newid, *roff;
+  uint32_t n;
+  int32_t *rdst;
+  uint32_t *map;
+};
+__device__ __forceinline__ uint32_t relabel_key(const relabel_view &g, uint32_t e) {
+  const uint32_t v = (uint32_t)__ldg(g.dst + e);
+  return v < g.n ? __ldg(g.newid + v) : 0xffffffffu;
+}
+
+// Rows above 4096 entries, a CTA each: keys and original entries for the segmented sort.
+__global__ void __launch_bounds__(1024) k_big_rows(relabel_view g, uint32_t rows, uint32_t *__restrict__ key,
+                                                   uint32_t *__restrict__ val) {
+  for (uint32_t r = blockIdx.x; r < rows; r += gridDim.x) {
+    const uint32_t b = g.roff[r], d = g.roff[r + 1] - b, e0 = g.off[g.oldid[r]];
+    for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) {
+      key[b + i] = relabel_key(g, e0 + i);
+      val[b + i] = e0 + i;
+    }
+  }
+}
+__global__ void k_put_big(const uint32_t *__restrict__ key, const uint32_t *__restrict__ val, uint32_t m,
+                          int32_t *__restrict__ rdst, uint32_t *__restrict__ map) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x) {
+    rdst[p] = (int32_t)key[p];
+    map[val[p]] = p;
+  }
 }
 
 // One CTA per row of at most NT*IPT entries (rows r0..r1, CTAs loop over them):
-// block radix sort over the low `bits` bits.  Padding keys are all ones and
-// `bits` leaves them above every id, so they sort last.  The input arrangement
-// does not matter to the sort, so loads are striped (coalesced).
+// block radix sort over the low `bits` bits of (key, place in the row).  Padding keys are
+// all ones and `bits` leaves them above every id, so they sort last.  The input
+// arrangement does not matter to the sort, so loads are striped (coalesced).
 template <int NT, int IPT>
-__global__ void __launch_bounds__(NT) k_row_sort(uint32_t r0, uint32_t r1, const uint32_t *__restrict__ roff,
-                                                 const uint32_t *__restrict__ key, const uint32_t *__restrict__ val,
-                                                 int bits, int32_t *__restrict__ rdst, uint32_t *__restrict__ map) {
+__global__ void __launch_bounds__(NT) k_row_sort(relabel_view g, uint32_t r0, uint32_t r1, int bits) {
   using Sort = cub::BlockRadixSort<uint32_t, NT, IPT, uint32_t, 5>;  // 5-bit digits: 4 and 6 measured slower
   __shared__ typename Sort::TempStorage tmp;
   for (uint32_t r = r0 + blockIdx.x; r < r1; r += gridDim.x) {
-    const uint32_t b = roff[r], d = roff[r + 1] - b;
+    const uint32_t b = g.roff[r], d = g.roff[r + 1] - b, e0 = g.off[g.oldid[r]];
     uint32_t k[IPT], v[IPT];
 #pragma unroll
     for (int i = 0; i < IPT; i++) {
       const uint32_t idx = (uint32_t)i * NT + threadIdx.x;
-      k[i] = idx < d ? key[b + idx] : 0xffffffffu;
-      v[i] = idx < d ? val[b + idx] : 0u;
+      k[i] = idx < d ? relabel_key(g, e0 + idx) : 0xffffffffu;
+      v[i] = idx;
     }
     Sort(tmp).SortBlockedToStriped(k, v, 0, bits);
 #pragma unroll
     for (int i = 0; i < IPT; i++) {
       const uint32_t idx = (uint32_t)i * NT + threadIdx.x;
-      if (idx < d) relabel_put(b + idx, k[i], v[i], rdst, map);
+      if (idx < d) {
+        g.rdst[b + idx] = (int32_t)k[i];
+        g.map[e0 + v[i]] = b + idx;
+      }
     }
     __syncthreads();  // tmp is reused by the next row
   }
 }
 
-// One warp per row of at most 32 entries: bitonic sort across the lanes.
-__global__ void k_warp_row_sort(uint32_t r0, uint32_t r1, const uint32_t *__restrict__ roff,
-                                const uint32_t *__restrict__ key, const uint32_t *__restrict__ val,
-                                int32_t *__restrict__ rdst, uint32_t *__restrict__ map) {
+// One warp per row of at most 32 E entries: a bitonic network over lanes and registers
+// (element 32 k + lane in register k, so loads and stores are coalesced).  One word an
+// element when key and place in the row (its low log2(32 E) bits) fit (PACKED), else a
+// pair.  Rows of 33 to 256 entries took a 64-thread radix sort of 256 pairs before,
+// whatever their length, after a pass that wrote the pairs to memory (757 and 433 us at
+// R-MAT 21; without that pass and with these sorts the whole host job takes 1.07 ms
+// less).  Rows of 513 to 1024 in 32 registers a lane measured slower than the CTA radix
+// sort (354 us against 268 for 257 to 1024).
+__host__ __device__ constexpr int relabel_place_bits(int e) { return e == 1 ? 5 : 1 + relabel_place_bits(e / 2); }
+template <int E, bool PACKED>
+__global__ void __launch_bounds__(256) k_warp_row_sort(relabel_view g, uint32_t r0, uint32_t r1) {
+  constexpr int SHIFT = relabel_place_bits(E);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t r = r0 + w; r < r1; r += nw) {
-    const uint32_t b = roff[r], d = roff[r + 1] - b;
-    uint32_t k = lane < d ? key[b + lane] : 0xffffffffu, v = lane < d ? val[b + lane] : 0u;
+    const uint32_t b = g.roff[r], d = g.roff[r + 1] - b, e0 = g.off[g.oldid[r]];
+    uint32_t k[E], v[E];
 #pragma unroll
-    for (uint32_t sz = 2; sz <= 32; sz <<= 1) {
+    for (int i = 0; i < E; i++) {
+      const uint32_t idx = 32u * i + lane, x = idx < d ? relabel_key(g, e0 + idx) : 0xffffffffu;
+      k[i] = PACKED ? (idx < d ? (x << SHIFT) | idx : 0xffffffffu) : x;
+      v[i] = idx;
+    }
+#pragma unroll
+    for (uint32_t sz = 2; sz <= 32u * E; sz <<= 1) {
 #pragma unroll
       for (uint32_t j = sz >> 1; j > 0; j >>= 1) {
-        const uint32_t ok = __shfl_xor_sync(ACCX_FULL_MASK, k, j), ov = __shfl_xor_sync(ACCX_FULL_MASK, v, j);
-        // ascending runs of sz lanes alternate with descending ones; the lower
-        // lane of a pair keeps the smaller key in an ascending run
-        const bool keep_min = ((lane & j) == 0) == ((lane & sz) == 0);
-        if (keep_min ? (ok < k) : (ok > k)) {
-          k = ok;
-          v = ov;
+        if (j >= 32u) {  // both elements in this lane
+#pragma unroll
+          for (int i = 0; i < E; i++) {
+            const int o = i ^ (int)(j >> 5);
+            if (o <= i) continue;
+            const bool up = ((32u * i) & sz) == 0;  // ascending runs of sz alternate with descending ones
+            if (up ? k[i] > k[o] : k[i] < k[o]) {
+              const uint32_t t = k[i], q = v[i];
+              k[i] = k[o];
+              k[o] = t;
+              v[i] = v[o];
+              v[o] = q;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < E; i++) {
+            const uint32_t ok = __shfl_xor_sync(ACCX_FULL_MASK, k[i], j);
+            // the lower lane of a pair keeps the smaller key in an ascending run
+            const bool keep_min = ((lane & j) == 0) == (((32u * i + lane) & sz) == 0);
+            if (PACKED) {
+              k[i] = keep_min ? min(k[i], ok) : max(k[i], ok);
+            } else {
+              const uint32_t ov = __shfl_xor_sync(ACCX_FULL_MASK, v[i], j);
+              if (keep_min ? ok < k[i] : ok > k[i]) {
+                k[i] = ok;
+                v[i] = ov;
+              }
+            }
+          }
         }
       }
     }
-    if (lane < d) relabel_put(b + lane, k, v, rdst, map);
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+      const uint32_t idx = 32u * i + lane;
+      if (idx < d) {
+        g.rdst[b + idx] = (int32_t)(PACKED ? k[i] >> SHIFT : k[i]);
+        g.map[e0 + (PACKED ? k[i] & ((1u << SHIFT) - 1u) : v[i])] = b + idx;
+      }
+    }
   }
 }
 
-// Entries [p0, p1) that are already in order (rows of at most one entry, or rows
-// sorted by the segmented sort).
-__global__ void k_put_range(const uint32_t *__restrict__ key, const uint32_t *__restrict__ val, uint32_t p0,
-                            uint32_t p1, int32_t *__restrict__ rdst, uint32_t *__restrict__ map) {
-  for (uint32_t p = p0 + blockIdx.x * blockDim.x + threadIdx.x; p < p1; p += gridDim.x * blockDim.x)
-    relabel_put(p, key[p], val[p], rdst, map);
+// Rows of at most one entry: entries p0.. of rows r0..r1 in order.
+__global__ void k_put_single(relabel_view g, uint32_t r0, uint32_t r1) {
+  for (uint32_t r = r0 + blockIdx.x * blockDim.x + threadIdx.x; r < r1; r += gridDim.x * blockDim.x) {
+    const uint32_t b = g.roff[r];
+    if (g.roff[r + 1] == b) continue;
+    const uint32_t e = g.off[g.oldid[r]];
+    g.rdst[b] = (int32_t)relabel_key(g, e);
+    g.map[e] = b;
+  }
 }
 
 // Four entries per thread and step, their index loads and then their gathers
@@ -260,18 +323,16 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
   ACCX_CUDA_TRY(cudaSetDevice(g->device));
   const uint32_t n = g->n, m = (uint32_t)g->m;
   const int grid = accx_sm_count(g->device) * 8;
-  unsigned long long *vkeys = nullptr, *vkeys2 = nullptr;
-  uint32_t *key = nullptr, *val = nullptr, *key2 = nullptr, *val2 = nullptr, *rdeg = nullptr, *bounds = nullptr;
+  // temporaries: vertex keys and ids (two buffers each; the plan lies in them later),
+  // degrees, class bounds
+  uint32_t *vtmp = nullptr, *rdeg = nullptr, *key = nullptr;
   void *tmp = nullptr;
   size_t tb = 0;
   int rc = ACCX_OK;
+  const size_t vn = ((size_t)n + 64) & ~(size_t)63;
   do {
-    if (accx_dev_alloc((void **)&vkeys, sizeof(unsigned long long) * ((size_t)n + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&vkeys2, sizeof(unsigned long long) * ((size_t)n + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&key, sizeof(uint32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&val, sizeof(uint32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&rdeg, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&bounds, sizeof(uint32_t) * 8, g->home) != cudaSuccess ||
+    if (accx_dev_alloc((void **)&vtmp, sizeof(uint32_t) * (4 * vn + (DENSE_KINDS + 1) * DENSE_BLOCKS), g->home) != cudaSuccess ||
+        accx_dev_alloc((void **)&rdeg, sizeof(uint32_t) * (vn + 2 * RELABEL_NCLASS + 2), g->home) != cudaSuccess ||
         accx_dev_alloc((void **)&g->d_roff, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
         accx_dev_alloc((void **)&g->d_rdst, sizeof(int32_t) * ((size_t)m + ACCX_DST_PAD), g->home) != cudaSuccess ||
         accx_dev_alloc((void **)&g->d_rmap, sizeof(uint32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
@@ -281,13 +342,14 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
       rc = ACCX_ERR_OOM;
       break;
     }
-    if (g->home && cudaStreamSynchronize(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-    // sort keys: ids need `bits` bits with the all-ones pattern left above every id
-    int bits = 1;
+    uint32_t *bounds = rdeg + vn;
+    // sort keys: ids need `bits` bits with the all-ones pattern left above every id, degrees `dbits`
+    int bits = 1, dbits = 1;
     while (bits < 32 && (1ull << bits) <= (unsigned long long)n) bits++;
-    cub::DoubleBuffer<unsigned long long> dk(vkeys, vkeys2);
+    while (dbits < 32 && (1ull << dbits) <= (unsigned long long)m) dbits++;
+    cub::DoubleBuffer<uint32_t> dk(vtmp, vtmp + vn), dv(vtmp + 2 * vn, vtmp + 3 * vn);
     size_t b1 = 0, b2 = 0;
-    if (cub::DeviceRadixSort::SortKeys(nullptr, b1, dk, (int64_t)n, 0, 64, s) != cudaSuccess ||
+    if (cub::DeviceRadixSort::SortPairs(nullptr, b1, dk, dv, (int64_t)n, 0, dbits, s) != cudaSuccess ||
         cub::DeviceScan::ExclusiveSum(nullptr, b2, rdeg, g->d_roff, (int64_t)n + 1, s) != cudaSuccess) {
       rc = ACCX_ERR_CUDA;
       break;
@@ -297,82 +359,75 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
     if (g->home && cudaStreamSynchronize(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     // 1. vertex order: degree descending, ties by id
     if (n) {
-      k_vertex_keys<<<grid, 256, 0, s>>>(g->d_off, n, vkeys);
-      if (cub::DeviceRadixSort::SortKeys(tmp, tb, dk, (int64_t)n, 0, 64, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-      k_perm<<<grid, 256, 0, s>>>(dk.Current(), n, g->d_off, g->d_oldid, g->d_newid, rdeg);
+      k_vertex_keys<<<grid, 256, 0, s>>>(g->d_off, n, (uint32_t)((1ull << dbits) - 1), vtmp, vtmp + 2 * vn);
+      if (cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dv, (int64_t)n, 0, dbits, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
+      k_perm<<<grid, 256, 0, s>>>(dv.Current(), n, g->d_off, g->d_oldid, g->d_newid, rdeg);
     }
     if (cudaMemsetAsync(rdeg + n, 0, sizeof(uint32_t), s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if (cub::DeviceScan::ExclusiveSum(tmp, tb, rdeg, g->d_roff, (int64_t)n + 1, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if (m) {
-      // 2. rows to their new places, keyed by the neighbours' new ids
-      k_row_scatter<256><<<(m + 255) / 256, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, n, m, g->d_newid,
-                                                         g->d_roff, key, val);
-      // 3. sort every row by key, with a kernel sized for its degree class
+      // 2. every row sorted by its neighbours' new ids, with a kernel sized for its degree class
+      const relabel_view view{g->d_off, g->d_dst, g->d_oldid, g->d_newid, g->d_roff, n, g->d_rdst, g->d_rmap};
       uint32_t hb[2 * RELABEL_NCLASS];
-      k_class_bounds<<<1, 32, 0, s>>>(rdeg, n, bounds);
-      if (cudaMemcpyAsync(hb, bounds, sizeof(uint32_t) * RELABEL_NCLASS, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      k_class_bounds<<<1, 32, 0, s>>>(rdeg, n, g->d_roff, bounds);
+      if (cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
           cudaStreamSynchronize(s) != cudaSuccess) {
         rc = ACCX_ERR_CUDA;
         break;
       }
-      for (int i = 0; i < RELABEL_NCLASS; i++)
-        if (cudaMemcpyAsync(hb + RELABEL_NCLASS + i, g->d_roff + hb[i], sizeof(uint32_t), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess) rc = ACCX_ERR_CUDA;
-      if (rc || cudaStreamSynchronize(s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
       const uint32_t *rb = hb, *pb = hb + RELABEL_NCLASS;  // class row bounds and their entry positions
       const int sms = accx_sm_count(g->device);
       // rows above 4096 entries: segmented radix sort (one CTA per row)
       if (rb[0] > 0) {
         size_t b3 = 0;
-        if (cub::DeviceSegmentedRadixSort::SortPairs(nullptr, b3, key, key, val, val, (int64_t)pb[0], (int64_t)rb[0],
+        uint32_t *none = nullptr;
+        if (cub::DeviceSegmentedRadixSort::SortPairs(nullptr, b3, none, none, none, none, (int64_t)pb[0], (int64_t)rb[0],
                                                      g->d_roff, g->d_roff + 1, 0, bits, s) != cudaSuccess) {
           rc = ACCX_ERR_CUDA;
           break;
         }
-        if (b3 > tb) {
-          if (cudaStreamSynchronize(s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-          accx_dev_free(tmp, g->home);
-          tmp = nullptr;
-          tb = b3;
-          if (accx_dev_alloc(&tmp, tb + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
-          if (g->home && cudaStreamSynchronize(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-        }
-        if (accx_dev_alloc((void **)&key2, sizeof(uint32_t) * ((size_t)pb[0] + 1), g->home) != cudaSuccess ||
-            accx_dev_alloc((void **)&val2, sizeof(uint32_t) * ((size_t)pb[0] + 1), g->home) != cudaSuccess) {
-          rc = ACCX_ERR_OOM;
-          break;
-        }
+        // keys and entries, sorted into a second pair; the scratch behind them
+        const size_t kn = ((size_t)pb[0] + 64) & ~(size_t)63;
+        if (accx_dev_alloc((void **)&key, sizeof(uint32_t) * 4 * kn + b3 + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
         if (g->home && cudaStreamSynchronize(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
-        if (cub::DeviceSegmentedRadixSort::SortPairs(tmp, tb, key, key2, val, val2, (int64_t)pb[0], (int64_t)rb[0],
+        uint32_t *val = key + kn, *key2 = key + 2 * kn, *val2 = key + 3 * kn;
+        k_big_rows<<<rb[0] < (uint32_t)sms * 2 ? rb[0] : sms * 2, 1024, 0, s>>>(view, rb[0], key, val);
+        if (cub::DeviceSegmentedRadixSort::SortPairs(key + 4 * kn, b3, key, key2, val, val2, (int64_t)pb[0], (int64_t)rb[0],
                                                      g->d_roff, g->d_roff + 1, 0, bits, s) != cudaSuccess) {
           rc = ACCX_ERR_CUDA;
           break;
         }
-        k_put_range<<<sms * 8, 256, 0, s>>>(key2, val2, 0u, pb[0], g->d_rdst, g->d_rmap);
+        k_put_big<<<sms * 8, 256, 0, s>>>(key2, val2, pb[0], g->d_rdst, g->d_rmap);
       }
       auto rows_grid = [&](uint32_t rows, int per_sm) { return (int)(rows < (uint32_t)(sms * per_sm) ? rows : sms * per_sm); };
-      if (rb[1] > rb[0])
-        k_row_sort<256, 16><<<rows_grid(rb[1] - rb[0], 8), 256, 0, s>>>(rb[0], rb[1], g->d_roff, key, val, bits,
-                                                                           g->d_rdst, g->d_rmap);
+      auto warps_grid = [&](uint32_t rows) { return rows_grid((rows + 7) / 8, 16); };
+      // words of (key, place) where both fit
+      auto fits = [&](int e) { return bits + relabel_place_bits(e) <= 32; };
+      if (rb[1] > rb[0]) k_row_sort<256, 16><<<rows_grid(rb[1] - rb[0], 8), 256, 0, s>>>(view, rb[0], rb[1], bits);
       if (rb[2] > rb[1])
-        k_row_sort<128, 8><<<rows_grid(rb[2] - rb[1], 16), 128, 0, s>>>(rb[1], rb[2], g->d_roff, key, val, bits,
-                                                                          g->d_rdst, g->d_rmap);
-      if (rb[3] > rb[2])
-        k_row_sort<64, 4><<<rows_grid(rb[3] - rb[2], 32), 64, 0, s>>>(rb[2], rb[3], g->d_roff, key, val, bits,
-                                                                        g->d_rdst, g->d_rmap);
+        k_row_sort<128, 8><<<rows_grid(rb[2] - rb[1], 16), 128, 0, s>>>(view, rb[1], rb[2], bits);
+      if (rb[3] > rb[2] && fits(16))
+        k_warp_row_sort<16, true><<<warps_grid(rb[3] - rb[2]), 256, 0, s>>>(view, rb[2], rb[3]);
+      else if (rb[3] > rb[2])
+        k_row_sort<128, 8><<<rows_grid(rb[3] - rb[2], 16), 128, 0, s>>>(view, rb[2], rb[3], bits);
       if (rb[4] > rb[3])
-        k_warp_row_sort<<<rows_grid((rb[4] - rb[3] + 7) / 8, 16), 256, 0, s>>>(rb[3], rb[4], g->d_roff, key, val,
-                                                                                g->d_rdst, g->d_rmap);
-      if (m > pb[4]) k_put_range<<<sms * 8, 256, 0, s>>>(key, val, pb[4], m, g->d_rdst, g->d_rmap);
+        (fits(8) ? k_warp_row_sort<8, true> : k_warp_row_sort<8, false>)<<<warps_grid(rb[4] - rb[3]), 256, 0, s>>>(view, rb[3], rb[4]);
+      if (rb[5] > rb[4])
+        (fits(4) ? k_warp_row_sort<4, true> : k_warp_row_sort<4, false>)<<<warps_grid(rb[5] - rb[4]), 256, 0, s>>>(view, rb[4], rb[5]);
+      if (rb[6] > rb[5])
+        (fits(2) ? k_warp_row_sort<2, true> : k_warp_row_sort<2, false>)<<<warps_grid(rb[6] - rb[5]), 256, 0, s>>>(view, rb[5], rb[6]);
+      if (rb[7] > rb[6])
+        (fits(1) ? k_warp_row_sort<1, true> : k_warp_row_sort<1, false>)<<<warps_grid(rb[7] - rb[6]), 256, 0, s>>>(view, rb[6], rb[7]);
+      if (m > pb[7]) k_put_single<<<sms * 8, 256, 0, s>>>(view, rb[7], n);
     }
     if (cudaMemsetAsync(g->d_rdst + m, 0xff, sizeof(int32_t) * ACCX_DST_PAD, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if ((rc = accx_tilerow_build(g, g->d_roff, &g->d_rtilerow, s)) != ACCX_OK) break;
-    // 4. the dense rows of oriented counts (the vertex keys are dead by now)
+    // 3. the dense rows of oriented counts
     float plan[(DENSE_KINDS + 1) * DENSE_BLOCKS];
-    const bool dense = m && n && sizeof(plan) <= sizeof(unsigned long long) * ((size_t)n + 1);
+    const bool dense = m && n;
     if (dense) {
       const uint32_t pb = (n + 1023u) / 1024u;
-      float *d_plan = reinterpret_cast<float *>(vkeys);
+      float *d_plan = reinterpret_cast<float *>(vtmp + 4 * vn);
       k_dense_plan<<<pb < DENSE_BLOCKS ? pb : DENSE_BLOCKS, 1024, 0, s>>>(g->d_roff, g->d_rdst, n, DENSE_COST, d_plan);
       if (cudaMemcpyAsync(plan, d_plan, sizeof(plan), cudaMemcpyDeviceToHost, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     }
@@ -383,9 +438,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
     cudaGetLastError();
     cudaStreamSynchronize(s);  // nothing of this call may still be running on the temporaries
   }
-  for (void *p : {(void *)vkeys, (void *)vkeys2, (void *)key, (void *)val, (void *)key2, (void *)val2, (void *)rdeg,
-                  (void *)bounds, tmp})
-    accx_dev_free(p, g->home);
+  for (void *p : {(void *)vtmp, (void *)rdeg, (void *)key, tmp}) accx_dev_free(p, g->home);
   if (!rc && g->d_rev_orig) {  // counts run on the relabeled CSR from now on
     accx_dev_free(g->d_rev_orig, g->home);
     g->d_rev_orig = nullptr;

@@ -218,8 +218,8 @@ int accx_grid_for(int device, int block, int per_sm) {
 // bijection onto the other half: the graph is symmetric.
 // Symmetry fingerprints: two published 64-bit finalisers (SplitMix64's, and
 // MurmurHash3's fmix64 applied to the key plus an odd constant) of the key
-// (a << 32 | b).  Over all entries, sum of f(u,v) - f(v,u) is zero (mod 2^64) on
-// a symmetric graph.
+// (smaller id << 32 | larger id) of an entry (u,v), added for u < v and subtracted for
+// u > v: zero (mod 2^64) over all entries of a symmetric graph.
 __device__ __forceinline__ unsigned long long fp_splitmix(unsigned long long z) {
   z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
   z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
@@ -235,12 +235,76 @@ __device__ __forceinline__ unsigned long long fp_fmix(unsigned long long k) {
 }
 #define FP_SLOTS 64  // fingerprint accumulators (CTAs spread their atomics over them)
 
+// The checks and the fingerprints of a full validation: a thread takes eight consecutive
+// entries, with one row search inside their 256-entry tile, and keeps the sums in
+// registers to the end (one entry a thread, with a CTA reduction for every 256 entries,
+// took 501 us for 64M entries; now 259).  Bound by the finalisers' 64-bit multiplications.
+__global__ void __launch_bounds__(256) k_validate_fp(const uint32_t *__restrict__ off,
+                                                     const uint32_t *__restrict__ tilerow,
+                                                     const int32_t *__restrict__ dst, uint32_t n, uint32_t m,
+                                                     int *__restrict__ status, unsigned long long *__restrict__ fp) {
+  __shared__ unsigned long long s_fp[2][8];
+  const uint32_t nb = m / 8 + (m % 8 ? 1 : 0);
+  unsigned long long d1 = 0, d2 = 0;
+  int flag = 0;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nb; c += gridDim.x * blockDim.x) {
+    const uint32_t e0 = c * 8, k = min(m - e0, 8u), t = e0 / 256u;
+    int32_t v[8];
+    if (k == 8) {
+      const int4 a = __ldg(reinterpret_cast<const int4 *>(dst + e0)), b = __ldg(reinterpret_cast<const int4 *>(dst + e0) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] = (uint32_t)i < k ? __ldg(dst + e0 + i) : 0;
+    }
+    int32_t prev = e0 ? __ldg(dst + e0 - 1) : -1;
+    uint32_t u = accx_row_of(off, __ldg(tilerow + t), __ldg(tilerow + t + 1) + 1, e0);
+    uint32_t rb = __ldg(off + u), re = __ldg(off + u + 1);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      if ((uint32_t)i >= k) break;
+      while (re <= e0 + i) {  // the next non-empty row
+        u++;
+        rb = re;
+        re = __ldg(off + u + 1);
+      }
+      if (v[i] < 0 || (uint32_t)v[i] >= n) flag |= V_RANGE;
+      else if ((uint32_t)v[i] == u) flag |= V_SELF;
+      else if (e0 + i > rb && prev >= v[i]) flag |= V_UNSORTED;
+      else {
+        // the pair's key, smaller id first, counted up from one side and down from the other
+        const uint32_t w = (uint32_t)v[i];
+        const unsigned long long a = ((unsigned long long)min(u, w) << 32) | max(u, w);
+        const unsigned long long f1 = fp_splitmix(a), f2 = fp_fmix(a);
+        d1 += u < w ? f1 : 0ull - f1;
+        d2 += u < w ? f2 : 0ull - f2;
+      }
+      prev = v[i];
+    }
+  }
+  if (flag) atomicOr(status, flag);
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) {
+    d1 += __shfl_xor_sync(ACCX_FULL_MASK, d1, d);
+    d2 += __shfl_xor_sync(ACCX_FULL_MASK, d2, d);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_fp[0][threadIdx.x >> 5] = d1;
+    s_fp[1][threadIdx.x >> 5] = d2;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long t = 0;
+    for (int w = 0; w < 8; w++) t += s_fp[threadIdx.x][w];
+    if (t) atomicAdd(&fp[threadIdx.x * FP_SLOTS + blockIdx.x % FP_SLOTS], t);  // wraps mod 2^64
+  }
+}
+
 template <bool SEARCH>
 __global__ void k_validate(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow, const int32_t *__restrict__ dst, uint32_t n,
                            uint32_t m, int full, int *__restrict__ status, unsigned long long *__restrict__ searched,
-                           uint32_t *__restrict__ rev, unsigned long long *__restrict__ fp) {
+                           uint32_t *__restrict__ rev) {
   __shared__ accx_tile_rows<256> sh;
-  __shared__ unsigned long long s_fp[2][8];
   uint32_t base = blockIdx.x * 256u;
   uint32_t e = base + threadIdx.x;
   uint32_t u = accx_tile_row<256>(off, tilerow, n, m, base, e, &sh);
@@ -274,30 +338,6 @@ __global__ void k_validate(const uint32_t *__restrict__ off, const uint32_t *__r
   if (SEARCH && full) {  // uniform over the block
     const int c = __syncthreads_count(chk);
     if (threadIdx.x == 0 && c) atomicAdd(searched, (unsigned long long)c);
-  }
-  if (fp) {  // uniform over the grid: the fingerprints of this block's entries
-    unsigned long long d1 = 0, d2 = 0;
-    if (e < m && !flag) {
-      const unsigned long long v = (uint32_t)dst[e];
-      const unsigned long long a = ((unsigned long long)u << 32) | v, b = (v << 32) | u;
-      d1 = fp_splitmix(a) - fp_splitmix(b);
-      d2 = fp_fmix(a) - fp_fmix(b);
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-      d1 += __shfl_xor_sync(ACCX_FULL_MASK, d1, d);
-      d2 += __shfl_xor_sync(ACCX_FULL_MASK, d2, d);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      s_fp[0][threadIdx.x >> 5] = d1;
-      s_fp[1][threadIdx.x >> 5] = d2;
-    }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-      unsigned long long t = 0;
-      for (int w = 0; w < 8; w++) t += s_fp[threadIdx.x][w];
-      if (t) atomicAdd(&fp[threadIdx.x * FP_SLOTS + blockIdx.x % FP_SLOTS], t);  // wraps mod 2^64
-    }
   }
 }
 
@@ -446,8 +486,12 @@ int accx_graph_validate_device(accx_graph *g, int full, int exact, cudaStream_t 
     }
     const uint32_t blocks = (uint32_t)((g->m + 255) / 256);
     const bool fingerprints = full && !exact;
-    k_validate<false><<<blocks, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->n, (uint32_t)g->m, full, d_status,
-                                             nullptr, nullptr, fingerprints ? d_fp : nullptr);
+    if (fingerprints)
+      k_validate_fp<<<accx_grid_for(g->device, 256, 8), 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->n, (uint32_t)g->m,
+                                                                    d_status, d_fp);
+    else
+      k_validate<false><<<blocks, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->n, (uint32_t)g->m, full, d_status,
+                                               nullptr, nullptr);
     unsigned long long fp[2 * FP_SLOTS];
     if (cudaMemcpyAsync(&st, d_status, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         (fingerprints && cudaMemcpyAsync(fp, d_fp, sizeof(fp), cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
@@ -472,7 +516,7 @@ int accx_graph_validate_device(accx_graph *g, int full, int exact, cudaStream_t 
           rev = nullptr;  // no room: counts build the index themselves
         }
         k_validate<true><<<blocks, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->n, (uint32_t)g->m, full, d_status,
-                                                d_searched, rev, nullptr);
+                                                d_searched, rev);
         unsigned long long searched = 0;
         if (cudaMemcpyAsync(&st, d_status, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaMemcpyAsync(&searched, d_searched, sizeof(searched), cudaMemcpyDeviceToHost, s) != cudaSuccess ||

@@ -61,8 +61,9 @@ typedef struct accx_graph accx_graph;
 /* Flags for accx_graph_create. */
 #define ACCX_GRAPH_VALIDATE 1u       /* check self loops, order, range, symmetry on the GPU */
 /* With ACCX_GRAPH_VALIDATE, how symmetry is checked.  By default in the same pass
- * as the other checks, by two 64-bit multiset fingerprints (the sums over all
- * entries (u,v) of two mixing functions of (u,v), against the same sums of (v,u));
+ * as the other checks, by two 64-bit multiset fingerprints (the sums of two
+ * mixing functions of the pair {u,v} over the entries with u < v, against the same
+ * sums over those with u > v);
  * rows are already checked strictly increasing, so an asymmetric graph passes
  * only if both 64-bit sums collide.  ACCX_GRAPH_VALIDATE_EXACT instead sorts the
  * entries by neighbour id (about 16 bytes per entry of scratch, several times the

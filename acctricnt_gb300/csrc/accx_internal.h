@@ -119,10 +119,13 @@ struct accx_graph {
 
 void accx_set_cuda_error(cudaError_t e, const char *what, const char *file, int line);
 
-// Device memory on a stream's pool when s != NULL (no device-wide synchronisation
-// on free), else plain cudaMalloc/cudaFree.
+// Device memory from the device's pool, ordered on s (the legacy stream when NULL).
+// accx_dev_wait(s) before any other stream uses it.  Freed on s; without a stream after a
+// device-wide synchronisation.
 cudaError_t accx_dev_alloc(void **p, size_t bytes, cudaStream_t s);
+cudaError_t accx_dev_wait(cudaStream_t s);
 void accx_dev_free(void *p, cudaStream_t s);
+void accx_dev_free_all(void *const *p, int k, cudaStream_t s);
 
 // True when p is a device (or managed) pointer.
 bool accx_is_device_ptr(const void *p);

@@ -92,6 +92,7 @@ extern "C" int accx_batch_create(accx_graph *const *graphs, int k, void *stream,
     if (accx_dev_alloc((void **)&u->d_off, sizeof(uint32_t) * (N + 1), nullptr) != cudaSuccess ||
         accx_dev_alloc((void **)&u->d_dst, sizeof(int32_t) * (M + ACCX_DST_PAD), nullptr) != cudaSuccess ||
         cudaMalloc(&d_ds, sizeof(accx_batch_desc) * k) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+    if (accx_dev_wait(nullptr) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if (cudaMemcpyAsync(d_ds, ds.data(), sizeof(accx_batch_desc) * k, cudaMemcpyHostToDevice, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     uint32_t last = (uint32_t)M;
     if (cudaMemcpyAsync(u->d_off + N, &last, sizeof(uint32_t), cudaMemcpyHostToDevice, s) != cudaSuccess ||

@@ -761,7 +761,7 @@ int accx_ensure_count_scratch(accx_graph *g) {
   if (!g->d_table) {
     ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_table, ACCX_NB * ACCX_NB, h));
     // pool allocations are ordered on the home stream; counts may run on another
-    if (h) ACCX_CUDA_TRY(cudaStreamSynchronize(h));
+    ACCX_CUDA_TRY(accx_dev_wait(h));
   }
   return ACCX_OK;
 }
@@ -808,7 +808,7 @@ static bool alloc_dense(accx_graph *g) {
   bool ok = accx_dev_alloc((void **)&g->d_dense_t, tb, g->home) == cudaSuccess &&
             accx_dev_alloc((void **)&g->d_dense_low, sizeof(uint32_t) * ((size_t)g->dense_m + 4), g->home) == cudaSuccess &&
             accx_dev_alloc((void **)&g->d_dense_items, sizeof(uint4) * (size_t)dense_cap(g), g->home) == cudaSuccess;
-  if (ok && g->home) ok = cudaStreamSynchronize(g->home) == cudaSuccess;
+  if (ok) ok = accx_dev_wait(g->home) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     for (void **p : {(void **)&g->d_dense_t, (void **)&g->d_dense_low, (void **)&g->d_dense_items}) {
@@ -825,7 +825,7 @@ static bool alloc_dense(accx_graph *g) {
 static bool alloc_degree(accx_graph *g) {
   const size_t words = 2 * (size_t)g->m + 3 * (size_t)g->n + 2 + 2 * ((size_t)g->m / DG_ROW_SMALL + (size_t)g->m / DG_SLICE + 2);
   bool ok = accx_dev_alloc((void **)&g->d_dg, sizeof(uint32_t) * words, g->home) == cudaSuccess;
-  if (ok && g->home) ok = cudaStreamSynchronize(g->home) == cudaSuccess;
+  if (ok) ok = accx_dev_wait(g->home) == cudaSuccess;
   if (!ok) cudaGetLastError();
   return ok;
 }
@@ -966,7 +966,7 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
       if (!g->d_vinfo) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_vinfo, sizeof(uint2) * (size_t)n, g->home));
       if (!g->d_or_items)
         ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_or_items, sizeof(uint32_t) * (size_t)items_cap, g->home));
-      if (g->home) ACCX_CUDA_TRY(cudaStreamSynchronize(g->home));
+      ACCX_CUDA_TRY(accx_dev_wait(g->home));
     }
     // prefix lengths: an index of the counting CSR, built on its first oriented count
     if (g->pre_csr != off) {
@@ -992,7 +992,7 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
         } else if (rc == ACCX_ERR_OOM) {
           if (!g->d_rev) {
             ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_rev, sizeof(uint32_t) * (size_t)m, g->home));
-            if (g->home) ACCX_CUDA_TRY(cudaStreamSynchronize(g->home));
+            ACCX_CUDA_TRY(accx_dev_wait(g->home));
           }
           ACCX_CUDA_TRY(cudaMemsetAsync(g->d_rev, 0xff, sizeof(uint32_t) * (size_t)m, s));
           k_rev_build<256><<<tiles, 256, 0, s>>>(off, tilerow, dst, g->d_pre, n, m, g->d_rev);

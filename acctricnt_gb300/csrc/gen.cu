@@ -88,6 +88,7 @@ static int build_csr(accx_graph *g, K *d_keys, uint64_t nkeys, uint32_t n, const
     g->m = nu;
     if (accx_dev_alloc((void **)&g->d_off, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
         accx_dev_alloc((void **)&g->d_dst, sizeof(int32_t) * ((size_t)nu + ACCX_DST_PAD), g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+    if (g->home != s && accx_dev_wait(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if (cudaMemsetAsync(g->d_dst + nu, 0xff, sizeof(int32_t) * ACCX_DST_PAD, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     int grid = accx_grid_for(g->device, 256, 8);
     k_keys_to_csr<<<grid, 256, 0, s>>>(uniq, nu, n, b, g->d_off, g->d_dst);

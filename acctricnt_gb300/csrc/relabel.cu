@@ -356,7 +356,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
     }
     tb = b1 > b2 ? b1 : b2;
     if (accx_dev_alloc(&tmp, tb + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
-    if (g->home && cudaStreamSynchronize(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
+    if (accx_dev_wait(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     // 1. vertex order: degree descending, ties by id
     if (n) {
       k_vertex_keys<<<grid, 256, 0, s>>>(g->d_off, n, (uint32_t)((1ull << dbits) - 1), vtmp, vtmp + 2 * vn);
@@ -389,7 +389,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
         // keys and entries, sorted into a second pair; the scratch behind them
         const size_t kn = ((size_t)pb[0] + 64) & ~(size_t)63;
         if (accx_dev_alloc((void **)&key, sizeof(uint32_t) * 4 * kn + b3 + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
-        if (g->home && cudaStreamSynchronize(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
+        if (accx_dev_wait(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
         uint32_t *val = key + kn, *key2 = key + 2 * kn, *val2 = key + 3 * kn;
         k_big_rows<<<rb[0] < (uint32_t)sms * 2 ? rb[0] : sms * 2, 1024, 0, s>>>(view, rb[0], key, val);
         if (cub::DeviceSegmentedRadixSort::SortPairs(key + 4 * kn, b3, key, key2, val, val2, (int64_t)pb[0], (int64_t)rb[0],
@@ -438,7 +438,8 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
     cudaGetLastError();
     cudaStreamSynchronize(s);  // nothing of this call may still be running on the temporaries
   }
-  for (void *p : {(void *)vtmp, (void *)rdeg, (void *)key, tmp}) accx_dev_free(p, g->home);
+  void *temps[] = {vtmp, rdeg, key, tmp};
+  accx_dev_free_all(temps, 4, g->home);
   if (!rc && g->d_rev_orig) {  // counts run on the relabeled CSR from now on
     accx_dev_free(g->d_rev_orig, g->home);
     g->d_rev_orig = nullptr;

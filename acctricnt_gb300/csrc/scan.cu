@@ -476,8 +476,7 @@ __global__ void __launch_bounds__(TILE) k_pairs(const uint32_t *__restrict__ off
 void accx_query_ctx_release(accx_query_ctx *q) {
   void *ptrs[] = {q->d_simbits, q->d_corelist,  q->d_label, q->d_parent,    q->d_hubmin,   q->d_hubmax,
                   q->d_push,    q->d_qcounters, q->d_pairs, q->d_pairs_tmp, q->d_corebits, q->d_big};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  accx_dev_free_all(ptrs, (int)(sizeof(ptrs) / sizeof(ptrs[0])), nullptr);
   *q = accx_query_ctx();
 }
 
@@ -485,18 +484,20 @@ static int ensure_query_arrays(const accx_graph *g, accx_query_ctx *q) {
   if (q->d_simbits && (q->n != g->n || q->m != g->m)) return ACCX_ERR_INVALID_ARG;  // made for another graph
   q->n = g->n;
   q->m = g->m;
+  if (q->d_big) return ACCX_OK;  // the last of them
   const size_t n = g->n ? g->n : 1, words = (g->m + 31) / 32 + 1;
-  if (!q->d_simbits) ACCX_CUDA_TRY(cudaMalloc(&q->d_simbits, sizeof(uint32_t) * words));
-  if (!q->d_corelist) ACCX_CUDA_TRY(cudaMalloc(&q->d_corelist, sizeof(uint32_t) * n));
+  if (!q->d_simbits) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_simbits, sizeof(uint32_t) * words, nullptr));
+  if (!q->d_corelist) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_corelist, sizeof(uint32_t) * n, nullptr));
   // rows above PUSH_ROW have at most 1 + degree/PUSH_SLICE slices
-  if (!q->d_push) ACCX_CUDA_TRY(cudaMalloc(&q->d_push, sizeof(uint2) * (g->m / PUSH_ROW + g->m / PUSH_SLICE + 2)));
-  if (!q->d_label) ACCX_CUDA_TRY(cudaMalloc(&q->d_label, sizeof(int32_t) * n));
-  if (!q->d_parent) ACCX_CUDA_TRY(cudaMalloc(&q->d_parent, sizeof(int32_t) * n));
-  if (!q->d_hubmin) ACCX_CUDA_TRY(cudaMalloc(&q->d_hubmin, sizeof(int32_t) * n));
-  if (!q->d_hubmax) ACCX_CUDA_TRY(cudaMalloc(&q->d_hubmax, sizeof(int32_t) * n));
-  if (!q->d_qcounters) ACCX_CUDA_TRY(cudaMalloc(&q->d_qcounters, sizeof(unsigned long long) * Q_NUM));
-  if (!q->d_corebits) ACCX_CUDA_TRY(cudaMalloc(&q->d_corebits, sizeof(uint32_t) * (n / 32 + 2)));
-  if (!q->d_big) ACCX_CUDA_TRY(cudaMalloc(&q->d_big, sizeof(uint32_t) * (g->m / BIG_ROW + 2)));
+  if (!q->d_push) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_push, sizeof(uint2) * (g->m / PUSH_ROW + g->m / PUSH_SLICE + 2), nullptr));
+  if (!q->d_label) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_label, sizeof(int32_t) * n, nullptr));
+  if (!q->d_parent) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_parent, sizeof(int32_t) * n, nullptr));
+  if (!q->d_hubmin) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_hubmin, sizeof(int32_t) * n, nullptr));
+  if (!q->d_hubmax) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_hubmax, sizeof(int32_t) * n, nullptr));
+  if (!q->d_qcounters) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_qcounters, sizeof(unsigned long long) * Q_NUM, nullptr));
+  if (!q->d_corebits) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_corebits, sizeof(uint32_t) * (n / 32 + 2), nullptr));
+  if (!q->d_big) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_big, sizeof(uint32_t) * (g->m / BIG_ROW + 2), nullptr));
+  ACCX_CUDA_TRY(accx_dev_wait(nullptr));
   return ACCX_OK;
 }
 
@@ -522,7 +523,7 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
       if (!gm->d_simkey) {
         ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_simkey, sizeof(float) * (size_t)m, g->home));
         ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_src, sizeof(uint32_t) * (size_t)m, g->home));
-        if (g->home) ACCX_CUDA_TRY(cudaStreamSynchronize(g->home));
+        ACCX_CUDA_TRY(accx_dev_wait(g->home));
       }
       k_simkey<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->d_cnt, m, g->cnt_bias, gm->d_simkey,
                                        gm->d_src);
@@ -575,7 +576,7 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
   if (sim_tmp) {
     cudaError_t e1 = cudaMemcpyAsync(sim, sim_tmp, m, cudaMemcpyDeviceToHost, s);
     cudaError_t e2 = cudaStreamSynchronize(s);
-    accx_dev_free(sim_tmp, s);
+    cudaFreeAsync(sim_tmp, s);
     if (e1 != cudaSuccess || e2 != cudaSuccess) return ACCX_ERR_CUDA;
   }
   if (label) {
@@ -638,12 +639,13 @@ static int build_pairs(accx_graph *g, accx_query_ctx *q, cudaStream_t s) {
   ACCX_CUDA_TRY(cudaMemcpyAsync(&h, q->d_qcounters + Q_PAIRS, sizeof(h), cudaMemcpyDeviceToHost, s));
   ACCX_CUDA_TRY(cudaStreamSynchronize(s));
   if (h > q->pairs_cap) {
-    if (q->d_pairs) cudaFree(q->d_pairs);
-    if (q->d_pairs_tmp) cudaFree(q->d_pairs_tmp);
+    accx_dev_free(q->d_pairs, nullptr);
+    accx_dev_free(q->d_pairs_tmp, nullptr);
     q->d_pairs = q->d_pairs_tmp = nullptr;
     q->pairs_cap = 0;
-    ACCX_CUDA_TRY(cudaMalloc(&q->d_pairs, sizeof(unsigned long long) * h));
-    ACCX_CUDA_TRY(cudaMalloc(&q->d_pairs_tmp, sizeof(unsigned long long) * h));
+    ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_pairs, sizeof(unsigned long long) * h, nullptr));
+    ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_pairs_tmp, sizeof(unsigned long long) * h, nullptr));
+    ACCX_CUDA_TRY(accx_dev_wait(nullptr));
     q->pairs_cap = h;
   }
   q->npairs = 0;
@@ -657,7 +659,7 @@ static int build_pairs(accx_graph *g, accx_query_ctx *q, cudaStream_t s) {
     ACCX_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (int64_t)h, 0, 64, s));
     ACCX_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, tb2, q->d_pairs, q->d_pairs_tmp, d_nsel, (int64_t)h, s));
     void *tmp = nullptr;
-    ACCX_CUDA_TRY(cudaMalloc(&tmp, std::max(tb, tb2) + 64));
+    ACCX_CUDA_TRY(accx_dev_alloc(&tmp, std::max(tb, tb2) + 64, s));
     d_nsel = reinterpret_cast<unsigned long long *>(static_cast<char *>(tmp) + ((std::max(tb, tb2) + 15) & ~size_t(15)));
     cudaError_t e1 = cub::DeviceRadixSort::SortKeys(tmp, tb, db, (int64_t)h, 0, 64, s);
     unsigned long long *sorted = db.Current(), *other = db.Alternate();
@@ -665,7 +667,7 @@ static int build_pairs(accx_graph *g, accx_query_ctx *q, cudaStream_t s) {
     unsigned long long nu = 0;
     cudaError_t e3 = cudaMemcpyAsync(&nu, d_nsel, sizeof(nu), cudaMemcpyDeviceToHost, s);
     cudaError_t e4 = cudaStreamSynchronize(s);
-    cudaFree(tmp);
+    cudaFreeAsync(tmp, s);
     if (e1 || e2 || e3 || e4) return ACCX_ERR_CUDA;
     if (other != q->d_pairs) std::swap(q->d_pairs, q->d_pairs_tmp);  // unique result lives in d_pairs
     q->npairs = nu;
@@ -696,13 +698,13 @@ extern "C" int accx_scan_pairs(accx_graph *g, int32_t *pairs, uint64_t cap, uint
   if (!q->npairs) return ACCX_OK;
   int32_t *tmp = nullptr;
   bool dev = accx_is_device_ptr(pairs);
-  if (dev) tmp = pairs; else ACCX_CUDA_TRY(cudaMalloc(&tmp, sizeof(int32_t) * 2 * q->npairs));
+  if (dev) tmp = pairs; else ACCX_CUDA_TRY(accx_dev_alloc((void **)&tmp, sizeof(int32_t) * 2 * q->npairs, s));
   k_keys_to_pairs<<<accx_sm_count(g->device) * 8, 256, 0, s>>>(q->d_pairs, q->npairs, tmp);
   ACCX_CUDA_TRY(cudaGetLastError());
   if (!dev) {
     cudaError_t e1 = cudaMemcpyAsync(pairs, tmp, sizeof(int32_t) * 2 * q->npairs, cudaMemcpyDeviceToHost, s);
     cudaError_t e2 = cudaStreamSynchronize(s);
-    cudaFree(tmp);
+    cudaFreeAsync(tmp, s);
     if (e1 || e2) return ACCX_ERR_CUDA;
   }
   return ACCX_OK;

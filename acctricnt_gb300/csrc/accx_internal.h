@@ -84,7 +84,7 @@ struct accx_graph {
   // dense rows of the relabeled CSR (planned by the relabel; 0 rows: none worth it)
   uint32_t dense_k = 0, dense_m = 0;       // hub ids (bits a row) and rows
   uint32_t plan_rows = 0, plan_maxpre = 0; // rows the relabel's plan looked at, and their longest prefix
-  uint32_t dense_built = 0;                // rows the arrays below were built for
+  bool dense_built = false;                // the arrays below hold the counting CSR's rows
   uint32_t *d_dense_t = nullptr;           // dense_m x dense_k bits
   uint32_t *d_dense_low = nullptr;         // dense_m: set bits of each row
   uint4 *d_dense_items = nullptr;          // (row, first entry, entries) pieces of the rows

@@ -803,6 +803,14 @@ static uint32_t dense_cap(const accx_graph *g) { return g->dense_m + (uint32_t)(
 static unsigned long long *dense_ctr(const accx_graph *g) {
   return reinterpret_cast<unsigned long long *>(g->d_dense_low + ((g->dense_m + 1u) & ~1u));
 }
+// Whether s is being captured in a CUDA graph: an index built there would exist only
+// after a replay, and nothing can be allocated.
+static bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (s && cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  if (s) cudaGetLastError();
+  return false;
+}
 static bool alloc_dense(accx_graph *g) {
   const size_t tb = (size_t)g->dense_m * (g->dense_k / 8u);
   bool ok = accx_dev_alloc((void **)&g->d_dense_t, tb, g->home) == cudaSuccess &&
@@ -894,10 +902,11 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   unsigned long long *ctr = g->d_counters;
   unsigned long long *work_u = g->d_counters + C_NUM;
   // the default policy on a CSR known to be symmetric (degree.cuh): ids in the warps'
-  // tables have 24 bits; without that, or without room, an intersection per edge
+  // tables have 24 bits; without that, or without room (or a way to ask for it, in a
+  // capture), an intersection per edge
   bool degree = !orient && policy == ACCX_POLICY_HEURISTIC && g->symmetric && n <= OW_MAX_N && m;
   const bool small = degree && m <= DG_SMALL_M;
-  if (degree && !small && !g->d_dg && !alloc_degree(g)) degree = false;
+  if (degree && !small && !g->d_dg && (is_capturing(s) || !alloc_degree(g))) degree = false;
   // which kinds can occur; oriented bitmap owners lie below the dense window, so only
   // their part of work_u is used
   const bool any = policy == ACCX_POLICY_TABLE || policy == ACCX_POLICY_MODEL;
@@ -961,6 +970,10 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     // per-entry bitmap work and the item array (n + m/32 + 1 bounds the items:
     // an owner is cut into at most max(1, degree/32) slices)
     const uint32_t items_cap = n + m / 32u + 1u;
+    if ((g->pre_csr != off || g->rev_csr != off) && is_capturing(s)) {  // the CSR's first oriented count
+      accx_set_cuda_error(cudaErrorStreamCaptureUnsupported, "indices of the counting CSR", __FILE__, __LINE__);
+      return ACCX_ERR_CUDA;
+    }
     if (!g->d_or_sl || !g->d_or_items || !g->d_vinfo) {
       if (!g->d_or_sl) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_or_sl, sizeof(uint2) * (size_t)m, g->home));
       if (!g->d_vinfo) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_vinfo, sizeof(uint2) * (size_t)n, g->home));
@@ -1002,17 +1015,19 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
       }
       g->rev_csr = off;
     }
-    // dense rows, where the relabel planned some and bitmap-kind edges can occur
+    // dense rows, where the relabel planned some and bitmap-kind edges can occur.  They are
+    // built once, so that a captured count finds the ones it was recorded with whatever
+    // other windows were counted since; a window below them probes every id.
     const uint32_t wpl = g->dense_k / 1024u;
-    uint32_t dm = rel && can_bitmap ? (g->dense_m < W ? g->dense_m : W) : 0u;
+    uint32_t dm = rel && can_bitmap && g->dense_m <= W ? g->dense_m : 0u;
     const uint32_t dchunk = dense_chunk(g), dcap = dense_cap(g);
-    if (dm && !g->d_dense_t && !alloc_dense(g)) dm = 0;  // no room: every id is probed
-    if (dm && g->dense_built != dm) {  // an index of the relabeled CSR, for this many rows
+    if (dm && !g->dense_built && (is_capturing(s) || (!g->d_dense_t && !alloc_dense(g)))) dm = 0;  // no room, or not now
+    if (dm && !g->dense_built) {
       auto kr = wpl == 4 ? k_dense_rows<4> : wpl == 2 ? k_dense_rows<2> : k_dense_rows<1>;
       ACCX_CUDA_TRY(cudaMemsetAsync(dense_ctr(g), 0, sizeof(unsigned long long), s));
       kr<<<sms * 8, 256, 0, s>>>(off, dst, g->d_pre, dm, dchunk, g->d_dense_t, g->d_dense_low, g->d_dense_items, dcap,
                                  dense_ctr(g));
-      g->dense_built = dm;
+      g->dense_built = true;
     }
     k_classify<true><<<classify_grid(sms, m), 256, 0, s>>>(off, tilerow, dst, n, m, policy, g->d_table, g->d_edge_list,
                                                           list_cap, work_u, ctr, g->d_pre, W, pcap, g->d_or_sl, g->d_rev,

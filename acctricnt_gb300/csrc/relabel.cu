@@ -286,13 +286,14 @@ __global__ void __launch_bounds__(1024) k_dense_plan(const uint32_t *__restrict_
 // gained, at most 64 MiB of bits (half of L2), and only if that spares more than the
 // two extra launches (DENSE_MIN probes).
 #define DENSE_MIN 4e6f
+#define DENSE_ROWS_MAX 192u  // blocks of 1024 ids in the default bitmap window
 static void dense_choose(accx_graph *g, const float *out) {
   const uint32_t blocks = (g->n + 1023u) / 1024u < DENSE_BLOCKS ? (g->n + 1023u) / 1024u : DENSE_BLOCKS;
   float best = DENSE_MIN;
   for (uint32_t k = 0; k < DENSE_KINDS; k++) {
     const uint32_t K = 1024u << k, lim = (64u << 20) / (K / 8u) / 1024u;
     float acc = 0.f;
-    for (uint32_t i = 0; i < blocks && i < lim; i++) {
+    for (uint32_t i = 0; i < blocks && i < lim && i < DENSE_ROWS_MAX; i++) {
       acc += out[k * DENSE_BLOCKS + i];
       if (acc > best) {
         best = acc;

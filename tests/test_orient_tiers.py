@@ -146,3 +146,40 @@ def test_gallop_skewed(p):
     G = accx.Graph.from_csr(off, dst)
     G.relabel()
     assert np.array_equal(G.count(policy="gallop", bias=2, orient=True), ref)
+
+
+def test_captured_counts_keep_their_indices():
+    """A captured count replays with the dense rows it was recorded with whatever windows
+    were counted in between; a first oriented count is refused in a capture, and a
+    default count that has no room for its lists there falls back."""
+    import torch
+    G = accx.Graph.generate(accx.rmat_params(16, 32, seed=16))
+    B = accx.Batch([G])
+    U = B.union
+    U.relabel()
+    want = U.count(policy="merge", bias=2, orient=True)
+    s = torch.cuda.Stream()
+    B.capture(policy="bitmap", bias=2, stream=s.cuda_stream, orient=True)
+    for kb in (1, 2, 24):
+        assert np.array_equal(U.count(policy="bitmap", bias=2, orient=True, window_kb=kb), want)
+        U.count(policy="merge", bias=7, out=None)
+        torch.cuda.synchronize()
+        B.launch(stream=s.cuda_stream)
+        s.synchronize()
+        assert np.array_equal(U.read_counts(), want)
+    for first in ({"policy": "bitmap"}, {"policy": "gallop", "orient": True}):
+        H = accx.Graph.generate(accx.rmat_params(16, 32, seed=16))
+        off, dst = H.download()
+        H = accx.Graph.from_csr(off, dst)
+        H.count(bias=2, **first)
+        torch.cuda.synchronize()
+        cg = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(cg, stream=s):
+            if "orient" not in first:
+                with pytest.raises(accx.AccxError):
+                    H.count(policy="bitmap", bias=2, orient=True, out=None, stream=s.cuda_stream)
+            H.count(bias=2, out=None, stream=s.cuda_stream)
+        cg.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(H.read_counts(), want)
+        assert np.array_equal(H.count(policy="bitmap", bias=2, orient=True), want)

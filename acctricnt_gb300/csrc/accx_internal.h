@@ -78,7 +78,7 @@ struct accx_graph {
   uint2 *d_vinfo = nullptr;                // n (offset, prefix length) of the counting CSR, oriented counts
   uint2 *d_or_sl = nullptr;                // m oriented bitmap entries: (partner prefix start, cut length), 0 length = not bitmap
   uint32_t *d_or_items = nullptr;          // n + m/32 + 1 oriented bitmap work items: owner of each
-  uint32_t *d_rev = nullptr;               // m reverse entry of every entry of the counting CSR (oriented counts)
+  uint32_t *d_rev = nullptr;               // m reverse entry of (at least) every suffix entry of the counting CSR (oriented counts)
   uint32_t *d_rev_orig = nullptr;          // m reverse entries of the handle's own CSR, recorded by full validation
   uint32_t *d_dg = nullptr;                // the default policy's degree-ordered count
   // dense rows of the relabeled CSR (planned by the relabel; 0 rows: none worth it)
@@ -158,9 +158,12 @@ int accx_model_plan_ms(accx_model *m, accx_graph *g, int mode, cudaStream_t s, d
 // Row index of every 256-entry tile of a CSR (graph.cu), allocated on g's home stream.
 int accx_tilerow_build(accx_graph *g, const uint32_t *off, uint32_t **out, cudaStream_t s);
 // Reverse index of g's CSR (off, tilerow, dst) by a stable sort of the entries
-// by neighbour id; with d_status the symmetry it relies on is checked (graph.cu).
+// by neighbour id; the symmetry it relies on is checked (graph.cu).
 int accx_rev_by_sort(accx_graph *g, const uint32_t *off, const uint32_t *tilerow, const int32_t *dst, int *d_status,
                      cudaStream_t s, uint32_t **rev_out);
+// The same for the suffix entries of a CSR known to be symmetric, with prefix lengths pre.
+int accx_rev_suffix(accx_graph *g, const uint32_t *off, const uint32_t *tilerow, const int32_t *dst, const uint32_t *pre,
+                    cudaStream_t s, uint32_t **rev_out);
 
 // Relabeled counts -> the handle's entry order (relabel.cu).
 int accx_relabel_gather(accx_graph *g, int32_t *out, cudaStream_t s);

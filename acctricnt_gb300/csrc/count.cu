@@ -988,8 +988,8 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     }
     // reverse entries: built on the first oriented count of this CSR and kept
     // (an index of the graph, like the tile rows).  The original CSR's comes
-    // from validation; a known-symmetric CSR's from the sort (accx_rev_by_sort);
-    // otherwise, or when the sort's scratch does not fit, a search per entry
+    // from validation; a known-symmetric CSR's suffix entries' from a sort
+    // (accx_rev_suffix); otherwise, or when the sort's scratch does not fit, a search per entry
     // pair, which leaves 0xffffffff where an asymmetric CSR has no reverse.
     if (g->rev_csr != off) {
       uint32_t *sorted = nullptr;
@@ -998,7 +998,7 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
         accx_dev_free(g->d_rev_orig, g->home);
         g->d_rev_orig = nullptr;
       } else {
-        rc = g->symmetric ? accx_rev_by_sort(g, off, tilerow, dst, nullptr, s, &sorted) : ACCX_ERR_OOM;
+        rc = g->symmetric ? accx_rev_suffix(g, off, tilerow, dst, g->d_pre, s, &sorted) : ACCX_ERR_OOM;
         if (rc == ACCX_OK) {
           accx_dev_free(g->d_rev, g->home);
           g->d_rev = sorted;

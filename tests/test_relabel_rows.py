@@ -9,6 +9,7 @@ pytestmark = pytest.mark.gpu
 
 if has_gpu():
     from acctricnt_gb300 import accx
+    from oracle import oracle
 
 
 @pytest.mark.parametrize("spare", [0, 1 << 20, (1 << 24) - 30000, 1 << 25])
@@ -40,3 +41,24 @@ def test_row_lengths(spare):
     ref = np.empty(len(dst), np.int64)
     ref[order] = np.arange(len(dst))
     assert np.array_equal(rmap, ref)
+
+
+# the reverse index of suffix entries: tiles of 256 entries with one row, many rows and
+# runs of empty rows, ids that are not relabeled (prefixes of every length)
+@pytest.mark.parametrize("n,k,spread", [(2, 1, 1), (3, 3, 1), (40, 300, 1), (256, 9000, 1), (257, 257, 1), (5000, 700, 1),
+                                        (600, 900, 1000), (3000, 40000, 7)])
+@pytest.mark.parametrize("relabel", [False, True])
+def test_reverse_of_suffix_entries(n, k, spread, relabel):
+    rng = np.random.default_rng(n + k)
+    u, v = rng.integers(0, n, k), rng.integers(0, n, k)
+    u[0], v[0] = 0, n - 1
+    u, v = u[u != v] * spread, v[u != v] * spread
+    N = n * spread
+    key = np.unique(np.concatenate([u * N + v, v * N + u]))
+    off, dst = np.searchsorted(key, np.arange(N + 1) * N).astype(np.uint32), (key % N).astype(np.int32)
+    ref = oracle.cn_count(off, dst, nthreads=4)
+    G = accx.Graph.from_csr(off, dst)
+    if relabel:
+        G.relabel()
+    for policy in ("merge", "gallop", "bitmap"):
+        assert np.array_equal(G.count(policy=policy, bias=2, orient=True), ref), policy

@@ -86,12 +86,20 @@ __device__ __forceinline__ bool accx_dense_edge(int policy, const uint8_t *table
 // owners' probe work is summed per row run, then per warp, before the atomic on
 // work_u; merge / gallop list slots are reserved with one device atomic per list
 // and block (a CTA scan of the threads' counts).
-#define CL_EPT 8
+// Bound by issue and the loads' latency (Erdos-Renyi, 40M entries: issue 51 %, DRAM 29 %,
+// 190 instructions an entry), so by the warps that fit: four entries a thread, with
+// 16-byte loads of ids and reverses, two entries' ranges a store and the rows of listed
+// entries in shared memory, take 48 registers and five CTAs an SM.  Eight entries, loaded
+// and stored one by one, with 64 registers and four CTAs: Erdos-Renyi 5M 1.46 ms, R-MAT 24
+// 5.16; now 1.18 and 4.45 (eight with wide loads 1.31 and 4.73, four with six CTAs 1.35
+// and 5.12).
+#define CL_EPT 4
 // partner ranges of galloping entries carry this flag in their length (the
 // bitmap kernel skips them); prefix lengths stay below 2^31 on a symmetric CSR
 #define OR_SL_GALLOP 0x80000000u
 struct cl_stats {
-  unsigned long long e[ACCX_NUM_KINDS] = {0, 0, 0}, w[ACCX_NUM_KINDS] = {0, 0, 0}, o[ACCX_NUM_KINDS] = {0, 0, 0};
+  uint32_t e[ACCX_NUM_KINDS] = {0, 0, 0};
+  unsigned long long w[ACCX_NUM_KINDS] = {0, 0, 0}, o[ACCX_NUM_KINDS] = {0, 0, 0};
   __device__ __forceinline__ void add(int kind, uint32_t dv, uint32_t du) {
 #pragma unroll
     for (int k = 0; k < ACCX_NUM_KINDS; k++)
@@ -104,7 +112,7 @@ struct cl_stats {
 };
 
 template <bool ORIENT>
-__global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
+__global__ void __launch_bounds__(256, 5) k_classify(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
                                                   const int32_t *__restrict__ dst, uint32_t n, uint32_t m, int policy,
                                                   const uint8_t *__restrict__ table, uint2 *__restrict__ list,
                                                   uint32_t list_cap, unsigned long long *__restrict__ work_u,
@@ -116,6 +124,7 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
   static_assert(256 % CL_EPT == 0, "chunks inside tile-row tiles");
   __shared__ uint8_t s_table[ACCX_NB * ACCX_NB];
   __shared__ uint32_t s_wc[2][8];              // per-warp merge / gallop entries of the block
+  __shared__ uint32_t s_u[CL_EPT][256];        // the rows of merge and gallop entries, each thread its own
   __shared__ unsigned long long s_base[2];     // the block's first slot in each list
   __shared__ unsigned long long s_st[3 * ACCX_NUM_KINDS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -133,7 +142,6 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
     const uint32_t e0 = blk * span + (uint32_t)tid * CL_EPT;
     uint32_t e1 = e0 + CL_EPT < m ? e0 + CL_EPT : m;
     if (e0 >= m) e1 = e0;
-    uint32_t uu[CL_EPT];
     uint32_t kinds = 0;            // 4 bits per entry (0xf: none)
     uint32_t cm = 0, cg = 0;       // this thread's merge / gallop entries
     uint32_t run_u = 0xffffffffu;  // the current row's bitmap work
@@ -150,9 +158,27 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
     if (e0 < e1) {
       // the partners and their sizes first (independent loads in flight)
       // (oriented: the partner's offset and prefix length from one 8-byte record)
-      uint32_t vv[CL_EPT], dd[CL_EPT], ss[CL_EPT];
+      uint32_t vv[CL_EPT], dd[CL_EPT], ss[CL_EPT], rr[ORIENT ? CL_EPT : 1];
+      if (e1 - e0 == CL_EPT) {
 #pragma unroll
-      for (int j = 0; j < CL_EPT; j++) vv[j] = e0 + j < e1 ? (uint32_t)__ldg(dst + e0 + j) : 0u;
+        for (int j = 0; j < CL_EPT; j += 4) {
+          const int4 q = __ldg(reinterpret_cast<const int4 *>(dst + e0 + j));
+          vv[j] = (uint32_t)q.x, vv[j + 1] = (uint32_t)q.y, vv[j + 2] = (uint32_t)q.z, vv[j + 3] = (uint32_t)q.w;
+        }
+        if (ORIENT) {
+#pragma unroll
+          for (int j = 0; j < CL_EPT; j += 4) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(rev + e0 + j));
+            rr[j] = q.x, rr[j + 1] = q.y, rr[j + 2] = q.z, rr[j + 3] = q.w;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < CL_EPT; j++) {
+          vv[j] = e0 + j < e1 ? (uint32_t)__ldg(dst + e0 + j) : 0u;
+          if (ORIENT) rr[j] = e0 + j < e1 ? __ldg(rev + e0 + j) : 0xffffffffu;
+        }
+      }
 #pragma unroll
       for (int j = 0; j < CL_EPT; j++) {
         if (ORIENT) {
@@ -168,10 +194,11 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
       uint32_t u = accx_row_of(off, __ldg(tilerow + t), __ldg(tilerow + t + 1) + 1, e0);
       uint32_t rb = __ldg(off + u), re = __ldg(off + u + 1);
       uint32_t du = ORIENT ? __ldg(pre + u) : re - rb;
+      uint4 sl2 = make_uint4(0u, 0u, 0u, 0u);  // two entries' ranges, written together if either is read
+      bool put = false;
 #pragma unroll
       for (int j = 0; j < CL_EPT; j++) {
         const uint32_t e = e0 + (uint32_t)j;
-        uu[j] = u;
         if (e >= e1) {
           kinds |= 0xfu << (4 * j);
           continue;
@@ -182,7 +209,6 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
           re = __ldg(off + u + 1);
           du = ORIENT ? __ldg(pre + u) : re - rb;
         }
-        uu[j] = u;
         const uint32_t v = vv[j];
         int kind = -1;
         const uint32_t dv = dd[j];
@@ -201,12 +227,13 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
           // its length cut at min(u, v) (galloping ones flagged in the top bit),
           // written where they are read: every entry of a row the bitmap kernel
           // walks (zero for the other kinds), and every galloping entry
+          if (!(j & 1)) sl2 = make_uint4(0u, 0u, 0u, 0u);
           uint2 sl = make_uint2(0u, 0u);
           if (kind == ACCX_KIND_BITMAP || kind == ACCX_KIND_GALLOP) {
             uint32_t sst = ss[j];
             uint32_t tt = sst + dv;
             if (v > u) {  // cut P(v) at u: u's position in N(v) is the reverse entry
-              const uint32_t r = __ldg(rev + e);
+              const uint32_t r = rr[j];
               tt = (r >= sst && r < tt) ? r : sst;
             }
             if (kind == ACCX_KIND_BITMAP) {
@@ -217,9 +244,14 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
             sl = make_uint2(sst, (tt - sst) | (kind == ACCX_KIND_GALLOP ? OR_SL_GALLOP : 0u));
             bwork = tt - sst;
           }
-          if ((u < bm_idlim && du <= bm_pcap) || kind == ACCX_KIND_GALLOP) or_sl[e] = sl;
+          if (j & 1) sl2.z = sl.x, sl2.w = sl.y;
+          else sl2.x = sl.x, sl2.y = sl.y;
+          put = ((j & 1) && put) || (u < bm_idlim && du <= bm_pcap) || kind == ACCX_KIND_GALLOP;
+          if (put && (j & 1)) *reinterpret_cast<uint4 *>(or_sl + e - 1) = sl2;
+          else if (put && e + 1 == e1) or_sl[e] = sl;
         }
         st.add(kind, dv, du);
+        if (kind == ACCX_KIND_MERGE || kind == ACCX_KIND_GALLOP) s_u[j][tid] = u;
         cm += kind == ACCX_KIND_MERGE;
         cg += kind == ACCX_KIND_GALLOP;
         if (kind == ACCX_KIND_BITMAP) {
@@ -275,10 +307,10 @@ __global__ void __launch_bounds__(256, 4) k_classify(const uint32_t *__restrict_
         // owned edges number exactly m/2 on a symmetric graph; the guard only
         // keeps unvalidated asymmetric input inside the list
         if (k == ACCX_KIND_MERGE) {
-          if (pm < list_cap) list[pm] = make_uint2(uu[j], e0 + (uint32_t)j);
+          if (pm < list_cap) list[pm] = make_uint2(s_u[j][tid], e0 + (uint32_t)j);
           pm++;
         } else if (k == ACCX_KIND_GALLOP) {
-          if (pg < list_cap) list[list_cap - 1 - pg] = make_uint2(uu[j], e0 + (uint32_t)j);
+          if (pg < list_cap) list[list_cap - 1 - pg] = make_uint2(s_u[j][tid], e0 + (uint32_t)j);
           pg++;
         }
       }
@@ -842,7 +874,7 @@ static bool alloc_degree(accx_graph *g) {
 // block of entries.
 static unsigned classify_grid(int sms, uint32_t m) {
   const unsigned long long blocks = ((unsigned long long)m + 256 * CL_EPT - 1) / (256 * CL_EPT);
-  const unsigned long long g = (unsigned long long)sms * 4;
+  const unsigned long long g = (unsigned long long)sms * 5;
   return (unsigned)(blocks < g ? (blocks ? blocks : 1) : g);
 }
 

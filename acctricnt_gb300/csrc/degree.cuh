@@ -8,10 +8,11 @@
 // vertices, as an id common to their F, and credited to its three edges; this is the
 // oriented count (orient.cuh) with the order computed on the fly instead of a
 // relabeled copy.  The vertex with the longer F owns the edge: it is staged, the other
-// one's ids are streamed, so the credits of the busy hub edges stay in shared counters.  Merging full lists up to a ratio of 50 cost 18.5 ms of an R-MAT 18
-// count: 19.4 -> 1.31 ms (14.8x); power law with 4.6M entries 7.0 -> 0.61 ms.
+// one's ids are streamed, so the credits of the busy hub edges stay in shared counters.
+// Merging full lists up to a ratio of 50 cost 18.5 ms of an R-MAT 18 count: 19.4 -> 1.31
+// ms (14.8x); power law with 4.6M entries 7.0 -> 0.61 ms.
 //
-// Small graphs: one kernel, eight lanes per owned edge (k_count_small).
+// Small graphs: one kernel, a warp per owned edge (k_count_small).
 //
 // Included by count.cu.
 #pragma once
@@ -459,9 +460,9 @@ __global__ void __launch_bounds__(TILE) k_dg_out(const uint32_t *__restrict__ of
 // A small graph in one kernel: a CTA takes DS_TILE entries, keeps the owned ones, and
 // gives a warp to each: its lanes search the shorter list's ids in the longer list, and
 // the count goes to both entries.  An R-MAT 10 count is launches and little else: nine
-// kernels and two fills took 61 us, with the caller's copy; now 22.  Few entries a CTA and whole warps, because
-// the hub's row would otherwise be the tail (64 entries and eight lanes an edge: 41 us
-// for this kernel alone).
+// kernels and two fills took 61 us, with the caller's copy; now 18.  Few entries a CTA and
+// whole warps, because the hub's row would otherwise be the tail (64 entries and eight
+// lanes an edge: 41 us for this kernel alone).
 #define DS_TILE 16
 __global__ void __launch_bounds__(256) k_count_small(const uint32_t *__restrict__ off,
                                                      const uint32_t *__restrict__ tilerow,

@@ -388,10 +388,12 @@ def measured_regret(model_ms, alternatives):
 
 
 def alg_bytes(G, dominant, stats, owner_work, matches=None):
-    """Algorithmic bytes of one launch of the dominant phase.  Oriented bitmap
-    kernel: the ids it probed, the owner prefixes it staged, 8 bytes per owned
-    edge (partner offset and prefix length) and a 4-byte read-modify-write of a
-    count per common id found (the credit of the partner-side entry)."""
+    """Algorithmic bytes of the dominant phase's launches in one count.  Oriented bitmap
+    kind (k_dense_pairs, k_bitmap_or and k_owner_warp): the ids its edges' partner lists
+    hold, the owner prefixes staged, 8 bytes per owned edge (partner offset and prefix
+    length) and a 4-byte read-modify-write of a count per common id found (the credit of
+    the partner-side entry).  The dense rows test the hub ids among them as bits of masks
+    that stay in L2, so the fraction is of a list-probing count's bytes; `traffic` is DRAM's."""
     if dominant == "bitmap" and matches is not None:
         found, probed = matches
         return 4 * probed + 4 * owner_work["bitmap"] + 8 * stats["bitmap"]["edges"] + 8 * found["bitmap"]
@@ -405,6 +407,23 @@ def alg_bytes(G, dominant, stats, owner_work, matches=None):
     if dominant == "mirror":
         return 4 * 4 * G.m
     return 8 * G.m
+
+
+def launches_per_count(policy, orient):
+    """This library's kernels in one count of a relabeled graph above 2^17 entries: model
+    inference (model policy); direct: six kernels (classify, item counts, merge, gallop, bitmap,
+    mirror; the ratio-50 rule's six are the degree-ordered count's); oriented: classify (which also
+    writes the bias), item lists, dense rows, bitmap and light owners where the bitmap kind can
+    occur, merge, the two galloping forms, combine; gather back to the caller's order."""
+    anyk = policy in ("model", "table")
+    k = 1 if policy == "model" else 0
+    if not orient:
+        return k + 6 + 1
+    k += 2 + 1
+    k += 4 if anyk or policy == "bitmap" else 0
+    k += 1 if anyk or policy in ("heuristic", "merge") else 0
+    k += 2 if policy != "merge" else 0
+    return k
 
 
 def workload_config(args, n, m, world):
@@ -467,6 +486,7 @@ def run_gb300(args):
     ab = alg_bytes(G, dominant, stats, owner_work, matches if dominant == "bitmap" else None)
     achieved = ab / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else None
     kname = dominant + ("_or" if orient and dominant in ("merge", "gallop", "bitmap") else "")
+    kernels = "k_dense_pairs + k_bitmap_or + k_owner_warp" if kname == "bitmap_or" else "k_" + kname
     traffic = None
     try:
         tr = json.load(open(os.path.join(ROOT, "profiles", "traffic.json"))).get(kname)
@@ -475,7 +495,7 @@ def run_gb300(args):
             traffic = int(tr["bytes_per_probe"] * probes)
     except Exception:
         pass
-    roofline = {"bound": "hbm", "kernel": "k_" + kname, "achieved": round(achieved, 1) if achieved else None,
+    roofline = {"bound": "hbm", "kernel": kernels, "achieved": round(achieved, 1) if achieved else None,
                 "peak": peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if peaks else "fallback",
                 "unit": "GB/s", "frac": round(achieved / peak, 4) if achieved else None, "traffic": traffic,
                 "alg_bytes_per_launch": int(ab), "launch_ms": round(dom_ms, 3),
@@ -508,11 +528,7 @@ def run_gb300(args):
             "phases_ms": {k: round(v, 3) for k, v in phases.items()}, "kinds": stats,
             "matches": ({"found": matches[0], "bitmap_probed": matches[1]} if matches else None),
             "scan": scan, "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-            # this library's kernels per count: model inference (model policy); direct: classify, item
-            # counts, merge, gallop, bitmap, mirror; oriented: prefix lengths, classify (which also
-            # writes the bias), item counts, item fill, merge, gallop, bitmap, combine; gather back
-            # (relabeled graph)
-            "gpu_launches": ((1 if policy == "model" else 0) + (8 if orient else 6) + 1) * args.steps,
+            "gpu_launches": launches_per_count(policy, orient) * args.steps,
             "clocks": clk.summary(),
             "sched": dict(sched_info, **(compared or {}))}
     G.free()

@@ -316,7 +316,6 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, GALLOP_CTAS) k_gallop_lane(c
 #define OW_SHARE 4096u
 #define OW_SPREAD 400000u
 #define OW_DEG 4096u
-#define OW_MAX_N (1u << 24)  // ids must fit 24 bits of a table word
 // CTA items aim at a 16th of a CTA's share of all probes, within these bounds (a
 // smaller item costs its staging more often, a larger one ends later than the rest)
 #define ITEM_TARGET_MIN 16384u

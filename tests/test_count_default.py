@@ -89,3 +89,21 @@ def test_rmat_relabeled_too(scale):
     off, dst = G.download()
     _check(off, dst)
     _check(off, dst, relabel=True)
+
+
+# ids of 24 and 25 bits beside the positions of a warp's table, and one bit more than fits
+@pytest.mark.parametrize("n", [(1 << 24) + 1, (1 << 25) - 1, 1 << 25])
+def test_wide_ids(n):
+    rng = np.random.default_rng(n)
+    us, vs = [], []
+    for c in (33, 129, 130):  # cliques of the highest ids and of random ones: |F| up to 32, 128, 129
+        for ids in (np.arange(n - c, n), np.sort(rng.choice(n, c, replace=False))):
+            a, b = np.triu_indices(c, 1)
+            us.append(ids[a])
+            vs.append(ids[b])
+    pool = np.concatenate([rng.choice(n, 4000, replace=False), np.arange(n - 500, n)])
+    us.append(rng.choice(pool, 150000))
+    vs.append(rng.choice(pool, 150000))
+    off, dst = _csr(n, np.concatenate(us), np.concatenate(vs))
+    assert len(dst) > SMALL_M
+    _check(off, dst)

@@ -934,10 +934,9 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   unsigned long long *ctr = g->d_counters;
   unsigned long long *work_u = g->d_counters + C_NUM;
   // the default policy on a CSR known to be symmetric (degree.cuh; power law with 20M
-  // vertices and 445M entries 3003 -> 109 ms, Erdos-Renyi with 480M 107 -> 49): ids in the warps'
-  // tables have 25 bits; without that, or without room (or a way to ask for it, in a
-  // capture), an intersection per edge
-  bool degree = !orient && policy == ACCX_POLICY_HEURISTIC && g->symmetric && n <= DG_MAX_N && m;
+  // vertices and 445M entries 3003 -> 108 ms, Erdos-Renyi with 480M 107 -> 48); without that,
+  // or without room (or a way to ask for it, in a capture), an intersection per edge
+  bool degree = !orient && policy == ACCX_POLICY_HEURISTIC && g->symmetric && m;
   const bool small = degree && m <= DG_SMALL_M;
   if (degree && !small && !g->d_dg && (is_capturing(s) || !alloc_degree(g))) degree = false;
   // which kinds can occur; oriented bitmap owners lie below the dense window, so only

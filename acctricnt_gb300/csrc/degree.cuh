@@ -30,8 +30,6 @@
 #define DG_SLICE 1024u         // entries of a row a CTA walks as one item
 #define DG_LIGHT 32u           // |F| up to which a warp walks a row where it finds it
 #define DG_WARP 128u           // |F| a warp's table takes: listed rows
-#define DG_POS 7               // bits of a position in a table word: DG_WARP ids
-#define DG_MAX_N ((1u << (32 - DG_POS)) - 1u)  // the ids take the others, and no word is all ones
 #define DG_KEEP 1024u          // list entries a CTA gathers before one atomic places them
 #define DG_CAP 1024u           // |F| staged at once by a CTA
 #define DG_SLOTS 4096u
@@ -279,13 +277,15 @@ __device__ __forceinline__ uint32_t dg_partner(const uint32_t *__restrict__ off,
 }
 
 // The shorter rows with 2..CAP ids in F, a warp each: F(x) in a hash table of
-// (id << DG_POS | position), the row's entries 32 at a time.  CAP = DG_LIGHT: every row, a
+// ids, with their positions beside it, the row's entries 32 at a time.  (Words of id and
+// position took the same time, but only ids of 24 bits.)  CAP = DG_LIGHT: every row, a
 // warp's rows spread over the graph (ids near each other often have like degrees); CAP =
 // DG_WARP: the listed rows, from a counter.
 #define DG_WARPS (DG_THREADS / 32)
 template <uint32_t CAP>
 struct dg_warp {
   uint32_t tab[4 * CAP];
+  uint8_t pos[4 * CAP];
   uint32_t oc[CAP];
   or_seg seg;
 };
@@ -312,16 +312,17 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_warp(const uint32_t *__restri
     for (uint32_t i = lane; i < px; i += 32) {
       const uint32_t y = (uint32_t)__ldg(f + b + i);
       uint32_t h = ow_hash(y, sh);
-      while (atomicCAS(&S.tab[h], 0xffffffffu, (y << DG_POS) | i) != 0xffffffffu) h = (h + 1) & mask;
+      while (atomicCAS(&S.tab[h], 0xffffffffu, y) != 0xffffffffu) h = (h + 1) & mask;
+      S.pos[h] = (uint8_t)i;
     }
     __syncwarp();
     auto look = [&](uint32_t id) {
       uint32_t h = ow_hash(id, sh), t = S.tab[h];
-      while ((t >> DG_POS) != id && t != 0xffffffffu) {
+      while (t != id && t != 0xffffffffu) {
         h = (h + 1) & mask;
         t = S.tab[h];
       }
-      return t == 0xffffffffu ? t : (t & ((1u << DG_POS) - 1u));
+      return t == 0xffffffffu ? t : (uint32_t)S.pos[h];
     };
     for (uint32_t e0 = b; e0 < ee; e0 += 32) {
       uint32_t v, sst;

@@ -91,7 +91,7 @@ def test_rmat_relabeled_too(scale):
     _check(off, dst, relabel=True)
 
 
-# ids of 24 and 25 bits beside the positions of a warp's table, and one bit more than fits
+# graphs whose ids need 25 and 26 bits
 @pytest.mark.parametrize("n", [(1 << 24) + 1, (1 << 25) - 1, 1 << 25])
 def test_wide_ids(n):
     rng = np.random.default_rng(n)

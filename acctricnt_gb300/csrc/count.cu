@@ -86,8 +86,8 @@ __device__ __forceinline__ bool accx_dense_edge(int policy, const uint8_t *table
 // owners' probe work is summed per row run, then per warp, before the atomic on
 // work_u; merge / gallop list slots are reserved with one device atomic per list
 // and block (a CTA scan of the threads' counts).
-// Bound by issue and the loads' latency (Erdos-Renyi, 40M entries: issue 51 %, DRAM 29 %,
-// 190 instructions an entry), so by the warps that fit: four entries a thread, with
+// Bound by its gathers' latency (Erdos-Renyi, 40M entries: issue 51 %, DRAM 29 %; fewer
+// scans and barriers changed nothing), so by the warps that fit: four entries a thread, with
 // 16-byte loads of ids and reverses, two entries' ranges a store and the rows of listed
 // entries in shared memory, take 48 registers and five CTAs an SM.  Eight entries, loaded
 // and stored one by one, with 64 registers and four CTAs: Erdos-Renyi 5M 1.46 ms, R-MAT 24

@@ -26,6 +26,7 @@
 
 #include "accx_internal.h"
 #include "devutil.cuh"
+#include "entries.h"
 #include "merge.cuh"
 
 // counters layout
@@ -146,15 +147,7 @@ __global__ void __launch_bounds__(256, 5) k_classify(const uint32_t *__restrict_
     uint32_t cm = 0, cg = 0;       // this thread's merge / gallop entries
     uint32_t run_u = 0xffffffffu;  // the current row's bitmap work
     unsigned long long run_w = 0;
-    if (fill && e0 < e1) {  // oriented counts start every entry at the bias
-      if (e1 - e0 == CL_EPT) {
-        const int4 b4 = make_int4(bias, bias, bias, bias);
-        reinterpret_cast<int4 *>(fill + e0)[0] = b4;  // e0 is a multiple of 8: 32-byte aligned
-        reinterpret_cast<int4 *>(fill + e0)[1] = b4;
-      } else {
-        for (uint32_t e = e0; e < e1; e++) fill[e] = bias;
-      }
-    }
+    if (fill) accx_fill_chunk<CL_EPT>(fill, e0, e1, bias);  // oriented counts start every entry at the bias
     if (e0 < e1) {
       // the partners and their sizes first (independent loads in flight)
       // (oriented: the partner's offset and prefix length from one 8-byte record)
@@ -870,7 +863,7 @@ static bool alloc_degree(accx_graph *g) {
   return ok;
 }
 
-// Persistent classify CTAs: four per SM (64 registers a thread), at most one per
+// Persistent classify CTAs: five per SM (48 registers a thread), at most one per
 // block of entries.
 static unsigned classify_grid(int sms, uint32_t m) {
   const unsigned long long blocks = ((unsigned long long)m + 256 * CL_EPT - 1) / (256 * CL_EPT);

@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(1024, 1) k_bitmap(const uint32_t *__restrict__
     for (uint32_t i = ca + tid; i < cb; i += nt) accx_sparse_insert(slots, S, (uint32_t)__ldg(dst + i));
     __syncthreads();
     // probe, one round of up to nt owned entries at a time
-    for (uint32_t r0 = pa; r0 < pb; r0 += (uint32_t)nt) {
+    for (uint32_t r0 = pa; r0 < pb; r0 = accx_entry_step(r0, (uint32_t)nt, pb)) {
       const uint32_t k = r0 + (uint32_t)tid;
       uint32_t sst = 0, len = 0;
       if (k < pb) {
@@ -678,10 +678,10 @@ __global__ void __launch_bounds__(1024, 1) k_bitmap(const uint32_t *__restrict__
         uint32_t h = 0;
         if (a0 + (uint32_t)lane < al) h += accx_bm_test(bv, (uint32_t)__ldg(dst + a0 + lane));
         if (bl4 + (uint32_t)lane < a1) h += accx_bm_test(bv, (uint32_t)__ldg(dst + bl4 + lane));
-        for (uint32_t jj = al + 4u * (uint32_t)lane; jj < bl4; jj += 256u) {
+        for (uint32_t jj = al + 4u * (uint32_t)lane; jj < bl4; jj = accx_entry_step(jj, 256u, bl4)) {
           const int4 q0 = __ldg(reinterpret_cast<const int4 *>(dst + jj));
           int4 q1 = make_int4(-1, -1, -1, -1);
-          if (jj + 128u < bl4) q1 = __ldg(reinterpret_cast<const int4 *>(dst + jj + 128u));
+          if (bl4 - jj > 128u) q1 = __ldg(reinterpret_cast<const int4 *>(dst + jj + 128u));
           h += accx_bm_test(bv, (uint32_t)q0.x) + accx_bm_test(bv, (uint32_t)q0.y) +
                accx_bm_test(bv, (uint32_t)q0.z) + accx_bm_test(bv, (uint32_t)q0.w);
           if (q1.x >= 0)

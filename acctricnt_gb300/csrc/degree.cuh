@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_cta(const uint32_t *__restric
     if (s_q >= nh) break;
     const uint2 item = heavy[s_q];
     const uint32_t x = item.x, b = __ldg(off + x), px = __ldg(flen + x);
-    const uint32_t e0 = b + item.y * DG_SLICE, ee = min(e0 + DG_SLICE, __ldg(off + x + 1));
+    const uint32_t e0 = b + item.y * DG_SLICE, ee = accx_slice_end(e0, DG_SLICE, __ldg(off + x + 1));
     for (uint32_t c0 = 0; c0 < px; c0 += DG_CAP) {
       const uint32_t cn = min(px - c0, DG_CAP);
       int lg = 8;
@@ -415,8 +415,9 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_cta(const uint32_t *__restric
       for (;;) {
         uint32_t e = 0;
         if (lane == 0) e = atomicAdd(&s_next, 32u);
-        e = e0 + __shfl_sync(ACCX_FULL_MASK, e, 0);
-        if (e >= ee) break;
+        e = __shfl_sync(ACCX_FULL_MASK, e, 0);
+        if (e >= ee - e0) break;
+        e += e0;
         uint32_t v, sst;
         const uint32_t len = dg_partner(off, dst, flen, x, px, e + lane, ee, &v, &sst);
         const uint32_t h = dg_stream(f, fc, sst, len, S, oc, lane, look);

@@ -25,3 +25,13 @@ ACCX_EHD void accx_fill_chunk(int32_t *p, uint32_t e0, uint32_t e1, int32_t x) {
     for (uint32_t e = e0; e < e1; e++) p[e] = x;
   }
 }
+
+// Positions are 32-bit and a CSR may have nearly 2^32 entries, so a position plus a step can
+// wrap: these compare what is left instead.
+
+// The end of a slice of `len` entries from e0 of a range that ends at `end` (e0 <= end).
+ACCX_EHD uint32_t accx_slice_end(uint32_t e0, uint32_t len, uint32_t end) {
+  return end - e0 > len ? e0 + len : end;
+}
+// The position `stride` after e in a loop over [.., end), e < end: `end` when there is none.
+ACCX_EHD uint32_t accx_entry_step(uint32_t e, uint32_t stride, uint32_t end) { return accx_slice_end(e, stride, end); }

@@ -17,6 +17,7 @@
 
 #include "accx_internal.h"
 #include "devutil.cuh"
+#include "entries.h"
 
 static thread_local char g_last_cuda_error[512];
 
@@ -343,7 +344,8 @@ __global__ void k_validate(const uint32_t *__restrict__ off, const uint32_t *__r
 }
 
 __global__ void k_iota(uint32_t *__restrict__ v, uint32_t m) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) v[i] = i;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i = accx_entry_step(i, stride, m)) v[i] = i;
 }
 
 // The reverse index by a stable radix sort of (neighbour id, entry index) pairs

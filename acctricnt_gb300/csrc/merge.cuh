@@ -1,5 +1,6 @@
 // Warp merge-path intersection count, shared by the counting kernels.
 #pragma once
+#include "entries.h"
 #include <stdint.h>
 
 #include "devutil.cuh"
@@ -29,9 +30,7 @@ __device__ __forceinline__ int accx_load_window(const int32_t *__restrict__ dst,
       if (ii >= pos && ii < end) buf[ii - pos] = vals[t];
     }
   }
-  uint32_t lim = al + MERGE_WIN;
-  if (lim > end) lim = end;
-  return (int)(lim - pos);
+  return (int)(accx_slice_end(al, MERGE_WIN, end) - pos);
 }
 
 __device__ __forceinline__ uint32_t accx_warp_merge_count(const int32_t *__restrict__ dst, uint32_t ab, uint32_t ae,

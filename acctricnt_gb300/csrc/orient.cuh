@@ -958,8 +958,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
     for (;;) {
       uint32_t r0 = 0;
       if (lane == 0) r0 = atomicAdd(&s_next, 32u);
-      r0 = pa + __shfl_sync(ACCX_FULL_MASK, r0, 0);
-      if (r0 >= pb) break;
+      r0 = __shfl_sync(ACCX_FULL_MASK, r0, 0);
+      if (r0 >= pb - pa) break;
+      r0 += pa;
       const uint32_t k = r0 + (uint32_t)lane;
       uint32_t sst = 0, len = 0;
       if (k < pb) {
@@ -975,7 +976,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
         const uint32_t a0 = __shfl_sync(ACCX_FULL_MASK, sst, src);
         const uint32_t a1 = a0 + __shfl_sync(ACCX_FULL_MASK, len, src);
         uint32_t h = 0;
-        for (uint32_t j0 = a0 & ~1u; j0 < a1; j0 += LONG_PIECE) {
+        for (uint32_t j0 = a0 & ~1u; j0 < a1; j0 = accx_entry_step(j0, LONG_PIECE, a1)) {
           // the last piece loads only the pair groups it needs (the size class is
           // warp-uniform, and each class issues all its loads at once)
           const uint32_t rem = a1 - j0;

@@ -12,6 +12,7 @@
 
 #include "accx_internal.h"
 #include "devutil.cuh"
+#include "entries.h"
 
 // Sort keys of the vertex order: the top of the key range less the degree, so that an
 // ascending stable sort of the ids by key gives degree descending, then id.  The keys have
@@ -84,7 +85,8 @@ __global__ void __launch_bounds__(1024) k_big_rows(relabel_view g, uint32_t rows
 }
 __global__ void k_put_big(const uint32_t *__restrict__ key, const uint32_t *__restrict__ val, uint32_t m,
                           int32_t *__restrict__ rdst, uint32_t *__restrict__ map) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x) {
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p = accx_entry_step(p, stride, m)) {
     rdst[p] = (int32_t)key[p];
     map[val[p]] = p;
   }
@@ -212,7 +214,7 @@ __global__ void k_gather_counts(const int32_t *__restrict__ cnt_r, const uint32_
                                 int32_t *cnt, int32_t *out) {
   const uint32_t stride = gridDim.x * blockDim.x;
   uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-  for (; e + 3 * stride < m; e += 4 * stride) {
+  for (; e < m && m - e > 3 * stride; e = accx_entry_step(e, 4 * stride, m)) {
     const uint32_t a = __ldg(map + e), b = __ldg(map + e + stride), c = __ldg(map + e + 2 * stride),
                    d = __ldg(map + e + 3 * stride);
     const int32_t x = __ldg(cnt_r + a), y = __ldg(cnt_r + b), z = __ldg(cnt_r + c), w = __ldg(cnt_r + d);
@@ -227,7 +229,7 @@ __global__ void k_gather_counts(const int32_t *__restrict__ cnt_r, const uint32_
       out[e + 3 * stride] = w;
     }
   }
-  for (; e < m; e += stride) {
+  for (; e < m; e = accx_entry_step(e, stride, m)) {
     const int32_t x = __ldg(cnt_r + __ldg(map + e));
     cnt[e] = x;
     if (out) out[e] = x;

@@ -22,6 +22,7 @@
 
 #include "accx_internal.h"
 #include "devutil.cuh"
+#include "entries.h"
 #include "simpred.h"
 
 // query counters
@@ -370,10 +371,14 @@ __global__ void k_compress(uint32_t n, const uint32_t *__restrict__ corebits, in
 __device__ __forceinline__ void accx_hub_range(const int32_t *__restrict__ dst, uint32_t b, uint32_t e, int32_t r,
                                                int lane, const uint32_t *__restrict__ corebits,
                                                int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax) {
-  for (uint32_t j0 = b; j0 < e; j0 += 128) {
+  const uint32_t len = e - b;
+  for (uint32_t i0 = 0; i0 < len; i0 += 128) {
     uint32_t u[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) u[k] = j0 + 32 * k + lane < e ? (uint32_t)__ldg(dst + j0 + 32 * k + lane) : 0xffffffffu;
+    for (int k = 0; k < 4; k++) {
+      const uint32_t i = i0 + 32 * k + lane;
+      u[k] = i < len ? (uint32_t)__ldg(dst + b + i) : 0xffffffffu;
+    }
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (u[k] == 0xffffffffu || accx_is_core(corebits, u[k])) continue;
@@ -393,7 +398,7 @@ __global__ void __launch_bounds__(256) k_hub_push(const uint32_t *__restrict__ o
   const unsigned long long np = qc[Q_PUSH], nc = qc[Q_CORELIST];
   for (unsigned long long i = w0; i < np; i += nw) {
     const uint2 it = __ldg(push + i);
-    const uint32_t b = __ldg(off + it.x) + it.y * PUSH_SLICE, e = min(b + PUSH_SLICE, __ldg(off + it.x + 1));
+    const uint32_t b = __ldg(off + it.x) + it.y * PUSH_SLICE, e = accx_slice_end(b, PUSH_SLICE, __ldg(off + it.x + 1));
     accx_hub_range(dst, b, e, parent[it.x], lane, corebits, hubmin, hubmax);
   }
   for (unsigned long long i = w0; i < nc; i += nw) {
@@ -437,7 +442,8 @@ __global__ void k_finish(uint32_t n, int32_t *__restrict__ label, const int32_t 
 }
 
 __global__ void k_bits_to_bytes(const uint32_t *__restrict__ bits, uint32_t m, uint8_t *__restrict__ out) {
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x)
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e = accx_entry_step(e, stride, m))
     out[e] = (bits[e >> 5] >> (e & 31)) & 1u;
 }
 
@@ -797,7 +803,8 @@ extern "C" int accx_similar_exact_batch(uint64_t k, const uint32_t *cnn, const u
 
 __global__ void k_cnt_digest(const int32_t *__restrict__ cnt, uint32_t m, unsigned long long *__restrict__ out) {
   unsigned long long sum = 0, dig = 0;
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e = accx_entry_step(e, stride, m)) {
     const uint32_t c = (uint32_t)cnt[e];
     sum += c;
     dig += accx_mix64_dev(((unsigned long long)e << 32) | c);

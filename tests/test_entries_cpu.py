@@ -32,7 +32,24 @@ static int fill(uint32_t m) {
   return bad;
 }
 
+// slices and strided loops of ranges that end close to 2^32: every position once, in order
+static int walk(uint64_t b, uint64_t end, uint32_t len) {
+  uint64_t at = b;
+  for (uint32_t e = (uint32_t)b; e < (uint32_t)end;) {
+    const uint32_t to = accx_slice_end(e, len, (uint32_t)end);
+    if (e != at || to <= e || to - e > len || (to < end && to - e != len)) return 1;
+    at = to;
+    if (accx_entry_step(e, len, (uint32_t)end) != to) return 1;
+    e = to;
+  }
+  return at != end;
+}
+
 int main() {
+  for (uint32_t len : {1u, 31u, 32u, 128u, 512u, 1024u, 1000000u, 0x80000000u, 0xffffffffu})
+    for (uint64_t end : {100ull, 0x80000000ull, (1ull << 32) - 1025, (1ull << 32) - 1024, (1ull << 32) - 65, (1ull << 32) - 1})
+      for (uint64_t n : {0ull, 1ull, 31ull, 64ull, 100ull, 3000ull, 5000001ull})
+        if (n <= end && walk(end - n, end, len)) return printf("%u at %llu, %llu left\n", len, (unsigned long long)end, (unsigned long long)n), 1;
   for (uint32_t m = 0; m <= 300; m++) {
     if (fill<4>(m)) return printf("fill<4> of %u entries\n", m), 1;
     if (fill<8>(m)) return printf("fill<8> of %u entries\n", m), 1;

@@ -112,6 +112,7 @@ struct accx_graph {
     cudaError_t _e = (call);                                  \
     if (_e != cudaSuccess) {                                  \
       accx_set_cuda_error(_e, #call, __FILE__, __LINE__);     \
+      cudaGetLastError(); /* not the next call's error */     \
       return (_e == cudaErrorMemoryAllocation) ? ACCX_ERR_OOM \
                                                : ACCX_ERR_CUDA; \
     }                                                         \

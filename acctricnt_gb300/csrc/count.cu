@@ -770,10 +770,11 @@ int accx_ensure_count_scratch(accx_graph *g) {
   cudaStream_t h = g->home;
   if (!g->d_cnt) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_cnt, sizeof(int32_t) * (m ? m : 1), h));
   if (!g->d_edge_list) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_edge_list, sizeof(uint2) * (m / 2 + 1), h));
-  if (!g->d_icnt) {
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_icnt, sizeof(unsigned long long) * (n + 1), h));
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_prefix, sizeof(unsigned long long) * (n + 1), h));
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_pre, sizeof(uint32_t) * (n ? n : 1), h));
+  // each by itself: an earlier call may have run out of memory between two of them
+  if (!g->d_icnt) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_icnt, sizeof(unsigned long long) * (n + 1), h));
+  if (!g->d_prefix) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_prefix, sizeof(unsigned long long) * (n + 1), h));
+  if (!g->d_pre) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_pre, sizeof(uint32_t) * (n ? n : 1), h));
+  if (!g->d_scan_tmp) {
     size_t bytes = 0;
     ACCX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, g->d_icnt, g->d_prefix, (int64_t)n + 1));
     ACCX_CUDA_TRY(accx_dev_alloc(&g->d_scan_tmp, bytes ? bytes : 16, h));

@@ -526,9 +526,9 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
     std::lock_guard<std::mutex> lk(mu_key);
     if (!g->key_valid.load(std::memory_order_relaxed)) {
       accx_graph *gm = const_cast<accx_graph *>(g);
-      if (!gm->d_simkey) {
-        ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_simkey, sizeof(float) * (size_t)m, g->home));
-        ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_src, sizeof(uint32_t) * (size_t)m, g->home));
+      if (!gm->d_simkey || !gm->d_src) {
+        if (!gm->d_simkey) ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_simkey, sizeof(float) * (size_t)m, g->home));
+        if (!gm->d_src) ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_src, sizeof(uint32_t) * (size_t)m, g->home));
         ACCX_CUDA_TRY(accx_dev_wait(g->home));
       }
       k_simkey<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->d_cnt, m, g->cnt_bias, gm->d_simkey,

@@ -1,0 +1,132 @@
+"""Calls that run out of device memory, in a child process whose device pool has a size limit:
+each says so, leaves the handle usable, and answers right when called again with and
+without room.  Answers are compared with the oracle's."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+CHILD = r"""
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+LIMIT = 256 << 20
+
+class Loc(C.Structure):
+    _fields_ = [("type", C.c_int), ("id", C.c_int)]
+
+class Props(C.Structure):
+    _fields_ = [("alloc", C.c_int), ("handles", C.c_int), ("loc", Loc), ("sec", C.c_void_p), ("max_size", C.c_size_t),
+                ("usage", C.c_ushort), ("reserved", C.c_ubyte * 54)]
+
+cu = C.CDLL("libcuda.so.1")
+def ok(r):
+    assert r == 0, r
+dev, ctx, pool = C.c_int(), C.c_void_p(), C.c_void_p()
+ok(cu.cuInit(0)); ok(cu.cuDeviceGet(C.byref(dev), 0))
+ok(cu.cuDevicePrimaryCtxRetain(C.byref(ctx), dev)); ok(cu.cuCtxSetCurrent(ctx))
+ok(cu.cuMemPoolCreate(C.byref(pool), C.byref(Props(1, 0, Loc(1, 0), None, LIMIT, 0))))
+ok(cu.cuMemPoolSetAttribute(pool, 4, C.byref(C.c_uint64(2 ** 64 - 1))))  # the release threshold
+ok(cu.cuDeviceSetMemPool(dev, pool))
+
+def used():
+    ok(cu.cuCtxSynchronize())
+    v = C.c_uint64()
+    ok(cu.cuMemPoolGetAttribute(pool, 7, C.byref(v)))
+    return v.value
+
+def take(size):
+    p = C.c_uint64()
+    r = cu.cuMemAllocFromPoolAsync(C.byref(p), C.c_size_t(size), pool, None)
+    ok(cu.cuCtxSynchronize())
+    return p if r == 0 else None
+
+def leave(room):
+    "Takes blocks until about `room` bytes of the pool are free."
+    held, size = [], LIMIT
+    while size >= 1 << 16:
+        free = LIMIT - used() - room
+        p = take(size) if free >= size else None
+        if p:
+            held.append(p)
+        else:
+            size //= 2
+    return held
+
+def give(held):
+    for p in held:
+        ok(cu.cuMemFreeAsync(p, None))
+    ok(cu.cuCtxSynchronize())
+
+from acctricnt_gb300 import accx
+from oracle import oracle
+
+def sweep(prep, op, check, rooms):
+    "Calls op with less and less taken: right or out of memory, twice, then right with all the room."
+    seen = set()
+    base = used()
+    for room in rooms:
+        g = prep()
+        held = leave(room)
+        for _ in range(2):
+            try:
+                check(op(g))
+                seen.add("right")
+            except accx.AccxError as e:
+                assert e.status == accx.ERR_OOM, (room, e)
+                seen.add("oom")
+        give(held)
+        check(op(g))
+        g.free()
+        assert used() == base, (room, used(), base)
+    assert seen == {"right", "oom"}, seen
+    print(sorted(seen))
+
+off, dst = accx.generate_host(accx.rmat_params(14, 16, seed=3))
+assert len(dst) > 1 << 17
+ref = oracle.scan(off, dst, 0.3, 3)
+
+def graph(**count):
+    g = accx.Graph.from_csr(off, dst)
+    if count:
+        g.count(out=None, **count)
+    return g
+
+def same_scan(r):
+    for k in ("sim", "label", "cluster"):
+        assert np.array_equal(r[k], ref[k]), k
+
+def same_counts(c):
+    assert np.array_equal(c, ref["cnn"])
+
+ROOMS = [k << 18 for k in range(0, 100, 3)]
+"""
+
+
+def _child(code):
+    r = subprocess.run([sys.executable, "-c", CHILD + code, ROOT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_query_keys():
+    _child("sweep(lambda: graph(policy='gallop', bias=2), lambda g: g.scan(0.3, 3), same_scan, ROOMS)\n")
+
+
+@pytest.mark.parametrize("kw", ["dict()", "dict(policy='bitmap')", "dict(policy='merge')",
+                                "dict(policy='bitmap', orient=True)", "dict(policy='merge', orient=True)"])
+def test_counts(kw):
+    _child("sweep(graph, lambda g: g.count(bias=2, **%s), same_counts, ROOMS)\n" % kw)
+
+
+def test_relabel_and_count():
+    _child("""
+def op(g):
+    g.relabel()
+    return g.count(policy='bitmap', bias=2, orient=True)
+sweep(graph, op, same_counts, ROOMS)
+""")

@@ -961,8 +961,9 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   if (small) {
     int32_t *direct = !rel && on_device ? copy : nullptr;
     ACCX_MARK(1);
-    k_count_small<<<(m + DS_TILE - 1) / DS_TILE, 256, 0, s>>>(off, tilerow, dst, n, m, bias, cnt,
-                                                                direct, ctr);
+    const uint32_t st = (m + DS_TILE - 1) / DS_TILE;
+    k_count_small<<<sms < accx_sm_count(g->device) && st > sms * 8u ? sms * 8u : st, 256, 0, s>>>(off, tilerow, dst, n, m,
+                                                                                                 bias, cnt, direct, ctr);
     if (direct) *copied = true;
     ACCX_MARK(2);
     ACCX_MARK(3);

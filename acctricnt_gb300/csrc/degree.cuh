@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(TILE) k_dg_out(const uint32_t *__restrict__ of
 // the count goes to both entries.  An R-MAT 10 count is launches and little else: nine
 // kernels and two fills took 61 us, with the caller's copy; now 18.  Few entries a CTA and
 // whole warps, because the hub's row would otherwise be the tail (64 entries and eight
-// lanes an edge: 41 us for this kernel alone).
+// lanes an edge: 41 us for this kernel alone).  A CTA a tile, but with a limit on the SMs
+// only as many CTAs as fit them at once (eight an SM), which loop.
 #define DS_TILE 16
 __global__ void __launch_bounds__(256) k_count_small(const uint32_t *__restrict__ off,
                                                      const uint32_t *__restrict__ tilerow,
@@ -477,44 +478,48 @@ __global__ void __launch_bounds__(256) k_count_small(const uint32_t *__restrict_
   __shared__ uint4 s_own[DS_TILE];
   __shared__ uint2 s_list[DS_TILE];
   __shared__ uint32_t s_n;
-  const uint32_t e = blockIdx.x * DS_TILE + threadIdx.x;
-  cl_stats st;
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
-  if (threadIdx.x < DS_TILE && e < m) {
-    const uint32_t t = e / 256u;
-    const uint32_t v = (uint32_t)__ldg(dst + e);
-    const uint32_t u = accx_row_of(off, __ldg(tilerow + t), __ldg(tilerow + t + 1) + 1, e);
-    const uint32_t ab = __ldg(off + u), ae = __ldg(off + u + 1), vb = __ldg(off + v), ve = __ldg(off + v + 1);
-    if (accx_owns(u, ae - ab, v, ve - vb)) {
-      const uint32_t i = atomicAdd(&s_n, 1u);
-      s_own[i] = make_uint4(ab, ae, vb, ve);
-      s_list[i] = make_uint2(u, e);
-      dg_stat(st, ae - ab, ve - vb);
-    }
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31;
-  for (uint32_t i = threadIdx.x / 32; i < s_n; i += 8) {
-    const uint4 o = s_own[i];
-    uint32_t lo = o.x, c = 0, r = 0;
-    if (lane == 31) r = accx_lower_bound(dst, o.z, o.w, (int32_t)s_list[i].x);  // the reverse entry
-    for (uint32_t j0 = o.z; j0 < o.w && lo < o.y; j0 += 32) {
-      const uint32_t j = j0 + lane;
-      uint32_t p = o.y;
-      if (j < o.w) {
-        const int32_t id = __ldg(dst + j);
-        p = accx_lower_bound(dst, lo, o.y, id);
-        c += p < o.y && __ldg(dst + p) == id;
+  const uint32_t tiles = (m + DS_TILE - 1) / DS_TILE;
+  cl_stats st;
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint32_t e = tile * DS_TILE + threadIdx.x;
+    __syncthreads();  // the list is the last tile's no more
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    if (threadIdx.x < DS_TILE && e < m) {
+      const uint32_t t = e / 256u;
+      const uint32_t v = (uint32_t)__ldg(dst + e);
+      const uint32_t u = accx_row_of(off, __ldg(tilerow + t), __ldg(tilerow + t + 1) + 1, e);
+      const uint32_t ab = __ldg(off + u), ae = __ldg(off + u + 1), vb = __ldg(off + v), ve = __ldg(off + v + 1);
+      if (accx_owns(u, ae - ab, v, ve - vb)) {
+        const uint32_t i = atomicAdd(&s_n, 1u);
+        s_own[i] = make_uint4(ab, ae, vb, ve);
+        s_list[i] = make_uint2(u, e);
+        dg_stat(st, ae - ab, ve - vb);
       }
-      lo = __shfl_sync(ACCX_FULL_MASK, p, (int)min(o.w - j0 - 1u, 31u));
     }
-    c = __reduce_add_sync(ACCX_FULL_MASK, c);
-    // lane 0: the entry, lane 31: its reverse
-    if (lane == 0) r = s_list[i].y;
-    if (lane == 0 || (lane == 31 && r < o.w && __ldg(dst + r) == (int32_t)s_list[i].x)) {
-      cnt[r] = (int32_t)c + bias;
-      if (copy) copy[r] = (int32_t)c + bias;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x / 32; i < s_n; i += 8) {
+      const uint4 o = s_own[i];
+      uint32_t lo = o.x, c = 0, r = 0;
+      if (lane == 31) r = accx_lower_bound(dst, o.z, o.w, (int32_t)s_list[i].x);  // the reverse entry
+      for (uint32_t j0 = o.z; j0 < o.w && lo < o.y; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        uint32_t p = o.y;
+        if (j < o.w) {
+          const int32_t id = __ldg(dst + j);
+          p = accx_lower_bound(dst, lo, o.y, id);
+          c += p < o.y && __ldg(dst + p) == id;
+        }
+        lo = __shfl_sync(ACCX_FULL_MASK, p, (int)min(o.w - j0 - 1u, 31u));
+      }
+      c = __reduce_add_sync(ACCX_FULL_MASK, c);
+      // lane 0: the entry, lane 31: its reverse
+      if (lane == 0) r = s_list[i].y;
+      if (lane == 0 || (lane == 31 && r < o.w && __ldg(dst + r) == (int32_t)s_list[i].x)) {
+        cnt[r] = (int32_t)c + bias;
+        if (copy) copy[r] = (int32_t)c + bias;
+      }
     }
   }
   dg_stat_flush(st, s_st, ctr);

@@ -81,6 +81,7 @@ struct accx_graph {
   uint32_t *d_rev = nullptr;               // m reverse entry of (at least) every suffix entry of the counting CSR (oriented counts)
   uint32_t *d_rev_orig = nullptr;          // m reverse entries of the handle's own CSR, recorded by full validation
   uint32_t *d_dg = nullptr;                // the default policy's degree-ordered count
+  bool dg_captured = false;                // a captured count reads d_dg: it stays
   // dense rows of the relabeled CSR (planned by the relabel; 0 rows: none worth it)
   uint32_t dense_k = 0, dense_m = 0;       // hub ids (bits a row) and rows
   uint32_t plan_rows = 0, plan_maxpre = 0; // rows the relabel's plan looked at, and their longest prefix
@@ -125,6 +126,9 @@ void accx_set_cuda_error(cudaError_t e, const char *what, const char *file, int 
 // device-wide synchronisation.
 cudaError_t accx_dev_alloc(void **p, size_t bytes, cudaStream_t s);
 cudaError_t accx_dev_wait(cudaStream_t s);
+// The same for an array of g: when it does not fit, scratch that g keeps only to spare its next
+// count an allocation (d_dg, up to 8m + 12n bytes) is freed first.
+cudaError_t accx_graph_alloc(accx_graph *g, void **p, size_t bytes, cudaStream_t s);
 void accx_dev_free(void *p, cudaStream_t s);
 void accx_dev_free_all(void *const *p, int k, cudaStream_t s);
 

@@ -768,24 +768,24 @@ __global__ void __launch_bounds__(TILE) k_mirror(const uint32_t *__restrict__ of
 int accx_ensure_count_scratch(accx_graph *g) {
   const size_t m = g->m, n = g->n;
   cudaStream_t h = g->home;
-  if (!g->d_cnt) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_cnt, sizeof(int32_t) * (m ? m : 1), h));
-  if (!g->d_edge_list) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_edge_list, sizeof(uint2) * (m / 2 + 1), h));
+  if (!g->d_cnt) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_cnt, sizeof(int32_t) * (m ? m : 1), h));
+  if (!g->d_edge_list) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_edge_list, sizeof(uint2) * (m / 2 + 1), h));
   // each by itself: an earlier call may have run out of memory between two of them
-  if (!g->d_icnt) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_icnt, sizeof(unsigned long long) * (n + 1), h));
-  if (!g->d_prefix) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_prefix, sizeof(unsigned long long) * (n + 1), h));
-  if (!g->d_pre) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_pre, sizeof(uint32_t) * (n ? n : 1), h));
+  if (!g->d_icnt) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_icnt, sizeof(unsigned long long) * (n + 1), h));
+  if (!g->d_prefix) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_prefix, sizeof(unsigned long long) * (n + 1), h));
+  if (!g->d_pre) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_pre, sizeof(uint32_t) * (n ? n : 1), h));
   if (!g->d_scan_tmp) {
     size_t bytes = 0;
     ACCX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, g->d_icnt, g->d_prefix, (int64_t)n + 1));
-    ACCX_CUDA_TRY(accx_dev_alloc(&g->d_scan_tmp, bytes ? bytes : 16, h));
+    ACCX_CUDA_TRY(accx_graph_alloc(g, &g->d_scan_tmp, bytes ? bytes : 16, h));
     g->scan_tmp_bytes = bytes;
   }
   if (!g->d_counters) {
     // counters followed by the per-vertex bitmap work array
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_counters, sizeof(unsigned long long) * (C_NUM + n + 1), h));
+    ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_counters, sizeof(unsigned long long) * (C_NUM + n + 1), h));
   }
   if (!g->d_table) {
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_table, ACCX_NB * ACCX_NB, h));
+    ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_table, ACCX_NB * ACCX_NB, h));
     // pool allocations are ordered on the home stream; counts may run on another
     ACCX_CUDA_TRY(accx_dev_wait(h));
   }
@@ -839,9 +839,9 @@ static bool is_capturing(cudaStream_t s) {
 }
 static bool alloc_dense(accx_graph *g) {
   const size_t tb = (size_t)g->dense_m * (g->dense_k / 8u);
-  bool ok = accx_dev_alloc((void **)&g->d_dense_t, tb, g->home) == cudaSuccess &&
-            accx_dev_alloc((void **)&g->d_dense_low, sizeof(uint32_t) * ((size_t)g->dense_m + 4), g->home) == cudaSuccess &&
-            accx_dev_alloc((void **)&g->d_dense_items, sizeof(uint4) * (size_t)dense_cap(g), g->home) == cudaSuccess;
+  bool ok = accx_graph_alloc(g, (void **)&g->d_dense_t, tb, g->home) == cudaSuccess &&
+            accx_graph_alloc(g, (void **)&g->d_dense_low, sizeof(uint32_t) * ((size_t)g->dense_m + 4), g->home) == cudaSuccess &&
+            accx_graph_alloc(g, (void **)&g->d_dense_items, sizeof(uint4) * (size_t)dense_cap(g), g->home) == cudaSuccess;
   if (ok) ok = accx_dev_wait(g->home) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
@@ -932,7 +932,11 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   // or without room (or a way to ask for it, in a capture), an intersection per edge
   bool degree = !orient && policy == ACCX_POLICY_HEURISTIC && g->symmetric && m;
   const bool small = degree && m <= DG_SMALL_M;
-  if (degree && !small && !g->d_dg && (is_capturing(s) || !alloc_degree(g))) degree = false;
+  if (degree && !small) {
+    const bool capturing = is_capturing(s);
+    if (!g->d_dg && (capturing || !alloc_degree(g))) degree = false;
+    else if (capturing) g->dg_captured = true;
+  }
   // which kinds can occur; oriented bitmap owners lie below the dense window, so only
   // their part of work_u is used
   const bool any = policy == ACCX_POLICY_TABLE || policy == ACCX_POLICY_MODEL;
@@ -1002,10 +1006,10 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
       return ACCX_ERR_CUDA;
     }
     if (!g->d_or_sl || !g->d_or_items || !g->d_vinfo) {
-      if (!g->d_or_sl) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_or_sl, sizeof(uint2) * (size_t)m, g->home));
-      if (!g->d_vinfo) ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_vinfo, sizeof(uint2) * (size_t)n, g->home));
+      if (!g->d_or_sl) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_or_sl, sizeof(uint2) * (size_t)m, g->home));
+      if (!g->d_vinfo) ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_vinfo, sizeof(uint2) * (size_t)n, g->home));
       if (!g->d_or_items)
-        ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_or_items, sizeof(uint32_t) * (size_t)items_cap, g->home));
+        ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_or_items, sizeof(uint32_t) * (size_t)items_cap, g->home));
       ACCX_CUDA_TRY(accx_dev_wait(g->home));
     }
     // prefix lengths: an index of the counting CSR, built on its first oriented count
@@ -1031,7 +1035,7 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
           g->d_rev = sorted;
         } else if (rc == ACCX_ERR_OOM) {
           if (!g->d_rev) {
-            ACCX_CUDA_TRY(accx_dev_alloc((void **)&g->d_rev, sizeof(uint32_t) * (size_t)m, g->home));
+            ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&g->d_rev, sizeof(uint32_t) * (size_t)m, g->home));
             ACCX_CUDA_TRY(accx_dev_wait(g->home));
           }
           ACCX_CUDA_TRY(cudaMemsetAsync(g->d_rev, 0xff, sizeof(uint32_t) * (size_t)m, s));

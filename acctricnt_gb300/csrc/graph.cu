@@ -81,6 +81,29 @@ cudaError_t accx_dev_alloc(void **p, size_t bytes, cudaStream_t s) {
 }
 cudaError_t accx_dev_wait(cudaStream_t s) { return cudaStreamSynchronize(s); }
 
+// Queries of several threads may run out on one handle at once.
+static bool give_back(accx_graph *g) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!g->d_dg || g->dg_captured) return false;
+  bool ok = cudaDeviceSynchronize() == cudaSuccess;  // a count on any stream may still use it
+  if (ok) {
+    ok = cudaFreeAsync(g->d_dg, g->home) == cudaSuccess && cudaStreamSynchronize(g->home) == cudaSuccess;
+    g->d_dg = nullptr;
+  }
+  cudaGetLastError();
+  return ok;
+}
+cudaError_t accx_graph_alloc(accx_graph *g, void **p, size_t bytes, cudaStream_t s) {
+  cudaError_t e = accx_dev_alloc(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation) {
+    give_back(g);  // or another thread did
+    cudaGetLastError();
+    e = accx_dev_alloc(p, bytes, s);
+  }
+  return e;
+}
+
 // Without a stream the device is synchronised first, as cudaFree does: work on
 // any stream may still read the blocks.
 void accx_dev_free_all(void *const *p, int k, cudaStream_t s) {
@@ -510,8 +533,8 @@ int accx_rev_suffix(accx_graph *g, const uint32_t *off, const uint32_t *tilerow,
   }
   if (ts > tb) tb = ts;
   const size_t words = 4 * hn + (((size_t)n + 3) & ~(size_t)3);
-  if (accx_dev_alloc((void **)&rev, sizeof(uint32_t) * (size_t)m, g->home) != cudaSuccess ||
-      accx_dev_alloc((void **)&buf, sizeof(uint32_t) * words + tb + 16, s) != cudaSuccess ||
+  if (accx_graph_alloc(g, (void **)&rev, sizeof(uint32_t) * (size_t)m, g->home) != cudaSuccess ||
+      accx_graph_alloc(g, (void **)&buf, sizeof(uint32_t) * words + tb + 16, s) != cudaSuccess ||
       (g->home != s && accx_dev_wait(g->home) != cudaSuccess)) {
     cudaGetLastError();
     accx_dev_free(rev, g->home);
@@ -558,7 +581,7 @@ int accx_tilerow_build(accx_graph *g, const uint32_t *off, uint32_t **out, cudaS
   if (m == 0 || *out) return ACCX_OK;
   const uint32_t ntiles = (m + 255) / 256;
   uint32_t *p = nullptr;
-  ACCX_CUDA_TRY(accx_dev_alloc((void **)&p, sizeof(uint32_t) * ((size_t)ntiles + 2), g->home));
+  ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&p, sizeof(uint32_t) * ((size_t)ntiles + 2), g->home));
   if (g->home != s) ACCX_CUDA_TRY(accx_dev_wait(g->home));
   k_tilerow<<<accx_sm_count(g->device) * 8, 256, 0, s>>>(off, g->n, m, ntiles, p);
   ACCX_CUDA_TRY(cudaGetLastError());

@@ -334,14 +334,14 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
   int rc = ACCX_OK;
   const size_t vn = ((size_t)n + 64) & ~(size_t)63;
   do {
-    if (accx_dev_alloc((void **)&vtmp, sizeof(uint32_t) * (4 * vn + (DENSE_KINDS + 1) * DENSE_BLOCKS), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&rdeg, sizeof(uint32_t) * (vn + 2 * RELABEL_NCLASS + 2), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&g->d_roff, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&g->d_rdst, sizeof(int32_t) * ((size_t)m + ACCX_DST_PAD), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&g->d_rmap, sizeof(uint32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&g->d_rcnt, sizeof(int32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&g->d_oldid, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
-        accx_dev_alloc((void **)&g->d_newid, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess) {
+    if (accx_graph_alloc(g, (void **)&vtmp, sizeof(uint32_t) * (4 * vn + (DENSE_KINDS + 1) * DENSE_BLOCKS), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&rdeg, sizeof(uint32_t) * (vn + 2 * RELABEL_NCLASS + 2), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&g->d_roff, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&g->d_rdst, sizeof(int32_t) * ((size_t)m + ACCX_DST_PAD), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&g->d_rmap, sizeof(uint32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&g->d_rcnt, sizeof(int32_t) * ((size_t)m + 1), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&g->d_oldid, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
+        accx_graph_alloc(g, (void **)&g->d_newid, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess) {
       rc = ACCX_ERR_OOM;
       break;
     }
@@ -358,7 +358,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
       break;
     }
     tb = b1 > b2 ? b1 : b2;
-    if (accx_dev_alloc(&tmp, tb + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+    if (accx_graph_alloc(g, &tmp, tb + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
     if (accx_dev_wait(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     // 1. vertex order: degree descending, ties by id
     if (n) {
@@ -391,7 +391,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
         }
         // keys and entries, sorted into a second pair; the scratch behind them
         const size_t kn = ((size_t)pb[0] + 64) & ~(size_t)63;
-        if (accx_dev_alloc((void **)&key, sizeof(uint32_t) * 4 * kn + b3 + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+        if (accx_graph_alloc(g, (void **)&key, sizeof(uint32_t) * 4 * kn + b3 + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
         if (accx_dev_wait(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
         uint32_t *val = key + kn, *key2 = key + 2 * kn, *val2 = key + 3 * kn;
         k_big_rows<<<rb[0] < (uint32_t)sms * 2 ? rb[0] : sms * 2, 1024, 0, s>>>(view, rb[0], key, val);

@@ -488,21 +488,22 @@ void accx_query_ctx_release(accx_query_ctx *q) {
 
 static int ensure_query_arrays(const accx_graph *g, accx_query_ctx *q) {
   if (q->d_simbits && (q->n != g->n || q->m != g->m)) return ACCX_ERR_INVALID_ARG;  // made for another graph
+  accx_graph *gm = const_cast<accx_graph *>(g);  // which may give scratch back
   q->n = g->n;
   q->m = g->m;
   if (q->d_big) return ACCX_OK;  // the last of them
   const size_t n = g->n ? g->n : 1, words = (g->m + 31) / 32 + 1;
-  if (!q->d_simbits) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_simbits, sizeof(uint32_t) * words, nullptr));
-  if (!q->d_corelist) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_corelist, sizeof(uint32_t) * n, nullptr));
+  if (!q->d_simbits) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_simbits, sizeof(uint32_t) * words, nullptr));
+  if (!q->d_corelist) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_corelist, sizeof(uint32_t) * n, nullptr));
   // rows above PUSH_ROW have at most 1 + degree/PUSH_SLICE slices
-  if (!q->d_push) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_push, sizeof(uint2) * (g->m / PUSH_ROW + g->m / PUSH_SLICE + 2), nullptr));
-  if (!q->d_label) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_label, sizeof(int32_t) * n, nullptr));
-  if (!q->d_parent) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_parent, sizeof(int32_t) * n, nullptr));
-  if (!q->d_hubmin) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_hubmin, sizeof(int32_t) * n, nullptr));
-  if (!q->d_hubmax) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_hubmax, sizeof(int32_t) * n, nullptr));
-  if (!q->d_qcounters) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_qcounters, sizeof(unsigned long long) * Q_NUM, nullptr));
-  if (!q->d_corebits) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_corebits, sizeof(uint32_t) * (n / 32 + 2), nullptr));
-  if (!q->d_big) ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_big, sizeof(uint32_t) * (g->m / BIG_ROW + 2), nullptr));
+  if (!q->d_push) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_push, sizeof(uint2) * (g->m / PUSH_ROW + g->m / PUSH_SLICE + 2), nullptr));
+  if (!q->d_label) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_label, sizeof(int32_t) * n, nullptr));
+  if (!q->d_parent) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_parent, sizeof(int32_t) * n, nullptr));
+  if (!q->d_hubmin) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_hubmin, sizeof(int32_t) * n, nullptr));
+  if (!q->d_hubmax) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_hubmax, sizeof(int32_t) * n, nullptr));
+  if (!q->d_qcounters) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_qcounters, sizeof(unsigned long long) * Q_NUM, nullptr));
+  if (!q->d_corebits) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_corebits, sizeof(uint32_t) * (n / 32 + 2), nullptr));
+  if (!q->d_big) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&q->d_big, sizeof(uint32_t) * (g->m / BIG_ROW + 2), nullptr));
   ACCX_CUDA_TRY(accx_dev_wait(nullptr));
   return ACCX_OK;
 }
@@ -527,8 +528,8 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
     if (!g->key_valid.load(std::memory_order_relaxed)) {
       accx_graph *gm = const_cast<accx_graph *>(g);
       if (!gm->d_simkey || !gm->d_src) {
-        if (!gm->d_simkey) ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_simkey, sizeof(float) * (size_t)m, g->home));
-        if (!gm->d_src) ACCX_CUDA_TRY(accx_dev_alloc((void **)&gm->d_src, sizeof(uint32_t) * (size_t)m, g->home));
+        if (!gm->d_simkey) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&gm->d_simkey, sizeof(float) * (size_t)m, g->home));
+        if (!gm->d_src) ACCX_CUDA_TRY(accx_graph_alloc(gm, (void **)&gm->d_src, sizeof(uint32_t) * (size_t)m, g->home));
         ACCX_CUDA_TRY(accx_dev_wait(g->home));
       }
       k_simkey<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_tilerow, g->d_dst, g->d_cnt, m, g->cnt_bias, gm->d_simkey,
@@ -545,7 +546,7 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
   const bool sim_dev = sim && m && accx_is_device_ptr(sim);
   uint8_t *sim_tmp = nullptr, *sim_out = sim_dev && !((uintptr_t)sim & 7) ? sim : nullptr;
   if (sim && m && !sim_dev) {
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&sim_tmp, m, s));
+    ACCX_CUDA_TRY(accx_graph_alloc(const_cast<accx_graph *>(g), (void **)&sim_tmp, m, s));
     sim_out = sim_tmp;
   }
   if (m) k_sim_keys<<<sms * 8, 256, 0, s>>>(g->d_simkey, g->d_off, g->d_src, g->d_dst, g->d_cnt, m, g->cnt_bias, sq, klo,
@@ -649,8 +650,8 @@ static int build_pairs(accx_graph *g, accx_query_ctx *q, cudaStream_t s) {
     accx_dev_free(q->d_pairs_tmp, nullptr);
     q->d_pairs = q->d_pairs_tmp = nullptr;
     q->pairs_cap = 0;
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_pairs, sizeof(unsigned long long) * h, nullptr));
-    ACCX_CUDA_TRY(accx_dev_alloc((void **)&q->d_pairs_tmp, sizeof(unsigned long long) * h, nullptr));
+    ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&q->d_pairs, sizeof(unsigned long long) * h, nullptr));
+    ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&q->d_pairs_tmp, sizeof(unsigned long long) * h, nullptr));
     ACCX_CUDA_TRY(accx_dev_wait(nullptr));
     q->pairs_cap = h;
   }
@@ -665,7 +666,7 @@ static int build_pairs(accx_graph *g, accx_query_ctx *q, cudaStream_t s) {
     ACCX_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (int64_t)h, 0, 64, s));
     ACCX_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, tb2, q->d_pairs, q->d_pairs_tmp, d_nsel, (int64_t)h, s));
     void *tmp = nullptr;
-    ACCX_CUDA_TRY(accx_dev_alloc(&tmp, std::max(tb, tb2) + 64, s));
+    ACCX_CUDA_TRY(accx_graph_alloc(g, &tmp, std::max(tb, tb2) + 64, s));
     d_nsel = reinterpret_cast<unsigned long long *>(static_cast<char *>(tmp) + ((std::max(tb, tb2) + 15) & ~size_t(15)));
     cudaError_t e1 = cub::DeviceRadixSort::SortKeys(tmp, tb, db, (int64_t)h, 0, 64, s);
     unsigned long long *sorted = db.Current(), *other = db.Alternate();
@@ -704,7 +705,7 @@ extern "C" int accx_scan_pairs(accx_graph *g, int32_t *pairs, uint64_t cap, uint
   if (!q->npairs) return ACCX_OK;
   int32_t *tmp = nullptr;
   bool dev = accx_is_device_ptr(pairs);
-  if (dev) tmp = pairs; else ACCX_CUDA_TRY(accx_dev_alloc((void **)&tmp, sizeof(int32_t) * 2 * q->npairs, s));
+  if (dev) tmp = pairs; else ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&tmp, sizeof(int32_t) * 2 * q->npairs, s));
   k_keys_to_pairs<<<accx_sm_count(g->device) * 8, 256, 0, s>>>(q->d_pairs, q->npairs, tmp);
   ACCX_CUDA_TRY(cudaGetLastError());
   if (!dev) {

@@ -130,3 +130,73 @@ def op(g):
     return g.count(policy='bitmap', bias=2, orient=True)
 sweep(graph, op, same_counts, ROOMS)
 """)
+
+
+# the default policy's count of a larger graph keeps lists for the next one: what a query, an
+# oriented count or a relabel of the same graph needs after it may take their place
+@pytest.mark.parametrize("op,check", [
+    ("lambda g: g.scan(0.3, 3)", "same_scan"),
+    ("lambda g: g.count(policy='merge', bias=2, orient=True)", "same_counts"),
+    ("lambda g: (g.relabel(), g.count(policy='bitmap', bias=2, orient=True))[1]", "same_counts")])
+def test_lists_of_the_default_count_are_given_back(op, check):
+    _child("""
+op, check = %s, %s
+STEP = 1 << 18
+def least(**kw):
+    "after a count: what it took, and the smallest room (in steps) beside it at which op answers"
+    base = used()
+    for k in range(400):
+        g = graph()
+        b = used()
+        g.count(out=None, bias=2, **kw)
+        took = used() - b
+        held = leave(k * STEP)
+        try:
+            check(op(g))
+            done = True
+        except accx.AccxError as e:
+            assert e.status == accx.ERR_OOM
+            done = False
+        give(held)
+        check(op(g))
+        same_counts(g.count(bias=2))
+        g.free()
+        assert used() == base
+        if done:
+            return took, k
+    assert False
+took, room = least(policy='gallop')
+took2, room2 = least()
+lists = (took2 - took) // STEP
+print(room, room2, lists)
+assert lists * STEP > 7 * len(dst)  # two words an entry and more
+assert room2 <= max(0, room - lists) + 2, (room, room2, lists)
+""" % (op, check))
+
+
+def test_captured_lists_stay():
+    _child("""
+import torch
+g = graph(bias=2)
+before = used()
+s = torch.cuda.Stream()
+torch.cuda.synchronize()
+cg = torch.cuda.CUDAGraph()
+with torch.cuda.graph(cg, stream=s):
+    g.count(bias=2, out=None, stream=s.cuda_stream)
+held = leave(1 << 16)
+for op in (lambda: g.scan(0.3, 3), lambda: g.count(policy='merge', bias=2, orient=True), lambda: g.relabel()):
+    try:
+        op()
+        assert False
+    except accx.AccxError as e:
+        assert e.status == accx.ERR_OOM
+g2 = g.count(policy='gallop', bias=9)
+assert np.array_equal(g2, ref["cnn"] + 7)
+cg.replay()
+torch.cuda.synchronize()
+same_counts(g.read_counts())
+give(held)
+g.count(bias=2, out=None)  # the handle's bias is the last count's, not the replay's
+same_scan(g.scan(0.3, 3))
+""")

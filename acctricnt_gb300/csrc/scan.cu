@@ -486,6 +486,18 @@ void accx_query_ctx_release(accx_query_ctx *q) {
   *q = accx_query_ctx();
 }
 
+// A temporary of the pool, freed on its stream on every way out of a call.
+struct stream_block {
+  void *p = nullptr;
+  cudaStream_t s;
+  explicit stream_block(cudaStream_t st) : s(st) {}
+  ~stream_block() {
+    if (p) cudaFreeAsync(p, s);
+  }
+  stream_block(const stream_block &) = delete;
+  stream_block &operator=(const stream_block &) = delete;
+};
+
 static int ensure_query_arrays(const accx_graph *g, accx_query_ctx *q) {
   if (q->d_simbits && (q->n != g->n || q->m != g->m)) return ACCX_ERR_INVALID_ARG;  // made for another graph
   accx_graph *gm = const_cast<accx_graph *>(g);  // which may give scratch back
@@ -544,10 +556,11 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
   // the caller's similarity bytes come from the same pass: into device memory that allows
   // 8-byte stores, or into a buffer that is then copied to the host
   const bool sim_dev = sim && m && accx_is_device_ptr(sim);
-  uint8_t *sim_tmp = nullptr, *sim_out = sim_dev && !((uintptr_t)sim & 7) ? sim : nullptr;
+  stream_block sim_tmp(s);
+  uint8_t *sim_out = sim_dev && !((uintptr_t)sim & 7) ? sim : nullptr;
   if (sim && m && !sim_dev) {
-    ACCX_CUDA_TRY(accx_graph_alloc(const_cast<accx_graph *>(g), (void **)&sim_tmp, m, s));
-    sim_out = sim_tmp;
+    ACCX_CUDA_TRY(accx_graph_alloc(const_cast<accx_graph *>(g), &sim_tmp.p, m, s));
+    sim_out = static_cast<uint8_t *>(sim_tmp.p);
   }
   if (m) k_sim_keys<<<sms * 8, 256, 0, s>>>(g->d_simkey, g->d_off, g->d_src, g->d_dst, g->d_cnt, m, g->cnt_bias, sq, klo,
                                             khi, reinterpret_cast<uint8_t *>(q->d_simbits), sim_out, q->d_qcounters);
@@ -580,10 +593,9 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
     k_bits_to_bytes<<<sms * 8, 256, 0, s>>>(q->d_simbits, m, sim);
     ACCX_CUDA_TRY(cudaGetLastError());
   }
-  if (sim_tmp) {
-    cudaError_t e1 = cudaMemcpyAsync(sim, sim_tmp, m, cudaMemcpyDeviceToHost, s);
+  if (sim_tmp.p) {
+    cudaError_t e1 = cudaMemcpyAsync(sim, sim_out, m, cudaMemcpyDeviceToHost, s);
     cudaError_t e2 = cudaStreamSynchronize(s);
-    cudaFreeAsync(sim_tmp, s);
     if (e1 != cudaSuccess || e2 != cudaSuccess) return ACCX_ERR_CUDA;
   }
   if (label) {
@@ -703,15 +715,15 @@ extern "C" int accx_scan_pairs(accx_graph *g, int32_t *pairs, uint64_t cap, uint
   if (!pairs) return ACCX_OK;
   if (cap < q->npairs) return ACCX_ERR_TOO_LARGE;
   if (!q->npairs) return ACCX_OK;
-  int32_t *tmp = nullptr;
-  bool dev = accx_is_device_ptr(pairs);
-  if (dev) tmp = pairs; else ACCX_CUDA_TRY(accx_graph_alloc(g, (void **)&tmp, sizeof(int32_t) * 2 * q->npairs, s));
+  stream_block block(s);
+  const bool dev = accx_is_device_ptr(pairs);
+  if (!dev) ACCX_CUDA_TRY(accx_graph_alloc(g, &block.p, sizeof(int32_t) * 2 * q->npairs, s));
+  int32_t *tmp = dev ? pairs : static_cast<int32_t *>(block.p);
   k_keys_to_pairs<<<accx_sm_count(g->device) * 8, 256, 0, s>>>(q->d_pairs, q->npairs, tmp);
   ACCX_CUDA_TRY(cudaGetLastError());
   if (!dev) {
     cudaError_t e1 = cudaMemcpyAsync(pairs, tmp, sizeof(int32_t) * 2 * q->npairs, cudaMemcpyDeviceToHost, s);
     cudaError_t e2 = cudaStreamSynchronize(s);
-    cudaFreeAsync(tmp, s);
     if (e1 || e2) return ACCX_ERR_CUDA;
   }
   return ACCX_OK;

@@ -200,3 +200,19 @@ give(held)
 g.count(bias=2, out=None)  # the handle's bias is the last count's, not the replay's
 same_scan(g.scan(0.3, 3))
 """)
+
+
+def test_query_and_pairs():
+    _child("""
+def op(g):
+    r = g.scan(0.3, 3)
+    r["pairs"] = g.pairs()
+    return r
+want = graph(bias=2)
+want.scan(0.3, 3)
+pairs = want.pairs()
+def check(r):
+    same_scan(r)
+    assert np.array_equal(r["pairs"], pairs)
+sweep(lambda: graph(policy='gallop', bias=2), op, check, ROOMS)
+""")

@@ -70,7 +70,14 @@ static int build_csr(accx_graph *g, K *d_keys, uint64_t nkeys, uint32_t n, const
         cub::DeviceSelect::Unique(nullptr, t2, d_keys, d_keys, d_res, (int64_t)nkeys, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     const size_t alt = (sizeof(K) * (nkeys ? nkeys : 1) + 255) & ~(size_t)255;
     size_t tb = t1 > t2 ? t1 : t2;
-    if (accx_dev_alloc((void **)&tmp, alt + 256 + (tb ? tb : 1), s) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+    if (accx_dev_alloc((void **)&tmp, alt + 256 + (tb ? tb : 1), s) != cudaSuccess) {
+      // no room to sort them, but a defect of the edges comes first
+      int bad = 0;
+      rc = d_bad && cudaMemcpyAsync(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+           cudaStreamSynchronize(s) == cudaSuccess && bad ? ACCX_ERR_RANGE : ACCX_ERR_OOM;
+      cudaGetLastError();
+      break;
+    }
     d_res = reinterpret_cast<unsigned long long *>(tmp + alt);
     void *d_tmp = tmp + alt + 256;
     db = cub::DoubleBuffer<K>(d_keys, reinterpret_cast<K *>(tmp));

@@ -216,3 +216,36 @@ def check(r):
     assert np.array_equal(r["pairs"], pairs)
 sweep(lambda: graph(policy='gallop', bias=2), op, check, ROOMS)
 """)
+
+
+def test_edge_lists_with_an_id_out_of_range():
+    """Named as such wherever the keys themselves fit, also where their sort does not."""
+    _child("""
+n = len(off) - 1
+src = np.repeat(np.arange(n), np.diff(off)).astype(np.uint32)
+bad = dst.astype(np.uint32).copy()
+bad[len(bad) // 3] = n
+block = 4 * 2 * len(src) + 2 * 4 * len(src)  # 32-bit keys of both directions, the two lists
+base = used()
+good = {}
+for room in [k << 18 for k in range(0, 120, 2)]:
+    held = leave(room)
+    for what, d in (("good", dst.astype(np.uint32)), ("bad", bad)):
+        try:
+            g = accx.Graph.from_edges(src, d, n)
+            assert what == "good"
+            o, a = g.download()
+            assert np.array_equal(o, off) and np.array_equal(a, dst)
+            g.free()
+            good[room] = True
+        except accx.AccxError as e:
+            assert e.status in ((accx.ERR_OOM,) if what == "good" else (accx.ERR_OOM, accx.ERR_RANGE)), (room, e)
+            if what == "good":
+                good[room] = False
+            elif room > block + (2 << 20):
+                assert e.status == accx.ERR_RANGE, (room, block)
+    give(held)
+    assert used() == base
+assert any(not v and r > block + (2 << 20) for r, v in good.items())  # rooms where only the sort does not fit
+assert good[max(good)]
+""")

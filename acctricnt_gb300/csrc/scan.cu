@@ -354,11 +354,20 @@ __global__ void __launch_bounds__(HOOK_WARPS * 32) k_hook_words(const uint32_t *
   }
 }
 
+// Every core's parent to its root.  Other threads shorten the same paths: all writes are
+// minima, so that one with an ancestor read earlier never undoes a root written since (with
+// plain stores a core could keep an ancestor for its cluster).
 __global__ void k_compress(uint32_t n, const uint32_t *__restrict__ corebits, int32_t *parent) {
   volatile int32_t *vp = parent;
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
     if (!accx_is_core(corebits, u)) continue;
-    parent[u] = uf_find(vp, (int32_t)u);
+    int32_t prev = (int32_t)u, cur = vp[u], next;
+    while (cur > (next = vp[cur])) {
+      atomicMin(&parent[prev], next);
+      prev = cur;
+      cur = next;
+    }
+    atomicMin(&parent[u], cur);
   }
 }
 

@@ -35,7 +35,8 @@
 #define Q_DIGEST 6
 #define Q_BIG 7
 #define Q_CORELIST 8   // cores with short rows, in the core list
-#define Q_PUSH 9       // slices of the other cores' rows
+#define Q_PUSH 9       // slices of the other cores' rows, and those cores times Q_LONG
+#define Q_LONG (1ull << 40)
 #define Q_NUM 10
 
 __device__ __forceinline__ unsigned long long accx_mix64_dev(unsigned long long x) {
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(256) k_sim_keys(const float *__restrict__ key,
 #define BIG_ROW 4096
 #define PUSH_ROW 256u     // cores with rows up to this are one warp's work
 #define PUSH_SLICE 512u   // entries of a longer core row a warp pushes
+#define CORE_KEEP 64u     // groups of 32 vertices with listed cores a warp gathers before one atomic places them
 __device__ __forceinline__ uint32_t accx_row_word(const uint32_t *__restrict__ bits, uint32_t w, uint32_t b,
                                                   uint32_t e) {
   uint32_t x = __ldg(bits + w);
@@ -212,7 +214,7 @@ __device__ __forceinline__ uint32_t accx_row_word(const uint32_t *__restrict__ b
 __device__ __forceinline__ void accx_push_slices(uint32_t u, uint32_t deg, uint2 *__restrict__ push,
                                                  unsigned long long *__restrict__ qc) {
   const uint32_t ns = (deg + PUSH_SLICE - 1) / PUSH_SLICE;
-  const unsigned long long p = atomicAdd(&qc[Q_PUSH], (unsigned long long)ns);
+  const unsigned long long p = atomicAdd(&qc[Q_PUSH], Q_LONG + ns) % Q_LONG;
   for (uint32_t j = 0; j < ns; j++) push[p + j] = make_uint2(u, j);
 }
 
@@ -222,8 +224,24 @@ __global__ void __launch_bounds__(256) k_cores(const uint32_t *__restrict__ off,
                                                int32_t *__restrict__ hubmax, uint32_t *__restrict__ corebits,
                                                uint32_t *__restrict__ big, uint32_t *__restrict__ corelist,
                                                uint2 *__restrict__ push, unsigned long long *__restrict__ qc) {
+  __shared__ uint2 s_keep[8][CORE_KEEP];  // first vertex and which of its 32
+  uint2 *keep = s_keep[threadIdx.x >> 5];
+  uint32_t groups = 0, kept = 0;
   const uint32_t stride = gridDim.x * blockDim.x;  // a multiple of 32
   const int lane = threadIdx.x & 31;
+  auto flush = [&]() {
+    __syncwarp();
+    unsigned long long p = 0;
+    if (lane == 0) p = atomicAdd(&qc[Q_CORELIST], (unsigned long long)kept);
+    p = __shfl_sync(ACCX_FULL_MASK, p, 0);
+    for (uint32_t i = 0; i < groups; i++) {
+      const uint2 g = keep[i];
+      if ((g.y >> lane) & 1u) corelist[p + __popc(g.y & ((1u << lane) - 1u))] = g.x + lane;
+      p += __popc(g.y);
+    }
+    __syncwarp();
+    groups = kept = 0;
+  };
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < ((n + 31) & ~31u); u += stride) {
     uint32_t b = 0, e = 0, c = 0;
     if (u < n) {
@@ -250,13 +268,13 @@ __global__ void __launch_bounds__(256) k_cores(const uint32_t *__restrict__ off,
     const bool brief = core && deg <= PUSH_ROW;
     const unsigned bw = __ballot_sync(ACCX_FULL_MASK, brief);
     if (bw) {
-      unsigned long long p = 0;
-      if (lane == 0) p = atomicAdd(&qc[Q_CORELIST], (unsigned long long)__popc(bw));
-      p = __shfl_sync(ACCX_FULL_MASK, p, 0);
-      if (brief) corelist[p + __popc(bw & ((1u << lane) - 1u))] = u;
+      if (lane == 0) keep[groups] = make_uint2(u, bw);
+      kept += __popc(bw);
+      if (++groups == CORE_KEEP) flush();
     }
     if (core && !brief) accx_push_slices(u, deg, push, qc);
   }
+  if (groups) flush();
 }
 
 __global__ void __launch_bounds__(256) k_cores_big(const uint32_t *__restrict__ off, int mu,
@@ -304,27 +322,79 @@ __device__ __forceinline__ int32_t uf_find(volatile int32_t *parent, int32_t x) 
   return cur;
 }
 
-// Union over similar core-core entries.  A warp takes 32 similarity words, gathers the
-// entries of their set bits in shared memory and then gives every lane one entry: an
-// entry is a chain of dependent random reads, so a thread working off a word's bits alone
-// left most of the machine waiting (R-MAT 22: 96 us; R-MAT 16: 61).  UnionThreadSafe
-// (union_find.h:22-35): hook the larger root under the smaller.
-// FIRST: a first pass that only lowers each core's parent to its smallest similar core
-// neighbour (one atomic minimum an entry, nothing to wait for or to retry).  It loses
-// links, but the second pass unites over every entry again and finds nearly all of them
-// done, where without it the cores of one big cluster fight over the same roots (both
-// passes: R-MAT 22 55 us, R-MAT 16 27; the second alone 112 and 73).
-#define HOOK_WARPS 4
-template <bool FIRST>
+// Union of two cores' components.  UnionThreadSafe (union_find.h:22-35): hook the larger
+// root under the smaller.
+__device__ __forceinline__ void uf_unite(volatile int32_t *vp, int32_t *parent, uint32_t u, uint32_t v) {
+  for (;;) {
+    int32_t ru = uf_find(vp, (int32_t)u), rv = uf_find(vp, (int32_t)v);
+    if (ru == rv) break;
+    int32_t lo = ru < rv ? ru : rv, hi = ru < rv ? rv : ru;
+    if (atomicCAS(&parent[hi], hi, lo) == hi) break;
+  }
+}
+
+// Union over similar core-core entries, in one of two forms; a kernel returns at once when
+// the query is not its own.
+// hook_words, few similar entries a core (below HOOK_DENSE): a thread a word of the similarity
+// bits, whose entries are mostly one row's and are united one after another.  There is little
+// to fight over.  On graphs of HOOK_OWN entries and more it is a kernel of its own, which has the
+// L1 to itself (with the other form's shared memory a ring of 16 entries a vertex took 714
+// us, without 576); on smaller ones the launch costs more (2 us) than that.
+// By lanes, many: a warp takes 32 words, gathers the entries of their set bits in shared
+// memory and gives every lane one entry (an entry is a chain of dependent random reads: a
+// thread working off a word's bits alone left most of the machine waiting).  A first pass
+// (FIRST) lowers cores' parents to their smallest similar core neighbour, one atomic minimum
+// an entry, nothing to wait for or to retry.  It loses links, but the second unites over
+// every entry again and finds nearly all of them done, where without it the cores of one big
+// cluster fight over the same roots.  An eighth of the vertices, by a hash, stay out of the
+// first pass: where ids follow the graph's layout (a ring, a lattice) the minima would make
+// chains of many thousands of links that the second has to walk.
+// The whole union, us, by lanes / by words: R-MAT 22 50 / 176, R-MAT 16 with 64 edges a
+// vertex 58 / 204, cliques of 1500 91 / 334; Erdos-Renyi 2M with 6 similar entries a core
+// 1350 / 666, power law 1M 546 / 145, ring of 16 entries a vertex 1170 / 576, cliques of 20
+// 56 / 58.
+#define HOOK_WARPS 8
+#define HOOK_DENSE 32ull
+__device__ __forceinline__ int hook_kind(const unsigned long long *__restrict__ qc) {  // 0: nothing to unite
+  const unsigned long long cores = qc[Q_CORELIST] + qc[Q_PUSH] / Q_LONG;
+  return cores < 2 ? 0 : qc[Q_SIMILAR] < HOOK_DENSE * cores ? 1 : 2;
+}
+#define HOOK_OWN (1u << 22)
+__device__ __forceinline__ void hook_words(const uint32_t *__restrict__ src, const int32_t *__restrict__ dst, uint32_t m,
+                                           const uint32_t *__restrict__ simbits,
+                                           const uint32_t *__restrict__ corebits, int32_t *parent) {
+  volatile int32_t *vp = parent;
+  const uint32_t words = (m + 31) / 32;
+  for (uint32_t wi = blockIdx.x * blockDim.x + threadIdx.x; wi < words; wi += gridDim.x * blockDim.x)
+    for (uint32_t w = __ldg(simbits + wi); w; w &= w - 1) {
+      const uint32_t e = wi * 32u + (uint32_t)(__ffs(w) - 1), v = (uint32_t)__ldg(dst + e);
+      if (!accx_is_core(corebits, v)) continue;
+      const uint32_t u = __ldg(src + e);
+      if (u < v && accx_is_core(corebits, u)) uf_unite(vp, parent, u, v);
+    }
+}
 __global__ void __launch_bounds__(HOOK_WARPS * 32) k_hook_words(const uint32_t *__restrict__ src,
                                                                 const int32_t *__restrict__ dst, uint32_t m,
                                                                 const uint32_t *__restrict__ simbits,
                                                                 const uint32_t *__restrict__ corebits,
+                                                                const unsigned long long *__restrict__ qc,
                                                                 int32_t *parent) {
-  __shared__ uint32_t s_q[HOOK_WARPS][1024];
+  if (hook_kind(qc) == 1) hook_words(src, dst, m, simbits, corebits, parent);
+}
+template <bool FIRST>
+__global__ void __launch_bounds__(HOOK_WARPS * 32) k_hook_lanes(const uint32_t *__restrict__ src,
+                                                                const int32_t *__restrict__ dst, uint32_t m,
+                                                                const uint32_t *__restrict__ simbits,
+                                                                const uint32_t *__restrict__ corebits,
+                                                                const unsigned long long *__restrict__ qc,
+                                                                int32_t *parent) {
+  __shared__ uint16_t s_q[HOOK_WARPS][1024];  // places in the warp's 32 words
+  const int kind = hook_kind(qc);
+  if (FIRST && kind == 1 && m < HOOK_OWN) hook_words(src, dst, m, simbits, corebits, parent);
+  if (kind != 2) return;
   volatile int32_t *vp = parent;
   const int lane = threadIdx.x & 31;
-  uint32_t *q = s_q[threadIdx.x >> 5];
+  uint16_t *q = s_q[threadIdx.x >> 5];
   const uint32_t words = (m + 31) / 32, nw = gridDim.x * HOOK_WARPS;
   for (unsigned long long w0 = 32ull * (blockIdx.x * HOOK_WARPS + (threadIdx.x >> 5)); w0 < words; w0 += 32ull * nw) {
     const uint32_t wi = (uint32_t)w0 + lane;
@@ -337,18 +407,13 @@ __global__ void __launch_bounds__(HOOK_WARPS * 32) k_hook_words(const uint32_t *
     }
     const uint32_t total = __shfl_sync(ACCX_FULL_MASK, at, 31);
     at -= __popc(w);
-    for (; w; w &= w - 1) q[at++] = wi * 32u + (uint32_t)(__ffs(w) - 1);
+    for (; w; w &= w - 1) q[at++] = (uint16_t)(lane * 32 + __ffs(w) - 1);
     __syncwarp();
     for (uint32_t i = lane; i < total; i += 32) {
-      const uint32_t e = q[i], u = __ldg(src + e), v = (uint32_t)__ldg(dst + e);
+      const uint32_t e = (uint32_t)w0 * 32u + q[i], u = __ldg(src + e), v = (uint32_t)__ldg(dst + e);
       if (u >= v || !accx_is_core(corebits, v) || !accx_is_core(corebits, u)) continue;
-      if (FIRST) atomicMin(&parent[v], (int32_t)u);
-      while (!FIRST) {
-        int32_t ru = uf_find(vp, (int32_t)u), rv = uf_find(vp, (int32_t)v);
-        if (ru == rv) break;
-        int32_t lo = ru < rv ? ru : rv, hi = ru < rv ? rv : ru;
-        if (atomicCAS(&parent[hi], hi, lo) == hi) break;
-      }
+      if (!FIRST) uf_unite(vp, parent, u, v);
+      else if ((v * 0x9E3779B1u) >> 29) atomicMin(&parent[v], (int32_t)u);
     }
     __syncwarp();
   }
@@ -376,7 +441,16 @@ __global__ void k_compress(uint32_t n, const uint32_t *__restrict__ corebits, in
 // core neighbour counts).  A warp per listed core with a short row, or per slice of a
 // longer row: walking the core bitmap instead, one warp had all the cores of a word,
 // whose rows can be hubs' (R-MAT 13: 86 us, now 8; R-MAT 22, with a grid of CTAs for the
-// longest rows: 97, now 70).
+// longest rows: 97, now 70).  Where a warp has HUB_PACK listed cores and more, it takes 32 at a
+// time and streams their rows as one (a lattice of 6M cores with four entries each
+// 777 us with a row a step).
+#define HUB_PACK 16u
+__device__ __forceinline__ void accx_hub_credit(uint32_t u, int32_t r, const uint32_t *__restrict__ corebits,
+                                                int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax) {
+  if (u == 0xffffffffu || accx_is_core(corebits, u)) return;
+  atomicMin(&hubmin[u], r);
+  atomicMax(&hubmax[u], r);
+}
 __device__ __forceinline__ void accx_hub_range(const int32_t *__restrict__ dst, uint32_t b, uint32_t e, int32_t r,
                                                int lane, const uint32_t *__restrict__ corebits,
                                                int32_t *__restrict__ hubmin, int32_t *__restrict__ hubmax) {
@@ -389,11 +463,7 @@ __device__ __forceinline__ void accx_hub_range(const int32_t *__restrict__ dst, 
       u[k] = i < len ? (uint32_t)__ldg(dst + b + i) : 0xffffffffu;
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (u[k] == 0xffffffffu || accx_is_core(corebits, u[k])) continue;
-      atomicMin(&hubmin[u[k]], r);
-      atomicMax(&hubmax[u[k]], r);
-    }
+    for (int k = 0; k < 4; k++) accx_hub_credit(u[k], r, corebits, hubmin, hubmax);
   }
 }
 __global__ void __launch_bounds__(256) k_hub_push(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst,
@@ -402,17 +472,60 @@ __global__ void __launch_bounds__(256) k_hub_push(const uint32_t *__restrict__ o
                                                   const uint32_t *__restrict__ corebits,
                                                   const int32_t *__restrict__ parent, int32_t *__restrict__ hubmin,
                                                   int32_t *__restrict__ hubmax) {
-  const int lane = threadIdx.x & 31;
+  // the rows of 32 cores: where each begins in their concatenation, less its place in dst
+  __shared__ uint32_t s_pre[8][32], s_beg[8][32];
+  __shared__ int32_t s_root[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned long long nw = (gridDim.x * blockDim.x) >> 5, w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long np = qc[Q_PUSH], nc = qc[Q_CORELIST];
+  const unsigned long long np = qc[Q_PUSH] % Q_LONG, nc = qc[Q_CORELIST];
   for (unsigned long long i = w0; i < np; i += nw) {
     const uint2 it = __ldg(push + i);
     const uint32_t b = __ldg(off + it.x) + it.y * PUSH_SLICE, e = accx_slice_end(b, PUSH_SLICE, __ldg(off + it.x + 1));
     accx_hub_range(dst, b, e, parent[it.x], lane, corebits, hubmin, hubmax);
   }
-  for (unsigned long long i = w0; i < nc; i += nw) {
-    const uint32_t v = __ldg(corelist + i);
-    accx_hub_range(dst, __ldg(off + v), __ldg(off + v + 1), parent[v], lane, corebits, hubmin, hubmax);
+  if (nc < HUB_PACK * nw) {
+    for (unsigned long long i = w0; i < nc; i += nw) {
+      const uint32_t v = __ldg(corelist + i);
+      accx_hub_range(dst, __ldg(off + v), __ldg(off + v + 1), parent[v], lane, corebits, hubmin, hubmax);
+    }
+    return;
+  }
+  uint32_t *pre = s_pre[warp], *beg = s_beg[warp];
+  int32_t *root = s_root[warp];
+  for (unsigned long long i = 32 * w0; i < nc; i += 32 * nw) {
+    uint32_t b = 0, len = 0;
+    if (i + lane < nc) {
+      const uint32_t v = __ldg(corelist + i + lane);
+      b = __ldg(off + v);
+      len = __ldg(off + v + 1) - b;
+      root[lane] = parent[v];
+    }
+    uint32_t incl = len;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t a = __shfl_up_sync(ACCX_FULL_MASK, incl, d);
+      if (lane >= d) incl += a;
+    }
+    const uint32_t tot = __shfl_sync(ACCX_FULL_MASK, incl, 31);
+    pre[lane] = incl - len;  // an empty row begins where the next one does
+    beg[lane] = b;
+    __syncwarp();
+    for (uint32_t c0 = 0; c0 < tot; c0 += 128) {
+      uint32_t u[4], s[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t c = c0 + 32 * k + lane;
+        // the last row that begins at or before c
+        uint32_t j = 0;
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) j += pre[j + d] <= c ? d : 0;
+        s[k] = j;
+        u[k] = c < tot ? (uint32_t)__ldg(dst + beg[j] + (c - pre[j])) : 0xffffffffu;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) accx_hub_credit(u[k], root[s[k]], corebits, hubmin, hubmax);
+    }
+    __syncwarp();
   }
 }
 
@@ -581,10 +694,12 @@ extern "C" int accx_scan_query_ctx(const accx_graph *g, accx_query_ctx *q, doubl
                                           q->d_qcounters);
   }
   if (m) {
-    k_hook_words<true><<<sms * 12, HOOK_WARPS * 32, 0, s>>>(g->d_src, g->d_dst, m, q->d_simbits, q->d_corebits,
-                                                           q->d_parent);
-    k_hook_words<false><<<sms * 12, HOOK_WARPS * 32, 0, s>>>(g->d_src, g->d_dst, m, q->d_simbits, q->d_corebits,
-                                                            q->d_parent);
+    const auto hook = [&](auto k) {
+      k<<<sms * 8, HOOK_WARPS * 32, 0, s>>>(g->d_src, g->d_dst, m, q->d_simbits, q->d_corebits, q->d_qcounters, q->d_parent);
+    };
+    if (m >= HOOK_OWN) hook(k_hook_words);
+    hook(k_hook_lanes<true>);
+    hook(k_hook_lanes<false>);
   }
   if (n) k_compress<<<sms * 4, 256, 0, s>>>(n, q->d_corebits, q->d_parent);
   if (n) k_hub_push<<<sms * 8, 256, 0, s>>>(g->d_off, g->d_dst, q->d_corelist, q->d_push, q->d_qcounters, q->d_corebits,

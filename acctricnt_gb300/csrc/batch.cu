@@ -91,7 +91,7 @@ extern "C" int accx_batch_create(accx_graph *const *graphs, int k, void *stream,
   do {
     if (accx_dev_alloc((void **)&u->d_off, sizeof(uint32_t) * (N + 1), nullptr) != cudaSuccess ||
         accx_dev_alloc((void **)&u->d_dst, sizeof(int32_t) * (M + ACCX_DST_PAD), nullptr) != cudaSuccess ||
-        cudaMalloc(&d_ds, sizeof(accx_batch_desc) * k) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
+        accx_dev_alloc((void **)&d_ds, sizeof(accx_batch_desc) * k, s) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
     if (accx_dev_wait(nullptr) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if (cudaMemcpyAsync(d_ds, ds.data(), sizeof(accx_batch_desc) * k, cudaMemcpyHostToDevice, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     uint32_t last = (uint32_t)M;
@@ -103,7 +103,7 @@ extern "C" int accx_batch_create(accx_graph *const *graphs, int k, void *stream,
     if ((rc = accx_tilerow_build(u, u->d_off, &u->d_tilerow, s)) != ACCX_OK) break;
     if (cudaStreamSynchronize(s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
   } while (0);
-  if (d_ds) cudaFree(d_ds);
+  accx_dev_free(d_ds, s);
   if (rc) {
     cudaGetLastError();
     accx_graph_free(u);

@@ -156,10 +156,10 @@ extern "C" int accx_vertex_ranges(const accx_graph *g, int parts, uint32_t *rang
   unsigned long long *cost = nullptr, *pre = nullptr;
   void *tmp = nullptr;
   size_t tb = 0;
-  ACCX_CUDA_TRY(cudaMalloc(&cost, sizeof(unsigned long long) * ((size_t)n + 1)));
-  cudaError_t e = cudaMalloc(&pre, sizeof(unsigned long long) * ((size_t)n + 1));
+  ACCX_CUDA_TRY(accx_dev_alloc((void **)&cost, sizeof(unsigned long long) * ((size_t)n + 1), s));
+  cudaError_t e = accx_dev_alloc((void **)&pre, sizeof(unsigned long long) * ((size_t)n + 1), s);
   if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, tb, cost, pre, (int64_t)n, s);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, tb + 16);
+  if (e == cudaSuccess) e = accx_dev_alloc(&tmp, tb + 16, s);
   std::vector<unsigned long long> h((size_t)n + 1, 0);
   if (e == cudaSuccess && n) {
     k_filtered_cost<<<accx_sm_count(g->device) * 8, 256, 0, s>>>(g->d_off, g->d_dst, n, cost);
@@ -167,10 +167,10 @@ extern "C" int accx_vertex_ranges(const accx_graph *g, int parts, uint32_t *rang
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data() + 1, pre, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
-  cudaFree(cost);
-  if (pre) cudaFree(pre);
-  if (tmp) cudaFree(tmp);
+  void *blocks[] = {cost, pre, tmp};
+  accx_dev_free_all(blocks, 3, s);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     accx_set_cuda_error(e, "vertex_ranges", __FILE__, __LINE__);
     return ACCX_ERR_CUDA;
   }

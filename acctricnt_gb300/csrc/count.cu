@@ -42,7 +42,8 @@
 #define C_LIGHT 17  // owners of the warp-per-owner kernel
 #define C_TICKET 18 // rows taken from the degree-ordered count's list
 #define C_DGBIG 19  // long rows of the default policy's degree-ordered count
-#define C_NUM 20
+#define C_DGLONG 20 // pieces of its longest rows
+#define C_NUM 21
 
 #define MERGE_WARPS 8        // warps per merge/gallop CTA
 #define ITEM_TARGET_DEFAULT (1u << 20)  // probe elements per bitmap work item
@@ -854,10 +855,13 @@ static bool alloc_dense(accx_graph *g) {
 }
 
 // Scratch of the degree-ordered count: entries and counters of the F lists (m each), the
-// F lengths and two lists of rows (n each), and the CTAs' items: at most a slice for each row of more than
-// DG_ROW_SMALL entries and one more per DG_SLICE entries.
+// F lengths and two lists of rows (n each), the CTAs' items: at most a slice for each row of more than
+// DG_ROW_SMALL entries and one more per DG_SLICE entries, and for the longest rows' pieces, at
+// most two a tile, their list and how many ids of F each has.
+static size_t dg_items(const accx_graph *g) { return (size_t)g->m / DG_ROW_SMALL + (size_t)g->m / DG_SLICE + 2; }
+static size_t dg_pieces(const accx_graph *g) { return 2 * ((size_t)g->m / DG_TILE + 1); }
 static bool alloc_degree(accx_graph *g) {
-  const size_t words = 2 * (size_t)g->m + 3 * (size_t)g->n + 2 + 2 * ((size_t)g->m / DG_ROW_SMALL + (size_t)g->m / DG_SLICE + 2);
+  const size_t words = 2 * (size_t)g->m + 3 * (size_t)g->n + 2 + 2 * dg_items(g) + 3 * dg_pieces(g);
   bool ok = accx_dev_alloc((void **)&g->d_dg, sizeof(uint32_t) * words, g->home) == cudaSuccess;
   if (ok) ok = accx_dev_wait(g->home) == cudaSuccess;
   if (!ok) cudaGetLastError();
@@ -978,8 +982,10 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
     const uint32_t row = m < DG_ROW_M ? DG_ROW_SMALL : DG_ROW;
     uint32_t *ent = g->d_dg, *mid = ent + 2 * (size_t)m, *big = mid + n, *flen = big + n;
     uint2 *heavy = reinterpret_cast<uint2 *>(g->d_dg + ((2 * (size_t)m + 3 * (size_t)n + 1) & ~(size_t)1));
-    k_dg_rows<<<sms * 8, DG_THREADS, 0, s>>>(off, dst, n, f, ent, fc, flen, big, mid, row, ctr);
-    k_dg_big<<<sms * 4, DG_THREADS, 0, s>>>(off, dst, f, ent, fc, flen, big, heavy, ctr);
+    uint2 *pieces = heavy + dg_items(g);
+    uint32_t *kept = reinterpret_cast<uint32_t *>(pieces + dg_pieces(g));
+    k_dg_rows<<<sms * 8, DG_THREADS, 0, s>>>(off, tilerow, dst, n, m, f, ent, fc, flen, big, mid, row, pieces, kept, ctr);
+    k_dg_big<<<sms * 4, DG_THREADS, 0, s>>>(off, dst, f, ent, fc, flen, big, pieces, kept, heavy, ctr);
     ACCX_MARK(1);
     const size_t smem = DG_SLOTS * 6u + DG_CAP * 4u;
     const size_t smid = sizeof(dg_warp<DG_WARP>) * DG_WARPS, slight = sizeof(dg_warp<DG_LIGHT>) * DG_WARPS;

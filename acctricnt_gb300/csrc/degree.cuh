@@ -34,6 +34,11 @@
 #define DG_CAP 1024u           // |F| staged at once by a CTA
 #define DG_SLOTS 4096u
 #define DG_THREADS 256
+// Rows above two tiles are cut at the entry tiles' ends and filtered by a CTA a piece: the keepers of
+// each piece are counted first (k_dg_rows), so that a piece knows where its part of F begins.
+// A CTA a row spent 1.5 us on 1024 entries: a star of 16M leaves took 25.1 ms (7.5 by an
+// intersection per edge), now 2.5; of 100K leaves 126 us (92), now 64.
+#define DG_TILE 8192u
 
 // Per-kind statistics of an edge whose larger degree is dl, the smaller ds.
 __device__ __forceinline__ void dg_stat(cl_stats &st, uint32_t dl, uint32_t ds) {
@@ -65,13 +70,70 @@ __device__ __forceinline__ bool dg_before(uint32_t v, uint32_t dv, uint32_t u, u
   return dv > du || (dv == du && v < u);
 }
 
+// The long rows' pieces in tile t: slot 2t, the row u that has the tile's first entry, and slot
+// 2t + 1, the row that begins inside the tile and has the next one's first entry (a long row
+// is longer than two tiles, so there are no others).  Keepers of every piece into kept[slot],
+// the pieces into a list.
+__device__ __forceinline__ void dg_count_pieces(const uint32_t *__restrict__ off, const uint32_t *__restrict__ tilerow,
+                                                const int32_t *__restrict__ dst, uint32_t m,
+                                                uint2 *__restrict__ pieces, uint32_t *__restrict__ kept,
+                                                unsigned long long *__restrict__ ctr) {
+  static_assert(DG_TILE % 256 == 0, "tiles of the row index");
+  __shared__ uint2 s_piece[2 * DG_THREADS];
+  __shared__ uint32_t s_pieces, s_sum;
+  const uint32_t tiles = m / DG_TILE + (m % DG_TILE ? 1u : 0u);
+  // neighbouring tiles to different CTAs
+  for (uint32_t t0 = 0; t0 < tiles; t0 += gridDim.x * DG_THREADS) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_pieces = 0;
+    __syncthreads();
+    const uint32_t t = t0 + threadIdx.x * gridDim.x + blockIdx.x;
+    if (t < tiles) {
+      const uint32_t u = __ldg(tilerow + t * (DG_TILE / 256u));
+      if (__ldg(off + u + 1) - __ldg(off + u) > 2 * DG_TILE) s_piece[atomicAdd(&s_pieces, 1u)] = make_uint2(u, 2 * t);
+      if (t + 1 < tiles) {
+        const uint32_t w = __ldg(tilerow + (t + 1) * (DG_TILE / 256u)), b = __ldg(off + w);
+        if (w != u && b < (t + 1) * DG_TILE && __ldg(off + w + 1) - b > 2 * DG_TILE)
+          s_piece[atomicAdd(&s_pieces, 1u)] = make_uint2(w, 2 * t + 1);
+      }
+    }
+    __syncthreads();
+    const uint32_t np = s_pieces;
+    for (uint32_t i = 0; i < np; i++) {
+      const uint2 pc = s_piece[i];
+      const uint32_t u = pc.x, b = __ldg(off + u), end = __ldg(off + u + 1), du = end - b, lo = (pc.y >> 1) * DG_TILE;
+      const uint32_t e0 = max(b, lo), len = accx_slice_end(lo, DG_TILE, end) - e0;
+      uint32_t c = 0;
+      for (uint32_t j0 = threadIdx.x; j0 < len; j0 += 4 * DG_THREADS) {
+        uint32_t v[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) v[r] = j0 + r * DG_THREADS < len ? (uint32_t)__ldg(dst + e0 + j0 + r * DG_THREADS) : u;
+#pragma unroll
+        for (int r = 0; r < 4; r++) c += dg_before(v[r], __ldg(off + v[r] + 1) - __ldg(off + v[r]), u, du);
+      }
+      if (threadIdx.x == 0) s_sum = 0;
+      __syncthreads();
+      c = __reduce_add_sync(ACCX_FULL_MASK, c);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, c);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        kept[pc.y] = s_sum;
+        pieces[atomicAdd(&ctr[C_DGLONG], 1ull)] = pc;
+      }
+    }
+  }
+}
+
 // F(u) into f[off[u] ..], the entries they came from into ent, their counters zeroed:
 // eight lanes a row, 32 entries a step.  Longer rows go to a list.
-__global__ void __launch_bounds__(DG_THREADS) k_dg_rows(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst,
-                                                        uint32_t n, int32_t *__restrict__ f, uint32_t *__restrict__ ent,
+__global__ void __launch_bounds__(DG_THREADS) k_dg_rows(const uint32_t *__restrict__ off,
+                                                        const uint32_t *__restrict__ tilerow,
+                                                        const int32_t *__restrict__ dst, uint32_t n, uint32_t m,
+                                                        int32_t *__restrict__ f, uint32_t *__restrict__ ent,
                                                         int32_t *__restrict__ fc, uint32_t *__restrict__ flen,
                                                         uint32_t *__restrict__ big, uint32_t *__restrict__ mid,
-                                                        uint32_t row, unsigned long long *__restrict__ ctr) {
+                                                        uint32_t row, uint2 *__restrict__ pieces,
+                                                        uint32_t *__restrict__ kept, unsigned long long *__restrict__ ctr) {
   static_assert(DG_ROW <= DG_WARP, "a listed row's F fits a warp's table");
   // the CTA's rows for the list, placed by one atomic at the end
   __shared__ unsigned long long s_st[9], s_at;
@@ -79,13 +141,14 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_rows(const uint32_t *__restri
   const int lane = threadIdx.x & 31, gl = lane & 7;
   if (threadIdx.x == 0) s_cnt = 0;
   __syncthreads();
+  dg_count_pieces(off, tilerow, dst, m, pieces, kept, ctr);
   const unsigned gmask = 0xffu << (lane & 24);
   cl_stats st;
   const uint32_t ng = gridDim.x * (DG_THREADS / 8);
   for (uint32_t u = blockIdx.x * (DG_THREADS / 8) + threadIdx.x / 8; u < n; u += ng) {
     const uint32_t b = __ldg(off + u), du = __ldg(off + u + 1) - b;
     if (du > row) {
-      if (gl == 0) big[atomicAdd(&ctr[C_DGBIG], 1ull)] = u;
+      if (gl == 0 && du <= 2 * DG_TILE) big[atomicAdd(&ctr[C_DGBIG], 1ull)] = u;
       continue;
     }
     uint32_t k = 0;
@@ -119,35 +182,51 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_rows(const uint32_t *__restri
     }
   }
   dg_stat_flush(st, s_st, ctr);  // its barriers come after the last row
-  const uint32_t kept = min(s_cnt, DG_KEEP);
-  if (threadIdx.x == 0 && kept) s_at = atomicAdd(&ctr[C_LIGHT], (unsigned long long)kept);
+  const uint32_t rows = min(s_cnt, DG_KEEP);
+  if (threadIdx.x == 0 && rows) s_at = atomicAdd(&ctr[C_LIGHT], (unsigned long long)rows);
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < kept; i += DG_THREADS) mid[s_at + i] = s_list[i];
+  for (uint32_t i = threadIdx.x; i < rows; i += DG_THREADS) mid[s_at + i] = s_list[i];
 }
 
-// The same for the listed rows, a CTA a row.
+// The same for the listed rows, a CTA a row or a piece of a long one.
 __global__ void __launch_bounds__(DG_THREADS) k_dg_big(const uint32_t *__restrict__ off, const int32_t *__restrict__ dst,
                                                        int32_t *__restrict__ f, uint32_t *__restrict__ ent,
                                                        int32_t *__restrict__ fc, uint32_t *__restrict__ flen,
-                                                       const uint32_t *__restrict__ big, uint2 *__restrict__ heavy,
+                                                       const uint32_t *__restrict__ big,
+                                                       const uint2 *__restrict__ pieces,
+                                                       const uint32_t *__restrict__ kept, uint2 *__restrict__ heavy,
                                                        unsigned long long *__restrict__ ctr) {
-  __shared__ unsigned long long s_st[9];
+  __shared__ unsigned long long s_st[9], s_at;
   __shared__ uint32_t s_w[DG_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   cl_stats st;
-  const uint32_t nb = (uint32_t)ctr[C_DGBIG];
-  for (uint32_t q = blockIdx.x; q < nb; q += gridDim.x) {
-    const uint32_t u = big[q], b = __ldg(off + u), du = __ldg(off + u + 1) - b;
-    uint32_t k = 0;
-    for (uint32_t i0 = 0; i0 < du; i0 += DG_THREADS * 4) {
+  const uint32_t np = (uint32_t)ctr[C_DGLONG], nb = (uint32_t)ctr[C_DGBIG];
+  for (uint32_t q = blockIdx.x; q < np + nb; q += gridDim.x) {
+    const uint2 pc = q < np ? pieces[q] : make_uint2(big[q - np], 0u);
+    const uint32_t u = pc.x, b = __ldg(off + u), end = __ldg(off + u + 1), du = end - b;
+    uint32_t e0 = b, e1 = end, k = 0;
+    if (q < np) {
+      const uint32_t lo = (pc.y >> 1) * DG_TILE, t = b / DG_TILE, pr = (pc.y >> 1) - t;  // pr earlier pieces
+      e0 = max(b, lo);
+      e1 = accx_slice_end(lo, DG_TILE, end);
+      for (uint32_t j = threadIdx.x; j < pr; j += DG_THREADS) k += kept[2 * (t + j) + (j == 0 && b % DG_TILE ? 1 : 0)];
+      k = __reduce_add_sync(ACCX_FULL_MASK, k);
+      if (lane == 0) s_w[warp] = k;
+      __syncthreads();
+      k = 0;
+      for (int w = 0; w < DG_THREADS / 32; w++) k += s_w[w];
+      __syncthreads();
+    }
+    const uint32_t len = e1 - e0;
+    for (uint32_t i0 = 0; i0 < len; i0 += DG_THREADS * 4) {
       uint32_t v[4], dv[4], mine = 0;  // a thread's entries are consecutive: ranks stay in order
       const uint32_t i = i0 + threadIdx.x * 4;
 #pragma unroll
-      for (int r = 0; r < 4; r++) v[r] = i + r < du ? (uint32_t)__ldg(dst + b + i + r) : 0u;
+      for (int r = 0; r < 4; r++) v[r] = i + r < len ? (uint32_t)__ldg(dst + e0 + i + r) : 0u;
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         dv[r] = __ldg(off + v[r] + 1) - __ldg(off + v[r]);
-        if (i + r < du && dg_before(v[r], dv[r], u, du)) mine |= 1u << r;
+        if (i + r < len && dg_before(v[r], dv[r], u, du)) mine |= 1u << r;
       }
       const uint32_t c = __popc(mine), incl = accx_warp_incl_sum(c, lane);
       if (lane == 31) s_w[warp] = incl;
@@ -160,20 +239,22 @@ __global__ void __launch_bounds__(DG_THREADS) k_dg_big(const uint32_t *__restric
       for (int r = 0; r < 4; r++)
         if ((mine >> r) & 1u) {
           f[p] = (int32_t)v[r];
-          ent[p] = b + i + r;
+          ent[p] = e0 + i + r;
           fc[p] = 0;
           p++;
           dg_stat(st, dv[r], du);
         }
       __syncthreads();
     }
-    if (threadIdx.x == 0) {
-      flen[u] = k;
+    if (e1 == end) {  // the row's last piece: k is all of F now
       const uint32_t ns = k > 1 ? (du + DG_SLICE - 1) / DG_SLICE : 0u;
-      if (ns) {
-        const unsigned long long p0 = atomicAdd(&ctr[C_HEAVY], (unsigned long long)ns);
-        for (uint32_t j = 0; j < ns; j++) heavy[p0 + j] = make_uint2(u, j);
+      if (threadIdx.x == 0) {
+        flen[u] = k;
+        if (ns) s_at = atomicAdd(&ctr[C_HEAVY], (unsigned long long)ns);
       }
+      __syncthreads();
+      for (uint32_t j = threadIdx.x; j < ns; j += DG_THREADS) heavy[s_at + j] = make_uint2(u, j);
+      __syncthreads();
     }
   }
   dg_stat_flush(st, s_st, ctr);

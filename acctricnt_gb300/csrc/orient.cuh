@@ -140,10 +140,16 @@ __device__ __forceinline__ uint32_t or_gallop_group(const int32_t *__restrict__ 
 // and the edge's credit goes to e; otherwise to the end of the partner range (x's
 // position in N(y)).  Two kernels, each of which returns at once when the edges are the
 // other's: where the partner lists average more than GALLOP_MEAN ids, groups of G lanes
-// take one edge each (k_gallop_or), else a lane does (k_gallop_lane).
+// take one edge each (k_gallop_or), else a lane does (k_gallop_lane).  Groups also take fewer
+// edges than k_gallop_lane has lanes (GALLOP_FEW): no lane has a second one then, and the
+// longest is the time (counts, us, lanes / groups: R-MAT 14 with 111K galloping edges in its
+// own numbering 196 / 97, R-MAT 13 152 / 79, a mixed table at R-MAT 12 148 / 118; cliques of
+// 20 with 380K 71 / 114, Erdos-Renyi with 1M 91 / 143).
 #define GALLOP_MEAN 24ull
+#define GALLOP_FEW 196608ull
 __device__ __forceinline__ bool or_gallop_long(const unsigned long long *__restrict__ ctr) {
-  return ctr[C_WORK + ACCX_KIND_GALLOP] > GALLOP_MEAN * ctr[C_EDGES + ACCX_KIND_GALLOP];
+  return ctr[C_WORK + ACCX_KIND_GALLOP] > GALLOP_MEAN * ctr[C_EDGES + ACCX_KIND_GALLOP] ||
+         ctr[C_EDGES + ACCX_KIND_GALLOP] < GALLOP_FEW;
 }
 struct or_gallop_edge {
   uint32_t xb, xe, yb, ye, at;  // owner range, partner range, the edge's prefix entry

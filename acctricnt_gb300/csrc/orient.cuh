@@ -883,7 +883,7 @@ __device__ __forceinline__ uint32_t or_piece(const int32_t *__restrict__ dst, ui
 // x, which the classifier keeps below W -- is staged as a dense bitmap over [0, W)
 // plus, per non-empty 32-bit word, the prefix position of the word's first id (rank of
 // an id = that base + popcount of the lower bits).  The warps then take the slice's
-// entries 32 at a time from a shared queue and need no barrier until its end: the
+// entries a ticket (at most 32) at a time from a shared queue and need no barrier until its end: the
 // classifier stored, per bitmap entry (x,y), where P(y) starts and its length cut at
 // min(x,y) (0 for other entries), one coalesced load.  A long probe list is walked by
 // the whole warp in pieces of LONG_PIECE ids, its bounds and hits staying in registers;
@@ -896,9 +896,20 @@ __device__ __forceinline__ uint32_t or_piece(const int32_t *__restrict__ dst, ui
 // entries with CTA scans and four barriers each, and one queue entry per long list:
 // ~0.15 ns a list and 0.84 ps an id at R-MAT 22 and 24 (R-MAT 24 count 69.2 -> 64.0 ms,
 // Chung-Lu 3M 4.12 -> 3.90).
+// A ticket is 32 entries of a long item, fewer of a short one, so that every warp gets four:
+// with 32 always, the items of graphs with long lists and short rows, down to 32 entries,
+// were one warp's work (counts, us, earlier form / 32 always / now: 3000 vertices of degree 850
+// in their own numbering 700 / 924 / 652, 100 cliques of 200 relabeled 558 / 607 / 473, with
+// 1024 threads 955 / 1457 / 602; R-MAT 22 12.4 -> 11.7 ms; two tickets a warp 11.8, one 12.4).
+// A ticket with more than four warps' share of the item's probes in long lists leaves them to
+// all warps, after a barrier that other items do without (vertices joined to all of 2000 hubs
+// and to a few of each other, in their own numbering: 279 / 478 / 274; R-MAT 24 +0.6 %).
 struct or_seg {
   uint32_t pre[33], beg[32], hit[32];
 };
+#define TICKET_MIN 4u     // entries of the smallest ticket
+#define TICKETS_PER 4u    // tickets a warp that an item is cut into, if they are 32 entries at most
+#define LEFT_CAP 64u      // lists that an item leaves to all warps
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__restrict__ off,
                                                        const int32_t *__restrict__ dst,
@@ -918,8 +929,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
   uint16_t *wbase = reinterpret_cast<uint16_t *>(ocnt + pcap + 32);  // nwords first-id positions
   __shared__ or_seg s_seg[NT / 32];
   // the next item, fetched while the current one is walked: x, its first and last entry
-  // to walk, row start and prefix length (x = 0xffffffff: none)
-  __shared__ uint32_t s_item[5], s_next;
+  // to walk, row start, prefix length and probes (x = 0xffffffff: none)
+  __shared__ uint32_t s_item[6], s_next;
+  __shared__ uint4 s_left[LEFT_CAP];  // (first entry, end, edge) of lists left to all warps
+  __shared__ uint32_t s_lists, s_taken;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31;
   or_seg &S = s_seg[tid >> 5];
@@ -938,6 +951,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
       s_item[2] = ub + (uint32_t)((unsigned long long)du * (sp + 1) / nsplit);
       s_item[3] = ub;
       s_item[4] = pre[x];
+      s_item[5] = (uint32_t)min(work_u[x] / nsplit, 0xffffffffull);
     }
     s_item[0] = x;
   };
@@ -947,6 +961,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
   __syncthreads();
   for (;;) {
     const uint32_t x = s_item[0], pa = s_item[1], pb = s_item[2], ub = s_item[3], px = s_item[4];
+    const uint32_t heavy = s_item[5] / max((uint32_t)nt >> 7, 1u);  // four warps' even share of the probes
     if (x == 0xffffffffu) break;
     const uint32_t pxs = px <= pcap ? px : 0;  // the classifier guarantees px <= pcap for bitmap owners
     for (uint32_t i = tid; i < pxs; i += nt) {
@@ -957,25 +972,37 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
       }
       ocnt[i] = 0;
     }
-    if (tid == 0) s_next = 0;
+    if (tid == 0) s_next = s_lists = s_taken = 0;
     __syncthreads();
     if (tid == 0) fetch();  // read by all after this item's last barrier
     __syncwarp();
+    const uint32_t tk = min(32u, max(TICKET_MIN, (pb - pa) / (TICKETS_PER * ((uint32_t)nt >> 5))));
     for (;;) {
       uint32_t r0 = 0;
-      if (lane == 0) r0 = atomicAdd(&s_next, 32u);
+      if (lane == 0) r0 = atomicAdd(&s_next, tk);
       r0 = __shfl_sync(ACCX_FULL_MASK, r0, 0);
       if (r0 >= pb - pa) break;
       r0 += pa;
       const uint32_t k = r0 + (uint32_t)lane;
       uint32_t sst = 0, len = 0;
-      if (k < pb) {
+      if ((uint32_t)lane < tk && k < pb) {
         const uint2 e = sl[k];
         sst = e.x;
         len = (e.y & OR_SL_GALLOP) ? 0u : e.y;  // galloping entries are not this kernel's
       }
       uint32_t hits = 0;
-      for (unsigned lm = __ballot_sync(ACCX_FULL_MASK, len >= LONG_SEG); lm; lm &= lm - 1) {
+      unsigned lm = __ballot_sync(ACCX_FULL_MASK, len >= LONG_SEG);
+      if (lm & (lm - 1)) {
+        if (__reduce_add_sync(ACCX_FULL_MASK, len >= LONG_SEG ? min(len, 1u << 26) : 0u) > heavy) {
+          // all warps take these after the last ticket
+          uint32_t p = 0;
+          if (lane == 0) p = atomicAdd(&s_lists, (uint32_t)__popc(lm));
+          p = __shfl_sync(ACCX_FULL_MASK, p, 0) + __popc(lm & ((1u << lane) - 1u));
+          if (len >= LONG_SEG && p < LEFT_CAP) s_left[p] = make_uint4(sst, sst + len, k, 0u);
+          lm = __ballot_sync(ACCX_FULL_MASK, len >= LONG_SEG && p >= LEFT_CAP);
+        }
+      }
+      for (; lm; lm &= lm - 1) {
         // a long list, walked in pieces of LONG_PIECE ids from the even entry at or
         // before its start
         const int src = __ffs(lm) - 1;
@@ -1052,6 +1079,25 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bitmap_or(const uint32_t *__r
       }
     }
     __syncthreads();
+    if (s_lists) {
+      for (;;) {
+        uint32_t i = 0;
+        if (lane == 0) i = atomicAdd(&s_taken, 1u);
+        i = __shfl_sync(ACCX_FULL_MASK, i, 0);
+        if (i >= min(s_lists, LEFT_CAP)) break;
+        const uint4 q = s_left[i];
+        uint32_t h = 0;
+        for (uint32_t j0 = q.x & ~1u; j0 < q.y; j0 = accx_entry_step(j0, 64u * 4u, q.y))
+          h += or_piece<4>(dst, j0, q.x, q.y, lane, W, words, wbase, ocnt, pxs, cnt);
+        h = __reduce_add_sync(ACCX_FULL_MASK, h);
+        if (lane == 0 && h) {
+          found += h;
+          if (q.z - ub < pxs) atomicAdd(&ocnt[q.z - ub], h);
+          else atomicAdd(cnt + (q.z - ub < px ? q.z : q.y), (int32_t)h);
+        }
+      }
+      __syncthreads();
+    }
     // owner-side credits to HBM, then clear what was staged
     for (uint32_t i = tid; i < pxs; i += nt) {
       const uint32_t h = ocnt[i];

@@ -241,63 +241,83 @@ __global__ void k_gather_counts(const int32_t *__restrict__ cnt_r, const uint32_
 // counting the block's prefix edges with K-bit rows.  An edge (c, b) of row c spares
 // about |P(c) ∩ [0, K)| probes (its partner's ids below K; within 20 % of the true
 // mean from scale 15 to 24) and costs two reads of a K-bit row, DENSE_COST probes
-// each.  Out: the gains, then the longest prefix of each block.
+// each.  Beside it the same with the partner's ids below K of one edge of each row, taken by a
+// hash: on a graph whose hubs are not joined to each other the first promises probes that
+// nothing makes (3000 x 3000 vertices, all joined to all, 297 us, with dense rows 787, now
+// 241; choosing K and M by the second alone cost R-MAT 24 3 %, the costs are fitted to the
+// first).  Out: both gains, then the longest prefix of each block.
 #define DENSE_COST make_float3(14.f, 22.f, 41.f)
 #define DENSE_KINDS 3
 #define DENSE_BLOCKS 256
+#define DENSE_ROWS_MAX 192u  // blocks of 1024 ids in the default bitmap window
 __global__ void __launch_bounds__(1024) k_dense_plan(const uint32_t *__restrict__ roff, const int32_t *__restrict__ rdst,
                                                      uint32_t n, float3 cost, float *__restrict__ out) {
-  __shared__ float s_g[DENSE_KINDS][32];
+  __shared__ float s_g[2 * DENSE_KINDS][32];
   __shared__ uint32_t s_p[32];
   const uint32_t x = blockIdx.x * 1024u + threadIdx.x;
   uint32_t p = 0;
-  float gain[DENSE_KINDS] = {0.f, 0.f, 0.f};
+  float gain[2 * DENSE_KINDS] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (x < n) {
     const uint32_t b = roff[x], e = roff[x + 1];
-    uint32_t hi = accx_lower_bound(rdst, b, e, (int32_t)x);
-    p = hi - b;
+    p = accx_lower_bound(rdst, b, e, (int32_t)x) - b;
     const float c[DENSE_KINDS] = {cost.x, cost.y, cost.z};
+    uint32_t hi = b + p;
 #pragma unroll
     for (int k = DENSE_KINDS - 1; k >= 0; k--) {
       hi = accx_lower_bound(rdst, b, hi, (int32_t)(1024u << k));
       gain[k] = (float)p * ((float)(hi - b) - 2.f * c[k]);
     }
+    if (p && blockIdx.x < DENSE_ROWS_MAX) {
+      const uint32_t at = __umulhi(x * 0x9E3779B1u, p);  // the edge's place in P(x)
+      const uint32_t y = (uint32_t)rdst[b + at], yb = roff[y], ye = roff[y + 1];
+      // the ids below K of P(y), or of P(x) below y where y owns the edge
+      uint32_t low = accx_lower_bound(rdst, yb, ye, (int32_t)min(y, 4096u));
+      const uint32_t py = (y > 4096u ? accx_lower_bound(rdst, low, ye, (int32_t)y) : low) - yb;
+      const bool own = p > py;
+      const uint32_t lb = own ? yb : b;
+      uint32_t le = own ? low : b + at;
+#pragma unroll
+      for (int k = DENSE_KINDS - 1; k >= 0; k--) {
+        le = accx_lower_bound(rdst, lb, le, (int32_t)(1024u << k));
+        gain[DENSE_KINDS + k] = (float)p * ((float)(le - lb) - 2.f * c[k]);
+      }
+    }
   }
 #pragma unroll
   for (int d = 16; d >= 1; d >>= 1)
 #pragma unroll
-    for (int k = 0; k < DENSE_KINDS; k++) gain[k] += __shfl_xor_sync(ACCX_FULL_MASK, gain[k], d);
+    for (int k = 0; k < 2 * DENSE_KINDS; k++) gain[k] += __shfl_xor_sync(ACCX_FULL_MASK, gain[k], d);
   p = __reduce_max_sync(ACCX_FULL_MASK, p);
   if ((threadIdx.x & 31) == 0) {
-    for (int k = 0; k < DENSE_KINDS; k++) s_g[k][threadIdx.x >> 5] = gain[k];
+    for (int k = 0; k < 2 * DENSE_KINDS; k++) s_g[k][threadIdx.x >> 5] = gain[k];
     s_p[threadIdx.x >> 5] = p;
   }
   __syncthreads();
-  if (threadIdx.x < DENSE_KINDS) {
+  if (threadIdx.x < 2 * DENSE_KINDS) {
     float t = 0.f;
     for (int w = 0; w < 32; w++) t += s_g[threadIdx.x][w];
     out[threadIdx.x * DENSE_BLOCKS + blockIdx.x] = t;
-  } else if (threadIdx.x == DENSE_KINDS) {
+  } else if (threadIdx.x == 2 * DENSE_KINDS) {
     uint32_t t = 0;
     for (int w = 0; w < 32; w++) t = max(t, s_p[w]);
-    reinterpret_cast<uint32_t *>(out)[DENSE_KINDS * DENSE_BLOCKS + blockIdx.x] = t;
+    reinterpret_cast<uint32_t *>(out)[2 * DENSE_KINDS * DENSE_BLOCKS + blockIdx.x] = t;
   }
 }
 
 // Picks K and M from the gains: the rows up to the block after which no more is
 // gained, at most 64 MiB of bits (half of L2), and only if that spares more than the
-// two extra launches (DENSE_MIN probes).
+// two extra launches (DENSE_MIN probes) and the rows' sampled edges gain too.
 #define DENSE_MIN 4e6f
-#define DENSE_ROWS_MAX 192u  // blocks of 1024 ids in the default bitmap window
 static void dense_choose(accx_graph *g, const float *out) {
   const uint32_t blocks = (g->n + 1023u) / 1024u < DENSE_BLOCKS ? (g->n + 1023u) / 1024u : DENSE_BLOCKS;
   float best = DENSE_MIN;
   for (uint32_t k = 0; k < DENSE_KINDS; k++) {
     const uint32_t K = 1024u << k, lim = (64u << 20) / (K / 8u) / 1024u;
-    float acc = 0.f;
+    float acc = 0.f, sampled = 0.f;
     for (uint32_t i = 0; i < blocks && i < lim && i < DENSE_ROWS_MAX; i++) {
       acc += out[k * DENSE_BLOCKS + i];
-      if (acc > best) {
+      sampled += out[(DENSE_KINDS + k) * DENSE_BLOCKS + i];
+      if (acc > best && sampled > 0.f) {
         best = acc;
         g->dense_k = K;
         g->dense_m = (i + 1) * 1024u < g->n ? (i + 1) * 1024u : g->n;
@@ -306,7 +326,7 @@ static void dense_choose(accx_graph *g, const float *out) {
   }
   g->plan_rows = blocks * 1024u;
   for (uint32_t i = 0; i < blocks; i++) {
-    const uint32_t p = reinterpret_cast<const uint32_t *>(out)[DENSE_KINDS * DENSE_BLOCKS + i];
+    const uint32_t p = reinterpret_cast<const uint32_t *>(out)[2 * DENSE_KINDS * DENSE_BLOCKS + i];
     if (p > g->plan_maxpre) g->plan_maxpre = p;
   }
 }
@@ -334,7 +354,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
   int rc = ACCX_OK;
   const size_t vn = ((size_t)n + 64) & ~(size_t)63;
   do {
-    if (accx_graph_alloc(g, (void **)&vtmp, sizeof(uint32_t) * (4 * vn + (DENSE_KINDS + 1) * DENSE_BLOCKS), g->home) != cudaSuccess ||
+    if (accx_graph_alloc(g, (void **)&vtmp, sizeof(uint32_t) * (4 * vn + (2 * DENSE_KINDS + 1) * DENSE_BLOCKS), g->home) != cudaSuccess ||
         accx_graph_alloc(g, (void **)&rdeg, sizeof(uint32_t) * (vn + 2 * RELABEL_NCLASS + 2), g->home) != cudaSuccess ||
         accx_graph_alloc(g, (void **)&g->d_roff, sizeof(uint32_t) * ((size_t)n + 1), g->home) != cudaSuccess ||
         accx_graph_alloc(g, (void **)&g->d_rdst, sizeof(int32_t) * ((size_t)m + ACCX_DST_PAD), g->home) != cudaSuccess ||
@@ -426,7 +446,7 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
     if (cudaMemsetAsync(g->d_rdst + m, 0xff, sizeof(int32_t) * ACCX_DST_PAD, s) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
     if ((rc = accx_tilerow_build(g, g->d_roff, &g->d_rtilerow, s)) != ACCX_OK) break;
     // 3. the dense rows of oriented counts
-    float plan[(DENSE_KINDS + 1) * DENSE_BLOCKS];
+    float plan[(2 * DENSE_KINDS + 1) * DENSE_BLOCKS];
     const bool dense = m && n;
     if (dense) {
       const uint32_t pb = (n + 1023u) / 1024u;

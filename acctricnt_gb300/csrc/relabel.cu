@@ -72,14 +72,34 @@ __device__ __forceinline__ uint32_t relabel_key(const relabel_view &g, uint32_t 
   return v < g.n ? __ldg(g.newid + v) : 0xffffffffu;
 }
 
-// Rows above 4096 entries, a CTA each: keys and original entries for the segmented sort.
-__global__ void __launch_bounds__(1024) k_big_rows(relabel_view g, uint32_t rows, uint32_t *__restrict__ key,
-                                                   uint32_t *__restrict__ val) {
-  for (uint32_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const uint32_t b = g.roff[r], d = g.roff[r + 1] - b, e0 = g.off[g.oldid[r]];
-    for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) {
-      key[b + i] = relabel_key(g, e0 + i);
-      val[b + i] = e0 + i;
+// Rows above 4096 entries: keys and original entries for the segmented sort.  A CTA takes
+// 4096 positions, which belong to one row or two (a CTA a row took 13 ms of
+// a star of 16M leaves).
+#define BIG_CHUNK 4096u
+__global__ void __launch_bounds__(256) k_big_rows(relabel_view g, uint32_t rows, uint32_t total,
+                                                  uint32_t *__restrict__ key, uint32_t *__restrict__ val) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t chunks = total / BIG_CHUNK + (total % BIG_CHUNK ? 1u : 0u);
+  for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+    const uint32_t p0 = c * BIG_CHUNK;
+    // the row of p0, by every warp
+    uint32_t r = 0, hi = rows;
+    while (hi - r > 1) {
+      const uint32_t step = (hi - r + 31) / 32, q = r + (uint32_t)lane * step;
+      const unsigned in = __ballot_sync(ACCX_FULL_MASK, q < hi && __ldg(g.roff + q) <= p0);
+      r += (31 - __clz(in)) * step;
+      hi = min(hi, r + step);
+    }
+    const uint32_t end = __ldg(g.roff + r + 1);
+    // an entry's place in the original less its position
+    const uint32_t d0 = __ldg(g.off + __ldg(g.oldid + r)) - __ldg(g.roff + r);
+    const uint32_t d1 = r + 1 < rows ? __ldg(g.off + __ldg(g.oldid + r + 1)) - end : 0u;
+    const uint32_t len = min(total - p0, BIG_CHUNK);
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < len; i += 256) {
+      const uint32_t p = p0 + i, e = p + (p < end ? d0 : d1);
+      key[p] = relabel_key(g, e);
+      val[p] = e;
     }
   }
 }
@@ -414,7 +434,8 @@ extern "C" int accx_graph_relabel(accx_graph *g, void *stream) {
         if (accx_graph_alloc(g, (void **)&key, sizeof(uint32_t) * 4 * kn + b3 + 16, g->home) != cudaSuccess) { rc = ACCX_ERR_OOM; break; }
         if (accx_dev_wait(g->home) != cudaSuccess) { rc = ACCX_ERR_CUDA; break; }
         uint32_t *val = key + kn, *key2 = key + 2 * kn, *val2 = key + 3 * kn;
-        k_big_rows<<<rb[0] < (uint32_t)sms * 2 ? rb[0] : sms * 2, 1024, 0, s>>>(view, rb[0], key, val);
+        const uint32_t chunks = pb[0] / BIG_CHUNK + 1;
+        k_big_rows<<<chunks < (uint32_t)sms * 8 ? chunks : sms * 8, 256, 0, s>>>(view, rb[0], pb[0], key, val);
         if (cub::DeviceSegmentedRadixSort::SortPairs(key + 4 * kn, b3, key, key2, val, val2, (int64_t)pb[0], (int64_t)rb[0],
                                                      g->d_roff, g->d_roff + 1, 0, bits, s) != cudaSuccess) {
           rc = ACCX_ERR_CUDA;

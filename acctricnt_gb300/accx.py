@@ -459,7 +459,7 @@ class Graph:
         return {KIND_NAMES[k]: {"edges": int(e[k]), "work": int(w[k])} for k in range(3)}
 
     def last_matches(self):
-        """Oriented counts: (common ids found per kind, ids probed by the bitmap kind)."""
+        """Oriented counts: (common ids found per kind, ids in the partner lists of the bitmap kind's edges)."""
         mt = np.zeros(3, np.uint64)
         pr = C.c_uint64()
         _check(lib.accx_cn_last_matches(self._h, _ptr(mt), C.byref(pr)), "cn_last_matches")

@@ -91,10 +91,10 @@ __device__ __forceinline__ bool accx_dense_edge(int policy, const uint8_t *table
 // Bound by its gathers' latency (Erdos-Renyi, 40M entries: issue 51 %, DRAM 29 %; fewer
 // scans and barriers changed nothing), so by the warps that fit: four entries a thread, with
 // 16-byte loads of ids and reverses, two entries' ranges a store and the rows of listed
-// entries in shared memory, take 48 registers and five CTAs an SM.  Eight entries, loaded
-// and stored one by one, with 64 registers and four CTAs: Erdos-Renyi 5M 1.46 ms, R-MAT 24
-// 5.16; now 1.18 and 4.45 (eight with wide loads 1.31 and 4.73, four with six CTAs 1.35
-// and 5.12).
+// entries in shared memory, take 48 registers and five CTAs an SM, without spills.  Eight
+// entries, loaded and stored one by one, with 64 registers and four CTAs: Erdos-Renyi 5M 1.46
+// ms, R-MAT 24 5.16; now 1.17 and 4.18 (before the fill of the counts was a store an entry less:
+// eight with wide loads 1.31 and 4.73, four with six CTAs 1.35 and 5.12, with five 1.18 and 4.45).
 #define CL_EPT 4
 // partner ranges of galloping entries carry this flag in their length (the
 // bitmap kernel skips them); prefix lengths stay below 2^31 on a symmetric CSR
@@ -809,22 +809,33 @@ static int g_block_warps = 32;
 static int g_dense_kb = 128;
 static int g_sparse_kb = 64;
 // Oriented bitmap kind: 256-thread CTAs, four per SM, with a 24 KiB window (owners
-// with ids below 196,608 use the bitmap kind, the others gallop).  Small CTAs run
-// a round's scans and barriers with fewer idle threads (most owners' rows are far
-// shorter than a CTA), and the low-degree owners past the window are cheaper to
-// gallop than to stage.  Whole counts (ms) by (CTA threads, window KiB):
-//   R-MAT 22: 256/24 18.9, 512/56 24.1 (the earlier default), 256/16 18.4
-//   R-MAT 24: 256/24 96.7, 512/56 98.6, 256/16 110.9 (too many owners gallop)
-//   Chung-Lu 20M (exponent 2.1): 256/24 46.0, 512/56 ~49; Erdos-Renyi 20M: 32.1, ~33.3
-// and with 256 threads a 32 KiB window (three CTAs per SM) or 128-thread CTAs
-// were slower at R-MAT 24 (95.4 and 93.5-127.4 ms for the bitmap phase alone).
+// with ids below 196,608 use the bitmap kind, the others gallop).  Small CTAs have fewer idle
+// threads at an item's barriers (most owners' rows are far shorter than a CTA), and the
+// low-degree owners past the window are cheaper to gallop than to stage.  Whole counts (ms)
+// by (CTA threads / window KiB):
+//                  256/16  256/20  256/24  256/28  256/32  512/40  512/56  1024/64
+//   R-MAT 18        0.58    0.58    0.59    0.59    0.59    0.60    0.60    0.64
+//   R-MAT 20        2.43    2.45    2.47    2.47    2.67    2.68    2.71    3.11
+//   R-MAT 22       11.83   11.77   11.88   11.81   13.19   12.45   12.57   13.92
+//   R-MAT 24       77.36   69.85   63.09   62.76   69.32   63.55   62.59   65.65
+//   Chung-Lu 3M     2.97    2.96    3.00    3.01    3.14    3.16    3.25    3.62
+//   Chung-Lu 20M   27.31   26.71   26.63   26.31   27.09   25.87   25.73   27.08
+//   Erdos-Renyi 20M galloping: 26.4-26.5 with all of them
+// (with 32 KiB three CTAs fit an SM; 16 and 20 send too many owners of R-MAT 24 to galloping).
 static int g_or_dense_kb = 24;
 static int g_or_counter_kb = 8;
 static int g_or_block_warps = 8;
 
 
 // Dense rows' scratch: item size, item capacity and the arrays (all or none).
-static uint32_t dense_chunk(const accx_graph *g) { return g->m < (1ull << 25) ? 256u : 512u; }
+// Entries an item: 256 on graphs below 2^25 entries, for more items than warps, else 512, for
+// fewer row ends.  Whole counts with 256 / 512: R-MAT 18 (7.6M entries) 592 / 603 us, R-MAT 20
+// (31M) 2.45 / 2.41 ms, R-MAT 22 (128M) 11.72 / 11.80, R-MAT 24 (521M) 63.8 / 63.1, Chung-Lu 3M
+// (62M) 2.99 / 3.00: never more than 2 % apart.
+#define DENSE_CHUNK_SMALL 256u
+#define DENSE_CHUNK 512u
+static_assert(DENSE_CHUNK < 1u << DENSE_PLANES && DENSE_CHUNK_SMALL < 1u << DENSE_PLANES, "an item's counters fit their planes");
+static uint32_t dense_chunk(const accx_graph *g) { return g->m < (1ull << 25) ? DENSE_CHUNK_SMALL : DENSE_CHUNK; }
 static uint32_t dense_cap(const accx_graph *g) { return g->dense_m + (uint32_t)(g->m / dense_chunk(g)) + 1u; }
 // the item counter lies behind the rows' lengths, 8-byte aligned
 static unsigned long long *dense_ctr(const accx_graph *g) {
@@ -893,8 +904,10 @@ static int launch_count(accx_graph *g, const accx_count_opts *o, cudaStream_t s,
   if (warps < 1 || warps > 32 || dkb < 1 || skb < 1) return ACCX_ERR_INVALID_ARG;
   if (orient ? (dkb + dkb / 2 + skb > 196 || skb > 200) : (dkb + skb > 200)) return ACCX_ERR_INVALID_ARG;
   // shapes past a block's 227 KB are refused for every policy, whether or not this count
-  // launches a bitmap kernel: windows and tables plus the per-round arrays (direct 29664
-  // bytes; oriented 32 a thread of the instance and 416)
+  // launches a bitmap kernel: windows and tables plus 29664 bytes for the direct kernel's
+  // per-round arrays, and for the oriented one 32 bytes a thread of the instance and 416: what an
+  // earlier form kept.  The present one keeps less (4176, 7280 or 13488 bytes by instance),
+  // so it fits wherever this lets a shape through; the limit stays where callers know it.
   const uint32_t inst = warps <= 8 ? 256u : warps <= 16 ? 512u : 1024u;
   const size_t need = orient ? (size_t)dkb * 1536u + (size_t)skb * 1024u + 144u + 32u * inst + 416u
                              : ((size_t)dkb + skb) * 1024u + 29664u;

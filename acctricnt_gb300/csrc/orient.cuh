@@ -599,8 +599,7 @@ __global__ void __launch_bounds__(OW_WARPS * 32) k_owner_warp(const uint32_t *__
 // 65-98 % of their ids below 4096.  K and M come from k_dense_plan.  Measured at
 // R-MAT 24 (K 4096, M 131072): list probing 71.2 -> 39.6 ms for 8.6 ms here; Chung-Lu 3M:
 // 4.2 -> 2.4 ms for both.
-#define DENSE_PLANES 10   // a counter holds at most DENSE_CHUNK neighbours: < 2^10
-#define DENSE_CHUNK_MAX 960u
+#define DENSE_PLANES 10   // bits of a counter: it takes every neighbour of an item
 #define DENSE_WARPS 8
 
 // T, low[x] = |T[x]| and the work items of the rows below M: a warp per row.

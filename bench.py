@@ -393,7 +393,7 @@ def alg_bytes(G, dominant, stats, owner_work, matches=None):
     hold, the owner prefixes staged, 8 bytes per owned edge (partner offset and prefix
     length) and a 4-byte read-modify-write of a count per common id found (the credit of
     the partner-side entry).  The dense rows test the hub ids among them as bits of masks
-    that stay in L2, so the fraction is of a list-probing count's bytes; `traffic` is DRAM's."""
+    that stay in L2: these are the bytes of a count that reads every list; `traffic` is DRAM's."""
     if dominant == "bitmap" and matches is not None:
         found, probed = matches
         return 4 * probed + 4 * owner_work["bitmap"] + 8 * stats["bitmap"]["edges"] + 8 * found["bitmap"]
@@ -484,7 +484,6 @@ def run_gb300(args):
     dominant = max(("merge", "gallop", "bitmap", "mirror", "plan"), key=lambda k: phases.get(k, 0.0))
     dom_ms = phases.get(dominant, 0.0)
     ab = alg_bytes(G, dominant, stats, owner_work, matches if dominant == "bitmap" else None)
-    achieved = ab / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else None
     kname = dominant + ("_or" if orient and dominant in ("merge", "gallop", "bitmap") else "")
     kernels = "k_dense_pairs + k_bitmap_or + k_owner_warp" if kname == "bitmap_or" else "k_" + kname
     traffic = None
@@ -495,10 +494,15 @@ def run_gb300(args):
             traffic = int(tr["bytes_per_probe"] * probes)
     except Exception:
         pass
-    roofline = {"bound": "hbm", "kernel": kernels, "achieved": round(achieved, 1) if achieved else None,
+    # DRAM bytes that move, where they were measured, against the HBM peak.  "list_bytes" are those of
+    # a count that reads every partner id from a list: dense rows and L2 spare most of them
+    moved = traffic if traffic else int(ab)
+    achieved = moved / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else None
+    roofline = {"bound": "instruction issue and latency" if traffic else "hbm", "kernel": kernels,
+                "achieved": round(achieved, 1) if achieved else None,
                 "peak": peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if peaks else "fallback",
                 "unit": "GB/s", "frac": round(achieved / peak, 4) if achieved else None, "traffic": traffic,
-                "alg_bytes_per_launch": int(ab), "launch_ms": round(dom_ms, 3),
+                "list_bytes_per_launch": int(ab), "launch_ms": round(dom_ms, 3),
                 "merge_equiv_bytes": int(4 * float(np.sum(np.diff(G.download()[0]).astype(np.float64) ** 2)) + 4 * G.m)}
     e2e = None
     if not args.no_e2e and rank == 0:

@@ -226,8 +226,9 @@ int accx_cn_last_stats(const accx_graph *g, uint64_t edges[ACCX_NUM_KINDS], uint
 int accx_cn_last_owner_work(const accx_graph *g, uint64_t owner_work[ACCX_NUM_KINDS]);
 
 /* Oriented counts: common ids found per kind (each a triangle) in the last
- * count, and the ids the bitmap kind actually probed (partner prefixes after the
- * cut at the smaller id).  Zero after a direct count. */
+ * count, and the ids in the partner lists of the bitmap kind's edges (partner prefixes after
+ * the cut at the smaller id): looked up one by one, or, between dense rows, many at a time as
+ * bits of a mask.  Zero after a direct count. */
 int accx_cn_last_matches(const accx_graph *g, uint64_t matches[ACCX_NUM_KINDS], uint64_t *probed);
 
 /* Phases timed when accx_count_opts.timing is set. */
